@@ -4,9 +4,9 @@ from __future__ import annotations
 
 import torch
 import torch.nn as nn
-from torch.autograd.function import Function, once_differentiable
+from torch.autograd.function import Function
 
-from . import config, kernels
+from . import _native, config, kernels
 
 
 # The few most recently quantized activations: (tensor kept alive so its address cannot be recycled, version, key,
@@ -23,70 +23,37 @@ def _input_key(X, mode):
     return (X.data_ptr(), tuple(X.shape), tuple(X.stride()), X.device, mode, config.seed())
 
 
-def _forward_common(ctx, X, W, b, want_scale):
-    """Forward of cuda/QLinear.py:28-35,52-60: absmax scales of X and W, fused quantize + GEMM (+ output scale),
-    and the quantized operands cached for the backward pass.  With config.share_quantized_inputs() a layer whose
-    input is the tensor the previous layer just quantized (same memory, same version) re-uses that int8 copy."""
-    mode = config.mode_for("gemm_fwd")
-    sW = kernels.cuda_kernels.get_scale(W)
-    hit = None
-    if config.sharing_quantized_inputs() and mode != kernels.ROUND_STOCHASTIC:
-        key = _input_key(X, mode)
+def _linear(X, W, b, want_scale):
+    """Forward of cuda/QLinear.py:28-35,52-60 (absmax scales of X and W, quantize, GEMM, optional output scale) with its
+    native autograd node, which keeps the quantized operands for the backward pass (cuda/QLinear.py:37-47,62-72: dY
+    quantized to nearest, dX and dW by int8 GEMMs, bias gradient in fp32).  With config.share_quantized_inputs() a layer
+    whose input is the tensor a previous layer just quantized (same memory, same version) re-uses that int8 copy."""
+    share = config.sharing_quantized_inputs() and config.mode_for("gemm_fwd") != kernels.ROUND_STOCHASTIC
+    Xq = sX = None
+    if share:
+        key = _input_key(X, config.mode_for("gemm_fwd"))
         for ent in _shared_input:
             if ent[1] == X._version and ent[2] == key:
-                hit = ent
-    if hit is not None:
-        Xq, sX = hit[3], hit[4]
-        Wq, _ = kernels.quantize(W, sW, mode=mode, seed=config.seed())
-        out = torch.empty((X.size(0), W.size(0)), dtype=torch.float32, device=X.device)
-        sY = torch.zeros_like(sX) if want_scale else None
-        kernels._qgemm_nt(out, Xq, Wq, sX, sW, b, sY)
-        res = (out, sY) if want_scale else out
-    else:
-        sX = kernels.cuda_kernels.get_scale(X)
-        Xq = kernels.alloc_int8(X.shape, X.device)
-        Wq = kernels.alloc_int8(W.shape, X.device)
-        res = kernels.QGEMM_forward(X, Xq, sX, W, Wq, sW, b, want_scale, mode=mode, seed=config.seed())
-        if config.sharing_quantized_inputs() and mode != kernels.ROUND_STOCHASTIC:
-            _shared_input.append((X, X._version, _input_key(X, mode), Xq, sX))
-            del _shared_input[:-_SHARED_SLOTS]
-    ctx.backward_cache = (Xq, sX, Wq, sW, b)
-    return res
+                Xq, sX = ent[3], ent[4]
+    Y, sY, Xq_used, sX_used = _native.ops.qlinear(X, W, b, want_scale, Xq, sX)
+    if share and Xq is None:
+        _shared_input.append((X, X._version, key, Xq_used, sX_used))
+        del _shared_input[:-_SHARED_SLOTS]
+    return (Y, sY) if want_scale else Y
 
 
-def _backward_common(ctx, grad_output):
-    """Backward of cuda/QLinear.py:37-47,62-72: quantize dY (nearest), dX and dW by int8 GEMMs, bias grad in fp32."""
-    Xq, sX, Wq, sW, b = ctx.backward_cache
-    dYq, sdY = kernels.quantize(grad_output, mode=config.mode_for("quantize"), seed=config.seed())
-    dX, dW = kernels.QGEMM_backward(dYq, Xq, Wq, sdY, sX, sW, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
-    db = grad_output.sum(0) if (b is not None and ctx.needs_input_grad[2]) else None
-    return dX, dW, db
-
-
-class Qlinear_func(Function):
+class Qlinear_func:
     @staticmethod
-    def forward(ctx, X, W, b=None):
-        return _forward_common(ctx, X, W, b, False)
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, grad_output):
-        return _backward_common(ctx, grad_output)
+    def apply(X, W, b=None):
+        return _linear(X, W, b, False)
 
 
-class Qlinear_func_reduce(Function):
+class Qlinear_func_reduce:
     """Also returns max|Y|/127 computed in the GEMM epilogue, so the consumer can skip its own absmax pass."""
 
     @staticmethod
-    def forward(ctx, X, W, b=None):
-        out, scale_out = _forward_common(ctx, X, W, b, True)
-        ctx.mark_non_differentiable(scale_out)
-        return out, scale_out
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, grad_output, _grad_scale):
-        return _backward_common(ctx, grad_output)
+    def apply(X, W, b=None):
+        return _linear(X, W, b, True)
 
 
 class QgemmNT_func(Function):

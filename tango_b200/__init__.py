@@ -23,5 +23,5 @@ def install_as_cuda() -> None:
     import sys
     sys.modules["cuda"] = sys.modules[__name__]
     # looked up by module name: the package attribute `QLinear` is the class, not the module
-    for name in ("kernels", "QLinear", "SPMM", "SDDMM", "util", "config", "graph", "_lib", "gnn", "dist", "peer"):
+    for name in ("kernels", "QLinear", "SPMM", "SDDMM", "util", "config", "graph", "_lib", "_native", "gnn", "dist", "peer"):
         sys.modules[f"cuda.{name}"] = importlib.import_module(f"{__name__}.{name}")

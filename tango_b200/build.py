@@ -3,19 +3,28 @@
 nvcc cross-compiles without a GPU.  The explicit -gencode pair is required: tcgen05 kind::i8 only assembles for the
 architecture-specific target compute_100a/sm_100a.  --fmad=false keeps every fp32 epilogue a sequence of single
 IEEE operations so results are bit-reproducible against the CPU checker.
+
+The host layer (csrc/torch_*.cpp -> lib/_torch_ops.so) is a Python extension over the torch C++ headers, compiled with
+g++ and linked against the library above, which it finds beside itself.
 """
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+import sysconfig
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
+HEADER = os.path.join(ROOT, "include", "tango_b200.h")
+CUDA_HOME = os.environ.get("CUDA_HOME") or "/usr/local/cuda"
 LIB_PATH = os.path.join(LIB_DIR, "libtango_b200.so")
 SOURCES = ["quantize.cu", "spmm.cu", "sddmm.cu", "gat_softmax.cu", "igemm_tcgen05.cu", "peer.cu"]
+HOST_SOURCES = ["torch_ops.cpp", "torch_autograd.cpp", "torch_bind.cpp"]
+HOST_LIB_PATH = os.path.join(LIB_DIR, "_torch_ops.so")
 # measurement aid of the benchmark, a library of its own (not part of the product ABI)
 PROBE_SRC = os.path.join(CSRC, "bench", "row_gather_probe.cu")
 PROBE_LIB_PATH = os.path.join(LIB_DIR, "libtango_bench_probe.so")
@@ -26,37 +35,62 @@ def _nvcc() -> str:
     return cand if os.path.exists(cand) else "nvcc"
 
 
-def needs_build() -> bool:
-    if not os.path.exists(LIB_PATH) or not os.path.exists(PROBE_LIB_PATH):
-        return True
-    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(PROBE_LIB_PATH))
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))]
-    deps += [PROBE_SRC, os.path.join(ROOT, "include", "tango_b200.h")]
-    return any(os.path.getmtime(d) > t for d in deps)
+def _newer(target: str, deps) -> bool:
+    return not os.path.exists(target) or any(os.path.getmtime(d) > os.path.getmtime(target) for d in deps)
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not needs_build():
-        return LIB_PATH
-    os.makedirs(LIB_DIR, exist_ok=True)
-    cmd = [_nvcc(), "-shared", "-Xcompiler", "-fPIC", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
-           "-O3", "--fmad=false", "-std=c++17", "-diag-suppress", "128", "-I", os.path.join(ROOT, "include"),
-           "-o", LIB_PATH] + [os.path.join(CSRC, s) for s in SOURCES]
-    if verbose:
-        cmd.insert(1, "-Xptxas")
-        cmd.insert(2, "-v")
+def _run(cmd, what: str):
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         sys.stderr.write(res.stdout + res.stderr)
-        raise RuntimeError("nvcc failed building libtango_b200.so")
-    if verbose:
-        sys.stderr.write(res.stderr)
-    res = subprocess.run([_nvcc(), "-shared", "-Xcompiler", "-fPIC", "-gencode", "arch=compute_100a,code=sm_100a",
-                          "-lineinfo", "-O3", "-std=c++17", "-o", PROBE_LIB_PATH, PROBE_SRC],
-                         capture_output=True, text=True)
-    if res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
-        raise RuntimeError("nvcc failed building libtango_bench_probe.so")
+        raise RuntimeError(f"{os.path.basename(cmd[0])} failed building {what}")
+    return res
+
+
+def _sources(*suffixes):
+    return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(suffixes)] + [HEADER]
+
+
+def needs_build() -> bool:
+    return (_newer(LIB_PATH, _sources(".cu", ".cuh")) or _newer(PROBE_LIB_PATH, [PROBE_SRC])
+            or _newer(HOST_LIB_PATH, _sources(".cpp", "torch_ops.h", "torch_autograd.h")))
+
+
+def _build_host() -> None:
+    """g++ over the torch headers (no nvcc: the host layer holds no device code)."""
+    from torch.utils.cpp_extension import include_paths, library_paths
+    import torch
+    flags = ["-O2", "-fPIC", "-std=c++17", "-fvisibility=hidden", "-DTORCH_API_INCLUDE_EXTENSION_H",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I" + os.path.dirname(HEADER),
+             "-I" + os.path.join(CUDA_HOME, "include"), "-I" + sysconfig.get_paths()["include"]]
+    flags += ["-isystem" + p for p in include_paths()]
+    objects = [os.path.join(LIB_DIR, os.path.splitext(s)[0] + ".o") for s in HOST_SOURCES]
+    with ThreadPoolExecutor() as pool:
+        list(pool.map(lambda so: _run(["g++", *flags, "-c", os.path.join(CSRC, so[0]), "-o", so[1]], so[0]),
+                      zip(HOST_SOURCES, objects)))
+    link = ["g++", "-shared", "-o", HOST_LIB_PATH, *objects, "-L" + LIB_DIR, "-ltango_b200", "-Wl,-rpath,$ORIGIN"]
+    link += [f for p in library_paths() for f in ("-L" + p, "-Wl,-rpath," + p)]
+    _run(link + ["-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda"], "_torch_ops.so")
+    for o in objects:
+        os.remove(o)
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    os.makedirs(LIB_DIR, exist_ok=True)
+    nvcc = [_nvcc(), "-shared", "-Xcompiler", "-fPIC", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3",
+            "-std=c++17"]
+    if force or _newer(LIB_PATH, _sources(".cu", ".cuh")):
+        cmd = nvcc + ["--fmad=false", "-diag-suppress", "128", "-I", os.path.dirname(HEADER), "--threads", "0",
+                      "-Xlinker", "-soname=libtango_b200.so", "-o", LIB_PATH] + [os.path.join(CSRC, s) for s in SOURCES]
+        if verbose:
+            cmd[1:1] = ["-Xptxas", "-v"]
+        res = _run(cmd, "libtango_b200.so")
+        if verbose:
+            sys.stderr.write(res.stderr)
+    if force or _newer(PROBE_LIB_PATH, [PROBE_SRC]):
+        _run(nvcc + ["-o", PROBE_LIB_PATH, PROBE_SRC], "libtango_bench_probe.so")
+    if force or _newer(HOST_LIB_PATH, _sources(".cpp", "torch_ops.h", "torch_autograd.h")):
+        _build_host()
     return LIB_PATH
 
 

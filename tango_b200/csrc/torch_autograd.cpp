@@ -1,0 +1,531 @@
+// Autograd nodes of the quantized operators, in C++: the backward of a node runs in the engine's thread without the
+// Python interpreter.  Each operator is a forward function and a node whose backward() returns one gradient per tensor
+// input.  int8 operands and scales of the forward pass are kept by the node itself (they are not differentiable);
+// forward results that the backward reads are kept as SavedVariables, so that a write to them in between is noticed.
+#include "torch_autograd.h"
+
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/variable.h>
+
+namespace tango_host {
+
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+// Below the autograd and view-tracking layers: forward and backward bodies only produce fresh, non-differentiable tensors.
+using Raw = at::AutoDispatchBelowADInplaceOrView;
+
+struct OnceNode : Node {
+    virtual variable_list backward(const variable_list &grads) = 0;
+
+    variable_list apply(variable_list &&grads) override {
+        variable_list out;
+        {
+            const c10::AutoGradMode no_grad(false);
+            const Raw raw;
+            out = backward(grads);
+        }
+        if (!c10::GradMode::is_enabled()) return out;
+        bool differentiable = false;
+        for (const Tensor &g : grads) differentiable |= g.defined() && g.requires_grad();
+        if (!differentiable) return out;
+        // a graph of the gradients was asked for: results that raise when they are differentiated again
+        for (Tensor &t : out)
+            if (t.defined()) {
+                t = t.detach();
+                t.set_requires_grad(true);
+            }
+        return torch::autograd::DelayedError("trying to differentiate twice a function that was marked with "
+                                             "@once_differentiable", (int)out.size())(std::move(out));
+    }
+    bool needs(size_t input) const { return task_should_compute_output(input); }
+};
+
+// The node of an operation on `inputs`, or null when no gradient is recorded.
+template <class N, class... T>
+static std::shared_ptr<N> make_node(const T &...inputs) {
+    if (!torch::autograd::compute_requires_grad(inputs...)) return nullptr;
+    auto node = std::shared_ptr<N>(new N(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(inputs...));
+    return node;
+}
+
+static Tensor zeros1(const Tensor &like) { return at::zeros({1}, like.options().dtype(at::kFloat)); }
+static uint64_t call_if(int mode) { return mode == TANGO_ROUND_STOCHASTIC ? next_call() : 0; }
+
+// ------------------------------------------------------------------------------------------------ QLinear
+struct QLinearBackward : OnceNode {
+    std::string name() const override { return "QLinearBackward"; }
+    Tensor xq, sx, wq, sw;
+    bool has_bias = false;
+    variable_list backward(const variable_list &grads) override {
+        const Tensor &dy = grads[0];
+        if (!dy.defined()) return variable_list(3);
+        const Quantized q = quantize(dy);
+        Tensor dx = needs(0) ? gemm_dx(q.q, wq, q.scale, sw) : Tensor();
+        Tensor dw = needs(1) ? gemm_dw(q.q, xq, q.scale, sx) : Tensor();
+        Tensor db = has_bias && needs(2) ? dy.sum(0) : Tensor();
+        return {dx, dw, db};
+    }
+};
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> qlinear(const Tensor &x, const Tensor &w, const Tensor &b, bool want_scale,
+                                                   const Tensor &xq_, const Tensor &sx_) {
+    require(x.is_cuda() && w.is_cuda() && (!b.defined() || b.is_cuda()), "x, w and b must be on the GPU");
+    require(x.size(1) == w.size(1), "x and w must have the same number of columns");
+    Tensor y, sy, xq = xq_, sx = sx_, wq, sw;
+    {
+        const Raw raw;
+        const int mode = settings().mode_gemm;
+        const uint64_t seed = settings().seed, call = call_if(mode);
+        if (mode == TANGO_ROUND_STOCHASTIC) next_call();       // the weight draws from call + 1
+        if (!xq.defined()) {
+            const Quantized q = quantize(x, {}, mode, seed, call, 16);
+            xq = q.q; sx = q.scale;
+        }
+        const Quantized q = quantize(w, {}, mode, seed, call + 1, 16);
+        wq = q.q; sw = q.scale;
+        y = floats({x.size(0), w.size(0)}, x);
+        if (want_scale) sy = zeros1(x);
+        gemm_nt(y, xq, wq, sx, sw, b.defined() ? b.detach() : b, sy);
+    }
+    if (auto node = make_node<QLinearBackward>(x, w, b)) {
+        node->xq = xq; node->sx = sx; node->wq = wq; node->sw = sw; node->has_bias = b.defined();
+        torch::autograd::set_history(y, node);
+    }
+    return {y, sy, xq, sx};
+}
+
+// ------------------------------------------------------------------------------------------------ aggregation
+struct SpmmCopyUBackward : OnceNode {
+    std::string name() const override { return "SpmmCopyUBackward"; }
+    GraphPtr g;
+    variable_list backward(const variable_list &grads) override {
+        if (!grads[0].defined() || !needs(0)) return variable_list(1);
+        const Quantized q = quantize(grads[0]);
+        return {spmm_copy_u(*g, true, q.q, q.scale)};
+    }
+};
+
+Tensor spmm_copy_u_fn(const GraphPtr &g, const Tensor &n, const Tensor &scale) {
+    Tensor out;
+    {
+        const Raw raw;
+        const Quantized q = quantize(n, scale);
+        out = spmm_copy_u(*g, false, q.q, q.scale);
+    }
+    if (auto node = make_node<SpmmCopyUBackward>(n)) {
+        node->g = g;
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+// True when the edge feature broadcasts over the node feature's last dimension, so that dE is a per-head dot product
+// (cuda/SPMM.py:26-34 of the reference).
+static bool reduces_last_dim(const Tensor &n, const Tensor &e) {
+    if (e.dim() < 2 || n.dim() != e.dim() || e.size(-1) != 1 || n.size(-1) <= 1) return false;
+    for (int64_t d = 1; d < n.dim() - 1; ++d)
+        if (n.size(d) != e.size(d)) return false;
+    return true;
+}
+
+struct SpmmUMulEBackward : OnceNode {
+    std::string name() const override { return "SpmmUMulEBackward"; }
+    GraphPtr g;
+    Tensor nq, sn, eq, se, scale;
+    bool reduce_last = false, compat = false;
+    std::vector<int64_t> e_shape;
+    variable_list backward(const variable_list &grads) override {
+        if (!grads[0].defined()) return variable_list(2);
+        const Quantized z = quantize(grads[0]);
+        Tensor dn, de;
+        if (needs(0)) dn = spmm_u_mul_e(*g, true, z.q, eq, compat ? scale : z.scale.mul(se));
+        if (needs(1)) de = sddmm(*g, reduce_last ? "dot" : "mul", nq, z.q, sn, z.scale, {}, false).reshape(e_shape);
+        return {dn, de};
+    }
+};
+
+Tensor spmm_u_mul_e_fn(const GraphPtr &g, const Tensor &n, const Tensor &e, const Tensor &scale_e, bool compat_dn_scale) {
+    Tensor out, sn, se, scale;
+    Quantized eq, nq;
+    {
+        const Raw raw;
+        sn = absmax_scale(n);
+        se = scale_e.defined() ? scale_e : absmax_scale(e);     // the producer may already know max|E| / 127
+        eq = quantize(e.reshape({e.size(0), -1}), se, 1);       // [E, H] int8, edge-id order (no transposed copy)
+        nq = quantize(n, sn);
+        scale = sn.mul(se);
+        out = spmm_u_mul_e(*g, false, nq.q, eq.q, scale);
+    }
+    if (auto node = make_node<SpmmUMulEBackward>(n, e)) {
+        node->g = g; node->nq = nq.q; node->sn = sn; node->eq = eq.q; node->se = se; node->scale = scale;
+        node->reduce_last = reduces_last_dim(n, e);
+        node->compat = compat_dn_scale;
+        node->e_shape = e.sizes().vec();
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+// ------------------------------------------------------------------------------------------------ edge scores
+// Per-edge and per-node tensors narrower than 16 bytes stay packed; wider rows are padded for 128-bit accesses.
+static int64_t row_align(const Tensor &t) {
+    const int64_t rows = t.size(0);
+    return (rows ? t.numel() / rows : 0) < 16 ? 1 : 16;
+}
+
+struct SddmmUAddVBackward : OnceNode {
+    std::string name() const override { return "SddmmUAddVBackward"; }
+    GraphPtr g;
+    variable_list backward(const variable_list &grads) override {
+        if (!grads[0].defined()) return variable_list(2);
+        const Quantized z = quantize(grads[0], {}, row_align(grads[0]));
+        Tensor du = needs(0) ? incidence_sum(*g, true, z.q, z.scale) : Tensor();
+        Tensor dv = needs(1) ? incidence_sum(*g, false, z.q, z.scale) : Tensor();
+        return {du, dv};
+    }
+};
+
+Tensor sddmm_u_add_v_fn(const GraphPtr &g, const Tensor &u, const Tensor &v, const Tensor &su, const Tensor &sv) {
+    Tensor out;
+    {
+        const Raw raw;
+        const int64_t align = row_align(u);
+        const Quantized uq = quantize(u, su, align);
+        const Quantized vq = u.is_same(v) ? uq : quantize(v, sv, align);
+        out = sddmm(*g, "add", uq.q, vq.q, uq.scale, vq.scale, {}, false);
+    }
+    if (auto node = make_node<SddmmUAddVBackward>(u, v)) {
+        node->g = g;
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+struct SddmmUDotVBackward : OnceNode {
+    std::string name() const override { return "SddmmUDotVBackward"; }
+    GraphPtr g;
+    Tensor uq, su, vq, sv;
+    variable_list backward(const variable_list &grads) override {
+        const Tensor &dz = grads[0];
+        if (!dz.defined()) return variable_list(2);
+        const Quantized z = quantize(dz.reshape({dz.size(0), -1}), {}, 1);
+        const bool flat = uq.dim() != 3;
+        auto side = [&](bool reverse, const Tensor &xq, const Tensor &sx) {
+            const Tensor d = spmm_u_mul_e(*g, reverse, flat ? xq.unsqueeze(1) : xq, z.q, sx.mul(z.scale));
+            return flat ? d.squeeze(1) : d;
+        };
+        Tensor du, dv;
+        if (needs(0)) du = side(true, vq, sv);
+        if (needs(1)) dv = side(false, uq, su);
+        return {du, dv};
+    }
+};
+
+Tensor sddmm_u_dot_v_fn(const GraphPtr &g, const Tensor &u, const Tensor &v) {
+    Tensor out;
+    Quantized uq, vq;
+    {
+        const Raw raw;
+        uq = quantize(u);
+        vq = u.is_same(v) ? uq : quantize(v);
+        out = sddmm(*g, "dot", uq.q, vq.q, uq.scale, vq.scale, {}, false);
+    }
+    if (auto node = make_node<SddmmUDotVBackward>(u, v)) {
+        node->g = g; node->uq = uq.q; node->su = uq.scale; node->vq = vq.q; node->sv = vq.scale;
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+// ------------------------------------------------------------------------------------------------ graph convolution
+// Backward of y = relu(.): int8 of (y > 0 ? g : 0) * row_scale, its scale, and the column sums of the masked gradient.
+static Quantized relu_grad_quantize(const Tensor &grad, const Tensor &y_, const Tensor &row_scale, Tensor *colsum, int mode,
+                                    uint64_t seed, uint64_t call) {
+    const c10::cuda::CUDAGuard guard(grad.device());
+    const Matrix g = matrix(grad), y = matrix(y_);
+    Quantized out{alloc_int8({g.rows, g.cols}, grad.device(), 16), floats({1}, grad)};
+    Tensor scratch;
+    int64_t bytes = 0;
+    if (colsum) {
+        *colsum = floats({g.cols}, grad);
+        bytes = tango_relu_grad_stats_scratch_bytes(g.rows, g.cols);
+        scratch = at::empty({std::max<int64_t>(bytes, 4)}, grad.options().dtype(at::kByte));
+    }
+    check(tango_relu_grad_stats(ptr<float>(g.t), g.ld, ptr<float>(y.t), y.ld, g.rows, g.cols, ptr<float>(row_scale),
+                                ptr<float>(out.scale), colsum ? ptr<float>(*colsum) : nullptr, ptr(scratch), bytes, cuda_stream()),
+          "relu_grad_stats");
+    check(tango_quantize_relu_grad(ptr<float>(g.t), g.ld, ptr<float>(y.t), y.ld, g.rows, g.cols, ptr<float>(row_scale),
+                                   ptr<float>(out.scale), ptr<int8_t>(out.q), out.q.stride(0), mode, seed, call,
+                                   settings().step, cuda_stream()), "quantize_relu_grad");
+    count(colsum ? 3 : 2);
+    return out;
+}
+
+struct GcnConvBackward : OnceNode {
+    std::string name() const override { return "GcnConvBackward"; }
+    GraphPtr g;
+    Tensor xq, sx, wq, sw, out_norm, in_norm;
+    SavedVariable out;
+    bool relu = false, has_bias = false, released = false;
+
+    void release_variables() override {
+        xq.reset(); wq.reset();
+        out.reset_data();
+        released = true;
+    }
+    variable_list backward(const variable_list &grads) override {
+        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+        if (!grads[0].defined()) return variable_list(3);
+        const int mode = settings().mode_quantize;
+        const uint64_t seed = settings().seed, call = call_if(mode);
+        const bool want_db = has_bias && needs(2);
+        Tensor db;
+        Quantized z;
+        if (relu) {
+            z = relu_grad_quantize(grads[0], out.unpack(shared_from_this()), in_norm, want_db ? &db : nullptr, mode, seed, call);
+        } else {
+            const Tensor d = grads[0].contiguous();
+            if (want_db) db = d.sum(0);
+            z = quantize(d, {}, mode, seed, call, 16, in_norm);
+        }
+        const Tensor dh = spmm_copy_u(*g, true, z.q, z.scale);
+        const Quantized h = quantize(dh);
+        // the backward of the left norm is the row factor in dX's epilogue
+        Tensor dx = needs(0) ? gemm_dx(h.q, wq, h.scale, sw, out_norm) : Tensor();
+        Tensor dw = needs(1) ? gemm_dw(h.q, xq, h.scale, sx) : Tensor();
+        return {dx, dw, db};
+    }
+};
+
+Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x_, const Tensor &w, const Tensor &b, const Tensor &out_norm,
+                   const Tensor &in_norm, bool relu) {
+    Tensor out;
+    Quantized xq, wq;
+    {
+        const Raw raw;
+        const int mode = settings().mode_gemm;
+        const uint64_t seed = settings().seed, call = call_if(mode);
+        if (mode == TANGO_ROUND_STOCHASTIC) next_call();
+        xq = quantize(x_.contiguous(), {}, mode, seed, call, 16, out_norm);
+        wq = quantize(w.contiguous(), {}, mode, seed, call + 1, 16);
+        const Tensor h = floats({x_.size(0), w.size(0)}, x_), sh = zeros1(x_);
+        gemm_nt(h, xq.q, wq.q, xq.scale, wq.scale, {}, sh);
+        const Quantized hq = quantize(h, sh);
+        out = spmm_copy_u(*g, false, hq.q, sh, in_norm, b, relu);
+    }
+    if (auto node = make_node<GcnConvBackward>(x_, w, b)) {
+        node->g = g; node->xq = xq.q; node->sx = xq.scale; node->wq = wq.q; node->sw = wq.scale;
+        node->out_norm = out_norm; node->in_norm = in_norm; node->relu = relu; node->has_bias = b.defined();
+        torch::autograd::set_history(out, node);
+        if (relu) node->out = SavedVariable(out, true);
+    }
+    return out;
+}
+
+// ------------------------------------------------------------------------------------------------ edge softmax
+static const int32_t *row_order(const Direction &d) { return d.sched.present ? ptr<int32_t>(d.sched.row_order) : nullptr; }
+
+struct EdgeSoftmaxBackward : OnceNode {
+    std::string name() const override { return "EdgeSoftmaxBackward"; }
+    GraphPtr g;
+    SavedVariable a;
+    float factor = 1.f;
+    bool released = false;
+    void release_variables() override {
+        a.reset_data();
+        released = true;
+    }
+    variable_list backward(const variable_list &grads) override {
+        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+        if (!grads[0].defined()) return variable_list(1);
+        const Tensor at = a.unpack(shared_from_this()), a2 = at.reshape({at.size(0), -1}).contiguous();
+        const c10::cuda::CUDAGuard guard(a2.device());
+        const Tensor da = grads[0].reshape(a2.sizes()).contiguous(), dz = at::empty_like(a2);
+        const Direction &d = g->dir(false);
+        check(tango_edge_softmax_bwd(ptr<int32_t>(d.indptr), ptr<int32_t>(d.edge_ids), row_order(d), d.sched.n_block_rows,
+                                     g->n_nodes, (int)a2.size(1), factor, ptr<float>(a2), ptr<float>(da), ptr<float>(dz),
+                                     nullptr, cuda_stream()), "edge_softmax_bwd");
+        count(1);
+        return {dz.view(at.sizes())};
+    }
+};
+
+std::tuple<Tensor, Tensor> edge_softmax_fn(const GraphPtr &g, const Tensor &z, double factor) {
+    require(z.is_cuda() && z.scalar_type() == at::kFloat, "fp32 CUDA scores expected");
+    Tensor a, sa;
+    {
+        const Raw raw;
+        const c10::cuda::CUDAGuard guard(z.device());
+        const Tensor z2 = z.reshape({z.size(0), -1}).contiguous();
+        require(z2.size(0) == g->n_edges(), "one score row per edge");
+        if (z2.size(1) > 8) throw std::invalid_argument("edge_softmax: at most 8 heads");
+        const Tensor a2 = at::empty_like(z2);
+        sa = zeros1(z);
+        const Direction &d = g->dir(false);
+        check(tango_edge_softmax(ptr<int32_t>(d.indptr), ptr<int32_t>(d.edge_ids), row_order(d), d.sched.n_block_rows,
+                                 g->n_nodes, ptr<float>(z2), (int)z2.size(1), (float)factor, ptr<float>(a2), ptr<float>(sa),
+                                 cuda_stream()), "edge_softmax");
+        count(1);
+        a = a2.view(z.sizes());
+    }
+    if (auto node = make_node<EdgeSoftmaxBackward>(z)) {
+        node->g = g; node->factor = (float)factor;
+        torch::autograd::set_history(a, node);
+        node->a = SavedVariable(a, true);
+    }
+    return {a, sa};
+}
+
+// ------------------------------------------------------------------------------------------------ graph attention
+// The two softmax flavours share everything but where the weights live; g, el, er as int8 [N, H] with their scales.
+struct GatLogits {
+    GraphPtr g;
+    Quantized el, er;
+    float slope;
+    int h;
+    const Direction &d() const { return g->dir(false); }
+    int64_t n_block() const { return d().sched.n_block_rows; }
+};
+
+static GatLogits gat_logits(const GraphPtr &g, const Tensor &el, const Tensor &er, double slope) {
+    const int64_t n = el.size(0), h = el.size(1);
+    const Quantized l = quantize(el.reshape({n, h}), {}, 1), r = quantize(er.reshape({n, h}), {}, 1);
+    return {g, l, r, (float)slope, (int)h};
+}
+
+// d_el / d_er from the gradient of the logits: int8, then summed over out-edges and in-edges.
+static std::pair<Tensor, Tensor> gat_logit_grads(const GatLogits &a, const Tensor &dz, const Tensor &sdz, bool want_l,
+                                                 bool want_r, at::IntArrayRef shape_l, at::IntArrayRef shape_r) {
+    const Quantized q = quantize(dz, sdz, 1);
+    Tensor dl = want_l ? incidence_sum(*a.g, true, q.q, sdz).view(shape_l) : Tensor();
+    Tensor dr = want_r ? incidence_sum(*a.g, false, q.q, sdz).view(shape_r) : Tensor();
+    return {dl, dr};
+}
+
+struct GatAttentionBackward : OnceNode {
+    std::string name() const override { return "GatAttentionBackward"; }
+    GatLogits l;
+    SavedVariable a;
+    std::vector<int64_t> shape_l, shape_r;
+    bool released = false;
+    void release_variables() override {
+        a.reset_data();
+        released = true;
+    }
+    variable_list backward(const variable_list &grads) override {
+        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+        if (!grads[0].defined()) return variable_list(2);
+        const Tensor at = a.unpack(shared_from_this());
+        const c10::cuda::CUDAGuard guard(at.device());
+        const Tensor a2 = at.reshape({-1, l.h}), da = grads[0].reshape({-1, l.h}).contiguous(), dz = at::empty_like(a2);
+        const Tensor sdz = zeros1(a2);
+        const Direction &d = l.d();
+        check(tango_gat_edge_softmax_bwd(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), ptr<int32_t>(d.edge_ids), row_order(d),
+                                         l.n_block(), l.g->n_nodes, ptr<int8_t>(l.el.q), ptr<int8_t>(l.er.q), l.h,
+                                         ptr<float>(l.el.scale), ptr<float>(l.er.scale), l.slope, ptr<float>(a2),
+                                         ptr<float>(da), ptr<float>(dz), ptr<float>(sdz), cuda_stream()), "gat_edge_softmax_bwd");
+        count(1);
+        const auto [dl, dr] = gat_logit_grads(l, dz, sdz, needs(0), needs(1), shape_l, shape_r);
+        return {dl, dr};
+    }
+};
+
+std::tuple<Tensor, Tensor> gat_attention_fn(const GraphPtr &g, const Tensor &el, const Tensor &er, double slope) {
+    Tensor a, sa;
+    GatLogits l;
+    {
+        const Raw raw;
+        const c10::cuda::CUDAGuard guard(el.device());
+        l = gat_logits(g, el, er, slope);
+        a = floats({g->n_edges(), l.h, 1}, el);
+        sa = zeros1(el);
+        const Direction &d = l.d();
+        check(tango_gat_edge_softmax(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), ptr<int32_t>(d.edge_ids), row_order(d),
+                                     l.n_block(), g->n_nodes, ptr<int8_t>(l.el.q), ptr<int8_t>(l.er.q), l.h,
+                                     ptr<float>(l.el.scale), ptr<float>(l.er.scale), l.slope, ptr<float>(a), ptr<float>(sa),
+                                     cuda_stream()), "gat_edge_softmax");
+        count(1);
+    }
+    if (auto node = make_node<GatAttentionBackward>(el, er)) {
+        node->l = l; node->shape_l = el.sizes().vec(); node->shape_r = er.sizes().vec();
+        torch::autograd::set_history(a, node);
+        node->a = SavedVariable(a, true);
+    }
+    return {a, sa};
+}
+
+struct GatAggregateBackward : OnceNode {
+    std::string name() const override { return "GatAggregateBackward"; }
+    GatLogits l;
+    Tensor m, inv, sa, aq, nq, sn;
+    std::vector<int64_t> shape_l, shape_r;
+    bool released = false;
+    void release_variables() override {
+        for (Tensor *t : {&m, &inv, &aq, &nq}) t->reset();
+        released = true;
+    }
+    variable_list backward(const variable_list &grads) override {
+        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+        if (!grads[0].defined()) return variable_list(3);
+        const c10::cuda::CUDAGuard guard(grads[0].device());
+        const Quantized z = quantize(grads[0]);
+        Tensor d_ft, dl, dr;
+        if (needs(0)) d_ft = spmm_u_mul_e(*l.g, true, z.q, aq, z.scale.mul(sa));
+        if (needs(1) || needs(2)) {
+            const Tensor da = sddmm(*l.g, "dot", nq, z.q, sn, z.scale, {}, false).reshape({-1, l.h});
+            const Tensor dz = at::empty_like(da), sdz = zeros1(da);
+            const Direction &d = l.d();
+            check(tango_gat_edge_softmax_bwd_stats(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), ptr<int32_t>(d.edge_ids),
+                                                   row_order(d), l.n_block(), l.g->n_nodes, ptr<int8_t>(l.el.q),
+                                                   ptr<int8_t>(l.er.q), l.h, ptr<float>(l.el.scale), ptr<float>(l.er.scale),
+                                                   l.slope, ptr<float>(m), ptr<float>(inv), ptr<float>(da), ptr<float>(dz),
+                                                   ptr<float>(sdz), cuda_stream()), "gat_edge_softmax_bwd_stats");
+            count(1);
+            std::tie(dl, dr) = gat_logit_grads(l, dz, sdz, needs(1), needs(2), shape_l, shape_r);
+        }
+        return {d_ft, dl, dr};
+    }
+};
+
+Tensor gat_aggregate_fn(const GraphPtr &g, const Tensor &ft, const Tensor &el, const Tensor &er, double slope) {
+    Tensor out, m, inv, sa, aq;
+    GatLogits l;
+    Quantized nq;
+    {
+        const Raw raw;
+        const c10::cuda::CUDAGuard guard(ft.device());
+        l = gat_logits(g, el, er, slope);
+        const Direction &d = l.d();
+        m = floats({g->n_nodes, l.h}, ft);
+        inv = at::empty_like(m);
+        sa = zeros1(ft);
+        check(tango_gat_edge_softmax_stats(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), row_order(d), l.n_block(),
+                                           g->n_nodes, ptr<int8_t>(l.el.q), ptr<int8_t>(l.er.q), l.h, ptr<float>(l.el.scale),
+                                           ptr<float>(l.er.scale), l.slope, ptr<float>(m), ptr<float>(inv), ptr<float>(sa),
+                                           cuda_stream()), "gat_edge_softmax_stats");
+        const int mode = settings().mode_quantize;
+        const uint64_t call = call_if(mode);
+        aq = at::empty({g->n_edges(), l.h}, ft.options().dtype(at::kChar));
+        check(tango_gat_edge_softmax_quantized(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), ptr<int32_t>(d.edge_ids),
+                                               row_order(d), l.n_block(), g->n_nodes, ptr<int8_t>(l.el.q), ptr<int8_t>(l.er.q),
+                                               l.h, ptr<float>(l.el.scale), ptr<float>(l.er.scale), l.slope, ptr<float>(m),
+                                               ptr<float>(inv), ptr<float>(sa), ptr<int8_t>(aq), mode, settings().seed, call,
+                                               settings().step, cuda_stream()), "gat_edge_softmax_quantized");
+        count(2);
+        nq = quantize(ft);
+        out = spmm_u_mul_e(*g, false, nq.q, aq, nq.scale.mul(sa));
+    }
+    if (auto node = make_node<GatAggregateBackward>(ft, el, er)) {
+        node->l = l; node->m = m; node->inv = inv; node->sa = sa; node->aq = aq; node->nq = nq.q; node->sn = nq.scale;
+        node->shape_l = el.sizes().vec(); node->shape_r = er.sizes().vec();
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+}  // namespace tango_host

@@ -1,0 +1,308 @@
+// The operators of this package over at::Tensor: shapes, allocation of outputs and scratch, and the C ABI calls.
+#include "torch_ops.h"
+
+#include <map>
+#include <mutex>
+
+namespace tango_host {
+
+void check(int rc, const char *what) {
+    if (rc == TANGO_OK) return;
+    std::string msg = std::string(what) + ": " + tango_strerror(rc);
+    if (rc == TANGO_ECUDA) msg += " (cudaError " + std::to_string(tango_last_cuda_error()) + ")";
+    throw Failure(msg);
+}
+
+Settings &settings() {
+    static Settings s;
+    return s;
+}
+
+Matrix matrix(const Tensor &t) {
+    if (t.dim() <= 1) {
+        Tensor c = t.contiguous();
+        const int64_t n = c.numel();
+        return {c, 1, n, std::max<int64_t>(n, 1)};
+    }
+    const int64_t rows = t.size(0), cols = rows ? t.numel() / rows : 0;
+    if (t.is_contiguous()) return {t, rows, cols, std::max<int64_t>(cols, 1)};
+    if (rows > 0 && t.stride(0) >= cols) {
+        int64_t want = 1;
+        bool packed = true;
+        for (int64_t d = t.dim() - 1; d >= 1 && packed; --d) {
+            packed = t.size(d) == 1 || t.stride(d) == want;
+            want *= t.size(d);
+        }
+        if (packed) return {t, rows, cols, t.stride(0)};
+    }
+    return {t.contiguous(), rows, cols, std::max<int64_t>(cols, 1)};
+}
+
+Tensor alloc_int8(at::IntArrayRef shape, const at::Device &device, int64_t align) {
+    const auto opt = at::TensorOptions().dtype(at::kChar).device(device);
+    if (shape.size() < 2) return at::empty(shape, opt);
+    int64_t cols = 1;
+    for (size_t d = 1; d < shape.size(); ++d) cols *= shape[d];
+    const int64_t ld = (std::max<int64_t>(cols, 1) + align - 1) / align * align;
+    if (ld == cols) return at::empty(shape, opt);
+    std::vector<int64_t> stride(shape.size(), 1);
+    for (size_t d = shape.size() - 1; d-- > 1;) stride[d] = stride[d + 1] * shape[d + 1];
+    stride[0] = ld;
+    return at::empty({shape[0] * ld}, opt).as_strided(shape, stride);
+}
+
+Tensor status_word(const at::Device &device) {
+    static std::mutex mutex;
+    static std::map<int, Tensor> words;      // one per device, for the life of the process
+    std::lock_guard<std::mutex> lock(mutex);
+    Tensor &w = words[device.index()];
+    if (!w.defined()) w = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(device));
+    return w;
+}
+
+// ------------------------------------------------------------------------------------------------ quantisation
+static void require_float(const Tensor &t) { require(t.is_cuda() && t.scalar_type() == at::kFloat, "fp32 CUDA tensor expected"); }
+
+Tensor absmax_scale(const Tensor &t, const Tensor &row_scale) {
+    require_float(t);
+    const c10::cuda::CUDAGuard guard(t.device());
+    const Matrix x = matrix(t);
+    Tensor scale = floats({1}, t);
+    check(tango_absmax_scale(ptr<float>(x.t), x.rows, x.cols, x.ld, ptr<float>(row_scale), ptr<float>(scale), cuda_stream()),
+          "get_scale");
+    count(1);
+    return scale;
+}
+
+void quantize_into(const Tensor &q, const Tensor &t, const Tensor &scale, int mode, uint64_t seed, uint64_t call,
+                   const Tensor &row_scale) {
+    require_float(t);
+    require(q.is_cuda() && q.scalar_type() == at::kChar && q.sizes() == t.sizes(), "int8 CUDA tensor of the input's shape expected");
+    const c10::cuda::CUDAGuard guard(t.device());
+    const Matrix x = matrix(t), o = matrix(q);
+    require(o.t.data_ptr() == q.data_ptr(), "output int8 tensor must be row-strided, not arbitrary-strided");
+    check(tango_quantize(ptr<float>(x.t), x.rows, x.cols, x.ld, ptr<float>(row_scale), ptr<float>(scale), ptr<int8_t>(q),
+                         o.ld, mode, seed, call, settings().step, cuda_stream()), "quantize");
+    count(1);
+}
+
+Quantized quantize(const Tensor &t, const Tensor &scale, int mode, uint64_t seed, uint64_t call, int64_t align,
+                   const Tensor &row_scale) {
+    require(t.is_cuda(), "tensor must be on GPU");
+    const Tensor s = scale.defined() ? scale : absmax_scale(t, row_scale);
+    Tensor q = alloc_int8(t.sizes(), t.device(), align);
+    quantize_into(q, t, s, mode, seed, call, row_scale);
+    return {q, s};
+}
+
+Quantized quantize(const Tensor &t, const Tensor &scale, int64_t align, const Tensor &row_scale) {
+    const int mode = settings().mode_quantize;
+    const uint64_t call = mode == TANGO_ROUND_STOCHASTIC ? next_call() : 0;
+    return quantize(t, scale, mode, settings().seed, call, align, row_scale);
+}
+
+// ------------------------------------------------------------------------------------------------ GEMMs
+void gemm_nt(const Tensor &y, const Tensor &xq, const Tensor &wq, const Tensor &sx, const Tensor &sw,
+             const Tensor &bias, const Tensor &scale_y) {
+    const c10::cuda::CUDAGuard guard(y.device());
+    const Matrix x = matrix(xq), w = matrix(wq), o = matrix(y);
+    check(tango_qgemm_nt(ptr<int8_t>(x.t), x.ld, ptr<int8_t>(w.t), w.ld, x.rows, w.rows, x.cols, ptr<float>(sx),
+                         ptr<float>(sw), ptr<float>(bias), ptr<float>(y), o.ld, ptr<float>(scale_y),
+                         ptr<int>(status_word(y.device())), cuda_stream()), "qgemm_nt");
+    count(1);
+}
+
+Tensor gemm_dx(const Tensor &dyq, const Tensor &wq, const Tensor &sdy, const Tensor &sw, const Tensor &row_scale) {
+    const c10::cuda::CUDAGuard guard(dyq.device());
+    const Matrix dy = matrix(dyq), w = matrix(wq);
+    Tensor dx = floats({dy.rows, w.cols}, sdy);
+    check(tango_qgemm_dx(ptr<int8_t>(dy.t), dy.ld, ptr<int8_t>(w.t), w.ld, dy.rows, dy.cols, w.cols, ptr<float>(sdy),
+                         ptr<float>(sw), ptr<float>(row_scale), ptr<float>(dx), w.cols,
+                         ptr<int>(status_word(dyq.device())), cuda_stream()), "QGEMM_backward_gradX");
+    count(1);
+    return dx;
+}
+
+Tensor gemm_dw(const Tensor &dyq, const Tensor &xq, const Tensor &sdy, const Tensor &sx) {
+    const c10::cuda::CUDAGuard guard(dyq.device());
+    const Matrix dy = matrix(dyq), x = matrix(xq);
+    Tensor dw = floats({dy.cols, x.cols}, sdy);
+    const int64_t bytes = tango_qgemm_dw_workspace_bytes(dy.cols, x.cols);
+    const Tensor ws = at::empty({std::max<int64_t>(bytes, 16)}, dyq.options().dtype(at::kByte));
+    check(tango_qgemm_dw(ptr<int8_t>(dy.t), dy.ld, ptr<int8_t>(x.t), x.ld, dy.rows, dy.cols, x.cols, ptr<float>(sdy),
+                         ptr<float>(sx), ptr<float>(dw), x.cols, ptr(ws), bytes, ptr<int>(status_word(dyq.device())),
+                         cuda_stream()), "QGEMM_backward_gradW");
+    count(2);
+    return dw;
+}
+
+// ------------------------------------------------------------------------------------------------ graph operators
+// The C ABI's view of a schedule, and the scratch that has to live until the call returns (the allocator orders its
+// reuse behind the launches on this stream).
+struct Plan {
+    tango_spmm_plan p{};
+    Tensor ws, packed;
+    const tango_spmm_plan *get(const Schedule &s) const { return s.present ? &p : nullptr; }
+};
+
+static Plan make_plan(const Schedule &s, int64_t f, const Tensor &like) {
+    Plan plan;
+    if (!s.present) return plan;
+    tango_spmm_plan &p = plan.p;
+    p.split_threshold = s.threshold;
+    p.row_order = ptr<int32_t>(s.row_order);
+    p.n_long_rows = p.row_order ? s.n_long : -1;
+    if (s.n_heavy == 0) return plan;
+    const int64_t ld = (f + 15) / 16 * 16;
+    plan.ws = at::empty({s.n_heavy, ld}, like.options().dtype(at::kInt));
+    p.units = ptr<int32_t>(s.units);
+    p.n_units = s.n_units;
+    p.heavy_rows = ptr<int32_t>(s.heavy_rows);
+    p.n_heavy = s.n_heavy;
+    p.ws = ptr<int32_t>(plan.ws);
+    p.ws_ld = ld;
+    if (s.has_hub) {
+        plan.packed = at::empty({s.dense_cols.numel(), ld}, like.options().dtype(at::kChar));
+        p.dense_a = ptr<int8_t>(s.dense);
+        p.dense_n_tiles = s.n_tiles;
+        p.dense_rows = s.dense_rows;
+        p.dense_units = ptr<int32_t>(s.dense_units);
+        p.dense_n_units = s.dense_units.size(0);
+        p.dense_cols = ptr<int32_t>(s.dense_cols);
+        p.dense_n_cols = s.dense_cols.numel();
+        p.dense_b = ptr<int8_t>(plan.packed);
+        p.dense_status = ptr<int>(status_word(like.device()));
+        p.n_skip_rows = s.n_skip;
+    }
+    return plan;
+}
+
+// Pointer of a mandatory index array; an empty one (graph without edges) still needs a valid address, and the row
+// pointers in front of it are one.
+static const int32_t *index_ptr(const Tensor &t, const Tensor &indptr) {
+    return t.numel() > 0 ? ptr<int32_t>(t) : ptr<int32_t>(indptr);
+}
+
+static int64_t short_launch(const Schedule &s) { return s.present && s.n_long < s.row_order.numel(); }
+
+Tensor spmm_copy_u(const Graph &g, bool reverse, const Tensor &nq, const Tensor &scale, const Tensor &row_scale,
+                   const Tensor &bias, bool relu) {
+    const c10::cuda::CUDAGuard guard(nq.device());
+    const Direction &d = g.dir(reverse);
+    const Matrix n = matrix(nq);
+    // the dense hub region takes feature rows at exactly their padded width, the layout every quantizer here writes
+    const bool hub = d.has_hub && nq.dim() >= 2 && nq.stride(0) == (n.cols + 15) / 16 * 16;
+    const Schedule &s = hub ? d.hub_sched : d.sched;
+    std::vector<int64_t> shape(nq.sizes().begin(), nq.sizes().end());
+    shape[0] = g.n_nodes;
+    Tensor out = floats(shape, scale);
+    const Plan plan = make_plan(s, n.cols, nq);
+    const Tensor &indptr = hub ? d.hub_indptr : d.indptr;
+    check(tango_spmm_copy_u(ptr<int32_t>(indptr), index_ptr(hub ? d.hub_indices : d.indices, indptr), g.n_nodes, 1,
+                            ptr<int8_t>(n.t), n.ld, n.cols, ptr<float>(scale), ptr<float>(row_scale), ptr<float>(bias),
+                            relu, ptr<float>(out), n.cols, nullptr, plan.get(s), cuda_stream()), "csr_SPMM");
+    count(1 + (s.n_heavy > 0) + short_launch(s) + (hub ? 2 : 0));
+    return out;
+}
+
+Tensor spmm_u_mul_e(const Graph &g, bool reverse, const Tensor &nq, const Tensor &eq, const Tensor &scale) {
+    require(nq.dim() == 3, "node features must be [N, H, D]");
+    const c10::cuda::CUDAGuard guard(nq.device());
+    const Direction &d = g.dir(reverse);
+    const Matrix n = matrix(nq);
+    const Tensor e = eq.numel() ? eq.contiguous() : at::zeros({1}, nq.options());
+    Tensor out = floats({d.n_rows(), nq.size(1), nq.size(2)}, scale);
+    const Plan plan = make_plan(d.sched, n.cols, nq);
+    check(tango_spmm_u_mul_e(ptr<int32_t>(d.indptr), index_ptr(d.indices, d.indptr), ptr<int32_t>(d.edge_ids), d.n_rows(),
+                             ptr<int8_t>(n.t), n.ld, (int)nq.size(1), (int)nq.size(2), ptr<int8_t>(e), ptr<float>(scale),
+                             ptr<float>(out), n.cols, plan.get(d.sched), cuda_stream()), "multi_cusparse_SPMM");
+    count(1 + (d.sched.n_units > 0) + short_launch(d.sched));
+    return out;
+}
+
+Tensor incidence_sum(const Graph &g, bool reverse, const Tensor &zq, const Tensor &scale) {
+    require(zq.is_cuda() && scale.is_cuda(), "CUDA tensors expected");
+    const c10::cuda::CUDAGuard guard(zq.device());
+    const Direction &d = g.dir(reverse);
+    const Matrix z = matrix(zq);
+    std::vector<int64_t> shape(zq.sizes().begin(), zq.sizes().end());
+    shape[0] = g.n_nodes;
+    Tensor out = floats(shape, scale);
+    const int64_t f = z.cols;
+    const Plan plan = make_plan(d.sched, f, zq);
+    check(tango_spmm_incidence(ptr<int32_t>(d.indptr), ptr<int32_t>(d.edge_ids), d.n_rows(), ptr<int8_t>(z.t), z.ld, f,
+                               ptr<float>(scale), ptr<float>(out), f, plan.get(d.sched), cuda_stream()), "incidence_SPMM");
+    const bool contiguous = !d.edge_ids.defined() && z.ld == f && (f == 1 || f == 2 || f == 4 || f == 8 || f == 16);
+    count(1 + (d.sched.n_units > 0) + (short_launch(d.sched) && (!contiguous || f == 4 || f == 8 || f == 16)));
+    return out;
+}
+
+// Average edges per row from which the dot product walks rows (the fixed operand stays in registers).  With a handful
+// of edges per row the endpoint-list kernel (32 edges per warp, whatever their rows) measured faster: 169,343 nodes /
+// 1.3 M edges, 4 heads x 32: 0.060 ms against 0.069 ms.
+constexpr int64_t kRowwiseDotMinDegree = 32;
+
+static bool sddmm_dot_rows(const Graph &g, bool reverse, const Matrix &u, const Matrix &v, int h, int dim, const Tensor &su,
+                           const Tensor &sv, const Tensor &out, const Tensor &scale) {
+    const Direction &d = g.dir(reverse);
+    const Schedule &s = d.sched;
+    tango_spmm_plan p{};
+    p.units = ptr<int32_t>(s.units); p.n_units = s.n_units; p.split_threshold = s.threshold;
+    p.row_order = ptr<int32_t>(s.row_order); p.n_long_rows = p.row_order ? s.n_long : -1;
+    const int rc = tango_sddmm_dot_rows(ptr<int32_t>(d.indptr), index_ptr(d.indices, d.indptr), ptr<int32_t>(d.edge_ids),
+                                        d.n_rows(), ptr<int8_t>(u.t), u.ld, ptr<int8_t>(v.t), v.ld, h, dim, ptr<float>(su),
+                                        ptr<float>(sv), ptr<float>(out), ptr<float>(scale), s.present ? &p : nullptr,
+                                        cuda_stream());
+    if (rc == TANGO_EALIGN) return false;      // an operand layout that only the endpoint-list kernel takes
+    check(rc, "mySDDMM_int8(dot, rows)");
+    count(1 + short_launch(s));
+    return true;
+}
+
+Tensor sddmm(const Graph &g, const std::string &op, const Tensor &u_, const Tensor &v_, const Tensor &su, const Tensor &sv,
+             const Tensor &scale, bool reverse) {
+    require(g.src.is_cuda() && g.dst.is_cuda() && u_.is_cuda() && v_.is_cuda() && su.is_cuda() && sv.is_cuda(),
+            "CUDA tensors expected");
+    const c10::cuda::CUDAGuard guard(u_.device());
+    const bool flat = u_.dim() == 2 && v_.dim() == 2;
+    const Tensor u = flat ? u_.unsqueeze(1) : u_, v = flat ? v_.unsqueeze(1) : v_;
+    const Tensor &src = reverse ? g.dst : g.src, &dst = reverse ? g.src : g.dst;
+    const int64_t n_edges = src.numel();
+    const bool dot = op == "dot";
+    // trailing-shape broadcast (dgl.sparse.infer_broadcast_shape in the reference); "dot" collapses the last dimension
+    if (dot && u.size(-1) != v.size(-1)) throw std::invalid_argument("dot needs equal feature sizes");
+    const int64_t nd = std::max(u.dim(), v.dim());
+    std::vector<int64_t> shape{n_edges};
+    for (int64_t k = 1; k < nd; ++k) {
+        const int64_t a = k - (nd - u.dim()) >= 1 ? u.size(k - (nd - u.dim())) : 1;
+        const int64_t b = k - (nd - v.dim()) >= 1 ? v.size(k - (nd - v.dim())) : 1;
+        if (a != b && a != 1 && b != 1) throw std::invalid_argument("cannot broadcast the feature shapes");
+        shape.push_back(std::max(a, b));
+    }
+    if (dot) shape.back() = 1;
+    Tensor out = floats(shape, su);
+    const Matrix um = matrix(u), vm = matrix(v);
+    if (dot) {
+        const int h = (int)u.size(-2), dim = (int)u.size(-1);
+        const bool rows = n_edges > 0 && n_edges >= kRowwiseDotMinDegree * g.n_nodes && u.dim() == 3 &&
+                          u.sizes().slice(1) == v.sizes().slice(1) && u.size(0) == g.n_nodes && v.size(0) == g.n_nodes;
+        if (!rows || !sddmm_dot_rows(g, reverse, um, vm, h, dim, su, sv, out, scale)) {
+            check(tango_sddmm_dot(ptr<int32_t>(src), ptr<int32_t>(dst), n_edges, ptr<int8_t>(um.t), um.ld, ptr<int8_t>(vm.t),
+                                  vm.ld, h, dim, ptr<float>(su), ptr<float>(sv), ptr<float>(out), ptr<float>(scale),
+                                  cuda_stream()), "mySDDMM_int8(dot)");
+            count(1);
+        }
+    } else {
+        const int code = op == "add" ? TANGO_OP_ADD : op == "sub" ? TANGO_OP_SUB : op == "mul" ? TANGO_OP_MUL
+                       : op == "div" ? TANGO_OP_DIV : -1;
+        if (code < 0) throw std::invalid_argument(op + " op not supported");
+        require(um.cols == vm.cols, "element-wise SDDMM needs equal feature shapes");
+        check(tango_sddmm_elementwise(code, ptr<int32_t>(src), ptr<int32_t>(dst), n_edges, ptr<int8_t>(um.t), um.ld,
+                                      ptr<int8_t>(vm.t), vm.ld, um.cols, ptr<float>(su), ptr<float>(sv), ptr<float>(out),
+                                      ptr<float>(scale), cuda_stream()), "mySDDMM_int8");
+        count(1);
+    }
+    return flat ? out.squeeze(1) : out;
+}
+
+}  // namespace tango_host

@@ -1,0 +1,122 @@
+// Shared by the host layer (torch_*.cpp): the operators of this package over at::Tensor, without Python.
+//
+// Why a native host layer: one training pass of a small model is a few dozen kernels of 2-10 microseconds each, and
+// the same calls issued operator by operator from Python cost 15-30 microseconds apiece (tensor wrappers, ctypes
+// marshalling, autograd nodes that take the interpreter lock in the engine's thread).  Here an autograd node is a C++
+// object whose backward runs without the interpreter, and a kernel call is a plain function call into the C ABI.
+#pragma once
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+
+#include <atomic>
+#include <memory>
+#include <string>
+#include <vector>
+
+#include "tango_b200.h"
+
+namespace tango_host {
+
+using at::Tensor;
+
+// A failed C ABI call (TangoError in Python) and a violated precondition (AssertionError).
+struct Failure : std::runtime_error {
+    using std::runtime_error::runtime_error;
+};
+struct Violation : std::runtime_error {
+    using std::runtime_error::runtime_error;
+};
+void check(int rc, const char *what);
+inline void require(bool ok, const char *what) {
+    if (!ok) throw Violation(what);
+}
+
+// Process-wide settings, written by tango_b200.config (see there for their meaning).
+struct Settings {
+    std::atomic<int> mode_gemm{TANGO_ROUND_TRUNC}, mode_quantize{TANGO_ROUND_NEAREST};
+    std::atomic<uint64_t> seed{0};
+    std::atomic<const uint64_t *> step{nullptr};
+    std::atomic<uint64_t> calls{0};      // keys the stochastic-rounding stream of successive calls
+    std::atomic<int64_t> launches{0};    // kernels launched so far
+};
+Settings &settings();
+inline uint64_t next_call() { return settings().calls.fetch_add(1) + 1; }
+inline void count(int64_t n) { settings().launches.fetch_add(n, std::memory_order_relaxed); }
+
+// The row schedule of one index bundle (tango_b200.graph.SpmmSchedule) and its dense hub region, if any.
+struct Schedule {
+    Tensor units, heavy_rows, row_order;
+    int64_t n_units = 0, n_heavy = 0, n_long = 0, n_block_rows = 0, n_skip = 0;
+    int threshold = 0;
+    bool present = false;
+    // hub region (tango_b200.graph.HubBlock)
+    Tensor dense, dense_units, dense_cols;
+    int64_t n_tiles = 0, dense_rows = 0;
+    bool has_hub = false;
+};
+
+// One direction of a graph: CSC rows are destinations, CSR rows are sources.
+struct Direction {
+    Tensor indptr, indices, edge_ids;    // edge_ids undefined: slot k holds edge k
+    Schedule sched;
+    bool has_hub = false;
+    Tensor hub_indptr, hub_indices;      // the edges outside the hub region
+    Schedule hub_sched;
+    int64_t n_rows() const { return indptr.numel() - 1; }
+};
+
+struct Graph {
+    std::shared_ptr<Direction> csc, csr;
+    Tensor src, dst;
+    int64_t n_nodes = 0;
+    const Direction &dir(bool reverse) const { return reverse ? *csr : *csc; }
+    int64_t n_edges() const { return src.numel(); }
+};
+using GraphPtr = std::shared_ptr<Graph>;
+
+// `t` seen as a row-major [rows, cols] matrix with leading dimension ld (elements); `t` may be a contiguous copy.
+struct Matrix {
+    Tensor t;
+    int64_t rows, cols, ld;
+};
+Matrix matrix(const Tensor &t);
+
+template <class T = void>
+inline T *ptr(const Tensor &t) {
+    return t.defined() && t.numel() > 0 ? static_cast<T *>(t.data_ptr()) : nullptr;
+}
+inline tango_stream_t cuda_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
+
+Tensor alloc_int8(at::IntArrayRef shape, const at::Device &device, int64_t align);
+inline Tensor floats(at::IntArrayRef shape, const Tensor &like) { return at::empty(shape, like.options().dtype(at::kFloat)); }
+Tensor status_word(const at::Device &device);
+
+// ---- quantisation
+struct Quantized {
+    Tensor q, scale;
+};
+Tensor absmax_scale(const Tensor &t, const Tensor &row_scale = {});
+void quantize_into(const Tensor &q, const Tensor &t, const Tensor &scale, int mode, uint64_t seed, uint64_t call,
+                   const Tensor &row_scale = {});
+Quantized quantize(const Tensor &t, const Tensor &scale, int mode, uint64_t seed, uint64_t call, int64_t align,
+                   const Tensor &row_scale = {});
+// with the rounding mode configured for the stand-alone quantizer, drawing a call number when it is stochastic
+Quantized quantize(const Tensor &t, const Tensor &scale = {}, int64_t align = 16, const Tensor &row_scale = {});
+
+// ---- GEMMs
+void gemm_nt(const Tensor &y, const Tensor &xq, const Tensor &wq, const Tensor &sx, const Tensor &sw,
+             const Tensor &bias, const Tensor &scale_y);
+Tensor gemm_dx(const Tensor &dyq, const Tensor &wq, const Tensor &sdy, const Tensor &sw, const Tensor &row_scale = {});
+Tensor gemm_dw(const Tensor &dyq, const Tensor &xq, const Tensor &sdy, const Tensor &sx);
+
+// ---- graph operators
+Tensor spmm_copy_u(const Graph &g, bool reverse, const Tensor &nq, const Tensor &scale, const Tensor &row_scale = {},
+                   const Tensor &bias = {}, bool relu = false);
+Tensor spmm_u_mul_e(const Graph &g, bool reverse, const Tensor &nq, const Tensor &eq, const Tensor &scale);
+Tensor incidence_sum(const Graph &g, bool reverse, const Tensor &zq, const Tensor &scale);
+// op: "dot", "add", "sub", "mul", "div"; U and V 2-D or 3-D; `scale` (optional, holding 0) receives max|out| / 127
+Tensor sddmm(const Graph &g, const std::string &op, const Tensor &u, const Tensor &v, const Tensor &su,
+             const Tensor &sv, const Tensor &scale, bool reverse);
+
+}  // namespace tango_host

@@ -10,9 +10,8 @@ import math
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
-from torch.autograd.function import Function, once_differentiable
 
-from . import config, kernels
+from . import _native
 from .QLinear import QLinear, Qlinear_func, Qlinear_func_reduce
 from .SDDMM import sddmm_u_add_v, sddmm_u_dot_v
 from .SPMM import spmm_copy_u, spmm_u_mul_e
@@ -41,7 +40,7 @@ def _cached_norm(graph, which: str) -> torch.Tensor:
     return cache[which]
 
 
-class _gcn_conv_fused(Function):
+def _gcn_conv_fused(graph, X, W, b, out_norm, in_norm, relu):
     """One "multiply first" graph convolution (in_feats > out_feats, norm='both') as a single autograd node:
 
         out = act( (A . Q(Q(X * d_out^-1/2) W^T)) * d_in^-1/2 + b )
@@ -50,49 +49,7 @@ class _gcn_conv_fused(Function):
     results), but the element-wise passes of the reference's layer (evaluation/test_gcn.py:86-94,123-137) are folded
     into the kernels next to them: the left norm into the absmax/quantize of X, the right norm + bias + ReLU into the
     aggregation's epilogue, and the right norm of the backward pass into the quantizer of the incoming gradient."""
-
-    @staticmethod
-    def forward(ctx, g, X, W, b, out_norm, in_norm, relu):
-        from .kernels import alloc_int8, next_call
-        mode_f, mode_q, seed = config.mode_for("gemm_fwd"), config.mode_for("quantize"), config.seed()
-        call = next_call() if mode_f == kernels.ROUND_STOCHASTIC else 0
-        if mode_f == kernels.ROUND_STOCHASTIC:
-            next_call()
-        X = X.contiguous()
-        sX = kernels._get_scale(X, out_norm)
-        sW = kernels._get_scale(W)
-        Xq, Wq = alloc_int8(X.shape, X.device), alloc_int8(W.shape, X.device)
-        H = torch.empty((X.shape[0], W.shape[0]), dtype=torch.float32, device=X.device)
-        sH = torch.zeros(1, dtype=torch.float32, device=X.device)
-        # X * d_out^-1/2 is quantized on load inside the GEMM kernel, which also writes Xq for the backward pass
-        kernels._qgemm_forward(H, X, Xq, W.contiguous(), Wq, None, sH, sX, sW, mode_f, seed, call, out_norm)
-        Hq, _ = kernels.quantize(H, sH, mode=mode_q, seed=seed)
-        out = kernels.csr_SPMM(g, Hq, sH, False, in_norm, b, relu)
-        ctx.g, ctx.relu, ctx.has_bias = g, relu, b is not None
-        ctx.save_for_backward(Xq, sX, Wq, sW, out_norm, in_norm, out if relu else None)
-        return out
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, d_out):
-        Xq, sX, Wq, sW, out_norm, in_norm, out = ctx.saved_tensors
-        mode_q, seed = config.mode_for("quantize"), config.seed()
-        want_db = ctx.has_bias and ctx.needs_input_grad[3]
-        call = kernels.next_call() if mode_q == kernels.ROUND_STOCHASTIC else 0
-        if ctx.relu:
-            # ReLU mask, bias gradient, right norm, absmax and quantisation in two passes over (d_out, out)
-            dZq, sdZ, db = kernels.relu_grad_quantize(d_out, out, in_norm, want_db, mode_q, seed, call)
-        else:
-            g1 = d_out.contiguous()
-            db = g1.sum(0) if want_db else None
-            sdZ = kernels._get_scale(g1, in_norm)
-            dZq = kernels.alloc_int8(g1.shape, g1.device)
-            kernels._quantize_into(dZq, g1, sdZ, mode_q, seed, call, in_norm)
-        dH = kernels.csr_SPMM(ctx.g, dZq, sdZ, True)
-        dHq, sdH = kernels.quantize(dH, mode=mode_q, seed=seed)
-        dX, dW = kernels.QGEMM_backward(dHq, Xq, Wq, sdH, sX, sW, ctx.needs_input_grad[1], ctx.needs_input_grad[2],
-                                        dx_row_scale=out_norm)   # backward of the left norm, in the GEMM epilogue
-        return None, dX, dW, db, None, None, None
+    return _native.ops.gcn_conv(_native.graph(graph), X, W, b, out_norm, in_norm, relu)
 
 
 class QGraphConv(nn.Module):
@@ -125,8 +82,8 @@ class QGraphConv(nn.Module):
         if (self._fused and self._norm == "both" and self.weight is not None and self._in_feats > self._out_feats
                 and feat.dim() == 2):
             relu = self._activation in (F.relu, torch.relu)
-            rst = _gcn_conv_fused.apply(graph, feat, self.weight, self.bias, _cached_norm(graph, "out"),
-                                        _cached_norm(graph, "in"), relu)
+            rst = _gcn_conv_fused(graph, feat, self.weight, self.bias, _cached_norm(graph, "out"),
+                                  _cached_norm(graph, "in"), relu)
             if self._activation is not None and not relu:
                 rst = self._activation(rst)
             return rst
@@ -175,34 +132,16 @@ class GCN(nn.Module):
 
 
 # ---------------------------------------------------------------------------------------------------- GAT
-class _edge_softmax_fn(Function):
-    """Softmax of edge scores (times a constant factor) over the incoming edges of every destination, per head (the
-    reference calls dgl.ops.edge_softmax, evaluation/test_gat.py:146, evaluation/test_HGT.py:60).  fp32, as in the
-    reference; one team-per-row kernel per direction."""
-
-    @staticmethod
-    def forward(ctx, g, e, factor):
-        a, sa = kernels.edge_softmax_fwd(g, e, factor, want_scale=True)
-        ctx.save_for_backward(a)
-        ctx.g, ctx.factor = g, factor
-        ctx.mark_non_differentiable(sa)
-        return a, sa
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, da, _dsa):
-        (a,) = ctx.saved_tensors
-        return None, kernels.edge_softmax_bwd(ctx.g, a, da, ctx.factor), None
-
-
 def edge_softmax(g, e, factor: float = 1.0, return_scale: bool = False):
-    """softmax over each destination's incoming edges of e * factor; with return_scale also max|a|/127, which the
-    kernel produces on the way and the consuming spmm_u_mul_e would otherwise recompute."""
-    a, sa = _edge_softmax_fn.apply(g, e, factor)
+    """softmax over each destination's incoming edges of e * factor, per head (the reference calls dgl.ops.edge_softmax,
+    evaluation/test_gat.py:146, evaluation/test_HGT.py:60); fp32, as in the reference, one team-per-row kernel per
+    direction.  With return_scale also max|a|/127, which the kernel produces on the way and the consuming spmm_u_mul_e
+    would otherwise recompute."""
+    a, sa = _native.ops.edge_softmax(_native.graph(g), e, factor)
     return (a, sa) if return_scale else a
 
 
-class _gat_attention_fused(Function):
+def _gat_attention_fused(g, el, er, slope):
     """Attention weights of a GAT layer in one pass per direction:
 
         a = edge_softmax(leaky_relu(Q(el)[src] + Q(er)[dst]))
@@ -211,32 +150,10 @@ class _gat_attention_fused(Function):
     without materialising the logits: el / er are quantized to int8 exactly as sddmm_u_add_v does, one kernel walks
     every destination's incoming edges (max, sum, normalise), and the backward kernel produces the gradient of the
     logits, which then takes sddmm_u_add_v's backward route (int8 quantisation + incidence sums)."""
-
-    @staticmethod
-    def forward(ctx, g, el, er, slope):
-        mode, seed = config.mode_for("quantize"), config.seed()
-        n, h = el.shape[0], el.shape[1]
-        elq, sl = kernels.quantize(el.reshape(n, h), mode=mode, seed=seed, align=1)
-        erq, sr = kernels.quantize(er.reshape(n, h), mode=mode, seed=seed, align=1)
-        a, sa = kernels.gat_edge_softmax(g, elq, erq, sl, sr, slope, want_scale=True)
-        ctx.g, ctx.slope, ctx.shapes = g, slope, (el.shape, er.shape)
-        ctx.save_for_backward(elq, erq, sl, sr, a)
-        ctx.mark_non_differentiable(sa)
-        return a.view(a.shape[0], h, 1), sa
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, da, _dsa):
-        elq, erq, sl, sr, a = ctx.saved_tensors
-        g = ctx.g
-        dz, sdz = kernels.gat_edge_softmax_bwd(g, elq, erq, sl, sr, a, da, ctx.slope, want_scale=True)
-        dzq, sdz = kernels.quantize(dz, sdz, mode=config.mode_for("quantize"), seed=config.seed(), align=1)
-        d_el = kernels.incidence_SPMM(g, dzq, sdz, True).view(ctx.shapes[0]) if ctx.needs_input_grad[1] else None
-        d_er = kernels.incidence_SPMM(g, dzq, sdz).view(ctx.shapes[1]) if ctx.needs_input_grad[2] else None
-        return None, d_el, d_er, None
+    return _native.ops.gat_attention(_native.graph(g), el, er, slope)
 
 
-class _gat_aggregate_fused(Function):
+def _gat_aggregate_fused(g, ft, el, er, slope):
     """Attention + aggregation of a GAT layer with no fp32 copy of the attention weights:
 
         out[v,h,:] = sum_e Q(a)[e,h] * Q(ft)[src(e),h,:],   a = edge_softmax(leaky_relu(Q(el)[src] + Q(er)[dst]))
@@ -246,41 +163,7 @@ class _gat_aggregate_fused(Function):
     cuda/SPMM.py:38-47), but the weights exist only as the int8 tensor the aggregation reads: one pass keeps the
     softmax statistics of every destination (which already fix the int8 scale), a second writes the int8 weights,
     and the backward pass recomputes the weights from the statistics."""
-
-    @staticmethod
-    def forward(ctx, g, ft, el, er, slope):
-        mode, seed = config.mode_for("quantize"), config.seed()
-        n, h = el.shape[0], el.shape[1]
-        elq, sl = kernels.quantize(el.reshape(n, h), mode=mode, seed=seed, align=1)
-        erq, sr = kernels.quantize(er.reshape(n, h), mode=mode, seed=seed, align=1)
-        m, inv, sa = kernels.gat_edge_softmax_stats(g, elq, erq, sl, sr, slope)
-        sN = kernels.cuda_kernels.get_scale(ft)
-        call = kernels.next_call() if mode == kernels.ROUND_STOCHASTIC else 0
-        aq = kernels.gat_edge_softmax_quantized(g, elq, erq, sl, sr, m, inv, sa, slope, mode, seed, call)
-        Nq, _ = kernels.quantize(ft, sN, mode=mode, seed=seed)
-        out = kernels.spmm_u_mul_e_int8(g, Nq, aq, sN * sa)
-        ctx.g, ctx.slope, ctx.shapes = g, slope, (el.shape, er.shape)
-        ctx.save_for_backward(elq, erq, sl, sr, m, inv, sa, aq, Nq, sN)
-        return out
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, d_out):
-        elq, erq, sl, sr, m, inv, sa, aq, Nq, sN = ctx.saved_tensors
-        g = ctx.g
-        mode, seed = config.mode_for("quantize"), config.seed()
-        dZq, sdZ = kernels.quantize(d_out, mode=mode, seed=seed)
-        d_ft = kernels.spmm_u_mul_e_int8(g, dZq, aq, sdZ * sa, True) if ctx.needs_input_grad[1] else None
-        d_el = d_er = None
-        if ctx.needs_input_grad[2] or ctx.needs_input_grad[3]:
-            da, _ = kernels.mySDDMM_int8(g, "dot", Nq, dZq, sN, sdZ, False)          # [E, H, 1] fp32
-            dz, sdz = kernels.gat_edge_softmax_bwd_stats(g, elq, erq, sl, sr, m, inv, da, ctx.slope)
-            dzq, sdz = kernels.quantize(dz, sdz, mode=mode, seed=seed, align=1)
-            if ctx.needs_input_grad[2]:
-                d_el = kernels.incidence_SPMM(g, dzq, sdz, True).view(ctx.shapes[0])
-            if ctx.needs_input_grad[3]:
-                d_er = kernels.incidence_SPMM(g, dzq, sdz).view(ctx.shapes[1])
-        return None, d_ft, d_el, d_er, None
+    return _native.ops.gat_aggregate(_native.graph(g), ft, el, er, slope)
 
 
 class QGATConv(nn.Module):
@@ -333,10 +216,10 @@ class QGATConv(nn.Module):
         int8_path = (self._fused == "int8" and not get_attention
                      and not (self.training and self.attn_drop.p > 0))
         if int8_path:
-            rst = _gat_aggregate_fused.apply(graph, ft, el, er, self._slope)
+            rst = _gat_aggregate_fused(graph, ft, el, er, self._slope)
         else:
             if self._fused:
-                a, sa = _gat_attention_fused.apply(graph, el, er, self._slope)
+                a, sa = _gat_attention_fused(graph, el, er, self._slope)
                 if self.training and self.attn_drop.p > 0:
                     a, sa = self.attn_drop(a), None   # dropout rescales a: its absmax has to be taken again
             else:

@@ -19,7 +19,7 @@ from typing import Optional
 
 import torch
 
-from . import _lib, config
+from . import _lib, _native, config
 from ._lib import ROUND_NEAREST, ROUND_STOCHASTIC, ROUND_TRUNC, SpmmPlan, check, lib
 from .graph import SpmmSchedule
 
@@ -86,15 +86,15 @@ def alloc_int8(shape, device, align: int = 16) -> torch.Tensor:
     return v.unflatten(1, shape[1:]) if len(shape) > 2 else v
 
 
-_status = {}
+_status = {}      # device -> the status word shared with the host layer
 
 
 def device_status(device=None, reset: bool = False) -> int:
     """Value of the per-device status word written by kernels with bounded waits (0 = no timeout).  Synchronises."""
-    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    t = _status.get(dev)
-    if t is None:
+    dev = torch.device("cuda" if device is None else device)
+    if dev.type != "cuda":
         return 0
+    t = _status_word(dev)
     v = int(t.item())
     if reset:
         t.zero_()
@@ -107,23 +107,20 @@ def _status_word(device) -> torch.Tensor:
         dev = torch.device("cuda", torch.cuda.current_device())
     t = _status.get(dev)
     if t is None:
-        t = torch.zeros(1, dtype=torch.int32, device=dev)
-        _status[dev] = t
+        t = _status[dev] = _native.ops.status_word(torch.empty(0, device=dev))
     return t
 
 
-launch_counter = [0]  # kernels of this library launched so far (benchmarks report it per step)
-_call_counter = [0]
+launch_counter = _native.LaunchCounter()
 
 
 def next_call() -> int:
     """Monotonic per-process counter that keys the stochastic-rounding stream of successive calls."""
-    _call_counter[0] += 1
-    return _call_counter[0]
+    return _native.ops.next_call()
 
 
 def set_call_counter(v: int) -> None:
-    _call_counter[0] = int(v)
+    _native.ops.set_call_counter(int(v))
 
 
 def infer_broadcast_shape(op, ushape, vshape):
@@ -147,13 +144,7 @@ def infer_broadcast_shape(op, ushape, vshape):
 
 # --------------------------------------------------------------------------------------------------- native module
 def _get_scale(t: torch.Tensor, row_scale: Optional[torch.Tensor] = None) -> torch.Tensor:
-    assert t.is_cuda and t.dtype == torch.float32
-    t, rows, cols, ld = _matrix(t)
-    scale = torch.empty(1, dtype=torch.float32, device=t.device)
-    with torch.cuda.device(t.device):
-        check(lib.tango_absmax_scale(_p(t), rows, cols, ld, _p(row_scale), _p(scale), _stream()), "get_scale")
-    launch_counter[0] += 1
-    return scale
+    return _native.ops.get_scale(t, row_scale)
 
 
 def _quantize_into(out: torch.Tensor, t: torch.Tensor, scale: torch.Tensor, mode: int = ROUND_NEAREST, seed: int = 0,
@@ -454,14 +445,9 @@ def _schedule(g, reverse: bool) -> Optional[SpmmSchedule]:
 def quantize(t: torch.Tensor, scale: torch.Tensor = None, mode: int = ROUND_NEAREST, seed: int = 0,
              call: Optional[int] = None, align: int = 16):
     """Quantize the input tensor to 8-bit (cuda/kernels.py:19-30).  Returns (int8 tensor, scale)."""
-    assert t.is_cuda, "tensor must be on GPU"
-    if scale is None:
-        scale = cuda_kernels.get_scale(t)
-    out = alloc_int8(t.shape, t.device, align)
     if mode == ROUND_STOCHASTIC and call is None:
         call = next_call()
-    _quantize_into(out, t, scale, mode, seed, call or 0)
-    return out, scale
+    return _native.ops.quantize(t, scale, mode, seed & 0xFFFFFFFFFFFFFFFF, call or 0, align)
 
 
 def mySDDMM_int8(g, op, U, V, scaleU, scaleV, isReduce, reverse=False):
