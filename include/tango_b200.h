@@ -99,6 +99,39 @@ int tango_quantize_relu_grad(const float *g, int64_t ldg, const float *y, int64_
                              const float *row_scale, const float *scale, int8_t *q, int64_t ldq, int mode,
                              uint64_t seed, uint64_t call, const uint64_t *step, tango_stream_t stream);
 
+/* One matrix of a fused absmax + quantise launch (host struct, read before the call returns): with
+ * m[r,c] = (gate ? (gate[r,c] > 0 ? x[r,c] : 0) : x[r,c]),
+ *   scale[0]  = max |m[r,c] * row_scale[r]| / 127            (fixed_scale: scale[0] is given instead)
+ *   q[r,c]    = round_mode(m[r,c] * row_scale[r] / scale[0])  (columns [cols, ldq) are zero; stream as in tango_quantize)
+ *   colsum[c] = sum_r m[r,c], added in a fixed order          (optional, not with fixed_scale)
+ *   product[i][0] = scale[0] * times[i][0]                    (optional; times[i] == NULL: the scale of job times_job) */
+typedef struct tango_quant_job {
+    const float *x;
+    int64_t rows, cols, ldx;
+    const float *gate;
+    int64_t ldgate;
+    const float *row_scale;
+    float *scale;
+    int fixed_scale;
+    int times_job;
+    const float *times[2];
+    float *product[2];
+    float *colsum;
+    int8_t *q;
+    int64_t ldq;
+    int mode;
+    uint64_t seed, call;
+} tango_quant_job;
+
+/* Up to four jobs of one rounding mode in one launch (a cooperative one: its CTAs meet once between the two sweeps).  Replaces the
+ * get_scale + quantize pairs in front of every int8 operator (cuda/QLinear.py:29-35, cuda/SPMM.py:9-20) and, with
+ * `gate` / `colsum`, the ReLU backward and bias gradient before them.  The scratch query returns a byte count or a
+ * negative error code; TANGO_ESIZE: a matrix of 2^32 elements or more in a row, or about 2^33 in all (use the calls
+ * above and below). */
+int64_t tango_quantize_fused_scratch_bytes(const tango_quant_job *jobs, int n_jobs);
+int tango_quantize_fused(const tango_quant_job *jobs, int n_jobs, const uint64_t *step, void *scratch,
+                         int64_t scratch_bytes, tango_stream_t stream);
+
 /* ---------------------------------------------------------------- int8 GEMMs (tcgen05 kind::i8) */
 
 /* Bytes of scratch tango_qgemm_dw needs for an [n, k] weight gradient. */

@@ -23,11 +23,15 @@ def _input_key(X, mode):
     return (X.data_ptr(), tuple(X.shape), tuple(X.stride()), X.device, mode, config.seed())
 
 
-def _linear(X, W, b, want_scale):
+def _linear(X, W, b, want_scale, copies=None):
     """Forward of cuda/QLinear.py:28-35,52-60 (absmax scales of X and W, quantize, GEMM, optional output scale) with its
     native autograd node, which keeps the quantized operands for the backward pass (cuda/QLinear.py:37-47,62-72: dY
     quantized to nearest, dX and dW by int8 GEMMs, bias gradient in fp32).  With config.share_quantized_inputs() a layer
-    whose input is the tensor a previous layer just quantized (same memory, same version) re-uses that int8 copy."""
+    whose input is the tensor a previous layer just quantized (same memory, same version) re-uses that int8 copy.  `copies` (a dict that the layers of
+    one forward pass hand to each other) does the same for layers that are known to read the same X."""
+    if copies is not None:
+        Y, sY, copies["Xq"], copies["sX"] = _native.ops.qlinear(X, W, b, want_scale, copies.get("Xq"), copies.get("sX"))
+        return (Y, sY) if want_scale else Y
     share = config.sharing_quantized_inputs() and config.mode_for("gemm_fwd") != kernels.ROUND_STOCHASTIC
     Xq = sX = None
     if share:
@@ -83,10 +87,27 @@ class QLinear(nn.Linear):
     def enable_reduce(self):
         self.isReduce = True
 
-    def forward(self, input):
+    def forward(self, input, copies=None):
         t = input.reshape(-1, input.size(-1))
         out_shape = input.shape[:-1] + (self.weight.size(0),)
+        out = _linear(t, self.weight, self.bias, self.isReduce, copies)
         if self.isReduce:
-            out, scale = Qlinear_func_reduce.apply(t, self.weight, self.bias)
-            return out.reshape(out_shape), scale
-        return Qlinear_func.apply(t, self.weight, self.bias).reshape(out_shape)
+            return out[0].reshape(out_shape), out[1]
+        return out.reshape(out_shape)
+
+
+def linear_group(layers, input):
+    """Yields the outputs of up to three QLinear layers that read the same input, whose absmax pass and int8 copy they
+    share; with config.share_quantized_inputs() the weights are quantized in the same launch as well.  Bit-identical to
+    calling the layers one by one, which is what happens with stochastic rounding (every layer draws its own numbers, in
+    the order in which the outputs are asked for)."""
+    plain = all(type(m) is QLinear and not m.isReduce for m in layers)
+    if not plain or config.mode_for("gemm_fwd") == kernels.ROUND_STOCHASTIC:
+        yield from (m(input) for m in layers)
+    elif config.sharing_quantized_inputs():
+        out = _native.ops.qlinear_group(input.reshape(-1, input.size(-1)), [m.weight for m in layers],
+                                        [m.bias for m in layers])
+        yield from (y.reshape(input.shape[:-1] + (y.size(1),)) for y in out)
+    else:
+        copies = {}
+        yield from (m(input, copies) for m in layers)

@@ -62,6 +62,8 @@ _SIGS = {
     "tango_relu_grad_stats": ([P, c_int64, P, c_int64, c_int64, c_int64, P, P, P, P, c_int64, P], c_int),
     "tango_quantize_relu_grad": ([P, c_int64, P, c_int64, c_int64, c_int64, P, P, P, c_int64, c_int, c_uint64,
                                   c_uint64, P, P], c_int),
+    "tango_quantize_fused_scratch_bytes": ([P, c_int], c_int64),
+    "tango_quantize_fused": ([P, c_int, P, P, c_int64, P], c_int),
     "tango_qgemm_dw_workspace_bytes": ([c_int64, c_int64], c_int64),
     "tango_qgemm_nt": ([P, c_int64, P, c_int64, c_int64, c_int64, c_int64, P, P, P, P, c_int64, P, P, P], c_int),
     "tango_qgemm_forward": ([P, c_int64, P, P, c_int64, c_int64, c_int64, c_int64, P, P, P, c_int64, P, c_int64, P, P,

@@ -414,6 +414,15 @@ static int launch_quantize(const float *x, int64_t rows, int64_t cols, int64_t l
 extern "C" int tango_quantize(const float *x, int64_t rows, int64_t cols, int64_t ldx, const float *row_scale,
                               const float *scale, int8_t *q, int64_t ldq, int mode, uint64_t seed, uint64_t call,
                               const uint64_t *step, tango_stream_t stream) {
+    if (rows < 0 || cols < 0 || ldx < cols || ldq < cols || mode < 0 || mode > 2) return TANGO_EINVAL;
+    if (rows == 0 || ldq == 0) return TANGO_OK;
+    if (!x || !scale || !q) return TANGO_EINVAL;
+    tango_quant_job job{};
+    job.x = x; job.rows = rows; job.cols = cols; job.ldx = ldx; job.row_scale = row_scale;
+    job.scale = const_cast<float *>(scale); job.fixed_scale = 1; job.q = q; job.ldq = ldq;
+    job.mode = mode; job.seed = seed; job.call = call;
+    const int rc = tango_quantize_fused(&job, 1, step, nullptr, 0, stream);
+    if (rc != TANGO_ESIZE) return rc;            // beyond 32-bit element indices: the 64-bit kernels below
     return launch_quantize(x, rows, cols, ldx, row_scale, scale, q, ldq, mode, seed, call, step, PushTargets{nullptr, 0, 0},
                            (cudaStream_t)stream);
 }

@@ -64,11 +64,12 @@ struct QLinearBackward : OnceNode {
     variable_list backward(const variable_list &grads) override {
         const Tensor &dy = grads[0];
         if (!dy.defined()) return variable_list(3);
-        const Quantized q = quantize(dy);
+        QuantJob job = quant_job(dy);
+        job.colsum = has_bias && needs(2);          // the bias gradient comes out of the quantizer's first sweep
+        const Quantized q = quantize(job);
         Tensor dx = needs(0) ? gemm_dx(q.q, wq, q.scale, sw) : Tensor();
         Tensor dw = needs(1) ? gemm_dw(q.q, xq, q.scale, sx) : Tensor();
-        Tensor db = has_bias && needs(2) ? dy.sum(0) : Tensor();
-        return {dx, dw, db};
+        return {dx, dw, q.colsum};
     }
 };
 
@@ -82,21 +83,53 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> qlinear(const Tensor &x, const Tensor
         const int mode = settings().mode_gemm;
         const uint64_t seed = settings().seed, call = call_if(mode);
         if (mode == TANGO_ROUND_STOCHASTIC) next_call();       // the weight draws from call + 1
-        if (!xq.defined()) {
-            const Quantized q = quantize(x, {}, mode, seed, call, 16);
-            xq = q.q; sx = q.scale;
+        const QuantJob jw{w, mode, seed, call + 1};
+        if (xq.defined()) {
+            const Quantized q = quantize(jw);
+            wq = q.q; sw = q.scale;
+        } else {
+            const auto q = quantize_all({jw, {x, mode, seed, call}});
+            wq = q[0].q; sw = q[0].scale; xq = q[1].q; sx = q[1].scale;
         }
-        const Quantized q = quantize(w, {}, mode, seed, call + 1, 16);
-        wq = q.q; sw = q.scale;
         y = floats({x.size(0), w.size(0)}, x);
         if (want_scale) sy = zeros1(x);
-        gemm_nt(y, xq, wq, sx, sw, b.defined() ? b.detach() : b, sy);
+        gemm_nt(y, xq, wq, sx, sw, b, sy);
     }
     if (auto node = make_node<QLinearBackward>(x, w, b)) {
         node->xq = xq; node->sx = sx; node->wq = wq; node->sw = sw; node->has_bias = b.defined();
         torch::autograd::set_history(y, node);
     }
     return {y, sy, xq, sx};
+}
+
+std::vector<Tensor> qlinear_group(const Tensor &x, const std::vector<Tensor> &w, const std::vector<Tensor> &b) {
+    const int mode = settings().mode_gemm;
+    const uint64_t seed = settings().seed;
+    require(w.size() >= 1 && w.size() <= 3 && w.size() == b.size(), "one to three layers");
+    require(mode != TANGO_ROUND_STOCHASTIC, "stochastic rounding draws anew for every layer");
+    std::vector<Tensor> y;
+    std::vector<Quantized> q;
+    {
+        const Raw raw;
+        std::vector<QuantJob> jobs;
+        for (const Tensor &t : w) {
+            require(x.is_cuda() && t.is_cuda() && x.size(1) == t.size(1), "x and w must be on the GPU and agree in columns");
+            jobs.push_back({t, mode, seed, 0});
+        }
+        jobs.push_back({x, mode, seed, 0});
+        q = quantize_all(jobs);
+        for (size_t k = 0; k < w.size(); ++k) {
+            y.push_back(floats({x.size(0), w[k].size(0)}, x));
+            gemm_nt(y[k], q.back().q, q[k].q, q.back().scale, q[k].scale, b[k], {});
+        }
+    }
+    for (size_t k = 0; k < w.size(); ++k)
+        if (auto node = make_node<QLinearBackward>(x, w[k], b[k])) {
+            node->xq = q.back().q; node->sx = q.back().scale; node->wq = q[k].q; node->sw = q[k].scale;
+            node->has_bias = b[k].defined();
+            torch::autograd::set_history(y[k], node);
+        }
+    return y;
 }
 
 // ------------------------------------------------------------------------------------------------ aggregation
@@ -114,7 +147,9 @@ Tensor spmm_copy_u_fn(const GraphPtr &g, const Tensor &n, const Tensor &scale) {
     Tensor out;
     {
         const Raw raw;
-        const Quantized q = quantize(n, scale);
+        QuantJob job = quant_job(n);
+        job.scale = scale;
+        const Quantized q = quantize(job);
         out = spmm_copy_u(*g, false, q.q, q.scale);
     }
     if (auto node = make_node<SpmmCopyUBackward>(n)) {
@@ -141,9 +176,11 @@ struct SpmmUMulEBackward : OnceNode {
     std::vector<int64_t> e_shape;
     variable_list backward(const variable_list &grads) override {
         if (!grads[0].defined()) return variable_list(2);
-        const Quantized z = quantize(grads[0]);
+        QuantJob job = quant_job(grads[0]);
+        if (!compat) job.times[0] = se;
+        const Quantized z = quantize(job);
         Tensor dn, de;
-        if (needs(0)) dn = spmm_u_mul_e(*g, true, z.q, eq, compat ? scale : z.scale.mul(se));
+        if (needs(0)) dn = spmm_u_mul_e(*g, true, z.q, eq, compat ? scale : z.product[0]);
         if (needs(1)) de = sddmm(*g, reduce_last ? "dot" : "mul", nq, z.q, sn, z.scale, {}, false).reshape(e_shape);
         return {dn, de};
     }
@@ -154,11 +191,13 @@ Tensor spmm_u_mul_e_fn(const GraphPtr &g, const Tensor &n, const Tensor &e, cons
     Quantized eq, nq;
     {
         const Raw raw;
-        sn = absmax_scale(n);
-        se = scale_e.defined() ? scale_e : absmax_scale(e);     // the producer may already know max|E| / 127
-        eq = quantize(e.reshape({e.size(0), -1}), se, 1);       // [E, H] int8, edge-id order (no transposed copy)
-        nq = quantize(n, sn);
-        scale = sn.mul(se);
+        QuantJob je = quant_job(e.reshape({e.size(0), -1}), 1);    // [E, H] int8, edge-id order (no transposed copy)
+        je.scale = scale_e;                                        // the producer may already know max|E| / 127
+        QuantJob jn = quant_job(n);
+        jn.times_job = 0;
+        const auto q = quantize_all({je, jn});
+        eq = q[0]; nq = q[1];
+        sn = nq.scale; se = eq.scale; scale = nq.product[0];
         out = spmm_u_mul_e(*g, false, nq.q, eq.q, scale);
     }
     if (auto node = make_node<SpmmUMulEBackward>(n, e)) {
@@ -183,7 +222,7 @@ struct SddmmUAddVBackward : OnceNode {
     GraphPtr g;
     variable_list backward(const variable_list &grads) override {
         if (!grads[0].defined()) return variable_list(2);
-        const Quantized z = quantize(grads[0], {}, row_align(grads[0]));
+        const Quantized z = quantize(grads[0], row_align(grads[0]));
         Tensor du = needs(0) ? incidence_sum(*g, true, z.q, z.scale) : Tensor();
         Tensor dv = needs(1) ? incidence_sum(*g, false, z.q, z.scale) : Tensor();
         return {du, dv};
@@ -195,8 +234,14 @@ Tensor sddmm_u_add_v_fn(const GraphPtr &g, const Tensor &u, const Tensor &v, con
     {
         const Raw raw;
         const int64_t align = row_align(u);
-        const Quantized uq = quantize(u, su, align);
-        const Quantized vq = u.is_same(v) ? uq : quantize(v, sv, align);
+        std::vector<QuantJob> jobs{quant_job(u, align)};
+        jobs[0].scale = su;
+        if (!u.is_same(v)) {
+            jobs.push_back(quant_job(v, align));
+            jobs[1].scale = sv;
+        }
+        const auto q = quantize_all(jobs);
+        const Quantized &uq = q.front(), &vq = q.back();
         out = sddmm(*g, "add", uq.q, vq.q, uq.scale, vq.scale, {}, false);
     }
     if (auto node = make_node<SddmmUAddVBackward>(u, v)) {
@@ -213,15 +258,17 @@ struct SddmmUDotVBackward : OnceNode {
     variable_list backward(const variable_list &grads) override {
         const Tensor &dz = grads[0];
         if (!dz.defined()) return variable_list(2);
-        const Quantized z = quantize(dz.reshape({dz.size(0), -1}), {}, 1);
+        QuantJob job = quant_job(dz.reshape({dz.size(0), -1}), 1);
+        job.times[0] = sv; job.times[1] = su;
+        const Quantized z = quantize(job);
         const bool flat = uq.dim() != 3;
-        auto side = [&](bool reverse, const Tensor &xq, const Tensor &sx) {
-            const Tensor d = spmm_u_mul_e(*g, reverse, flat ? xq.unsqueeze(1) : xq, z.q, sx.mul(z.scale));
+        auto side = [&](bool reverse, const Tensor &xq, const Tensor &scale) {
+            const Tensor d = spmm_u_mul_e(*g, reverse, flat ? xq.unsqueeze(1) : xq, z.q, scale);
             return flat ? d.squeeze(1) : d;
         };
         Tensor du, dv;
-        if (needs(0)) du = side(true, vq, sv);
-        if (needs(1)) dv = side(false, uq, su);
+        if (needs(0)) du = side(true, vq, z.product[0]);
+        if (needs(1)) dv = side(false, uq, z.product[1]);
         return {du, dv};
     }
 };
@@ -231,8 +278,10 @@ Tensor sddmm_u_dot_v_fn(const GraphPtr &g, const Tensor &u, const Tensor &v) {
     Quantized uq, vq;
     {
         const Raw raw;
-        uq = quantize(u);
-        vq = u.is_same(v) ? uq : quantize(v);
+        std::vector<QuantJob> jobs{quant_job(u)};
+        if (!u.is_same(v)) jobs.push_back(quant_job(v));
+        const auto q = quantize_all(jobs);
+        uq = q.front(); vq = q.back();
         out = sddmm(*g, "dot", uq.q, vq.q, uq.scale, vq.scale, {}, false);
     }
     if (auto node = make_node<SddmmUDotVBackward>(u, v)) {
@@ -243,29 +292,6 @@ Tensor sddmm_u_dot_v_fn(const GraphPtr &g, const Tensor &u, const Tensor &v) {
 }
 
 // ------------------------------------------------------------------------------------------------ graph convolution
-// Backward of y = relu(.): int8 of (y > 0 ? g : 0) * row_scale, its scale, and the column sums of the masked gradient.
-static Quantized relu_grad_quantize(const Tensor &grad, const Tensor &y_, const Tensor &row_scale, Tensor *colsum, int mode,
-                                    uint64_t seed, uint64_t call) {
-    const c10::cuda::CUDAGuard guard(grad.device());
-    const Matrix g = matrix(grad), y = matrix(y_);
-    Quantized out{alloc_int8({g.rows, g.cols}, grad.device(), 16), floats({1}, grad)};
-    Tensor scratch;
-    int64_t bytes = 0;
-    if (colsum) {
-        *colsum = floats({g.cols}, grad);
-        bytes = tango_relu_grad_stats_scratch_bytes(g.rows, g.cols);
-        scratch = at::empty({std::max<int64_t>(bytes, 4)}, grad.options().dtype(at::kByte));
-    }
-    check(tango_relu_grad_stats(ptr<float>(g.t), g.ld, ptr<float>(y.t), y.ld, g.rows, g.cols, ptr<float>(row_scale),
-                                ptr<float>(out.scale), colsum ? ptr<float>(*colsum) : nullptr, ptr(scratch), bytes, cuda_stream()),
-          "relu_grad_stats");
-    check(tango_quantize_relu_grad(ptr<float>(g.t), g.ld, ptr<float>(y.t), y.ld, g.rows, g.cols, ptr<float>(row_scale),
-                                   ptr<float>(out.scale), ptr<int8_t>(out.q), out.q.stride(0), mode, seed, call,
-                                   settings().step, cuda_stream()), "quantize_relu_grad");
-    count(colsum ? 3 : 2);
-    return out;
-}
-
 struct GcnConvBackward : OnceNode {
     std::string name() const override { return "GcnConvBackward"; }
     GraphPtr g;
@@ -281,24 +307,18 @@ struct GcnConvBackward : OnceNode {
     variable_list backward(const variable_list &grads) override {
         TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
         if (!grads[0].defined()) return variable_list(3);
-        const int mode = settings().mode_quantize;
-        const uint64_t seed = settings().seed, call = call_if(mode);
-        const bool want_db = has_bias && needs(2);
-        Tensor db;
-        Quantized z;
-        if (relu) {
-            z = relu_grad_quantize(grads[0], out.unpack(shared_from_this()), in_norm, want_db ? &db : nullptr, mode, seed, call);
-        } else {
-            const Tensor d = grads[0].contiguous();
-            if (want_db) db = d.sum(0);
-            z = quantize(d, {}, mode, seed, call, 16, in_norm);
-        }
+        // ReLU mask, bias gradient, right norm, absmax and quantisation: two sweeps of one launch over (grad, out)
+        QuantJob job = quant_job(grads[0]);
+        job.row_scale = in_norm;
+        job.colsum = has_bias && needs(2);
+        if (relu) job.gate = out.unpack(shared_from_this());
+        const Quantized z = quantize(job);
         const Tensor dh = spmm_copy_u(*g, true, z.q, z.scale);
         const Quantized h = quantize(dh);
         // the backward of the left norm is the row factor in dX's epilogue
         Tensor dx = needs(0) ? gemm_dx(h.q, wq, h.scale, sw, out_norm) : Tensor();
         Tensor dw = needs(1) ? gemm_dw(h.q, xq, h.scale, sx) : Tensor();
-        return {dx, dw, db};
+        return {dx, dw, z.colsum};
     }
 };
 
@@ -311,11 +331,15 @@ Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x_, const Tensor &w, const T
         const int mode = settings().mode_gemm;
         const uint64_t seed = settings().seed, call = call_if(mode);
         if (mode == TANGO_ROUND_STOCHASTIC) next_call();
-        xq = quantize(x_.contiguous(), {}, mode, seed, call, 16, out_norm);
-        wq = quantize(w.contiguous(), {}, mode, seed, call + 1, 16);
+        QuantJob jx{x_, mode, seed, call};
+        jx.row_scale = out_norm;
+        const auto q = quantize_all({{w, mode, seed, call + 1}, jx});
+        wq = q[0]; xq = q[1];
         const Tensor h = floats({x_.size(0), w.size(0)}, x_), sh = zeros1(x_);
         gemm_nt(h, xq.q, wq.q, xq.scale, wq.scale, {}, sh);
-        const Quantized hq = quantize(h, sh);
+        QuantJob jh = quant_job(h);
+        jh.scale = sh;
+        const Quantized hq = quantize(jh);
         out = spmm_copy_u(*g, false, hq.q, sh, in_norm, b, relu);
     }
     if (auto node = make_node<GcnConvBackward>(x_, w, b)) {
@@ -394,14 +418,17 @@ struct GatLogits {
 
 static GatLogits gat_logits(const GraphPtr &g, const Tensor &el, const Tensor &er, double slope) {
     const int64_t n = el.size(0), h = el.size(1);
-    const Quantized l = quantize(el.reshape({n, h}), {}, 1), r = quantize(er.reshape({n, h}), {}, 1);
-    return {g, l, r, (float)slope, (int)h};
+    const QuantJob jl = quant_job(el.reshape({n, h}), 1), jr = quant_job(er.reshape({n, h}), 1);
+    const auto q = quantize_all({jl, jr});
+    return {g, q[0], q[1], (float)slope, (int)h};
 }
 
 // d_el / d_er from the gradient of the logits: int8, then summed over out-edges and in-edges.
 static std::pair<Tensor, Tensor> gat_logit_grads(const GatLogits &a, const Tensor &dz, const Tensor &sdz, bool want_l,
                                                  bool want_r, at::IntArrayRef shape_l, at::IntArrayRef shape_r) {
-    const Quantized q = quantize(dz, sdz, 1);
+    QuantJob job = quant_job(dz, 1);
+    job.scale = sdz;
+    const Quantized q = quantize(job);
     Tensor dl = want_l ? incidence_sum(*a.g, true, q.q, sdz).view(shape_l) : Tensor();
     Tensor dr = want_r ? incidence_sum(*a.g, false, q.q, sdz).view(shape_r) : Tensor();
     return {dl, dr};
@@ -473,9 +500,11 @@ struct GatAggregateBackward : OnceNode {
         TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
         if (!grads[0].defined()) return variable_list(3);
         const c10::cuda::CUDAGuard guard(grads[0].device());
-        const Quantized z = quantize(grads[0]);
+        QuantJob job = quant_job(grads[0]);
+        job.times[0] = sa;
+        const Quantized z = quantize(job);
         Tensor d_ft, dl, dr;
-        if (needs(0)) d_ft = spmm_u_mul_e(*l.g, true, z.q, aq, z.scale.mul(sa));
+        if (needs(0)) d_ft = spmm_u_mul_e(*l.g, true, z.q, aq, z.product[0]);
         if (needs(1) || needs(2)) {
             const Tensor da = sddmm(*l.g, "dot", nq, z.q, sn, z.scale, {}, false).reshape({-1, l.h});
             const Tensor dz = at::empty_like(da), sdz = zeros1(da);
@@ -517,8 +546,10 @@ Tensor gat_aggregate_fn(const GraphPtr &g, const Tensor &ft, const Tensor &el, c
                                                ptr<float>(inv), ptr<float>(sa), ptr<int8_t>(aq), mode, settings().seed, call,
                                                settings().step, cuda_stream()), "gat_edge_softmax_quantized");
         count(2);
-        nq = quantize(ft);
-        out = spmm_u_mul_e(*g, false, nq.q, aq, nq.scale.mul(sa));
+        QuantJob jn = quant_job(ft);
+        jn.times[0] = sa;
+        nq = quantize(jn);
+        out = spmm_u_mul_e(*g, false, nq.q, aq, nq.product[0]);
     }
     if (auto node = make_node<GatAggregateBackward>(ft, el, er)) {
         node->l = l; node->m = m; node->inv = inv; node->sa = sa; node->aq = aq; node->nq = nq.q; node->sn = nq.scale;

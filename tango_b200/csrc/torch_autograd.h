@@ -9,6 +9,9 @@ namespace tango_host {
 std::tuple<Tensor, Tensor, Tensor, Tensor> qlinear(const Tensor &x, const Tensor &w, const Tensor &b, bool want_scale,
                                                    const Tensor &xq, const Tensor &sx);
 
+// Layers that read the same input: X and up to three weights quantized in one launch, one GEMM each.
+std::vector<Tensor> qlinear_group(const Tensor &x, const std::vector<Tensor> &w, const std::vector<Tensor> &b);
+
 Tensor spmm_copy_u_fn(const GraphPtr &g, const Tensor &n, const Tensor &scale);
 Tensor spmm_u_mul_e_fn(const GraphPtr &g, const Tensor &n, const Tensor &e, const Tensor &scale_e, bool compat_dn_scale);
 Tensor sddmm_u_add_v_fn(const GraphPtr &g, const Tensor &u, const Tensor &v, const Tensor &su, const Tensor &sv);

@@ -88,7 +88,10 @@ PYBIND11_MODULE(_torch_ops, m) {
     m.def("get_scale", [](const Tensor &t, const py::object &row_scale) { return absmax_scale(t, optional(row_scale)); },
           py::arg("t"), py::arg("row_scale") = py::none());
     m.def("quantize", [](const Tensor &t, const py::object &scale, int mode, uint64_t seed, uint64_t call, int64_t align) {
-        Quantized q = quantize(t, optional(scale), mode, seed, call, align);
+        require(t.is_cuda(), "tensor must be on GPU");
+        QuantJob job{t, mode, seed, call, align};
+        job.scale = optional(scale);
+        const Quantized q = quantize(job);
         return py::make_tuple(q.q, q.scale);
     });
 
@@ -96,6 +99,11 @@ PYBIND11_MODULE(_torch_ops, m) {
                         const py::object &sx) {
         auto [y, sy, xq2, sx2] = qlinear(x, w, optional(b), want_scale, optional(xq), optional(sx));
         return py::make_tuple(y, wrap(sy), xq2, sx2);
+    });
+    m.def("qlinear_group", [](const Tensor &x, const std::vector<Tensor> &w, const std::vector<py::object> &b) {
+        std::vector<Tensor> bias;
+        for (const py::object &o : b) bias.push_back(optional(o));
+        return qlinear_group(x, w, bias);
     });
     m.def("spmm_copy_u", [](const GraphPtr &g, const Tensor &n, const py::object &s) { return spmm_copy_u_fn(g, n, optional(s)); });
     m.def("spmm_u_mul_e", [](const GraphPtr &g, const Tensor &n, const Tensor &e, const py::object &s, bool compat) {

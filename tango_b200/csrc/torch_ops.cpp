@@ -74,32 +74,85 @@ Tensor absmax_scale(const Tensor &t, const Tensor &row_scale) {
     return scale;
 }
 
-void quantize_into(const Tensor &q, const Tensor &t, const Tensor &scale, int mode, uint64_t seed, uint64_t call,
-                   const Tensor &row_scale) {
-    require_float(t);
-    require(q.is_cuda() && q.scalar_type() == at::kChar && q.sizes() == t.sizes(), "int8 CUDA tensor of the input's shape expected");
-    const c10::cuda::CUDAGuard guard(t.device());
-    const Matrix x = matrix(t), o = matrix(q);
-    require(o.t.data_ptr() == q.data_ptr(), "output int8 tensor must be row-strided, not arbitrary-strided");
-    check(tango_quantize(ptr<float>(x.t), x.rows, x.cols, x.ld, ptr<float>(row_scale), ptr<float>(scale), ptr<int8_t>(q),
-                         o.ld, mode, seed, call, settings().step, cuda_stream()), "quantize");
+QuantJob quant_job(const Tensor &t, int64_t align) {
+    QuantJob j;
+    j.t = t;
+    j.mode = settings().mode_quantize;
+    j.seed = settings().seed;
+    j.call = j.mode == TANGO_ROUND_STOCHASTIC ? next_call() : 0;
+    j.align = align;
+    return j;
+}
+
+// A matrix too large for the fused kernel's 32-bit indices: scale, then quantize, then column sums, one after the other.
+static void quantize_large(const QuantJob &j, const tango_quant_job &c, Quantized &o) {
+    if (c.gate) {
+        const int64_t bytes = tango_relu_grad_stats_scratch_bytes(c.rows, c.cols);
+        const Tensor scratch = at::empty({std::max<int64_t>(bytes, 16)}, j.t.options().dtype(at::kByte));
+        check(tango_relu_grad_stats(c.x, c.ldx, c.gate, c.ldgate, c.rows, c.cols, c.row_scale, c.scale, c.colsum, ptr(scratch),
+                                    bytes, cuda_stream()), "relu_grad_stats");
+        check(tango_quantize_relu_grad(c.x, c.ldx, c.gate, c.ldgate, c.rows, c.cols, c.row_scale, c.scale, c.q, c.ldq, c.mode,
+                                       c.seed, c.call, settings().step, cuda_stream()), "quantize_relu_grad");
+    } else {
+        if (!c.fixed_scale)
+            check(tango_absmax_scale(c.x, c.rows, c.cols, c.ldx, c.row_scale, c.scale, cuda_stream()), "get_scale");
+        check(tango_quantize(c.x, c.rows, c.cols, c.ldx, c.row_scale, c.scale, c.q, c.ldq, c.mode, c.seed, c.call,
+                             settings().step, cuda_stream()), "quantize");
+        if (c.colsum) at::sum_out(o.colsum, j.t.reshape({c.rows, c.cols}), at::IntArrayRef{0});
+    }
+    count(3);
+}
+
+std::vector<Quantized> quantize_all(const std::vector<QuantJob> &jobs) {
+    const c10::cuda::CUDAGuard guard(jobs[0].t.device());
+    const size_t n = jobs.size();
+    std::vector<Quantized> out(n);
+    tango_quant_job c[4];
+    Matrix x[4], gate[4];
+    const auto fp = jobs[0].t.options().dtype(at::kFloat);
+    for (size_t k = 0; k < n; ++k) {
+        const QuantJob &j = jobs[k];
+        Quantized &o = out[k];
+        require_float(j.t);
+        x[k] = matrix(j.t);
+        o.q = alloc_int8(j.t.sizes(), j.t.device(), j.align);
+        o.scale = j.scale.defined() ? j.scale : at::empty({1}, fp);
+        if (j.gate.defined()) gate[k] = matrix(j.gate);
+        if (j.colsum) o.colsum = at::empty({x[k].cols}, fp);
+        const Matrix q = matrix(o.q);
+        c[k] = tango_quant_job{};
+        c[k].x = ptr<float>(x[k].t); c[k].rows = x[k].rows; c[k].cols = x[k].cols; c[k].ldx = x[k].ld;
+        c[k].gate = ptr<float>(gate[k].t); c[k].ldgate = gate[k].ld;
+        c[k].row_scale = ptr<float>(j.row_scale);
+        c[k].scale = ptr<float>(o.scale);
+        c[k].fixed_scale = j.scale.defined();
+        c[k].times_job = j.times_job;
+        for (int i = 0; i < 2; ++i)
+            if (j.times[i].defined() || (i == 0 && j.times_job >= 0)) {
+                o.product[i] = at::empty({1}, fp);
+                c[k].times[i] = ptr<float>(j.times[i]);
+                c[k].product[i] = ptr<float>(o.product[i]);
+            }
+        c[k].colsum = ptr<float>(o.colsum);
+        c[k].q = ptr<int8_t>(o.q); c[k].ldq = q.ld;
+        c[k].mode = j.mode; c[k].seed = j.seed; c[k].call = j.call;
+    }
+    const int64_t bytes = tango_quantize_fused_scratch_bytes(c, (int)n);
+    if (bytes < 0) {
+        for (size_t k = 0; k < n; ++k) quantize_large(jobs[k], c[k], out[k]);
+        for (size_t k = 0; k < n; ++k)
+            for (int i = 0; i < 2; ++i)
+                if (c[k].product[i])
+                    at::mul_out(out[k].product[i], out[k].scale, jobs[k].times[i].defined() ? jobs[k].times[i] : out[jobs[k].times_job].scale);
+        return out;
+    }
+    const Tensor scratch = at::empty({std::max<int64_t>(bytes, 16)}, fp.dtype(at::kByte));
+    check(tango_quantize_fused(c, (int)n, settings().step, ptr(scratch), bytes, cuda_stream()), "quantize");
     count(1);
+    return out;
 }
 
-Quantized quantize(const Tensor &t, const Tensor &scale, int mode, uint64_t seed, uint64_t call, int64_t align,
-                   const Tensor &row_scale) {
-    require(t.is_cuda(), "tensor must be on GPU");
-    const Tensor s = scale.defined() ? scale : absmax_scale(t, row_scale);
-    Tensor q = alloc_int8(t.sizes(), t.device(), align);
-    quantize_into(q, t, s, mode, seed, call, row_scale);
-    return {q, s};
-}
-
-Quantized quantize(const Tensor &t, const Tensor &scale, int64_t align, const Tensor &row_scale) {
-    const int mode = settings().mode_quantize;
-    const uint64_t call = mode == TANGO_ROUND_STOCHASTIC ? next_call() : 0;
-    return quantize(t, scale, mode, settings().seed, call, align, row_scale);
-}
+Quantized quantize(const QuantJob &job) { return quantize_all({job})[0]; }
 
 // ------------------------------------------------------------------------------------------------ GEMMs
 void gemm_nt(const Tensor &y, const Tensor &xq, const Tensor &wq, const Tensor &sx, const Tensor &sw,

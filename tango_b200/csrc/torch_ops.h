@@ -78,7 +78,7 @@ using GraphPtr = std::shared_ptr<Graph>;
 // `t` seen as a row-major [rows, cols] matrix with leading dimension ld (elements); `t` may be a contiguous copy.
 struct Matrix {
     Tensor t;
-    int64_t rows, cols, ld;
+    int64_t rows = 0, cols = 0, ld = 0;
 };
 Matrix matrix(const Tensor &t);
 
@@ -95,14 +95,29 @@ Tensor status_word(const at::Device &device);
 // ---- quantisation
 struct Quantized {
     Tensor q, scale;
+    Tensor colsum;        // when asked for: column sums of the (gated) input
+    Tensor product[2];    // when asked for: scale * times[i]
 };
+// What to quantize, with every option of the fused kernel (tango_quant_job).
+struct QuantJob {
+    Tensor t;
+    int mode;
+    uint64_t seed, call;
+    int64_t align = 16;
+    Tensor scale;         // given scale; undefined: max|t| / 127
+    Tensor gate;          // t counts only where gate > 0
+    Tensor row_scale;
+    bool colsum = false;
+    Tensor times[2];
+    int times_job = -1;   // product[0] = this scale * the scale of that job
+};
+// A job with the rounding mode configured for the stand-alone quantizer, drawing a call number when it is stochastic.
+QuantJob quant_job(const Tensor &t, int64_t align = 16);
+// One launch for up to four jobs.
+std::vector<Quantized> quantize_all(const std::vector<QuantJob> &jobs);
+Quantized quantize(const QuantJob &job);
+inline Quantized quantize(const Tensor &t, int64_t align = 16) { return quantize(quant_job(t, align)); }
 Tensor absmax_scale(const Tensor &t, const Tensor &row_scale = {});
-void quantize_into(const Tensor &q, const Tensor &t, const Tensor &scale, int mode, uint64_t seed, uint64_t call,
-                   const Tensor &row_scale = {});
-Quantized quantize(const Tensor &t, const Tensor &scale, int mode, uint64_t seed, uint64_t call, int64_t align,
-                   const Tensor &row_scale = {});
-// with the rounding mode configured for the stand-alone quantizer, drawing a call number when it is stochastic
-Quantized quantize(const Tensor &t, const Tensor &scale = {}, int64_t align = 16, const Tensor &row_scale = {});
 
 // ---- GEMMs
 void gemm_nt(const Tensor &y, const Tensor &xq, const Tensor &wq, const Tensor &sx, const Tensor &sw,

@@ -12,7 +12,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import _native
-from .QLinear import QLinear, Qlinear_func, Qlinear_func_reduce
+from .QLinear import QLinear, Qlinear_func, Qlinear_func_reduce, linear_group
 from .SDDMM import sddmm_u_add_v, sddmm_u_dot_v
 from .SPMM import spmm_copy_u, spmm_u_mul_e
 
@@ -283,9 +283,10 @@ class HGT(nn.Module):
         self.norm = nn.LayerNorm(out_dim) if use_norm else nn.Identity()
 
     def forward(self, g, h):
-        k = self.attn_linear(self.k_linear(h)).view(-1, self.n_heads, self.d_k)
-        v = self.msg_linear(self.v_linear(h)).view(-1, self.n_heads, self.d_k)
-        q = self.q_linear(h).view(-1, self.n_heads, self.d_k)
+        shared = linear_group([self.k_linear, self.v_linear, self.q_linear], h)
+        k = self.attn_linear(next(shared)).view(-1, self.n_heads, self.d_k)
+        v = self.msg_linear(next(shared)).view(-1, self.n_heads, self.d_k)
+        q = next(shared).view(-1, self.n_heads, self.d_k)
         t = sddmm_u_dot_v.apply(g, k, q)
         attn, s_attn = edge_softmax(g, t, 1.0 / self.sqrt_dk, True)   # the reference divides t by sqrt(d_k) first
         out = spmm_u_mul_e.apply(g, v, attn, s_attn).view(-1, self.out_dim)
