@@ -104,7 +104,8 @@ int tango_quantize_relu_grad(const float *g, int64_t ldg, const float *y, int64_
  *   scale[0]  = max |m[r,c] * row_scale[r]| / 127            (fixed_scale: scale[0] is given instead)
  *   q[r,c]    = round_mode(m[r,c] * row_scale[r] / scale[0])  (columns [cols, ldq) are zero; stream as in tango_quantize)
  *   colsum[c] = sum_r m[r,c], added in a fixed order          (optional, not with fixed_scale)
- *   product[i][0] = scale[0] * times[i][0]                    (optional; times[i] == NULL: the scale of job times_job) */
+ *   product[i][0] = scale[0] * times[i][0]                    (optional; times[i] == NULL: the scale of job times_job)
+ * `clear` (optional): clear_words 32-bit words that the launch sets to zero, for kernels behind it that accumulate. */
 typedef struct tango_quant_job {
     const float *x;
     int64_t rows, cols, ldx;
@@ -117,6 +118,8 @@ typedef struct tango_quant_job {
     const float *times[2];
     float *product[2];
     float *colsum;
+    void *clear;
+    int64_t clear_words;
     int8_t *q;
     int64_t ldq;
     int mode;
@@ -144,6 +147,14 @@ int tango_qgemm_nt(const int8_t *xq, int64_t ldx, const int8_t *wq, int64_t ldw,
                    const float *sx, const float *sw, const float *bias, float *y, int64_t ldy, float *scale_y,
                    int *status, tango_stream_t stream);
 
+/* The same product with the element-wise steps around it in the epilogue:
+ * Y = act(acc * (sx*sw) * row_scale[r] + bias[c]); scale_y = max|Y[r,c] * scale_row_factor[r]| / 127 (every optional
+ * argument may be NULL; relu = 0 or 1).  They are the norms, bias and activation of a graph convolution that multiplies
+ * last (evaluation/test_gcn.py:95-137). */
+int tango_qgemm_layer(const int8_t *xq, int64_t ldx, const int8_t *wq, int64_t ldw, int64_t m, int64_t n, int64_t k,
+                      const float *sx, const float *sw, const float *row_scale, const float *bias, int relu, float *y,
+                      int64_t ldy, float *scale_y, const float *scale_row_factor, int *status, tango_stream_t stream);
+
 /* The reference's fused forward: quantises X[M,K] (times row_scale[r] if given) and W[N,K] with the given rounding
  * mode and the scales sx, sw, writes the int8 copies xq, wq that the backward pass re-uses, and computes the GEMM
  * above.  Stochastic mode draws X with `call`, W with `call`+1.  (The reference quantizes on load inside the GEMM,
@@ -168,6 +179,14 @@ int tango_qgemm_dx(const int8_t *dyq, int64_t lddy, const int8_t *wq, int64_t ld
 int tango_qgemm_dw(const int8_t *dyq, int64_t lddy, const int8_t *xq, int64_t ldx, int64_t m, int64_t n, int64_t k,
                    const float *sdy, const float *sx, float *dw, int64_t lddw, void *workspace,
                    int64_t workspace_bytes, int *status, tango_stream_t stream);
+
+/* The same in one launch: the CTA that completes an output tile dequantises it.  `scratch` (16-byte aligned,
+ * tango_qgemm_dw_scratch_bytes; may be NULL when that is 0) must hold ZEROS on entry -- the quantizer launch in front can
+ * clear it (tango_quant_job.clear). */
+int64_t tango_qgemm_dw_scratch_bytes(int64_t m, int64_t n, int64_t k);
+int tango_qgemm_dw_cleared(const int8_t *dyq, int64_t lddy, const int8_t *xq, int64_t ldx, int64_t m, int64_t n,
+                           int64_t k, const float *sdy, const float *sx, float *dw, int64_t lddw, void *scratch,
+                           int64_t scratch_bytes, int *status, tango_stream_t stream);
 
 /* Weight gradient for callers that have no device memory to lend and must not allocate any: same result as
  * tango_qgemm_dw, but the split-K scratch is a fixed 4 MiB array that lives inside the library image, so no

@@ -44,6 +44,8 @@ struct Job {
     float *product[2];
     int times_job;
     float *colsum;              // optional
+    uint32_t *clear;            // optional: words set to zero for the kernels behind this one
+    int64_t clear_words;
     int8_t *q;
     int64_t ldx, ldgate, ldq;
     uint32_t rows, cols;
@@ -342,6 +344,7 @@ __global__ void __launch_bounds__(kThreads, MODE == TANGO_ROUND_STOCHASTIC ? (EX
     while (ji + 1 < p.n_jobs && (int)blockIdx.x >= p.job[ji + 1].first_block) ++ji;
     const Job &j = p.job[ji];
     const int block = blockIdx.x - j.first_block;
+    for (int64_t i = (int64_t)block * kThreads + threadIdx.x; i < j.clear_words; i += (int64_t)j.n_blocks * kThreads) j.clear[i] = 0;
     float scale;
     if (STATS) {
         float m = 0.f;
@@ -358,9 +361,10 @@ __global__ void __launch_bounds__(kThreads, MODE == TANGO_ROUND_STOCHASTIC ? (EX
             if (block == 0 && threadIdx.x == 0) *j.scale = scale;
         }
         if (EXT && j.colsum) {
-            // one warp per column: the CTAs' sums in 32 interleaved chains, then a fixed butterfly
+            // one warp per column, the columns spread over the CTAs: the CTAs' sums in 32 interleaved chains, then a fixed
+            // butterfly (the other warps are already quantising)
             const int lane = threadIdx.x & 31;
-            for (uint32_t c = block * (kThreads / 32) + (threadIdx.x >> 5); c < j.cols; c += j.n_blocks * (kThreads / 32)) {
+            for (uint32_t c = block + (threadIdx.x >> 5) * j.n_blocks; c < j.cols; c += j.n_blocks * (kThreads / 32)) {
                 float t = 0.f;
                 for (int b = lane; b < j.n_blocks; b += 32) t = __fadd_rn(t, __ldcg(j.part_sum + (int64_t)b * j.cols + c));
 #pragma unroll
@@ -438,7 +442,7 @@ int plan(const tango_quant_job *jobs, int n, const uint64_t *step, Launch &l) {
     for (int k = 0; k < n; ++k) {
         const tango_quant_job &s = jobs[k];
         if (s.rows < 0 || s.cols < 0 || s.ldx < s.cols || s.ldq < s.cols || s.mode < 0 || s.mode > 2 || !s.scale ||
-            (s.gate && s.ldgate < s.cols) || (s.colsum && s.fixed_scale))
+            (s.gate && s.ldgate < s.cols) || (s.colsum && s.fixed_scale) || s.clear_words < 0 || (s.clear_words > 0 && !s.clear))
             return TANGO_EINVAL;
         for (int i = 0; i < 2; ++i)
             if (s.product[i] && !s.times[i] && (s.times_job < 0 || s.times_job >= n || s.fixed_scale)) return TANGO_EINVAL;
@@ -448,6 +452,7 @@ int plan(const tango_quant_job *jobs, int n, const uint64_t *step, Launch &l) {
         j.x = s.x; j.gate = s.gate; j.row_scale = s.row_scale; j.scale = s.scale;
         j.times_job = s.times_job;
         for (int i = 0; i < 2; ++i) { j.times[i] = s.times[i]; j.product[i] = s.product[i]; }
+        j.clear = static_cast<uint32_t *>(s.clear); j.clear_words = s.clear_words;
         j.colsum = s.colsum; j.q = s.q; j.seed = s.seed; j.call = s.call; j.fixed = s.fixed_scale;
         int64_t rows = s.rows, cols = s.cols, ldx = s.ldx, ldq = s.ldq, ldg = s.ldgate;
         const bool packed = ldx == cols && (!s.gate || ldg == cols);

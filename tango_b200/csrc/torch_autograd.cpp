@@ -66,9 +66,10 @@ struct QLinearBackward : OnceNode {
         if (!dy.defined()) return variable_list(3);
         QuantJob job = quant_job(dy);
         job.colsum = has_bias && needs(2);          // the bias gradient comes out of the quantizer's first sweep
+        if (needs(1)) job.clear = dw_scratch(dy.size(0), dy.size(1), xq.size(1), dy);
         const Quantized q = quantize(job);
         Tensor dx = needs(0) ? gemm_dx(q.q, wq, q.scale, sw) : Tensor();
-        Tensor dw = needs(1) ? gemm_dw(q.q, xq, q.scale, sx) : Tensor();
+        Tensor dw = needs(1) ? gemm_dw(q.q, xq, q.scale, sx, job.clear) : Tensor();
         return {dx, dw, q.colsum};
     }
 };
@@ -83,7 +84,8 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> qlinear(const Tensor &x, const Tensor
         const int mode = settings().mode_gemm;
         const uint64_t seed = settings().seed, call = call_if(mode);
         if (mode == TANGO_ROUND_STOCHASTIC) next_call();       // the weight draws from call + 1
-        const QuantJob jw{w, mode, seed, call + 1};
+        QuantJob jw{w, mode, seed, call + 1};
+        if (want_scale) jw.clear = sy = floats({1}, x);
         if (xq.defined()) {
             const Quantized q = quantize(jw);
             wq = q.q; sw = q.scale;
@@ -92,7 +94,6 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> qlinear(const Tensor &x, const Tensor
             wq = q[0].q; sw = q[0].scale; xq = q[1].q; sx = q[1].scale;
         }
         y = floats({x.size(0), w.size(0)}, x);
-        if (want_scale) sy = zeros1(x);
         gemm_nt(y, xq, wq, sx, sw, b, sy);
     }
     if (auto node = make_node<QLinearBackward>(x, w, b)) {
@@ -314,10 +315,12 @@ struct GcnConvBackward : OnceNode {
         if (relu) job.gate = out.unpack(shared_from_this());
         const Quantized z = quantize(job);
         const Tensor dh = spmm_copy_u(*g, true, z.q, z.scale);
-        const Quantized h = quantize(dh);
+        QuantJob jh = quant_job(dh);
+        if (needs(1)) jh.clear = dw_scratch(dh.size(0), dh.size(1), xq.size(1), dh);
+        const Quantized h = quantize(jh);
         // the backward of the left norm is the row factor in dX's epilogue
         Tensor dx = needs(0) ? gemm_dx(h.q, wq, h.scale, sw, out_norm) : Tensor();
-        Tensor dw = needs(1) ? gemm_dw(h.q, xq, h.scale, sx) : Tensor();
+        Tensor dw = needs(1) ? gemm_dw(h.q, xq, h.scale, sx, jh.clear) : Tensor();
         return {dx, dw, z.colsum};
     }
 };
@@ -331,11 +334,12 @@ Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x_, const Tensor &w, const T
         const int mode = settings().mode_gemm;
         const uint64_t seed = settings().seed, call = call_if(mode);
         if (mode == TANGO_ROUND_STOCHASTIC) next_call();
+        const Tensor h = floats({x_.size(0), w.size(0)}, x_), sh = floats({1}, x_);
         QuantJob jx{x_, mode, seed, call};
         jx.row_scale = out_norm;
+        jx.clear = sh;
         const auto q = quantize_all({{w, mode, seed, call + 1}, jx});
         wq = q[0]; xq = q[1];
-        const Tensor h = floats({x_.size(0), w.size(0)}, x_), sh = zeros1(x_);
         gemm_nt(h, xq.q, wq.q, xq.scale, wq.scale, {}, sh);
         QuantJob jh = quant_job(h);
         jh.scale = sh;

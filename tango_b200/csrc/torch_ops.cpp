@@ -134,12 +134,16 @@ std::vector<Quantized> quantize_all(const std::vector<QuantJob> &jobs) {
                 c[k].product[i] = ptr<float>(o.product[i]);
             }
         c[k].colsum = ptr<float>(o.colsum);
+        if (j.clear.defined()) { c[k].clear = ptr(j.clear); c[k].clear_words = j.clear.numel(); }
         c[k].q = ptr<int8_t>(o.q); c[k].ldq = q.ld;
         c[k].mode = j.mode; c[k].seed = j.seed; c[k].call = j.call;
     }
     const int64_t bytes = tango_quantize_fused_scratch_bytes(c, (int)n);
     if (bytes < 0) {
-        for (size_t k = 0; k < n; ++k) quantize_large(jobs[k], c[k], out[k]);
+        for (size_t k = 0; k < n; ++k) {
+            if (jobs[k].clear.defined()) Tensor(jobs[k].clear).zero_();
+            quantize_large(jobs[k], c[k], out[k]);
+        }
         for (size_t k = 0; k < n; ++k)
             for (int i = 0; i < 2; ++i)
                 if (c[k].product[i])
@@ -176,16 +180,18 @@ Tensor gemm_dx(const Tensor &dyq, const Tensor &wq, const Tensor &sdy, const Ten
     return dx;
 }
 
-Tensor gemm_dw(const Tensor &dyq, const Tensor &xq, const Tensor &sdy, const Tensor &sx) {
+Tensor dw_scratch(int64_t m, int64_t n, int64_t k, const Tensor &like) {
+    return at::empty({tango_qgemm_dw_scratch_bytes(m, n, k) / 4}, like.options().dtype(at::kInt));
+}
+
+Tensor gemm_dw(const Tensor &dyq, const Tensor &xq, const Tensor &sdy, const Tensor &sx, const Tensor &scratch) {
     const c10::cuda::CUDAGuard guard(dyq.device());
     const Matrix dy = matrix(dyq), x = matrix(xq);
     Tensor dw = floats({dy.cols, x.cols}, sdy);
-    const int64_t bytes = tango_qgemm_dw_workspace_bytes(dy.cols, x.cols);
-    const Tensor ws = at::empty({std::max<int64_t>(bytes, 16)}, dyq.options().dtype(at::kByte));
-    check(tango_qgemm_dw(ptr<int8_t>(dy.t), dy.ld, ptr<int8_t>(x.t), x.ld, dy.rows, dy.cols, x.cols, ptr<float>(sdy),
-                         ptr<float>(sx), ptr<float>(dw), x.cols, ptr(ws), bytes, ptr<int>(status_word(dyq.device())),
-                         cuda_stream()), "QGEMM_backward_gradW");
-    count(2);
+    check(tango_qgemm_dw_cleared(ptr<int8_t>(dy.t), dy.ld, ptr<int8_t>(x.t), x.ld, dy.rows, dy.cols, x.cols, ptr<float>(sdy),
+                                 ptr<float>(sx), ptr<float>(dw), x.cols, ptr(scratch), scratch.numel() * 4,
+                                 ptr<int>(status_word(dyq.device())), cuda_stream()), "QGEMM_backward_gradW");
+    count(1);
     return dw;
 }
 
