@@ -105,7 +105,7 @@ int tango_quantize_relu_grad(const float *g, int64_t ldg, const float *y, int64_
  *   q[r,c]    = round_mode(m[r,c] * row_scale[r] / scale[0])  (columns [cols, ldq) are zero; stream as in tango_quantize)
  *   colsum[c] = sum_r m[r,c], added in a fixed order          (optional, not with fixed_scale)
  *   product[i][0] = scale[0] * times[i][0]                    (optional; times[i] == NULL: the scale of job times_job)
- * `clear` (optional): clear_words 32-bit words that the launch sets to zero, for kernels behind it that accumulate. */
+ * clear[i] (optional): clear_words[i] 32-bit words that the launch sets to zero, for kernels behind it that accumulate. */
 typedef struct tango_quant_job {
     const float *x;
     int64_t rows, cols, ldx;
@@ -118,8 +118,8 @@ typedef struct tango_quant_job {
     const float *times[2];
     float *product[2];
     float *colsum;
-    void *clear;
-    int64_t clear_words;
+    void *clear[2];
+    int64_t clear_words[2];
     int8_t *q;
     int64_t ldq;
     int mode;
@@ -172,6 +172,11 @@ int tango_qgemm_forward(const float *x, int64_t ldx_f, const float *row_scale, c
 int tango_qgemm_dx(const int8_t *dyq, int64_t lddy, const int8_t *wq, int64_t ldw, int64_t m, int64_t n, int64_t k,
                    const float *sdy, const float *sw, const float *row_scale, float *dx, int64_t lddx, int *status,
                    tango_stream_t stream);
+
+/* The same; scale_dx (holding 0 on entry) receives max|dX| / 127 for the quantizer behind it. */
+int tango_qgemm_dx_layer(const int8_t *dyq, int64_t lddy, const int8_t *wq, int64_t ldw, int64_t m, int64_t n, int64_t k,
+                         const float *sdy, const float *sw, const float *row_scale, float *dx, int64_t lddx,
+                         float *scale_dx, int *status, tango_stream_t stream);
 
 /* dW[N,K] = float(dYq^T[N,M] . Xq[M,K]) * (sdy[0]*sx[0]); split over M with int32 atomics into `workspace`
  * (tango_qgemm_dw_workspace_bytes; contents on entry are irrelevant), then dequantised.

@@ -745,17 +745,23 @@ extern "C" int tango_qgemm_forward(const float *x, int64_t ldx_f, const float *r
     return tango_qgemm_nt(xq, ldxq, wq, ldwq, m, n, k, sx, sw, bias, y, ldy, scale_y, status, stream);
 }
 
-extern "C" int tango_qgemm_dx(const int8_t *dyq, int64_t lddy, const int8_t *wq, int64_t ldw, int64_t m, int64_t n,
-                              int64_t k, const float *sdy, const float *sw, const float *row_scale, float *dx,
-                              int64_t lddx, int *status, tango_stream_t stream) {
+extern "C" int tango_qgemm_dx_layer(const int8_t *dyq, int64_t lddy, const int8_t *wq, int64_t ldw, int64_t m, int64_t n,
+                                    int64_t k, const float *sdy, const float *sw, const float *row_scale, float *dx,
+                                    int64_t lddx, float *scale_dx, int *status, tango_stream_t stream) {
     if (m < 0 || n <= 0 || k < 0 || lddy < n || ldw < k || lddx < k) return TANGO_EINVAL;
     if (m == 0 || k == 0) return TANGO_OK;
     if (!dyq || !wq || !sdy || !sw || !dx) return TANGO_EINVAL;
     // D[m, k] = A[m, n] . B[n, k]: reduction n; B is stored with the reduction index as its row
     GemmCall c{};
     c.a = dyq; c.lda = lddy; c.b = wq; c.ldb = ldw; c.b_mn = 1; c.M = m; c.N = k; c.K = n; c.mode = MODE_STORE; c.splits = 1;
-    c.out = dx; c.ldo = lddx; c.sa = sdy; c.sb = sw; c.out_row_scale = row_scale; c.status = status;
+    c.out = dx; c.ldo = lddx; c.sa = sdy; c.sb = sw; c.out_row_scale = row_scale; c.absmax = scale_dx; c.status = status;
     return launch_gemm(c, (cudaStream_t)stream);
+}
+
+extern "C" int tango_qgemm_dx(const int8_t *dyq, int64_t lddy, const int8_t *wq, int64_t ldw, int64_t m, int64_t n,
+                              int64_t k, const float *sdy, const float *sw, const float *row_scale, float *dx,
+                              int64_t lddx, int *status, tango_stream_t stream) {
+    return tango_qgemm_dx_layer(dyq, lddy, wq, ldw, m, n, k, sdy, sw, row_scale, dx, lddx, nullptr, status, stream);
 }
 
 // D[n, k] = A[n, m] . B[m, k]: both operands are stored with the reduction index m as their row

@@ -44,8 +44,8 @@ struct Job {
     float *product[2];
     int times_job;
     float *colsum;              // optional
-    uint32_t *clear;            // optional: words set to zero for the kernels behind this one
-    int64_t clear_words;
+    uint32_t *clear[2];         // optional: words set to zero for the kernels behind this one
+    int64_t clear_words[2];
     int8_t *q;
     int64_t ldx, ldgate, ldq;
     uint32_t rows, cols;
@@ -344,7 +344,10 @@ __global__ void __launch_bounds__(kThreads, MODE == TANGO_ROUND_STOCHASTIC ? (EX
     while (ji + 1 < p.n_jobs && (int)blockIdx.x >= p.job[ji + 1].first_block) ++ji;
     const Job &j = p.job[ji];
     const int block = blockIdx.x - j.first_block;
-    for (int64_t i = (int64_t)block * kThreads + threadIdx.x; i < j.clear_words; i += (int64_t)j.n_blocks * kThreads) j.clear[i] = 0;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        for (int64_t i = (int64_t)block * kThreads + threadIdx.x; i < j.clear_words[k]; i += (int64_t)j.n_blocks * kThreads)
+            j.clear[k][i] = 0;
     float scale;
     if (STATS) {
         float m = 0.f;
@@ -442,17 +445,19 @@ int plan(const tango_quant_job *jobs, int n, const uint64_t *step, Launch &l) {
     for (int k = 0; k < n; ++k) {
         const tango_quant_job &s = jobs[k];
         if (s.rows < 0 || s.cols < 0 || s.ldx < s.cols || s.ldq < s.cols || s.mode < 0 || s.mode > 2 || !s.scale ||
-            (s.gate && s.ldgate < s.cols) || (s.colsum && s.fixed_scale) || s.clear_words < 0 || (s.clear_words > 0 && !s.clear))
+            (s.gate && s.ldgate < s.cols) || (s.colsum && s.fixed_scale))
             return TANGO_EINVAL;
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < 2; ++i) {
+            if (s.clear_words[i] < 0 || (s.clear_words[i] > 0 && !s.clear[i])) return TANGO_EINVAL;
             if (s.product[i] && !s.times[i] && (s.times_job < 0 || s.times_job >= n || s.fixed_scale)) return TANGO_EINVAL;
+        }
         if (s.rows > 0 && s.cols > 0 && (!s.x || !s.q)) return TANGO_EINVAL;
         if (s.rows > 0 && s.ldq > 0 && !s.q) return TANGO_EINVAL;
         Job j{};
         j.x = s.x; j.gate = s.gate; j.row_scale = s.row_scale; j.scale = s.scale;
         j.times_job = s.times_job;
         for (int i = 0; i < 2; ++i) { j.times[i] = s.times[i]; j.product[i] = s.product[i]; }
-        j.clear = static_cast<uint32_t *>(s.clear); j.clear_words = s.clear_words;
+        for (int i = 0; i < 2; ++i) { j.clear[i] = static_cast<uint32_t *>(s.clear[i]); j.clear_words[i] = s.clear_words[i]; }
         j.colsum = s.colsum; j.q = s.q; j.seed = s.seed; j.call = s.call; j.fixed = s.fixed_scale;
         int64_t rows = s.rows, cols = s.cols, ldx = s.ldx, ldq = s.ldq, ldg = s.ldgate;
         const bool packed = ldx == cols && (!s.gate || ldg == cols);

@@ -59,17 +59,17 @@ static uint64_t call_if(int mode) { return mode == TANGO_ROUND_STOCHASTIC ? next
 // ------------------------------------------------------------------------------------------------ QLinear
 struct QLinearBackward : OnceNode {
     std::string name() const override { return "QLinearBackward"; }
-    Tensor xq, sx, wq, sw;
+    Quantized x, w;
     bool has_bias = false;
     variable_list backward(const variable_list &grads) override {
         const Tensor &dy = grads[0];
         if (!dy.defined()) return variable_list(3);
         QuantJob job = quant_job(dy);
         job.colsum = has_bias && needs(2);          // the bias gradient comes out of the quantizer's first sweep
-        if (needs(1)) job.clear = dw_scratch(dy.size(0), dy.size(1), xq.size(1), dy);
+        if (needs(1)) job.clear = dw_scratch(dy.size(0), dy.size(1), x.q.size(1), dy);
         const Quantized q = quantize(job);
-        Tensor dx = needs(0) ? gemm_dx(q.q, wq, q.scale, sw) : Tensor();
-        Tensor dw = needs(1) ? gemm_dw(q.q, xq, q.scale, sx, job.clear) : Tensor();
+        Tensor dx = needs(0) ? gemm_dx(q, w) : Tensor();
+        Tensor dw = needs(1) ? gemm_dw(q, x, job.clear) : Tensor();
         return {dx, dw, q.colsum};
     }
 };
@@ -78,7 +78,8 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> qlinear(const Tensor &x, const Tensor
                                                    const Tensor &xq_, const Tensor &sx_) {
     require(x.is_cuda() && w.is_cuda() && (!b.defined() || b.is_cuda()), "x, w and b must be on the GPU");
     require(x.size(1) == w.size(1), "x and w must have the same number of columns");
-    Tensor y, sy, xq = xq_, sx = sx_, wq, sw;
+    Tensor y, sy;
+    Quantized xq, wq;
     {
         const Raw raw;
         const int mode = settings().mode_gemm;
@@ -86,21 +87,20 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> qlinear(const Tensor &x, const Tensor
         if (mode == TANGO_ROUND_STOCHASTIC) next_call();       // the weight draws from call + 1
         QuantJob jw{w, mode, seed, call + 1};
         if (want_scale) jw.clear = sy = floats({1}, x);
-        if (xq.defined()) {
-            const Quantized q = quantize(jw);
-            wq = q.q; sw = q.scale;
+        if (xq_.defined()) {
+            xq.q = xq_; xq.scale = sx_;
+            wq = quantize(jw);
         } else {
             const auto q = quantize_all({jw, {x, mode, seed, call}});
-            wq = q[0].q; sw = q[0].scale; xq = q[1].q; sx = q[1].scale;
+            wq = q[0]; xq = q[1];
         }
-        y = floats({x.size(0), w.size(0)}, x);
-        gemm_nt(y, xq, wq, sx, sw, b, sy);
+        y = gemm_nt(xq, wq, b, sy);
     }
     if (auto node = make_node<QLinearBackward>(x, w, b)) {
-        node->xq = xq; node->sx = sx; node->wq = wq; node->sw = sw; node->has_bias = b.defined();
+        node->x = xq; node->w = wq; node->has_bias = b.defined();
         torch::autograd::set_history(y, node);
     }
-    return {y, sy, xq, sx};
+    return {y, sy, xq.q, xq.scale};
 }
 
 std::vector<Tensor> qlinear_group(const Tensor &x, const std::vector<Tensor> &w, const std::vector<Tensor> &b) {
@@ -119,15 +119,11 @@ std::vector<Tensor> qlinear_group(const Tensor &x, const std::vector<Tensor> &w,
         }
         jobs.push_back({x, mode, seed, 0});
         q = quantize_all(jobs);
-        for (size_t k = 0; k < w.size(); ++k) {
-            y.push_back(floats({x.size(0), w[k].size(0)}, x));
-            gemm_nt(y[k], q.back().q, q[k].q, q.back().scale, q[k].scale, b[k], {});
-        }
+        for (size_t k = 0; k < w.size(); ++k) y.push_back(gemm_nt(q.back(), q[k], b[k]));
     }
     for (size_t k = 0; k < w.size(); ++k)
         if (auto node = make_node<QLinearBackward>(x, w[k], b[k])) {
-            node->xq = q.back().q; node->sx = q.back().scale; node->wq = q[k].q; node->sw = q[k].scale;
-            node->has_bias = b[k].defined();
+            node->x = q.back(); node->w = q[k]; node->has_bias = b[k].defined();
             torch::autograd::set_history(y[k], node);
         }
     return y;
@@ -293,61 +289,105 @@ Tensor sddmm_u_dot_v_fn(const GraphPtr &g, const Tensor &u, const Tensor &v) {
 }
 
 // ------------------------------------------------------------------------------------------------ graph convolution
+// act((A . X') W^T ...) with the norms of both sides, bias and ReLU.  `first` says which product runs first: the linear
+// layer where it narrows the features (its int8 output is aggregated), else the aggregation (its fp32 output is quantized for
+// the linear layer).  Either way the element-wise steps sit in the kernels next to them, and every tensor that a kernel here
+// produces for a quantizer brings its scale along (epilogue maximum), so only the inputs of the layer are swept for theirs.
+enum class First { linear, aggregate };
+
 struct GcnConvBackward : OnceNode {
     std::string name() const override { return "GcnConvBackward"; }
     GraphPtr g;
-    Tensor xq, sx, wq, sw, out_norm, in_norm;
+    First first = First::linear;
+    Quantized x, w;                 // operands of the linear layer
+    Tensor out_norm, in_norm;
     SavedVariable out;
     bool relu = false, has_bias = false, released = false;
 
     void release_variables() override {
-        xq.reset(); wq.reset();
+        x.q.reset(); w.q.reset();
         out.reset_data();
         released = true;
     }
     variable_list backward(const variable_list &grads) override {
         TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
-        if (!grads[0].defined()) return variable_list(3);
+        const Tensor &d = grads[0];
+        if (!d.defined()) return variable_list(3);
         // ReLU mask, bias gradient, right norm, absmax and quantisation: two sweeps of one launch over (grad, out)
-        QuantJob job = quant_job(grads[0]);
+        QuantJob job = quant_job(d);
         job.row_scale = in_norm;
         job.colsum = has_bias && needs(2);
         if (relu) job.gate = out.unpack(shared_from_this());
+        const Tensor dw_tmp = needs(1) ? dw_scratch(d.size(0), w.q.size(0), x.q.size(1), d) : Tensor();
+        const Tensor scale = floats({1}, d);
+        Tensor dx, dw;
+        if (first == First::linear) {
+            job.clear = scale;
+            const Quantized z = quantize(job);
+            const Tensor dh = spmm_copy_u(*g, true, z.q, z.scale, {}, {}, false, scale);
+            QuantJob jh = quant_job(dh);
+            jh.scale = scale;
+            jh.clear = dw_tmp;
+            const Quantized h = quantize(jh);
+            // the backward of the left norm is the row factor in dX's epilogue
+            if (needs(0)) dx = gemm_dx(h, w, out_norm);
+            if (needs(1)) dw = gemm_dw(h, x, dw_tmp);
+            return {dx, dw, z.colsum};
+        }
+        job.clear = dw_tmp;
+        job.clear2 = scale;
         const Quantized z = quantize(job);
-        const Tensor dh = spmm_copy_u(*g, true, z.q, z.scale);
-        QuantJob jh = quant_job(dh);
-        if (needs(1)) jh.clear = dw_scratch(dh.size(0), dh.size(1), xq.size(1), dh);
-        const Quantized h = quantize(jh);
-        // the backward of the left norm is the row factor in dX's epilogue
-        Tensor dx = needs(0) ? gemm_dx(h.q, wq, h.scale, sw, out_norm) : Tensor();
-        Tensor dw = needs(1) ? gemm_dw(h.q, xq, h.scale, sx, jh.clear) : Tensor();
+        if (needs(1)) dw = gemm_dw(z, x, dw_tmp);
+        if (needs(0)) {
+            const Tensor da = gemm_dx(z, w, {}, scale);
+            QuantJob ja = quant_job(da);
+            ja.scale = scale;
+            const Quantized a = quantize(ja);
+            dx = spmm_copy_u(*g, true, a.q, a.scale, out_norm);
+        }
         return {dx, dw, z.colsum};
     }
 };
 
 Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x_, const Tensor &w, const Tensor &b, const Tensor &out_norm,
-                   const Tensor &in_norm, bool relu) {
+                   const Tensor &in_norm, bool relu, bool linear_first) {
     Tensor out;
-    Quantized xq, wq;
+    Quantized x, wq;
     {
         const Raw raw;
         const int mode = settings().mode_gemm;
-        const uint64_t seed = settings().seed, call = call_if(mode);
-        if (mode == TANGO_ROUND_STOCHASTIC) next_call();
-        const Tensor h = floats({x_.size(0), w.size(0)}, x_), sh = floats({1}, x_);
-        QuantJob jx{x_, mode, seed, call};
-        jx.row_scale = out_norm;
-        jx.clear = sh;
-        const auto q = quantize_all({{w, mode, seed, call + 1}, jx});
-        wq = q[0]; xq = q[1];
-        gemm_nt(h, xq.q, wq.q, xq.scale, wq.scale, {}, sh);
-        QuantJob jh = quant_job(h);
-        jh.scale = sh;
-        const Quantized hq = quantize(jh);
-        out = spmm_copy_u(*g, false, hq.q, sh, in_norm, b, relu);
+        const uint64_t seed = settings().seed;
+        const Tensor scale = floats({1}, x_);
+        if (linear_first) {
+            const uint64_t call = call_if(mode);
+            if (mode == TANGO_ROUND_STOCHASTIC) next_call();
+            QuantJob jx{x_, mode, seed, call};
+            jx.row_scale = out_norm;
+            jx.clear = scale;
+            const auto q = quantize_all({{w, mode, seed, call + 1}, jx});
+            wq = q[0]; x = q[1];
+            const Tensor h = gemm_nt(x, wq, {}, scale);
+            QuantJob jh = quant_job(h);
+            jh.scale = scale;
+            const Quantized hq = quantize(jh);
+            out = spmm_copy_u(*g, false, hq.q, scale, in_norm, b, relu);
+        } else {
+            QuantJob jx = quant_job(x_);
+            jx.row_scale = out_norm;
+            jx.clear = scale;
+            const Quantized xq = quantize(jx);
+            const Tensor a = spmm_copy_u(*g, false, xq.q, xq.scale, {}, {}, false, scale);
+            const uint64_t call = call_if(mode);
+            if (mode == TANGO_ROUND_STOCHASTIC) next_call();
+            QuantJob ja{a, mode, seed, call};
+            ja.scale = scale;
+            const auto q = quantize_all({{w, mode, seed, call + 1}, ja});
+            wq = q[0]; x = q[1];
+            out = gemm_nt(x, wq, b, {}, in_norm, relu);
+        }
     }
     if (auto node = make_node<GcnConvBackward>(x_, w, b)) {
-        node->g = g; node->xq = xq.q; node->sx = xq.scale; node->wq = wq.q; node->sw = wq.scale;
+        node->g = g; node->first = linear_first ? First::linear : First::aggregate; node->x = x; node->w = wq;
         node->out_norm = out_norm; node->in_norm = in_norm; node->relu = relu; node->has_bias = b.defined();
         torch::autograd::set_history(out, node);
         if (relu) node->out = SavedVariable(out, true);

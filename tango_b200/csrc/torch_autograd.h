@@ -17,9 +17,10 @@ Tensor spmm_u_mul_e_fn(const GraphPtr &g, const Tensor &n, const Tensor &e, cons
 Tensor sddmm_u_add_v_fn(const GraphPtr &g, const Tensor &u, const Tensor &v, const Tensor &su, const Tensor &sv);
 Tensor sddmm_u_dot_v_fn(const GraphPtr &g, const Tensor &u, const Tensor &v);
 
-// One "multiply first" graph convolution: act((A . Q(Q(X * out_norm) W^T)) * in_norm + b).
+// One graph convolution, norm='both', the linear layer or the aggregation first:
+// act((A . Q(Q(X * out_norm) W^T)) * in_norm + b)  or  act((Q(A . Q(X * out_norm)) W^T) * in_norm + b).
 Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x, const Tensor &w, const Tensor &b, const Tensor &out_norm,
-                   const Tensor &in_norm, bool relu);
+                   const Tensor &in_norm, bool relu, bool linear_first);
 
 // softmax(z * factor) over the incoming edges of every destination; (weights, max|weight| / 127).
 std::tuple<Tensor, Tensor> edge_softmax_fn(const GraphPtr &g, const Tensor &z, double factor);

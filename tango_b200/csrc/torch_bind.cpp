@@ -114,7 +114,9 @@ PYBIND11_MODULE(_torch_ops, m) {
     });
     m.def("sddmm_u_dot_v", &sddmm_u_dot_v_fn);
     m.def("gcn_conv", [](const GraphPtr &g, const Tensor &x, const Tensor &w, const py::object &b, const Tensor &out_norm,
-                         const Tensor &in_norm, bool relu) { return gcn_conv_fn(g, x, w, optional(b), out_norm, in_norm, relu); });
+                         const Tensor &in_norm, bool relu, bool linear_first) {
+        return gcn_conv_fn(g, x, w, optional(b), out_norm, in_norm, relu, linear_first);
+    });
     m.def("edge_softmax", &edge_softmax_fn);
     m.def("gat_attention", &gat_attention_fn);
     m.def("gat_aggregate", &gat_aggregate_fn);

@@ -134,14 +134,17 @@ std::vector<Quantized> quantize_all(const std::vector<QuantJob> &jobs) {
                 c[k].product[i] = ptr<float>(o.product[i]);
             }
         c[k].colsum = ptr<float>(o.colsum);
-        if (j.clear.defined()) { c[k].clear = ptr(j.clear); c[k].clear_words = j.clear.numel(); }
+        const Tensor *clear[2] = {&j.clear, &j.clear2};
+        for (int i = 0; i < 2; ++i)
+            if (clear[i]->defined()) { c[k].clear[i] = ptr(*clear[i]); c[k].clear_words[i] = clear[i]->numel(); }
         c[k].q = ptr<int8_t>(o.q); c[k].ldq = q.ld;
         c[k].mode = j.mode; c[k].seed = j.seed; c[k].call = j.call;
     }
     const int64_t bytes = tango_quantize_fused_scratch_bytes(c, (int)n);
     if (bytes < 0) {
         for (size_t k = 0; k < n; ++k) {
-            if (jobs[k].clear.defined()) Tensor(jobs[k].clear).zero_();
+            for (const Tensor &t : {jobs[k].clear, jobs[k].clear2})
+                if (t.defined()) t.zero_();
             quantize_large(jobs[k], c[k], out[k]);
         }
         for (size_t k = 0; k < n; ++k)
@@ -159,23 +162,26 @@ std::vector<Quantized> quantize_all(const std::vector<QuantJob> &jobs) {
 Quantized quantize(const QuantJob &job) { return quantize_all({job})[0]; }
 
 // ------------------------------------------------------------------------------------------------ GEMMs
-void gemm_nt(const Tensor &y, const Tensor &xq, const Tensor &wq, const Tensor &sx, const Tensor &sw,
-             const Tensor &bias, const Tensor &scale_y) {
-    const c10::cuda::CUDAGuard guard(y.device());
-    const Matrix x = matrix(xq), w = matrix(wq), o = matrix(y);
-    check(tango_qgemm_nt(ptr<int8_t>(x.t), x.ld, ptr<int8_t>(w.t), w.ld, x.rows, w.rows, x.cols, ptr<float>(sx),
-                         ptr<float>(sw), ptr<float>(bias), ptr<float>(y), o.ld, ptr<float>(scale_y),
-                         ptr<int>(status_word(y.device())), cuda_stream()), "qgemm_nt");
+Tensor gemm_nt(const Quantized &xq, const Quantized &wq, const Tensor &bias, const Tensor &scale_out, const Tensor &row_scale,
+               bool relu) {
+    const c10::cuda::CUDAGuard guard(xq.q.device());
+    const Matrix x = matrix(xq.q), w = matrix(wq.q);
+    Tensor y = floats({x.rows, w.rows}, xq.scale);
+    check(tango_qgemm_layer(ptr<int8_t>(x.t), x.ld, ptr<int8_t>(w.t), w.ld, x.rows, w.rows, x.cols, ptr<float>(xq.scale),
+                            ptr<float>(wq.scale), ptr<float>(row_scale), ptr<float>(bias), relu, ptr<float>(y), w.rows,
+                            ptr<float>(scale_out), nullptr, ptr<int>(status_word(y.device())), cuda_stream()), "qgemm_nt");
     count(1);
+    return y;
 }
 
-Tensor gemm_dx(const Tensor &dyq, const Tensor &wq, const Tensor &sdy, const Tensor &sw, const Tensor &row_scale) {
-    const c10::cuda::CUDAGuard guard(dyq.device());
-    const Matrix dy = matrix(dyq), w = matrix(wq);
-    Tensor dx = floats({dy.rows, w.cols}, sdy);
-    check(tango_qgemm_dx(ptr<int8_t>(dy.t), dy.ld, ptr<int8_t>(w.t), w.ld, dy.rows, dy.cols, w.cols, ptr<float>(sdy),
-                         ptr<float>(sw), ptr<float>(row_scale), ptr<float>(dx), w.cols,
-                         ptr<int>(status_word(dyq.device())), cuda_stream()), "QGEMM_backward_gradX");
+Tensor gemm_dx(const Quantized &dyq, const Quantized &wq, const Tensor &row_scale, const Tensor &scale_out) {
+    const c10::cuda::CUDAGuard guard(dyq.q.device());
+    const Matrix dy = matrix(dyq.q), w = matrix(wq.q);
+    Tensor dx = floats({dy.rows, w.cols}, dyq.scale);
+    check(tango_qgemm_dx_layer(ptr<int8_t>(dy.t), dy.ld, ptr<int8_t>(w.t), w.ld, dy.rows, dy.cols, w.cols,
+                               ptr<float>(dyq.scale), ptr<float>(wq.scale), ptr<float>(row_scale), ptr<float>(dx), w.cols,
+                               ptr<float>(scale_out), ptr<int>(status_word(dx.device())), cuda_stream()),
+          "QGEMM_backward_gradX");
     count(1);
     return dx;
 }
@@ -184,13 +190,13 @@ Tensor dw_scratch(int64_t m, int64_t n, int64_t k, const Tensor &like) {
     return at::empty({tango_qgemm_dw_scratch_bytes(m, n, k) / 4}, like.options().dtype(at::kInt));
 }
 
-Tensor gemm_dw(const Tensor &dyq, const Tensor &xq, const Tensor &sdy, const Tensor &sx, const Tensor &scratch) {
-    const c10::cuda::CUDAGuard guard(dyq.device());
-    const Matrix dy = matrix(dyq), x = matrix(xq);
-    Tensor dw = floats({dy.cols, x.cols}, sdy);
-    check(tango_qgemm_dw_cleared(ptr<int8_t>(dy.t), dy.ld, ptr<int8_t>(x.t), x.ld, dy.rows, dy.cols, x.cols, ptr<float>(sdy),
-                                 ptr<float>(sx), ptr<float>(dw), x.cols, ptr(scratch), scratch.numel() * 4,
-                                 ptr<int>(status_word(dyq.device())), cuda_stream()), "QGEMM_backward_gradW");
+Tensor gemm_dw(const Quantized &dyq, const Quantized &xq, const Tensor &scratch) {
+    const c10::cuda::CUDAGuard guard(dyq.q.device());
+    const Matrix dy = matrix(dyq.q), x = matrix(xq.q);
+    Tensor dw = floats({dy.cols, x.cols}, dyq.scale);
+    check(tango_qgemm_dw_cleared(ptr<int8_t>(dy.t), dy.ld, ptr<int8_t>(x.t), x.ld, dy.rows, dy.cols, x.cols,
+                                 ptr<float>(dyq.scale), ptr<float>(xq.scale), ptr<float>(dw), x.cols, ptr(scratch),
+                                 scratch.numel() * 4, ptr<int>(status_word(dw.device())), cuda_stream()), "QGEMM_backward_gradW");
     count(1);
     return dw;
 }
@@ -245,7 +251,7 @@ static const int32_t *index_ptr(const Tensor &t, const Tensor &indptr) {
 static int64_t short_launch(const Schedule &s) { return s.present && s.n_long < s.row_order.numel(); }
 
 Tensor spmm_copy_u(const Graph &g, bool reverse, const Tensor &nq, const Tensor &scale, const Tensor &row_scale,
-                   const Tensor &bias, bool relu) {
+                   const Tensor &bias, bool relu, const Tensor &scale_out) {
     const c10::cuda::CUDAGuard guard(nq.device());
     const Direction &d = g.dir(reverse);
     const Matrix n = matrix(nq);
@@ -259,7 +265,7 @@ Tensor spmm_copy_u(const Graph &g, bool reverse, const Tensor &nq, const Tensor 
     const Tensor &indptr = hub ? d.hub_indptr : d.indptr;
     check(tango_spmm_copy_u(ptr<int32_t>(indptr), index_ptr(hub ? d.hub_indices : d.indices, indptr), g.n_nodes, 1,
                             ptr<int8_t>(n.t), n.ld, n.cols, ptr<float>(scale), ptr<float>(row_scale), ptr<float>(bias),
-                            relu, ptr<float>(out), n.cols, nullptr, plan.get(s), cuda_stream()), "csr_SPMM");
+                            relu, ptr<float>(out), n.cols, ptr<float>(scale_out), plan.get(s), cuda_stream()), "csr_SPMM");
     count(1 + (s.n_heavy > 0) + short_launch(s) + (hub ? 2 : 0));
     return out;
 }

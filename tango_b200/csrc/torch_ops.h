@@ -110,7 +110,7 @@ struct QuantJob {
     bool colsum = false;
     Tensor times[2];
     int times_job = -1;   // product[0] = this scale * the scale of that job
-    Tensor clear;         // set to zero by the launch (4-byte elements), for the kernels behind it that accumulate
+    Tensor clear, clear2; // set to zero by the launch (4-byte elements), for the kernels behind it that accumulate
 };
 // A job with the rounding mode configured for the stand-alone quantizer, drawing a call number when it is stochastic.
 QuantJob quant_job(const Tensor &t, int64_t align = 16);
@@ -121,17 +121,17 @@ inline Quantized quantize(const Tensor &t, int64_t align = 16) { return quantize
 Tensor absmax_scale(const Tensor &t, const Tensor &row_scale = {});
 
 // ---- GEMMs
-// scale_y, if given, holds 0 and receives max|y| / 127
-void gemm_nt(const Tensor &y, const Tensor &xq, const Tensor &wq, const Tensor &sx, const Tensor &sw,
-             const Tensor &bias, const Tensor &scale_y);
-Tensor gemm_dx(const Tensor &dyq, const Tensor &wq, const Tensor &sdy, const Tensor &sw, const Tensor &row_scale = {});
+// Y = act(acc * scales * row_scale[r] + bias).  Here and below a `scale_out`, if given, holds 0 and receives max|.| / 127.
+Tensor gemm_nt(const Quantized &x, const Quantized &w, const Tensor &bias, const Tensor &scale_out = {},
+               const Tensor &row_scale = {}, bool relu = false);
+Tensor gemm_dx(const Quantized &dy, const Quantized &w, const Tensor &row_scale = {}, const Tensor &scale_out = {});
 // `scratch`: from dw_scratch, cleared by a launch in front
 Tensor dw_scratch(int64_t m, int64_t n, int64_t k, const Tensor &like);
-Tensor gemm_dw(const Tensor &dyq, const Tensor &xq, const Tensor &sdy, const Tensor &sx, const Tensor &scratch);
+Tensor gemm_dw(const Quantized &dy, const Quantized &x, const Tensor &scratch);
 
 // ---- graph operators
 Tensor spmm_copy_u(const Graph &g, bool reverse, const Tensor &nq, const Tensor &scale, const Tensor &row_scale = {},
-                   const Tensor &bias = {}, bool relu = false);
+                   const Tensor &bias = {}, bool relu = false, const Tensor &scale_out = {});
 Tensor spmm_u_mul_e(const Graph &g, bool reverse, const Tensor &nq, const Tensor &eq, const Tensor &scale);
 Tensor incidence_sum(const Graph &g, bool reverse, const Tensor &zq, const Tensor &scale);
 // op: "dot", "add", "sub", "mul", "div"; U and V 2-D or 3-D; `scale` (optional, holding 0) receives max|out| / 127

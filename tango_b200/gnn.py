@@ -41,15 +41,17 @@ def _cached_norm(graph, which: str) -> torch.Tensor:
 
 
 def _gcn_conv_fused(graph, X, W, b, out_norm, in_norm, relu):
-    """One "multiply first" graph convolution (in_feats > out_feats, norm='both') as a single autograd node:
+    """One graph convolution (norm='both') as a single autograd node, the linear layer first where it shrinks the features,
+    else the aggregation:
 
-        out = act( (A . Q(Q(X * d_out^-1/2) W^T)) * d_in^-1/2 + b )
+        out = act( (A . Q(Q(X * d_out^-1/2) W^T)) * d_in^-1/2 + b )     or     act( (Q(A . Q(X * d_out^-1/2)) W^T) * ... )
 
     Same arithmetic, operation for operation, as the unfused composition in QGraphConv.forward (bit-identical
     results), but the element-wise passes of the reference's layer (evaluation/test_gcn.py:86-94,123-137) are folded
     into the kernels next to them: the left norm into the absmax/quantize of X, the right norm + bias + ReLU into the
-    aggregation's epilogue, and the right norm of the backward pass into the quantizer of the incoming gradient."""
-    return _native.ops.gcn_conv(_native.graph(graph), X, W, b, out_norm, in_norm, relu)
+    epilogue of the aggregation or of the GEMM, and the right norm of the backward pass into the quantizer of the
+    incoming gradient."""
+    return _native.ops.gcn_conv(_native.graph(graph), X, W, b, out_norm, in_norm, relu, W.size(1) > W.size(0))
 
 
 class QGraphConv(nn.Module):
@@ -79,8 +81,7 @@ class QGraphConv(nn.Module):
     def forward(self, graph, feat):
         if not self._allow_zero_in_degree and _has_zero_in_degree(graph):
             raise RuntimeError("There are 0-in-degree nodes in the graph; add self loops first")
-        if (self._fused and self._norm == "both" and self.weight is not None and self._in_feats > self._out_feats
-                and feat.dim() == 2):
+        if self._fused and self._norm == "both" and self.weight is not None and feat.dim() == 2:
             relu = self._activation in (F.relu, torch.relu)
             rst = _gcn_conv_fused(graph, feat, self.weight, self.bias, _cached_norm(graph, "out"),
                                   _cached_norm(graph, "in"), relu)
