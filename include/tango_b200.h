@@ -252,6 +252,15 @@ typedef struct tango_spmm_plan {
     int8_t *dense_b;             /* scratch [dense_n_cols, round_up(f, 16)] int8: the region's feature rows, packed */
     int *dense_status;           /* optional device word that receives TANGO_ETIMEOUT if a bounded wait of the GEMM expires */
     int64_t n_skip_rows;         /* leading entries of row_order owned by units + finalize (0 without a dense region) */
+    /* Optional, with one segment per row and no dense region: arrival counters [n_heavy], one per heavy row.  ws and the
+     * counters must then hold ZEROS on entry (a quantizer launch in front can clear them, tango_quant_job.clear), and the
+     * call is a single launch: the warp that adds the last unit of a row finishes it. */
+    int32_t *arrivals;
+    int64_t unit_slots;          /* slots per unit: every heavy row is cut into ceil(length / unit_slots) units */
+    const int32_t *row_info;     /* optional [n_rows, 4], 16-byte aligned, in row_order's order: (row, first slot, end slot, 0);
+                                    row_order must then be sorted by decreasing length behind its first n_skip_rows entries, */
+    int64_t n_over_few;          /* and these two hold how many of its leading rows (skipped ones included) are longer than */
+    int64_t n_over_one;          /* 4 and than 1 slots; both at least n_long_rows */
 } tango_spmm_plan;
 
 /* out[v,:] = sum_k scales[k] * float(sum_{j in segment k of row v} Nq[indices[j], :]) for v < n_rows.

@@ -40,6 +40,11 @@ class SpmmPlan(Structure):
         ("dense_b", c_void_p),
         ("dense_status", c_void_p),
         ("n_skip_rows", c_int64),
+        ("arrivals", c_void_p),
+        ("unit_slots", c_int64),
+        ("row_info", c_void_p),
+        ("n_over_few", c_int64),
+        ("n_over_one", c_int64),
     ]
 
 

@@ -39,6 +39,14 @@ __device__ __forceinline__ void atomic_max_nonneg(float *addr, float v) {
     atomicMax(reinterpret_cast<int *>(addr), __float_as_int(v));
 }
 
+// 256-bit store (p 32-byte aligned): a whole sector per lane.  Two 128-bit stores of the same bytes reach L2 as two partial
+// sector writes.
+__device__ __forceinline__ void store_v8(float *p, const uint32_t *r) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+
 // Block-wide max of a non-negative value, then one atomic per block of (max / 127).
 __device__ __forceinline__ void block_absmax_to_scale(float thread_max, float *scale_out) {
     __shared__ float s_warp[32];

@@ -165,12 +165,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-__device__ __forceinline__ void store_v8(float *p, const uint32_t *r) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]),
-                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
-
 // ---- one 32 x 32 chunk of an accumulator: lane = row, register = column, `width` columns exist
 // 16-byte piece j of row `lane` goes to piece j ^ (lane & 7) of the staging tile: conflict-free both ways.
 __device__ __forceinline__ void stage_chunk(uint32_t *tile, const uint32_t (&r)[32]) {

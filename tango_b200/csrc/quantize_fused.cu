@@ -262,6 +262,7 @@ __device__ __forceinline__ uint32_t pack4(const float4 &v4, float inv, uint32_t 
 // Quantises units [beg, end) of a job, from the end to the beginning.  FLAT: x and q are packed alike (one row).
 template <int MODE, int VEC, bool WHOLE, bool FLAT, bool GATE>
 __device__ __forceinline__ void quantize_units(const Job &j, uint32_t beg, uint32_t end, float inv, uint64_t call) {
+    constexpr int S = MODE == TANGO_ROUND_STOCHASTIC ? 2 : kSteps;     // (bound by the random numbers, and by registers)
     const float *x = j.x, *gate = j.gate, *row_scale = j.row_scale;
     const Philox ph{(uint32_t)j.seed, (uint32_t)(j.seed >> 32)};
     const auto block_of = [&](uint64_t flat) {
@@ -269,14 +270,14 @@ __device__ __forceinline__ void quantize_units(const Job &j, uint32_t beg, uint3
         return ph((uint32_t)blk, (uint32_t)(blk >> 32), (uint32_t)call, (uint32_t)(call >> 32));
     };
     constexpr bool kOwnBlock = WHOLE || FLAT;      // units are aligned to the Philox blocks
-    const uint32_t trips = end > beg ? (end - beg + kSteps * kThreads - 1) / (kSteps * kThreads) : 0;
+    const uint32_t trips = end > beg ? (end - beg + S * kThreads - 1) / (S * kThreads) : 0;
     for (uint32_t t = trips; t-- > 0;) {
-        const uint32_t u0 = beg + t * (kSteps * kThreads) + threadIdx.x;
-        float4 v[kSteps];
-        float s[kSteps];
-        uint32_t row[kSteps], col[kSteps];
+        const uint32_t u0 = beg + t * (S * kThreads) + threadIdx.x;
+        float4 v[S];
+        float s[S];
+        uint32_t row[S], col[S];
 #pragma unroll
-        for (int k = 0; k < kSteps; ++k) {
+        for (int k = 0; k < S; ++k) {
             const uint32_t u = u0 + k * kThreads;
             v[k] = make_float4(0.f, 0.f, 0.f, 0.f); s[k] = 1.f;
             row[k] = FLAT ? 0 : j.by_upr.div(u);
@@ -292,13 +293,13 @@ __device__ __forceinline__ void quantize_units(const Job &j, uint32_t beg, uint3
         uint4 edge = make_uint4(0, 0, 0, 0);
         if (MODE == TANGO_ROUND_STOCHASTIC && !kOwnBlock) {
             // a unit that is not aligned to the Philox blocks needs the block of the unit after it, which the next lane
-            // computes for itself; for lane 31 the first kSteps lanes compute it, one step each
-            const uint32_t un = u0 - (threadIdx.x & 31) + 32 + (threadIdx.x & 31) % kSteps * kThreads;
+            // computes for itself; for lane 31 the first S lanes compute it, one step each
+            const uint32_t un = u0 - (threadIdx.x & 31) + 32 + (threadIdx.x & 31) % S * kThreads;
             const uint32_t rn = j.by_upr.div(un);
             edge = block_of((uint64_t)rn * j.cols + ((un - rn * j.upr) << 2));
         }
 #pragma unroll
-        for (int k = 0; k < kSteps; ++k) {
+        for (int k = 0; k < S; ++k) {
             const bool in = u0 + k * kThreads < end;
             const uint64_t flat = (uint64_t)row[k] * j.cols + col[k];
             uint4 r0 = make_uint4(0, 0, 0, 0), r1 = r0;
@@ -337,7 +338,7 @@ __device__ __forceinline__ void quantize_band(const Job &j, uint32_t beg, uint32
 
 // EXT: jobs with a gate or column sums take part; STATS: false when every scale is given (no barrier, ordinary launch).
 template <bool STATS, int MODE, bool EXT>
-__global__ void __launch_bounds__(kThreads, MODE == TANGO_ROUND_STOCHASTIC ? (EXT ? 2 : 3) : EXT ? 4 : 5) quantize_fused_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(kThreads, MODE == TANGO_ROUND_STOCHASTIC && EXT ? 3 : MODE == TANGO_ROUND_STOCHASTIC || EXT ? 4 : 5) quantize_fused_kernel(const __grid_constant__ Params p) {
     __shared__ float s_part[EXT && STATS ? kThreads * 4 : 1];
     __shared__ float s_warp[kThreads / 32];
     int ji = 0;

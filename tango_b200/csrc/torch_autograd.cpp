@@ -53,6 +53,11 @@ static std::shared_ptr<N> make_node(const T &...inputs) {
     return node;
 }
 
+static int64_t row_width(const Tensor &t) { return t.dim() > 1 && t.size(0) ? t.numel() / t.size(0) : t.numel(); }
+// the scratch of an aggregation of t's rows
+static Tensor aggregation_scratch(const Graph &g, bool reverse, const Tensor &t) {
+    return spmm_scratch(g, reverse, row_width(t), t);
+}
 static Tensor zeros1(const Tensor &like) { return at::zeros({1}, like.options().dtype(at::kFloat)); }
 static uint64_t call_if(int mode) { return mode == TANGO_ROUND_STOCHASTIC ? next_call() : 0; }
 
@@ -135,8 +140,9 @@ struct SpmmCopyUBackward : OnceNode {
     GraphPtr g;
     variable_list backward(const variable_list &grads) override {
         if (!grads[0].defined() || !needs(0)) return variable_list(1);
-        const Quantized q = quantize(grads[0]);
-        return {spmm_copy_u(*g, true, q.q, q.scale)};
+        QuantJob job = quant_job(grads[0]);
+        job.clear = aggregation_scratch(*g, true, grads[0]);
+        return {spmm_copy_u(*g, true, quantize(job), job.clear)};
     }
 };
 
@@ -146,8 +152,8 @@ Tensor spmm_copy_u_fn(const GraphPtr &g, const Tensor &n, const Tensor &scale) {
         const Raw raw;
         QuantJob job = quant_job(n);
         job.scale = scale;
-        const Quantized q = quantize(job);
-        out = spmm_copy_u(*g, false, q.q, q.scale);
+        job.clear = aggregation_scratch(*g, false, n);
+        out = spmm_copy_u(*g, false, quantize(job), job.clear);
     }
     if (auto node = make_node<SpmmCopyUBackward>(n)) {
         node->g = g;
@@ -175,9 +181,10 @@ struct SpmmUMulEBackward : OnceNode {
         if (!grads[0].defined()) return variable_list(2);
         QuantJob job = quant_job(grads[0]);
         if (!compat) job.times[0] = se;
+        if (needs(0)) job.clear = aggregation_scratch(*g, true, grads[0]);
         const Quantized z = quantize(job);
         Tensor dn, de;
-        if (needs(0)) dn = spmm_u_mul_e(*g, true, z.q, eq, compat ? scale : z.product[0]);
+        if (needs(0)) dn = spmm_u_mul_e(*g, true, z.q, eq, compat ? scale : z.product[0], job.clear);
         if (needs(1)) de = sddmm(*g, reduce_last ? "dot" : "mul", nq, z.q, sn, z.scale, {}, false).reshape(e_shape);
         return {dn, de};
     }
@@ -192,10 +199,11 @@ Tensor spmm_u_mul_e_fn(const GraphPtr &g, const Tensor &n, const Tensor &e, cons
         je.scale = scale_e;                                        // the producer may already know max|E| / 127
         QuantJob jn = quant_job(n);
         jn.times_job = 0;
+        jn.clear = aggregation_scratch(*g, false, n);
         const auto q = quantize_all({je, jn});
         eq = q[0]; nq = q[1];
         sn = nq.scale; se = eq.scale; scale = nq.product[0];
-        out = spmm_u_mul_e(*g, false, nq.q, eq.q, scale);
+        out = spmm_u_mul_e(*g, false, nq.q, eq.q, scale, jn.clear);
     }
     if (auto node = make_node<SpmmUMulEBackward>(n, e)) {
         node->g = g; node->nq = nq.q; node->sn = sn; node->eq = eq.q; node->se = se; node->scale = scale;
@@ -219,9 +227,12 @@ struct SddmmUAddVBackward : OnceNode {
     GraphPtr g;
     variable_list backward(const variable_list &grads) override {
         if (!grads[0].defined()) return variable_list(2);
-        const Quantized z = quantize(grads[0], row_align(grads[0]));
-        Tensor du = needs(0) ? incidence_sum(*g, true, z.q, z.scale) : Tensor();
-        Tensor dv = needs(1) ? incidence_sum(*g, false, z.q, z.scale) : Tensor();
+        QuantJob job = quant_job(grads[0], row_align(grads[0]));
+        if (needs(0)) job.clear = aggregation_scratch(*g, true, grads[0]);
+        if (needs(1)) job.clear2 = aggregation_scratch(*g, false, grads[0]);
+        const Quantized z = quantize(job);
+        Tensor du = needs(0) ? incidence_sum(*g, true, z, job.clear) : Tensor();
+        Tensor dv = needs(1) ? incidence_sum(*g, false, z, job.clear2) : Tensor();
         return {du, dv};
     }
 };
@@ -257,15 +268,17 @@ struct SddmmUDotVBackward : OnceNode {
         if (!dz.defined()) return variable_list(2);
         QuantJob job = quant_job(dz.reshape({dz.size(0), -1}), 1);
         job.times[0] = sv; job.times[1] = su;
+        if (needs(0)) job.clear = aggregation_scratch(*g, true, vq);
+        if (needs(1)) job.clear2 = aggregation_scratch(*g, false, uq);
         const Quantized z = quantize(job);
         const bool flat = uq.dim() != 3;
-        auto side = [&](bool reverse, const Tensor &xq, const Tensor &scale) {
-            const Tensor d = spmm_u_mul_e(*g, reverse, flat ? xq.unsqueeze(1) : xq, z.q, scale);
+        auto side = [&](bool reverse, const Tensor &xq, const Tensor &scale, const Tensor &scratch) {
+            const Tensor d = spmm_u_mul_e(*g, reverse, flat ? xq.unsqueeze(1) : xq, z.q, scale, scratch);
             return flat ? d.squeeze(1) : d;
         };
         Tensor du, dv;
-        if (needs(0)) du = side(true, vq, z.product[0]);
-        if (needs(1)) dv = side(false, uq, z.product[1]);
+        if (needs(0)) du = side(true, vq, z.product[0], job.clear);
+        if (needs(1)) dv = side(false, uq, z.product[1], job.clear2);
         return {du, dv};
     }
 };
@@ -323,8 +336,9 @@ struct GcnConvBackward : OnceNode {
         Tensor dx, dw;
         if (first == First::linear) {
             job.clear = scale;
+            job.clear2 = aggregation_scratch(*g, true, d);
             const Quantized z = quantize(job);
-            const Tensor dh = spmm_copy_u(*g, true, z.q, z.scale, {}, {}, false, scale);
+            const Tensor dh = spmm_copy_u(*g, true, z, job.clear2, {}, {}, false, scale);
             QuantJob jh = quant_job(dh);
             jh.scale = scale;
             jh.clear = dw_tmp;
@@ -342,8 +356,8 @@ struct GcnConvBackward : OnceNode {
             const Tensor da = gemm_dx(z, w, {}, scale);
             QuantJob ja = quant_job(da);
             ja.scale = scale;
-            const Quantized a = quantize(ja);
-            dx = spmm_copy_u(*g, true, a.q, a.scale, out_norm);
+            ja.clear = aggregation_scratch(*g, true, da);
+            dx = spmm_copy_u(*g, true, quantize(ja), ja.clear, out_norm);
         }
         return {dx, dw, z.colsum};
     }
@@ -369,14 +383,14 @@ Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x_, const Tensor &w, const T
             const Tensor h = gemm_nt(x, wq, {}, scale);
             QuantJob jh = quant_job(h);
             jh.scale = scale;
-            const Quantized hq = quantize(jh);
-            out = spmm_copy_u(*g, false, hq.q, scale, in_norm, b, relu);
+            jh.clear = aggregation_scratch(*g, false, h);
+            out = spmm_copy_u(*g, false, quantize(jh), jh.clear, in_norm, b, relu);
         } else {
             QuantJob jx = quant_job(x_);
             jx.row_scale = out_norm;
             jx.clear = scale;
-            const Quantized xq = quantize(jx);
-            const Tensor a = spmm_copy_u(*g, false, xq.q, xq.scale, {}, {}, false, scale);
+            jx.clear2 = aggregation_scratch(*g, false, x_);
+            const Tensor a = spmm_copy_u(*g, false, quantize(jx), jx.clear2, {}, {}, false, scale);
             const uint64_t call = call_if(mode);
             if (mode == TANGO_ROUND_STOCHASTIC) next_call();
             QuantJob ja{a, mode, seed, call};
@@ -472,9 +486,11 @@ static std::pair<Tensor, Tensor> gat_logit_grads(const GatLogits &a, const Tenso
                                                  bool want_r, at::IntArrayRef shape_l, at::IntArrayRef shape_r) {
     QuantJob job = quant_job(dz, 1);
     job.scale = sdz;
+    if (want_l) job.clear = aggregation_scratch(*a.g, true, dz);
+    if (want_r) job.clear2 = aggregation_scratch(*a.g, false, dz);
     const Quantized q = quantize(job);
-    Tensor dl = want_l ? incidence_sum(*a.g, true, q.q, sdz).view(shape_l) : Tensor();
-    Tensor dr = want_r ? incidence_sum(*a.g, false, q.q, sdz).view(shape_r) : Tensor();
+    Tensor dl = want_l ? incidence_sum(*a.g, true, q, job.clear).view(shape_l) : Tensor();
+    Tensor dr = want_r ? incidence_sum(*a.g, false, q, job.clear2).view(shape_r) : Tensor();
     return {dl, dr};
 }
 
@@ -546,9 +562,10 @@ struct GatAggregateBackward : OnceNode {
         const c10::cuda::CUDAGuard guard(grads[0].device());
         QuantJob job = quant_job(grads[0]);
         job.times[0] = sa;
+        if (needs(0)) job.clear = aggregation_scratch(*l.g, true, grads[0]);
         const Quantized z = quantize(job);
         Tensor d_ft, dl, dr;
-        if (needs(0)) d_ft = spmm_u_mul_e(*l.g, true, z.q, aq, z.product[0]);
+        if (needs(0)) d_ft = spmm_u_mul_e(*l.g, true, z.q, aq, z.product[0], job.clear);
         if (needs(1) || needs(2)) {
             const Tensor da = sddmm(*l.g, "dot", nq, z.q, sn, z.scale, {}, false).reshape({-1, l.h});
             const Tensor dz = at::empty_like(da), sdz = zeros1(da);
@@ -592,8 +609,9 @@ Tensor gat_aggregate_fn(const GraphPtr &g, const Tensor &ft, const Tensor &el, c
         count(2);
         QuantJob jn = quant_job(ft);
         jn.times[0] = sa;
+        jn.clear = aggregation_scratch(*g, false, ft);
         nq = quantize(jn);
-        out = spmm_u_mul_e(*g, false, nq.q, aq, nq.product[0]);
+        out = spmm_u_mul_e(*g, false, nq.q, aq, nq.product[0], jn.clear);
     }
     if (auto node = make_node<GatAggregateBackward>(ft, el, er)) {
         node->l = l; node->m = m; node->inv = inv; node->sa = sa; node->aq = aq; node->nq = nq.q; node->sn = nq.scale;

@@ -16,6 +16,10 @@ static Schedule schedule(const py::object &s, bool with_hub) {
     out.units = tensor_attr(s, "units");
     out.heavy_rows = tensor_attr(s, "heavy_rows");
     out.row_order = tensor_attr(s, "row_order");
+    if (const py::object info = s.attr("row_info"); !info.is_none()) out.row_info = info.cast<Tensor>();
+    out.n_over_few = s.attr("n_over_few").cast<int64_t>();
+    out.n_over_one = s.attr("n_over_one").cast<int64_t>();
+    out.unit = s.attr("unit").cast<int>();
     out.n_units = s.attr("n_units").cast<int64_t>();
     out.n_heavy = s.attr("n_heavy").cast<int64_t>();
     out.n_long = s.attr("n_long").cast<int64_t>();

@@ -210,16 +210,25 @@ struct Plan {
     const tango_spmm_plan *get(const Schedule &s) const { return s.present ? &p : nullptr; }
 };
 
-static Plan make_plan(const Schedule &s, int64_t f, const Tensor &like) {
+static Plan make_plan(const Schedule &s, int64_t f, const Tensor &like, const Tensor &scratch) {
     Plan plan;
     if (!s.present) return plan;
     tango_spmm_plan &p = plan.p;
     p.split_threshold = s.threshold;
     p.row_order = ptr<int32_t>(s.row_order);
     p.n_long_rows = p.row_order ? s.n_long : -1;
+    p.row_info = p.row_order ? ptr<int32_t>(s.row_info) : nullptr;
+    p.n_over_few = s.n_over_few;
+    p.n_over_one = s.n_over_one;
     if (s.n_heavy == 0) return plan;
     const int64_t ld = (f + 15) / 16 * 16;
-    plan.ws = at::empty({s.n_heavy, ld}, like.options().dtype(at::kInt));
+    if (scratch.defined()) {
+        plan.ws = scratch;
+        p.arrivals = ptr<int32_t>(scratch) + s.n_heavy * ld;
+        p.unit_slots = s.unit;
+    } else {
+        plan.ws = at::empty({s.n_heavy, ld}, like.options().dtype(at::kInt));
+    }
     p.units = ptr<int32_t>(s.units);
     p.n_units = s.n_units;
     p.heavy_rows = ptr<int32_t>(s.heavy_rows);
@@ -248,57 +257,65 @@ static const int32_t *index_ptr(const Tensor &t, const Tensor &indptr) {
     return t.numel() > 0 ? ptr<int32_t>(t) : ptr<int32_t>(indptr);
 }
 
-static int64_t short_launch(const Schedule &s) { return s.present && s.n_long < s.row_order.numel(); }
+static const Schedule &schedule_for(const Direction &d, bool hub) { return hub ? d.hub_sched : d.sched; }
+// the dense hub region takes feature rows at exactly their padded width, the layout every quantizer here writes
+static bool takes_hub(const Direction &d, const Tensor &nq, int64_t cols) {
+    return d.has_hub && nq.dim() >= 2 && nq.stride(0) == (cols + 15) / 16 * 16;
+}
 
-Tensor spmm_copy_u(const Graph &g, bool reverse, const Tensor &nq, const Tensor &scale, const Tensor &row_scale,
+Tensor spmm_scratch(const Graph &g, bool reverse, int64_t f, const Tensor &like) {
+    const Schedule &s = g.dir(reverse).sched;
+    if (!s.present || s.n_units == 0) return {};
+    return at::empty({s.n_heavy * ((f + 15) / 16 * 16 + 1)}, like.options().dtype(at::kInt));
+}
+
+Tensor spmm_copy_u(const Graph &g, bool reverse, const Quantized &nq, const Tensor &scratch, const Tensor &row_scale,
                    const Tensor &bias, bool relu, const Tensor &scale_out) {
-    const c10::cuda::CUDAGuard guard(nq.device());
+    const c10::cuda::CUDAGuard guard(nq.q.device());
     const Direction &d = g.dir(reverse);
-    const Matrix n = matrix(nq);
-    // the dense hub region takes feature rows at exactly their padded width, the layout every quantizer here writes
-    const bool hub = d.has_hub && nq.dim() >= 2 && nq.stride(0) == (n.cols + 15) / 16 * 16;
-    const Schedule &s = hub ? d.hub_sched : d.sched;
-    std::vector<int64_t> shape(nq.sizes().begin(), nq.sizes().end());
+    const Matrix n = matrix(nq.q);
+    const bool hub = takes_hub(d, nq.q, n.cols);
+    const Schedule &s = schedule_for(d, hub);
+    std::vector<int64_t> shape(nq.q.sizes().begin(), nq.q.sizes().end());
     shape[0] = g.n_nodes;
-    Tensor out = floats(shape, scale);
-    const Plan plan = make_plan(s, n.cols, nq);
+    Tensor out = floats(shape, nq.scale);
+    const Plan plan = make_plan(s, n.cols, nq.q, hub ? Tensor() : scratch);
     const Tensor &indptr = hub ? d.hub_indptr : d.indptr;
     check(tango_spmm_copy_u(ptr<int32_t>(indptr), index_ptr(hub ? d.hub_indices : d.indices, indptr), g.n_nodes, 1,
-                            ptr<int8_t>(n.t), n.ld, n.cols, ptr<float>(scale), ptr<float>(row_scale), ptr<float>(bias),
+                            ptr<int8_t>(n.t), n.ld, n.cols, ptr<float>(nq.scale), ptr<float>(row_scale), ptr<float>(bias),
                             relu, ptr<float>(out), n.cols, ptr<float>(scale_out), plan.get(s), cuda_stream()), "csr_SPMM");
-    count(1 + (s.n_heavy > 0) + short_launch(s) + (hub ? 2 : 0));
+    count(1 + (s.n_heavy > 0 && !plan.p.arrivals) + (hub ? 2 : 0));
     return out;
 }
 
-Tensor spmm_u_mul_e(const Graph &g, bool reverse, const Tensor &nq, const Tensor &eq, const Tensor &scale) {
+Tensor spmm_u_mul_e(const Graph &g, bool reverse, const Tensor &nq, const Tensor &eq, const Tensor &scale,
+                    const Tensor &scratch) {
     require(nq.dim() == 3, "node features must be [N, H, D]");
     const c10::cuda::CUDAGuard guard(nq.device());
     const Direction &d = g.dir(reverse);
     const Matrix n = matrix(nq);
     const Tensor e = eq.numel() ? eq.contiguous() : at::zeros({1}, nq.options());
     Tensor out = floats({d.n_rows(), nq.size(1), nq.size(2)}, scale);
-    const Plan plan = make_plan(d.sched, n.cols, nq);
+    const Plan plan = make_plan(d.sched, n.cols, nq, scratch);
     check(tango_spmm_u_mul_e(ptr<int32_t>(d.indptr), index_ptr(d.indices, d.indptr), ptr<int32_t>(d.edge_ids), d.n_rows(),
                              ptr<int8_t>(n.t), n.ld, (int)nq.size(1), (int)nq.size(2), ptr<int8_t>(e), ptr<float>(scale),
                              ptr<float>(out), n.cols, plan.get(d.sched), cuda_stream()), "multi_cusparse_SPMM");
-    count(1 + (d.sched.n_units > 0) + short_launch(d.sched));
+    count(1 + (d.sched.n_units > 0 && !plan.p.arrivals));
     return out;
 }
 
-Tensor incidence_sum(const Graph &g, bool reverse, const Tensor &zq, const Tensor &scale) {
-    require(zq.is_cuda() && scale.is_cuda(), "CUDA tensors expected");
-    const c10::cuda::CUDAGuard guard(zq.device());
+Tensor incidence_sum(const Graph &g, bool reverse, const Quantized &zq, const Tensor &scratch) {
+    const c10::cuda::CUDAGuard guard(zq.q.device());
     const Direction &d = g.dir(reverse);
-    const Matrix z = matrix(zq);
-    std::vector<int64_t> shape(zq.sizes().begin(), zq.sizes().end());
+    const Matrix z = matrix(zq.q);
+    std::vector<int64_t> shape(zq.q.sizes().begin(), zq.q.sizes().end());
     shape[0] = g.n_nodes;
-    Tensor out = floats(shape, scale);
+    Tensor out = floats(shape, zq.scale);
     const int64_t f = z.cols;
-    const Plan plan = make_plan(d.sched, f, zq);
+    const Plan plan = make_plan(d.sched, f, zq.q, scratch);
     check(tango_spmm_incidence(ptr<int32_t>(d.indptr), ptr<int32_t>(d.edge_ids), d.n_rows(), ptr<int8_t>(z.t), z.ld, f,
-                               ptr<float>(scale), ptr<float>(out), f, plan.get(d.sched), cuda_stream()), "incidence_SPMM");
-    const bool contiguous = !d.edge_ids.defined() && z.ld == f && (f == 1 || f == 2 || f == 4 || f == 8 || f == 16);
-    count(1 + (d.sched.n_units > 0) + (short_launch(d.sched) && (!contiguous || f == 4 || f == 8 || f == 16)));
+                               ptr<float>(zq.scale), ptr<float>(out), f, plan.get(d.sched), cuda_stream()), "incidence_SPMM");
+    count(1 + (d.sched.n_units > 0 && !plan.p.arrivals));
     return out;
 }
 
@@ -320,7 +337,7 @@ static bool sddmm_dot_rows(const Graph &g, bool reverse, const Matrix &u, const 
                                         cuda_stream());
     if (rc == TANGO_EALIGN) return false;      // an operand layout that only the endpoint-list kernel takes
     check(rc, "mySDDMM_int8(dot, rows)");
-    count(1 + short_launch(s));
+    count(1 + (s.present && s.n_long < s.row_order.numel()));
     return true;
 }
 

@@ -46,9 +46,9 @@ inline void count(int64_t n) { settings().launches.fetch_add(n, std::memory_orde
 
 // The row schedule of one index bundle (tango_b200.graph.SpmmSchedule) and its dense hub region, if any.
 struct Schedule {
-    Tensor units, heavy_rows, row_order;
-    int64_t n_units = 0, n_heavy = 0, n_long = 0, n_block_rows = 0, n_skip = 0;
-    int threshold = 0;
+    Tensor units, heavy_rows, row_order, row_info;
+    int64_t n_units = 0, n_heavy = 0, n_long = 0, n_block_rows = 0, n_skip = 0, n_over_few = 0, n_over_one = 0;
+    int threshold = 0, unit = 0;
     bool present = false;
     // hub region (tango_b200.graph.HubBlock)
     Tensor dense, dense_units, dense_cols;
@@ -130,10 +130,14 @@ Tensor dw_scratch(int64_t m, int64_t n, int64_t k, const Tensor &like);
 Tensor gemm_dw(const Quantized &dy, const Quantized &x, const Tensor &scratch);
 
 // ---- graph operators
-Tensor spmm_copy_u(const Graph &g, bool reverse, const Tensor &nq, const Tensor &scale, const Tensor &row_scale = {},
+// Scratch of an aggregation of `f` features (undefined if it needs none): cleared by a launch in front (QuantJob.clear), the
+// aggregation is then a single launch; without it, it clears and finishes its own.
+Tensor spmm_scratch(const Graph &g, bool reverse, int64_t f, const Tensor &like);
+Tensor spmm_copy_u(const Graph &g, bool reverse, const Quantized &n, const Tensor &scratch, const Tensor &row_scale = {},
                    const Tensor &bias = {}, bool relu = false, const Tensor &scale_out = {});
-Tensor spmm_u_mul_e(const Graph &g, bool reverse, const Tensor &nq, const Tensor &eq, const Tensor &scale);
-Tensor incidence_sum(const Graph &g, bool reverse, const Tensor &zq, const Tensor &scale);
+// `n` int8 [N, H, D], `e` int8 [E, H]; `scale` multiplies the integer sums
+Tensor spmm_u_mul_e(const Graph &g, bool reverse, const Tensor &n, const Tensor &e, const Tensor &scale, const Tensor &scratch);
+Tensor incidence_sum(const Graph &g, bool reverse, const Quantized &z, const Tensor &scratch);
 // op: "dot", "add", "sub", "mul", "div"; U and V 2-D or 3-D; `scale` (optional, holding 0) receives max|out| / 127
 Tensor sddmm(const Graph &g, const std::string &op, const Tensor &u, const Tensor &v, const Tensor &su,
              const Tensor &sv, const Tensor &scale, bool reverse);

@@ -254,15 +254,17 @@ class SpmmSchedule:
         if threshold is None:
             # A row is worked on by one warp, neighbour batch after neighbour batch, so the longest unsplit row sets
             # the critical path of the kernel.  Keep it short relative to the total work: about nnz / 16384 (one
-            # batch-chain per resident warp slot), between 256 and SPLIT_THRESHOLD.
+            # batch-chain per resident warp slot), between 512 and SPLIT_THRESHOLD (below that the atomics of the slices
+            # cost more than the shorter chain gains: 1.3 M edges, F = 128 / 40: 86 / 45 us at 256, 83 / 41 us at 512).
             nnz = int(indptr[-1]) if indptr.numel() else 0
-            threshold = 256
+            threshold = 512
             while threshold < SPLIT_THRESHOLD and threshold * 16384 < nnz:
                 threshold *= 2
         if unit is None:
             unit = max(128, threshold // 2)
         self.nseg = nseg
         self.threshold = threshold
+        self.unit = unit
         n_rows = (indptr.numel() - 1) // nseg
         ip = indptr.long()
         row_deg = ip[nseg::nseg] - ip[:-1:nseg][:n_rows] if nseg > 1 else ip[1:] - ip[:-1]
@@ -289,6 +291,14 @@ class SpmmSchedule:
             self.row_order = torch.cat([heavy, rest]).to(torch.int32)
             self.n_skip = int(heavy.numel())
             self.n_long = self.n_skip + n_rest_long
+        # row, first and end slot of every row in row_order's order: one 16-byte load for a short row instead of two trips
+        order = self.row_order.long()
+        self.row_info = None if nseg > 1 else torch.stack(
+            [self.row_order, indptr[order], indptr[order + 1], torch.zeros_like(self.row_order)], dim=1).to(torch.int32).contiguous()
+        # how many rows of that order have more than 4 and more than one slot
+        ranked = row_deg[order[self.n_skip:]]
+        self.n_over_few, self.n_over_one = [self.n_skip + c for c in
+                                            torch.stack([(ranked > 4).sum(), (ranked > 1).sum()]).tolist()]
         self.n_block_rows = int((row_deg > BLOCK_ROW_NNZ).sum())   # rows that deserve a whole CTA in row-team kernels
         self.n_heavy = int(heavy.numel())
         self.heavy_rows = heavy.to(torch.int32)

@@ -222,6 +222,11 @@ def _qgemm_gradW(dW, dY_q, X_q, scaledY, scaleX):
     launch_counter[0] += 2
 
 
+def _add_row_info(plan: SpmmPlan, sched: SpmmSchedule) -> None:
+    if plan.row_order and getattr(sched, "row_info", None) is not None:
+        plan.row_info, plan.n_over_few, plan.n_over_one = sched.row_info.data_ptr(), sched.n_over_few, sched.n_over_one
+
+
 def _make_plan(sched: Optional[SpmmSchedule], f: int, device):
     """ctypes plan + the tensors that must stay alive for the call."""
     if sched is None:
@@ -232,11 +237,13 @@ def _make_plan(sched: Optional[SpmmSchedule], f: int, device):
     hub = getattr(sched, "hub", None)
     if sched.n_heavy == 0:
         plan = SpmmPlan(None, 0, None, 0, None, 0, sched.threshold, order_ptr, n_long)
+        _add_row_info(plan, sched)
         return ctypes.byref(plan), (plan,)
     ws_ld = _round_up(f, 16)
     ws = torch.empty((sched.n_heavy * sched.nseg, ws_ld), dtype=torch.int32, device=device)
     plan = SpmmPlan(sched.units.data_ptr() if sched.n_units else None, sched.n_units, sched.heavy_rows.data_ptr(),
                     sched.n_heavy, ws.data_ptr(), ws_ld, sched.threshold, order_ptr, n_long)
+    _add_row_info(plan, sched)
     keep = [plan, ws]
     if hub is not None:
         packed = torch.empty((hub.cols.numel(), ws_ld), dtype=torch.int8, device=device)
@@ -259,7 +266,6 @@ def _csr_spmm(out, indptr, indices, U, scaleU, sched=None, nseg=1, row_scale=Non
         check(lib.tango_spmm_copy_u(_p(indptr), _pi(indices), n_rows, nseg, _p(U), ldn, f, _p(scaleU), _p(row_scale),
                                     _p(bias), int(relu), _p(out), ldo, _p(out_absmax), plan, _stream()), "csr_SPMM")
     launch_counter[0] += (1 + (sched is not None and sched.n_heavy > 0)
-                          + (sched is not None and sched.n_long < sched.row_order.numel())
                           + (2 if getattr(sched, "hub", None) is not None else 0))
     del keep
 
@@ -299,7 +305,7 @@ def _u_mul_e_spmm(indptr, indices, edge_ids, N, E, scale, sched=None):
     with torch.cuda.device(N.device):
         check(lib.tango_spmm_u_mul_e(_p(indptr), _pi(indices), _p(edge_ids), n_rows, _p(N), ldn, h, d, _p(E), _p(scale),
                                      _p(out), f, plan, _stream()), "multi_cusparse_SPMM")
-    launch_counter[0] += 1 + (sched is not None and sched.n_units > 0) + (sched is not None and sched.n_long < sched.row_order.numel())
+    launch_counter[0] += 1 + (sched is not None and sched.n_units > 0)
     del keep
     return out
 
@@ -312,9 +318,7 @@ def _incidence_spmm(out, indptr, edge_ids, E, scale, sched=None):
     with torch.cuda.device(E.device):
         check(lib.tango_spmm_incidence(_p(indptr), _p(edge_ids), n_rows, _p(E), ldz, f, _p(scale), _p(out), ldo, plan,
                                        _stream()), "incidence_SPMM")
-    contiguous = edge_ids is None and ldz == f and f in (1, 2, 4, 8, 16)    # streamed by the contiguous-row kernel
-    has_short = sched is not None and sched.n_long < sched.row_order.numel() and (not contiguous or f in (4, 8, 16))
-    launch_counter[0] += 1 + (sched is not None and sched.n_units > 0) + has_short
+    launch_counter[0] += 1 + (sched is not None and sched.n_units > 0)
     del keep
 
 
