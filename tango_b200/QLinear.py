@@ -27,10 +27,12 @@ def _linear(X, W, b, want_scale, copies=None):
     """Forward of cuda/QLinear.py:28-35,52-60 (absmax scales of X and W, quantize, GEMM, optional output scale) with its
     native autograd node, which keeps the quantized operands for the backward pass (cuda/QLinear.py:37-47,62-72: dY
     quantized to nearest, dX and dW by int8 GEMMs, bias gradient in fp32).  With config.share_quantized_inputs() a layer
-    whose input is the tensor a previous layer just quantized (same memory, same version) re-uses that int8 copy.  `copies` (a dict that the layers of
-    one forward pass hand to each other) does the same for layers that are known to read the same X."""
+    whose input is the tensor a previous layer just quantized (same memory, same version) re-uses that int8 copy.
+    `copies` (a dict that the layers of one forward pass hand to each other) does the same for layers that are known to
+    read the same X."""
     if copies is not None:
-        Y, sY, copies["Xq"], copies["sX"] = _native.ops.qlinear(X, W, b, want_scale, copies.get("Xq"), copies.get("sX"))
+        Y, sY, copies["Xq"], copies["sX"] = _native.call(_native.ops.qlinear, X, W, b, want_scale, copies.get("Xq"),
+                                                         copies.get("sX"))
         return (Y, sY) if want_scale else Y
     share = config.sharing_quantized_inputs() and config.mode_for("gemm_fwd") != kernels.ROUND_STOCHASTIC
     Xq = sX = None
@@ -39,7 +41,7 @@ def _linear(X, W, b, want_scale, copies=None):
         for ent in _shared_input:
             if ent[1] == X._version and ent[2] == key:
                 Xq, sX = ent[3], ent[4]
-    Y, sY, Xq_used, sX_used = _native.ops.qlinear(X, W, b, want_scale, Xq, sX)
+    Y, sY, Xq_used, sX_used = _native.call(_native.ops.qlinear, X, W, b, want_scale, Xq, sX)
     if share and Xq is None:
         _shared_input.append((X, X._version, key, Xq_used, sX_used))
         del _shared_input[:-_SHARED_SLOTS]
@@ -96,12 +98,18 @@ class QLinear(nn.Linear):
         return out.reshape(out_shape)
 
 
+def _hooked(m) -> bool:
+    """True when calling the module does more than its forward: hooks that want to see its input and output."""
+    own = (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks, m._backward_pre_hooks)
+    return any(own) or torch.nn.modules.module._has_any_global_hook() or "forward" in m.__dict__
+
+
 def linear_group(layers, input):
     """Yields the outputs of up to three QLinear layers that read the same input, whose absmax pass and int8 copy they
     share; with config.share_quantized_inputs() the weights are quantized in the same launch as well.  Bit-identical to
     calling the layers one by one, which is what happens with stochastic rounding (every layer draws its own numbers, in
     the order in which the outputs are asked for)."""
-    plain = all(type(m) is QLinear and not m.isReduce for m in layers)
+    plain = not _native.transformed() and all(type(m) is QLinear and not m.isReduce and not _hooked(m) for m in layers)
     if not plain or config.mode_for("gemm_fwd") == kernels.ROUND_STOCHASTIC:
         yield from (m(input) for m in layers)
     elif config.sharing_quantized_inputs():

@@ -13,7 +13,7 @@ class sddmm_u_add_v:
 
     @staticmethod
     def apply(g, U, V, scaleU_=None, scaleV_=None):
-        return _native.ops.sddmm_u_add_v(_native.graph(g), U, V, scaleU_, scaleV_)
+        return _native.call(_native.ops.sddmm_u_add_v, _native.graph(g), U, V, scaleU_, scaleV_)
 
 
 class sddmm_u_dot_v:
@@ -22,4 +22,4 @@ class sddmm_u_dot_v:
 
     @staticmethod
     def apply(g, U, V):
-        return _native.ops.sddmm_u_dot_v(_native.graph(g), U, V)
+        return _native.call(_native.ops.sddmm_u_dot_v, _native.graph(g), U, V)

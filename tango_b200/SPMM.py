@@ -12,7 +12,7 @@ class spmm_copy_u:
 
     @staticmethod
     def apply(g, N, scaleN=None):
-        return _native.ops.spmm_copy_u(_native.graph(g), N, scaleN)
+        return _native.call(_native.ops.spmm_copy_u, _native.graph(g), N, scaleN)
 
 
 class spmm_u_mul_e:
@@ -25,4 +25,4 @@ class spmm_u_mul_e:
 
     @staticmethod
     def apply(g, N, E, scaleE_=None):
-        return _native.ops.spmm_u_mul_e(_native.graph(g), N, E, scaleE_, spmm_u_mul_e.compat_dn_scale)
+        return _native.call(_native.ops.spmm_u_mul_e, _native.graph(g), N, E, scaleE_, spmm_u_mul_e.compat_dn_scale)

@@ -7,6 +7,9 @@ import importlib.util
 import os
 import sys
 
+import torch
+from torch.autograd.function import Function, once_differentiable
+
 from . import _lib
 
 PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "_torch_ops.so")
@@ -15,7 +18,6 @@ PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "_torch_o
 def _load():
     if not os.path.exists(PATH):
         raise ImportError(f"{PATH} is missing: build it first with `python tango_b200/build.py`")
-    import torch  # noqa: F401  (its libraries have to be loaded before the extension)
     loader = importlib.machinery.ExtensionFileLoader("_torch_ops", PATH)
     module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_torch_ops", PATH, loader=loader))
     # the extension names its exception class by the package it belongs to, under whatever name that was imported
@@ -25,6 +27,45 @@ def _load():
 
 
 ops = _load()
+
+
+def transformed() -> bool:
+    """True under tracing, forward-mode differentiation or a functorch transform."""
+    return (torch._C._get_tracing_state() is not None or torch.autograd.forward_ad._current_level >= 0
+            or torch._C._are_functorch_transforms_active())
+
+
+class _Opaque(Function):
+    """An operator as a Python autograd Function around its native node.  Tracing, forward mode and the functorch
+    transforms know only what passes through the dispatcher or a Function: a call to the extension would leave a constant in
+    the trace and drop a tangent without a word.  Through a Function it is recorded, or refused with an error."""
+
+    @staticmethod
+    def forward(ctx, op, *args):
+        leaf = {id(a): a.detach().requires_grad_(a.requires_grad) for a in args if isinstance(a, torch.Tensor)}
+        ctx.args = [leaf.get(id(a), a) for a in args]      # one tensor given twice stays one
+        with torch.enable_grad():
+            out = op(*ctx.args)
+        single = not isinstance(out, tuple)
+        ctx.outs = (out,) if single else out
+        res = [o.detach() if isinstance(o, torch.Tensor) else o for o in ctx.outs]
+        ctx.mark_non_differentiable(*[r for r, o in zip(res, ctx.outs) if isinstance(o, torch.Tensor) and not o.requires_grad])
+        return res[0] if single else tuple(res)
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, *grads):
+        outs = [(o, g) for o, g in zip(ctx.outs, grads) if isinstance(o, torch.Tensor) and o.requires_grad and g is not None]
+        leaf = {id(a): a for a in ctx.args if isinstance(a, torch.Tensor) and a.requires_grad}
+        found = torch.autograd.grad([o for o, _ in outs], list(leaf.values()), [g for _, g in outs], retain_graph=True,
+                                    allow_unused=True) if outs and leaf else ()
+        grad = dict(zip(leaf, found))
+        return (None, *(grad.pop(id(a), None) for a in ctx.args))      # the first of two places takes the whole gradient
+
+
+def call(op, *args):
+    """op(*args) for an operator of `ops` whose tensors are differentiable."""
+    return _Opaque.apply(op, *args) if transformed() else op(*args)
 
 
 class LaunchCounter:
@@ -52,19 +93,32 @@ def _direction(g, fmt: str, hub):
     return ops.Direction((indptr, indices, edge_ids), sched, hub)
 
 
+class _Kept:
+    """The view of a graph that is kept on the graph object, and the objects it was built from.  A copied or unpickled graph
+    gets an empty one."""
+    __slots__ = ("made_from", "handle")
+
+    def __init__(self, made_from=None, handle=None):
+        self.made_from, self.handle = made_from, handle
+
+    def __reduce__(self):
+        return _Kept, ()
+
+
 def graph(g):
     """The host layer's view of a graph object, built once and kept on it; built anew when the object's index bundles
     or hub regions are other objects than the ones it was built from."""
     csc, csr = g.adj_csc, g.adj_csr
     hubs = getattr(g, "_hubs", None)
     hub_csc, hub_csr = (hubs.get("csc"), hubs.get("csr")) if hubs else (None, None)
+    made_from = (csc, csr, hub_csc, hub_csr)
     kept = getattr(g, "_native", None)
-    if kept is not None and kept[0] is csc and kept[1] is csr and kept[2] is hub_csc and kept[3] is hub_csr:
-        return kept[4]
+    if isinstance(kept, _Kept) and kept.made_from is not None and all(a is b for a, b in zip(kept.made_from, made_from)):
+        return kept.handle
     src, dst = g.coo
     handle = ops.Graph(_direction(g, "csc", hub_csc), _direction(g, "csr", hub_csr), src, dst, g.num_nodes())
     try:
-        g._native = (csc, csr, hub_csc, hub_csr, handle)
+        g._native = _Kept(made_from, handle)
     except AttributeError:       # an object without room for it: rebuilt on every call
         pass
     return handle

@@ -44,6 +44,31 @@ struct OnceNode : Node {
     bool needs(size_t input) const { return task_should_compute_output(input); }
 };
 
+// A node whose operands pass through the saved-tensor hooks and are given back after the backward pass.
+struct SavingNode : OnceNode {
+    std::vector<SavedVariable> saved;
+    bool released = false;
+    // call it after set_history; the first `outputs` of them are outputs of the node
+    void keep(std::initializer_list<Tensor> tensors, size_t outputs = 0) {
+        saved.reserve(tensors.size());
+        for (const Tensor &t : tensors) {
+            saved.emplace_back(t, outputs > 0);
+            if (outputs > 0) --outputs;
+        }
+    }
+    std::vector<Tensor> kept() {
+        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+        std::vector<Tensor> t;
+        t.reserve(saved.size());
+        for (SavedVariable &s : saved) t.push_back(s.unpack(shared_from_this()));
+        return t;
+    }
+    void release_variables() override {
+        for (SavedVariable &s : saved) s.reset_data();
+        released = true;
+    }
+};
+
 // The node of an operation on `inputs`, or null when no gradient is recorded.
 template <class N, class... T>
 static std::shared_ptr<N> make_node(const T &...inputs) {
@@ -308,29 +333,24 @@ Tensor sddmm_u_dot_v_fn(const GraphPtr &g, const Tensor &u, const Tensor &v) {
 // produces for a quantizer brings its scale along (epilogue maximum), so only the inputs of the layer are swept for theirs.
 enum class First { linear, aggregate };
 
-struct GcnConvBackward : OnceNode {
+struct GcnConvBackward : SavingNode {
     std::string name() const override { return "GcnConvBackward"; }
     GraphPtr g;
     First first = First::linear;
-    Quantized x, w;                 // operands of the linear layer
-    Tensor out_norm, in_norm;
-    SavedVariable out;
-    bool relu = false, has_bias = false, released = false;
+    bool relu = false, has_bias = false;
 
-    void release_variables() override {
-        x.q.reset(); w.q.reset();
-        out.reset_data();
-        released = true;
-    }
     variable_list backward(const variable_list &grads) override {
-        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
         const Tensor &d = grads[0];
+        const std::vector<Tensor> k = kept();      // out (undefined without ReLU), the linear layer's operands, the norms
         if (!d.defined()) return variable_list(3);
+        Quantized x, w;
+        x.q = k[1]; x.scale = k[2]; w.q = k[3]; w.scale = k[4];
+        const Tensor &out = k[0], &out_norm = k[5], &in_norm = k[6];
         // ReLU mask, bias gradient, right norm, absmax and quantisation: two sweeps of one launch over (grad, out)
         QuantJob job = quant_job(d);
         job.row_scale = in_norm;
         job.colsum = has_bias && needs(2);
-        if (relu) job.gate = out.unpack(shared_from_this());
+        if (relu) job.gate = out;
         const Tensor dw_tmp = needs(1) ? dw_scratch(d.size(0), w.q.size(0), x.q.size(1), d) : Tensor();
         const Tensor scale = floats({1}, d);
         Tensor dx, dw;
@@ -365,6 +385,7 @@ struct GcnConvBackward : OnceNode {
 
 Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x_, const Tensor &w, const Tensor &b, const Tensor &out_norm,
                    const Tensor &in_norm, bool relu, bool linear_first) {
+    require(x_.size(1) == w.size(1), "features and weight must have the same number of columns");
     Tensor out;
     Quantized x, wq;
     {
@@ -401,10 +422,10 @@ Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x_, const Tensor &w, const T
         }
     }
     if (auto node = make_node<GcnConvBackward>(x_, w, b)) {
-        node->g = g; node->first = linear_first ? First::linear : First::aggregate; node->x = x; node->w = wq;
-        node->out_norm = out_norm; node->in_norm = in_norm; node->relu = relu; node->has_bias = b.defined();
+        node->g = g; node->first = linear_first ? First::linear : First::aggregate;
+        node->relu = relu; node->has_bias = b.defined();
         torch::autograd::set_history(out, node);
-        if (relu) node->out = SavedVariable(out, true);
+        node->keep({relu ? out : Tensor(), x.q, x.scale, wq.q, wq.scale, out_norm, in_norm}, 1);
     }
     return out;
 }
@@ -412,20 +433,14 @@ Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x_, const Tensor &w, const T
 // ------------------------------------------------------------------------------------------------ edge softmax
 static const int32_t *row_order(const Direction &d) { return d.sched.present ? ptr<int32_t>(d.sched.row_order) : nullptr; }
 
-struct EdgeSoftmaxBackward : OnceNode {
+struct EdgeSoftmaxBackward : SavingNode {
     std::string name() const override { return "EdgeSoftmaxBackward"; }
     GraphPtr g;
-    SavedVariable a;
     float factor = 1.f;
-    bool released = false;
-    void release_variables() override {
-        a.reset_data();
-        released = true;
-    }
     variable_list backward(const variable_list &grads) override {
-        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+        const std::vector<Tensor> k = kept();
         if (!grads[0].defined()) return variable_list(1);
-        const Tensor at = a.unpack(shared_from_this()), a2 = at.reshape({at.size(0), -1}).contiguous();
+        const Tensor &at = k[0], a2 = at.reshape({at.size(0), -1}).contiguous();
         const c10::cuda::CUDAGuard guard(a2.device());
         const Tensor da = grads[0].reshape(a2.sizes()).contiguous(), dz = at::empty_like(a2);
         const Direction &d = g->dir(false);
@@ -458,7 +473,7 @@ std::tuple<Tensor, Tensor> edge_softmax_fn(const GraphPtr &g, const Tensor &z, d
     if (auto node = make_node<EdgeSoftmaxBackward>(z)) {
         node->g = g; node->factor = (float)factor;
         torch::autograd::set_history(a, node);
-        node->a = SavedVariable(a, true);
+        node->keep({a}, 1);
     }
     return {a, sa};
 }
@@ -494,20 +509,16 @@ static std::pair<Tensor, Tensor> gat_logit_grads(const GatLogits &a, const Tenso
     return {dl, dr};
 }
 
-struct GatAttentionBackward : OnceNode {
+struct GatAttentionBackward : SavingNode {
     std::string name() const override { return "GatAttentionBackward"; }
-    GatLogits l;
-    SavedVariable a;
+    GatLogits l;                               // without el and er, which are saved
     std::vector<int64_t> shape_l, shape_r;
-    bool released = false;
-    void release_variables() override {
-        a.reset_data();
-        released = true;
-    }
     variable_list backward(const variable_list &grads) override {
-        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+        const std::vector<Tensor> k = kept();
         if (!grads[0].defined()) return variable_list(2);
-        const Tensor at = a.unpack(shared_from_this());
+        const Tensor &at = k[0];
+        GatLogits l = this->l;
+        l.el.q = k[1]; l.el.scale = k[2]; l.er.q = k[3]; l.er.scale = k[4];
         const c10::cuda::CUDAGuard guard(at.device());
         const Tensor a2 = at.reshape({-1, l.h}), da = grads[0].reshape({-1, l.h}).contiguous(), dz = at::empty_like(a2);
         const Tensor sdz = zeros1(a2);
@@ -539,26 +550,24 @@ std::tuple<Tensor, Tensor> gat_attention_fn(const GraphPtr &g, const Tensor &el,
         count(1);
     }
     if (auto node = make_node<GatAttentionBackward>(el, er)) {
-        node->l = l; node->shape_l = el.sizes().vec(); node->shape_r = er.sizes().vec();
+        node->l = l; node->l.el = node->l.er = {};
+        node->shape_l = el.sizes().vec(); node->shape_r = er.sizes().vec();
         torch::autograd::set_history(a, node);
-        node->a = SavedVariable(a, true);
+        node->keep({a, l.el.q, l.el.scale, l.er.q, l.er.scale}, 1);
     }
     return {a, sa};
 }
 
-struct GatAggregateBackward : OnceNode {
+struct GatAggregateBackward : SavingNode {
     std::string name() const override { return "GatAggregateBackward"; }
-    GatLogits l;
-    Tensor m, inv, sa, aq, nq, sn;
+    GatLogits l;                               // without el and er, which are saved
     std::vector<int64_t> shape_l, shape_r;
-    bool released = false;
-    void release_variables() override {
-        for (Tensor *t : {&m, &inv, &aq, &nq}) t->reset();
-        released = true;
-    }
     variable_list backward(const variable_list &grads) override {
-        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+        const std::vector<Tensor> k = kept();
         if (!grads[0].defined()) return variable_list(3);
+        GatLogits l = this->l;
+        l.el.q = k[0]; l.el.scale = k[1]; l.er.q = k[2]; l.er.scale = k[3];
+        const Tensor &m = k[4], &inv = k[5], &sa = k[6], &aq = k[7], &nq = k[8], &sn = k[9];
         const c10::cuda::CUDAGuard guard(grads[0].device());
         QuantJob job = quant_job(grads[0]);
         job.times[0] = sa;
@@ -614,9 +623,10 @@ Tensor gat_aggregate_fn(const GraphPtr &g, const Tensor &ft, const Tensor &el, c
         out = spmm_u_mul_e(*g, false, nq.q, aq, nq.product[0], jn.clear);
     }
     if (auto node = make_node<GatAggregateBackward>(ft, el, er)) {
-        node->l = l; node->m = m; node->inv = inv; node->sa = sa; node->aq = aq; node->nq = nq.q; node->sn = nq.scale;
+        node->l = l; node->l.el = node->l.er = {};
         node->shape_l = el.sizes().vec(); node->shape_r = er.sizes().vec();
         torch::autograd::set_history(out, node);
+        node->keep({l.el.q, l.el.scale, l.er.q, l.er.scale, m, inv, sa, aq, nq.q, nq.scale});
     }
     return out;
 }

@@ -51,7 +51,7 @@ def _gcn_conv_fused(graph, X, W, b, out_norm, in_norm, relu):
     into the kernels next to them: the left norm into the absmax/quantize of X, the right norm + bias + ReLU into the
     epilogue of the aggregation or of the GEMM, and the right norm of the backward pass into the quantizer of the
     incoming gradient."""
-    return _native.ops.gcn_conv(_native.graph(graph), X, W, b, out_norm, in_norm, relu, W.size(1) > W.size(0))
+    return _native.call(_native.ops.gcn_conv, _native.graph(graph), X, W, b, out_norm, in_norm, relu, W.size(1) > W.size(0))
 
 
 class QGraphConv(nn.Module):
@@ -138,7 +138,7 @@ def edge_softmax(g, e, factor: float = 1.0, return_scale: bool = False):
     evaluation/test_gat.py:146, evaluation/test_HGT.py:60); fp32, as in the reference, one team-per-row kernel per
     direction.  With return_scale also max|a|/127, which the kernel produces on the way and the consuming spmm_u_mul_e
     would otherwise recompute."""
-    a, sa = _native.ops.edge_softmax(_native.graph(g), e, factor)
+    a, sa = _native.call(_native.ops.edge_softmax, _native.graph(g), e, factor)
     return (a, sa) if return_scale else a
 
 
@@ -151,7 +151,7 @@ def _gat_attention_fused(g, el, er, slope):
     without materialising the logits: el / er are quantized to int8 exactly as sddmm_u_add_v does, one kernel walks
     every destination's incoming edges (max, sum, normalise), and the backward kernel produces the gradient of the
     logits, which then takes sddmm_u_add_v's backward route (int8 quantisation + incidence sums)."""
-    return _native.ops.gat_attention(_native.graph(g), el, er, slope)
+    return _native.call(_native.ops.gat_attention, _native.graph(g), el, er, slope)
 
 
 def _gat_aggregate_fused(g, ft, el, er, slope):
@@ -164,7 +164,7 @@ def _gat_aggregate_fused(g, ft, el, er, slope):
     cuda/SPMM.py:38-47), but the weights exist only as the int8 tensor the aggregation reads: one pass keeps the
     softmax statistics of every destination (which already fix the int8 scale), a second writes the int8 weights,
     and the backward pass recomputes the weights from the statistics."""
-    return _native.ops.gat_aggregate(_native.graph(g), ft, el, er, slope)
+    return _native.call(_native.ops.gat_aggregate, _native.graph(g), ft, el, er, slope)
 
 
 class QGATConv(nn.Module):

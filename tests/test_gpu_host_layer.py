@@ -1,0 +1,205 @@
+"""The native operators as a user's program meets them: differentiable entry points against the CPU oracle at the sizes where
+the fused quantizer, the GEMMs and the single-launch aggregation can go wrong, and the autograd features around them
+(saved-tensor hooks, tracing, forward mode, functorch, module hooks, copies and files of a model)."""
+import copy
+import io
+
+import numpy as np
+import pytest
+import torch
+import torch.nn.functional as F
+
+from oracle import tango_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _np(t):
+    return t.detach().cpu().numpy()
+
+
+def _graph(n=1500, e=20000, seed=3):
+    import tango_b200 as T
+    from tango_b200.graph import rmat_graph
+    return T.graph_preprocess(rmat_graph(n, e, seed, device="cuda"))
+
+
+def _star(n, hub_edges):
+    """Two rows far above the slicing threshold, rows of 0..70 neighbours, and rows with one."""
+    import tango_b200 as T
+    from tango_b200.graph import Graph
+    rng = np.random.default_rng(5)
+    deg = np.concatenate([[hub_edges, hub_edges // 2], np.arange(71), np.full(n - 73, 1)])
+    dst = np.repeat(np.arange(n), deg)
+    src = rng.integers(0, n, dst.size)
+    order = rng.permutation(dst.size)
+    g = Graph(torch.from_numpy(src[order].astype(np.int32)), torch.from_numpy(dst[order].astype(np.int32)), n).to("cuda")
+    return T.graph_preprocess(g)
+
+
+def _index(g, fmt):
+    return [_np(t).astype(np.int64) for t in (g.adj_csr if fmt == "csr" else g.adj_csc)]
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (3, 5, 2), (127, 16, 33), (129, 130, 41), (1000, 602, 64), (4099, 31, 257)])
+@pytest.mark.parametrize("expanded", [False, True])
+def test_linear_layer_against_oracle(cuda, m, k, n, expanded):
+    """Forward, dX and dW bit for bit; the bias gradient is an fp32 sum, in any order within m * 2^-24 * sum|dY|."""
+    import tango_b200 as T
+    rng = np.random.default_rng(m + k + n)
+    x, dy = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((m, n)).astype(np.float32)
+    if expanded:
+        dy[:] = dy[:1]
+    layer = T.QLinear(k, n).cuda()
+    xt = torch.from_numpy(x).cuda().requires_grad_()
+    y = layer(xt)
+    grad = torch.from_numpy(dy).cuda()
+    y.backward(grad[:1].expand(m, n) if expanded else grad)
+    ry, xq, wq, sx, sw, *_ = O.qgemm_forward(x, _np(layer.weight), _np(layer.bias))
+    sdy = O.absmax_scale(dy)
+    dyq = O.quantize(dy, sdy)
+    np.testing.assert_array_equal(_np(y), ry)
+    np.testing.assert_array_equal(_np(xt.grad), O.qgemm_backward_dx(dyq, wq, sdy, sw))
+    np.testing.assert_array_equal(_np(layer.weight.grad), O.qgemm_backward_dw(dyq, xq, sdy, sx))
+    d64 = dy.astype(np.float64)
+    assert (np.abs(_np(layer.bias.grad) - d64.sum(0)) <= m * 2.0 ** -24 * np.abs(d64).sum(0)).all()
+
+
+@pytest.mark.parametrize("f", [1, 4, 16, 17, 41, 64, 128, 130, 513, 602])
+def test_neighbour_sum_of_all_row_classes(cuda, f):
+    """Sliced, long, short and one-neighbour rows in one launch; twice, as the second finds the first one's scratch."""
+    import tango_b200 as T
+    g = _star(2000, 9000)
+    x = np.random.default_rng(f).standard_normal((2000, f)).astype(np.float32)
+    dz = np.random.default_rng(f + 1).standard_normal((2000, f)).astype(np.float32)
+    csc, csr = _index(g, "csc"), _index(g, "csr")
+    sx, sz = O.absmax_scale(x), O.absmax_scale(dz)
+    for _ in range(2):
+        xt = torch.from_numpy(x).cuda().requires_grad_()
+        out = T.spmm_copy_u.apply(g, xt)
+        out.backward(torch.from_numpy(dz).cuda())
+        np.testing.assert_array_equal(_np(out), O.spmm_copy_u(csc[0], csc[1], O.quantize(x, sx), sx))
+        np.testing.assert_array_equal(_np(xt.grad), O.spmm_copy_u(csr[0], csr[1], O.quantize(dz, sz), sz))
+
+
+@pytest.mark.parametrize("h,d", [(1, 16), (1, 41), (2, 8), (2, 24), (4, 4), (4, 32), (3, 5), (8, 16)])
+def test_weighted_sum_of_all_row_classes(cuda, h, d):
+    """One, two and four heads take their weights as a word, the others byte by byte; edge sums stream contiguous rows."""
+    import tango_b200 as T
+    g = _star(1500, 5000)
+    rng = np.random.default_rng(h * d)
+    x = rng.standard_normal((1500, h, d)).astype(np.float32)
+    e = rng.standard_normal((g.num_edges(), h, 1)).astype(np.float32)
+    out = T.spmm_u_mul_e.apply(g, torch.from_numpy(x).cuda(), torch.from_numpy(e).cuda())
+    csc = _index(g, "csc")
+    sx, se = O.absmax_scale(x), O.absmax_scale(e)
+    ref = O.spmm_u_mul_e(csc[0], csc[1], csc[2], O.quantize(x, sx), O.quantize(e[:, :, 0], se), np.float32(sx * se))
+    np.testing.assert_array_equal(_np(out), ref)
+    v = torch.zeros(1500, h, 1, device="cuda", requires_grad=True)
+    T.sddmm_u_add_v.apply(g, torch.zeros_like(v), v).backward(torch.from_numpy(e).cuda())
+    eq = O.quantize(e.reshape(-1, h), se)
+    np.testing.assert_array_equal(_np(v.grad)[:, :, 0], O.spmm_incidence(csc[0], csc[2], eq, se))
+
+
+def _models(g):
+    from tango_b200.gnn import GAT, GCN, HGT
+    torch.manual_seed(0)
+    yield "gcn", GCN(g, 40, 24, 30, 1).cuda()          # a layer that narrows the features and one that does not
+    yield "gat", GAT(g, 2, 40, 8, 5, [4, 1]).cuda()
+    yield "gat int8", GAT(g, 2, 40, 8, 5, [4, 1], fused="int8").cuda()
+    hgt = HGT(40, 32, 4).cuda()
+    hgt.graph = g
+    yield "hgt", hgt
+
+
+def _forward(m, x):
+    return m(m.graph, x) if type(m).__name__ == "HGT" else m(x)
+
+
+def _step(m, x):
+    m.zero_grad(set_to_none=True)
+    out = _forward(m, x)
+    out.square().sum().backward()
+    return [out.detach()] + [p.grad for p in m.parameters()]
+
+
+def test_saved_tensor_hooks_and_copies_of_models(cuda):
+    g = _graph()
+    x = torch.randn(g.num_nodes(), 40, device="cuda")
+    for name, m in _models(g):
+        want = _step(m, x)
+        seen = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: seen.append(t.dtype) or t.cpu(), lambda t: t.cuda()):
+            got = _step(m, x)
+        assert all(torch.equal(a, b) for a, b in zip(want, got)), name
+        assert name == "hgt" or torch.int8 in seen, name          # the int8 operands are offloaded too
+        for other in (copy.deepcopy(m), torch.load(io.BytesIO(_saved(m)), weights_only=False)):
+            assert all(torch.equal(a, b) for a, b in zip(want, _step(other, x))), name
+        out = _forward(m, x).sum()
+        out.backward(retain_graph=True)
+        out.backward()
+        if name != "hgt":
+            with pytest.raises(RuntimeError, match="backward through the graph a second time"):
+                out.backward()
+
+
+def _saved(m):
+    b = io.BytesIO()
+    torch.save(m, b)
+    return b.getvalue()
+
+
+def test_tracing_and_transforms_see_the_operators(cuda):
+    import tango_b200 as T
+    g = _graph(300, 3000)
+    layer = T.QLinear(40, 8).cuda()
+    a, b = torch.randn(2, 300, 40, device="cuda")
+    ops = {"linear": layer, "spmm": lambda t: T.spmm_copy_u.apply(g, t),
+           "dot": lambda t: T.sddmm_u_dot_v.apply(g, t.view(300, 4, 10), t.view(300, 4, 10))}
+    for name, op in ops.items():
+        with torch.no_grad():
+            traced = torch.jit.trace(op, a, check_trace=False)
+            assert torch.equal(traced(b), op(b)), name
+        with torch.autograd.forward_ad.dual_level(), pytest.raises(RuntimeError):
+            op(torch.autograd.forward_ad.make_dual(a, b))
+        with pytest.raises(RuntimeError):
+            torch.func.grad(lambda t: op(t).sum())(a)
+        with pytest.raises(RuntimeError):
+            torch.vmap(op)(torch.stack([a, b]))
+        with torch.autograd.forward_ad.dual_level():               # no tangent: an ordinary pass
+            x1, x2 = a.clone().requires_grad_(), a.clone().requires_grad_()
+            y1 = op(x1)
+        y2 = op(x2)
+        assert torch.equal(y1, y2)
+        dy = torch.randn_like(y1)
+        y1.backward(dy)
+        y2.backward(dy)
+        assert torch.equal(x1.grad, x2.grad), name
+
+
+@pytest.mark.parametrize("share", [False, True])
+def test_module_hooks_of_projections_that_share_their_input(cuda, share):
+    from tango_b200 import config
+    from tango_b200.gnn import HGT
+    g = _graph(400, 4000)
+    m = HGT(40, 32, 4).cuda()
+    x = torch.randn(400, 40, device="cuda")
+    config.share_quantized_inputs(share)
+    try:
+        plain = m(g, x)
+        seen = []
+        m.k_linear.register_forward_pre_hook(lambda mod, args: seen.append(len(args)))
+        m.q_linear.register_forward_hook(lambda mod, args, out: out * 1.0)
+        assert torch.equal(m(g, x), plain) and seen == [1]
+        m.v_linear.register_forward_pre_hook(lambda mod, args: (args[0] * 2,))
+        assert not torch.equal(m(g, x), plain)
+    finally:
+        config.share_quantized_inputs(False)
+
+
+def test_widths_that_do_not_match_are_refused(cuda):
+    from tango_b200.gnn import QGraphConv
+    g = _graph(300, 3000)
+    for feats, hidden in ((40, 8), (8, 40)):
+        with pytest.raises(AssertionError):
+            QGraphConv(feats, hidden).cuda()(g, torch.randn(300, feats - 1, device="cuda"))
