@@ -1,0 +1,252 @@
+// The attention projections of a GAT layer and their gradients, fp32 throughout:
+//   forward : el[n,h] = <x[n,h,:], al[h,:]>,  er[n,h] = <x[n,h,:], ar[h,:]>
+//   backward: dx[n,h,:] += dl[n,h] * al[h,:] + dr[n,h] * ar[h,:],  dal[h,:] = sum_n dl[n,h] * x[n,h,:],  dar likewise
+//
+// Bound: HBM.  Forward reads x once (both projections take the same registers); backward reads x and dx and writes dx.
+// Operator by operator each projection is a product of the size of x and a reduction over it, and the backward pass four
+// more products, two reductions and two sums: some 24 sweeps instead of four.
+#include "common.cuh"
+
+namespace tango {
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kItems = 4;      // (node, head) pairs in flight per lane group
+constexpr int kRows = 4;       // rows in flight per thread of the backward kernel
+
+struct ProjArgs {
+    const float *x, *al, *ar;
+    int64_t items, rows;
+    int H, D, F;
+    float *el, *er;            // forward
+    const float *dl, *dr;      // backward
+    float *dx;
+    float *part;               // [bands, 2, F]
+    int64_t band;              // rows per CTA
+    int groups_log2;           // forward: log2 of the lanes per item
+};
+
+template <int VEC>
+__device__ __forceinline__ void load(const float *p, float (&v)[VEC]) {
+    if (VEC == 4) {
+        const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
+        v[0] = t.x; v[1 % VEC] = t.y; v[2 % VEC] = t.z; v[3 % VEC] = t.w;
+    } else {
+        v[0] = __ldg(p);
+    }
+}
+
+// 2^groups_log2 lanes share an item and reduce with a fixed butterfly.
+template <int VEC>
+__global__ void __launch_bounds__(kThreads) project_kernel(const ProjArgs a) {
+    const int G = 1 << a.groups_log2, sub = threadIdx.x & (G - 1);
+    const int per_cta = kThreads >> a.groups_log2;
+    const int64_t i0 = (int64_t)blockIdx.x * per_cta * kItems + (threadIdx.x >> a.groups_log2);
+    float l[kItems], r[kItems];
+    int head[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        const int64_t i = i0 + (int64_t)k * per_cta;
+        l[k] = r[k] = 0.f;
+        head[k] = a.items <= 0xffffffffll ? (int)((uint32_t)i % (uint32_t)a.H) : (int)(i % a.H);
+    }
+    for (int c = sub * VEC; c < a.D; c += G * VEC) {
+        float v[kItems][VEC];
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            const int64_t i = i0 + (int64_t)k * per_cta;
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) v[k][e] = 0.f;
+            if (i < a.items) load<VEC>(a.x + i * a.D + c, v[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            float wl[VEC], wr[VEC];
+            load<VEC>(a.al + (int64_t)head[k] * a.D + c, wl);
+            load<VEC>(a.ar + (int64_t)head[k] * a.D + c, wr);
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) {
+                l[k] += v[k][e] * wl[e];
+                r[k] += v[k][e] * wr[e];
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        for (int o = G >> 1; o > 0; o >>= 1) {
+            l[k] += __shfl_xor_sync(0xffffffffu, l[k], o);
+            r[k] += __shfl_xor_sync(0xffffffffu, r[k], o);
+        }
+        const int64_t i = i0 + (int64_t)k * per_cta;
+        if (sub == 0 && i < a.items) { a.el[i] = l[k]; a.er[i] = r[k]; }
+    }
+}
+
+// Thread tx of a CTA owns VEC columns, the rows of the CTA's band are dealt to its thread rows; their sums are added in a
+// fixed order.  blockIdx.y: which kThreads * VEC columns.
+template <int VEC>
+__global__ void __launch_bounds__(kThreads) project_bwd_kernel(const ProjArgs a, int cw) {
+    __shared__ float s_part[2][kThreads * VEC];
+    const int tx = threadIdx.x % cw, ty = threadIdx.x / cw, nty = kThreads / cw;
+    const int c = (blockIdx.y * cw + tx) * VEC;
+    const int64_t r0 = (int64_t)blockIdx.x * a.band, r1 = min(a.rows, r0 + a.band);
+    float sl[VEC], sr[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) sl[e] = sr[e] = 0.f;
+    if (c < a.F) {
+        const int head = c / a.D;
+        float wl[VEC], wr[VEC];
+        load<VEC>(a.al + c, wl);
+        load<VEC>(a.ar + c, wr);
+        for (int64_t r = r0 + ty; r < r1; r += (int64_t)nty * kRows) {
+            float v[kRows][VEC], d[kRows][VEC], gl[kRows], gr[kRows];
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) {
+                const int64_t rr = r + (int64_t)k * nty;
+                gl[k] = gr[k] = 0.f;
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) v[k][e] = d[k][e] = 0.f;
+                if (rr < r1) {
+                    gl[k] = __ldg(a.dl + rr * a.H + head);
+                    gr[k] = __ldg(a.dr + rr * a.H + head);
+                    if (a.part) load<VEC>(a.x + rr * a.F + c, v[k]);
+                    if (a.dx) {
+#pragma unroll
+                        for (int e = 0; e < VEC; ++e)
+                            if (VEC == 1) d[k][e] = a.dx[rr * a.F + c + e];
+                        if (VEC == 4) {
+                            const float4 t = *reinterpret_cast<const float4 *>(a.dx + rr * a.F + c);
+                            d[k][0] = t.x; d[k][1 % VEC] = t.y; d[k][2 % VEC] = t.z; d[k][3 % VEC] = t.w;
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) {
+                const int64_t rr = r + (int64_t)k * nty;
+                if (rr >= r1) break;
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) {
+                    sl[e] += gl[k] * v[k][e];
+                    sr[e] += gr[k] * v[k][e];
+                    d[k][e] += gl[k] * wl[e];
+                    d[k][e] += gr[k] * wr[e];
+                }
+                if (a.dx) {
+                    float *o = a.dx + rr * a.F + c;
+                    if (VEC == 4) *reinterpret_cast<float4 *>(o) = make_float4(d[k][0], d[k][1 % VEC], d[k][2 % VEC], d[k][3 % VEC]);
+                    else o[0] = d[k][0];
+                }
+            }
+        }
+    }
+    if (!a.part) return;
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+        s_part[0][threadIdx.x * VEC + e] = sl[e];
+        s_part[1][threadIdx.x * VEC + e] = sr[e];
+    }
+    __syncthreads();
+    if (ty == 0 && c < a.F) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+            float tl = 0.f, tr = 0.f;
+            for (int y = 0; y < nty; ++y) {
+                tl += s_part[0][(y * cw + tx) * VEC + e];
+                tr += s_part[1][(y * cw + tx) * VEC + e];
+            }
+            float *p = a.part + (int64_t)blockIdx.x * 2 * a.F + c + e;
+            p[0] = tl;
+            p[a.F] = tr;
+        }
+    }
+}
+
+// One warp per column of the [bands, 2, F] partial sums: 32 interleaved chains, then a fixed butterfly.
+__global__ void __launch_bounds__(kThreads) project_sum_kernel(const float *__restrict__ part, int64_t bands, int F,
+                                                               float *__restrict__ dal, float *__restrict__ dar) {
+    const int64_t c = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (c >= 2 * (int64_t)F) return;
+    float t = 0.f;
+    for (int64_t b = lane; b < bands; b += 32) t += __ldg(part + b * 2 * F + c);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) (c < F ? dal : dar)[c < F ? c : c - F] = t;
+}
+
+struct Split {
+    int vec, cw;
+    int64_t band, bands;
+};
+
+Split split(int64_t n, int h, int d, bool wide) {
+    Split s;
+    const int64_t f = (int64_t)h * d;
+    s.vec = wide && d % 4 == 0 ? 4 : 1;
+    s.cw = 1;
+    while (s.cw < (f + s.vec - 1) / s.vec && s.cw < kThreads) s.cw <<= 1;
+    // four CTAs per SM if that leaves a thread a few trips over its rows, fewer where there are not enough rows
+    const int64_t trip = (int64_t)(kThreads / s.cw) * kRows;
+    const int64_t bands = n > 0 ? ceil_div(n, trip) : 0;
+    s.band = ceil_div(n, bands < kNumSMs * 4 ? (bands > 0 ? bands : 1) : kNumSMs * 4);
+    s.bands = s.band > 0 ? ceil_div(n, s.band) : 0;
+    return s;
+}
+
+bool valid(int64_t n, int h, int d) { return n >= 0 && h >= 1 && d >= 1 && (int64_t)h * d <= (1 << 20); }
+
+}  // namespace
+}  // namespace tango
+
+using namespace tango;
+
+extern "C" int tango_gat_project(const float *x, int64_t n, int h, int d, const float *al, const float *ar, float *el,
+                                 float *er, tango_stream_t stream) {
+    if (!valid(n, h, d)) return TANGO_EINVAL;
+    if (n == 0) return TANGO_OK;
+    if (!x || !al || !ar || !el || !er) return TANGO_EINVAL;
+    ProjArgs a{};
+    a.x = x; a.al = al; a.ar = ar; a.items = n * h; a.H = h; a.D = d; a.el = el; a.er = er;
+    const bool wide = d % 4 == 0 && aligned(x, 16) && aligned(al, 16) && aligned(ar, 16);
+    const int pieces = wide ? d / 4 : d;
+    while ((1 << a.groups_log2) < pieces && a.groups_log2 < 5) ++a.groups_log2;
+    const int64_t blocks = ceil_div(a.items, (int64_t)(kThreads >> a.groups_log2) * kItems);
+    if (blocks > 0x7fffffff) return TANGO_ESIZE;
+    if (wide) project_kernel<4><<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
+    else project_kernel<1><<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
+    TANGO_LAUNCH_CHECK();
+    return TANGO_OK;
+}
+
+extern "C" int64_t tango_gat_project_bwd_scratch_bytes(int64_t n, int h, int d) {
+    if (!valid(n, h, d)) return TANGO_EINVAL;
+    const Split wide = split(n, h, d, true), narrow = split(n, h, d, false);
+    return (wide.bands > narrow.bands ? wide.bands : narrow.bands) * 2 * h * d * (int64_t)sizeof(float);
+}
+
+extern "C" int tango_gat_project_bwd(const float *x, int64_t n, int h, int d, const float *al, const float *ar,
+                                     const float *dl, const float *dr, float *dx, float *dal, float *dar, void *scratch,
+                                     int64_t scratch_bytes, tango_stream_t stream) {
+    if (!valid(n, h, d) || (dal == nullptr) != (dar == nullptr)) return TANGO_EINVAL;
+    const int f = h * d;
+    if (n > 0 && (!al || !ar || !dl || !dr || (dal && !x))) return TANGO_EINVAL;
+    if (dal && n > 0 && (!scratch || scratch_bytes < tango_gat_project_bwd_scratch_bytes(n, h, d))) return TANGO_EINVAL;
+    ProjArgs a{};
+    a.x = x; a.al = al; a.ar = ar; a.rows = n; a.H = h; a.D = d; a.F = f; a.dl = dl; a.dr = dr; a.dx = dx;
+    a.part = dal ? static_cast<float *>(scratch) : nullptr;
+    const Split s = split(n, h, d, aligned(x, 16) && aligned(al, 16) && aligned(ar, 16) && aligned(dx, 16));
+    a.band = s.band;
+    if (n > 0 && (dx || dal)) {
+        const dim3 grid((unsigned)s.bands, (unsigned)ceil_div(ceil_div(f, s.vec), s.cw));
+        if (s.vec == 4) project_bwd_kernel<4><<<grid, kThreads, 0, (cudaStream_t)stream>>>(a, s.cw);
+        else project_bwd_kernel<1><<<grid, kThreads, 0, (cudaStream_t)stream>>>(a, s.cw);
+        TANGO_LAUNCH_CHECK();
+    }
+    if (dal) {
+        project_sum_kernel<<<(unsigned)ceil_div(2 * (int64_t)f, kThreads / 32), kThreads, 0, (cudaStream_t)stream>>>(
+            static_cast<const float *>(scratch), s.bands, f, dal, dar);
+        TANGO_LAUNCH_CHECK();
+    }
+    return TANGO_OK;
+}

@@ -69,6 +69,15 @@ struct SavingNode : OnceNode {
     }
 };
 
+// An int8 GEMM operand whose rows are padded to 16 bytes, as alloc_int8 lays it out: a saved-tensor hook may have given it back
+// packed.
+static Tensor padded(const Tensor &t) {
+    if (t.dim() < 2 || t.size(0) == 0 || t.stride(0) % 16 == 0) return t;
+    const Tensor p = alloc_int8(t.sizes(), t.device(), 16);
+    p.as_strided({t.size(0), p.stride(0)}, {p.stride(0), 1}).zero_();
+    return p.copy_(t);
+}
+
 // The node of an operation on `inputs`, or null when no gradient is recorded.
 template <class N, class... T>
 static std::shared_ptr<N> make_node(const T &...inputs) {
@@ -344,7 +353,7 @@ struct GcnConvBackward : SavingNode {
         const std::vector<Tensor> k = kept();      // out (undefined without ReLU), the linear layer's operands, the norms
         if (!d.defined()) return variable_list(3);
         Quantized x, w;
-        x.q = k[1]; x.scale = k[2]; w.q = k[3]; w.scale = k[4];
+        x.q = padded(k[1]); x.scale = k[2]; w.q = padded(k[3]); w.scale = k[4];
         const Tensor &out = k[0], &out_norm = k[5], &in_norm = k[6];
         // ReLU mask, bias gradient, right norm, absmax and quantisation: two sweeps of one launch over (grad, out)
         QuantJob job = quant_job(d);

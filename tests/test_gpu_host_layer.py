@@ -41,7 +41,7 @@ def _index(g, fmt):
     return [_np(t).astype(np.int64) for t in (g.adj_csr if fmt == "csr" else g.adj_csc)]
 
 
-@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (3, 5, 2), (127, 16, 33), (129, 130, 41), (1000, 602, 64), (4099, 31, 257)])
+@pytest.mark.parametrize("m,k,n", [(2, 1, 2), (3, 5, 2), (127, 16, 33), (129, 130, 41), (1000, 602, 64), (4099, 31, 257)])
 @pytest.mark.parametrize("expanded", [False, True])
 def test_linear_layer_against_oracle(cuda, m, k, n, expanded):
     """Forward, dX and dW bit for bit; the bias gradient is an fp32 sum, in any order within m * 2^-24 * sum|dY|."""
