@@ -8,7 +8,7 @@
 // weights (u_mul_e), so every accumulator is an exact int32.  Rows longer than the plan's threshold are cut into
 // units that add into an int32 scratch row with integer atomics (order independent => deterministic), and the last one to
 // arrive finishes the row; rows of at most 48 neighbours are handled by lane groups (short_rows); all three kinds share
-// one launch; in-edge sums over contiguous edge rows have their own streaming kernel (incidence_contig_kernel).
+// one launch; in-edge sums over contiguous edge rows have their own streaming kernel (incidence_kernel).
 #include "common.cuh"
 
 namespace tango {
@@ -724,9 +724,51 @@ __device__ __forceinline__ void contig_segment(int (&acc)[F], int beg, int end, 
         for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
 }
 
-// Units and medium rows as above, short rows (F of 4, 8 or 16) by lane groups in the CTAs behind them.
+// The same when the edge ids are a list: a lane takes a whole record of F bytes, eight (four) of them in flight.
+// Random records out of an array of E * F bytes are bound by L2 sectors in flight, not by bytes.
 template <int F>
-__global__ void __launch_bounds__(kSpmmThreads, 8) incidence_contig_kernel(const SpmmArgs a) {
+__device__ __forceinline__ void listed_segment(int (&acc)[F], int beg, int end, const SpmmArgs &a) {
+    constexpr int U = F <= 4 ? 8 : 4;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int c = 0; c < F; ++c) acc[c] = 0;
+    for (int j0 = beg + lane; j0 < end; j0 += 32 * U) {
+        int id[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) id[u] = j0 + 32 * u < end ? __ldg(a.indices + j0 + 32 * u) : -1;
+        uint4 w[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            w[u] = make_uint4(0, 0, 0, 0);
+            if (id[u] < 0) continue;
+            const int8_t *p = a.feat + (int64_t)id[u] * F;
+            if (F == 16) w[u] = __ldg(reinterpret_cast<const uint4 *>(p));
+            else if (F == 8) { const uint2 t = __ldg(reinterpret_cast<const uint2 *>(p)); w[u].x = t.x; w[u].y = t.y; }
+            else if (F == 4) w[u].x = __ldg(reinterpret_cast<const uint32_t *>(p));
+            else if (F == 2) w[u].x = __ldg(reinterpret_cast<const uint16_t *>(p));
+            else w[u].x = (uint32_t)(uint8_t)__ldg(p);
+        }
+        if (F == 4) {
+#pragma unroll
+            for (int u = 0; u < U; u += 4) add_chunk<F>(acc, make_uint4(w[u].x, w[u + 1].x, w[u + 2].x, w[u + 3].x));
+        } else {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const uint32_t ws[4] = {w[u].x, w[u].y, w[u].z, w[u].w};
+#pragma unroll
+                for (int c = 0; c < F; ++c) acc[c] += (int)(int8_t)(ws[c >> 2] >> (8 * (c & 3)));
+            }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < F; ++c)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+}
+
+// Units and medium rows as above, short rows (F of 4, 8 or 16) by lane groups in the CTAs behind them.
+template <int F, bool LISTED>
+__global__ void __launch_bounds__(kSpmmThreads, LISTED && F <= 4 ? 12 : 8) incidence_kernel(const SpmmArgs a) {
     if ((int64_t)blockIdx.x >= a.long_blocks) {
         float amax = 0.f;
         if (F >= 4) short_rows<F == 16 ? 16 : 4, MODE_COPY, false>(a, (int64_t)blockIdx.x - a.long_blocks, amax);
@@ -737,7 +779,8 @@ __global__ void __launch_bounds__(kSpmmThreads, 8) incidence_contig_kernel(const
     int acc[F];
     if (w < a.n_units) {
         const int4 u = __ldg(reinterpret_cast<const int4 *>(a.units) + w);
-        contig_segment<F>(acc, u.y, u.z, a);
+        if (LISTED) listed_segment<F>(acc, u.y, u.z, a);
+        else contig_segment<F>(acc, u.y, u.z, a);
 #pragma unroll
         for (int c = 0; c < F; ++c)
             if (lane == c && acc[c] != 0) atomicAdd(a.ws + (int64_t)u.w * a.ws_ld + c, acc[c]);
@@ -748,7 +791,8 @@ __global__ void __launch_bounds__(kSpmmThreads, 8) incidence_contig_kernel(const
         if (a.row_order) row = __ldg(a.row_order + row);
         const int beg = __ldg(a.indptr + row), end = __ldg(a.indptr + row + 1);
         if (a.n_heavy > 0 && end - beg > a.split_threshold) return;   // covered by units
-        contig_segment<F>(acc, beg, end, a);
+        if (LISTED) listed_segment<F>(acc, beg, end, a);
+        else contig_segment<F>(acc, beg, end, a);
         const float sc = __ldg(a.scales);
 #pragma unroll
         for (int c = 0; c < F; ++c)
@@ -929,10 +973,22 @@ static int launch_spmm(SpmmArgs &a, const tango_spmm_plan *plan, cudaStream_t st
     return (a.n_units > 0 && !a.arrivals) || dense ? finalize(a, stream) : TANGO_OK;
 }
 
-// Contiguous incidence sums (see incidence_contig_kernel); returns false when the layout does not qualify.
-static bool try_incidence_contig(SpmmArgs &a, const tango_spmm_plan *plan, cudaStream_t stream, int &rc) {
+template <bool LISTED>
+static void launch_incidence(const SpmmArgs &a, unsigned blocks, cudaStream_t stream) {
+    switch (a.f) {
+        case 1: incidence_kernel<1, LISTED><<<blocks, kSpmmThreads, 0, stream>>>(a); break;
+        case 2: incidence_kernel<2, LISTED><<<blocks, kSpmmThreads, 0, stream>>>(a); break;
+        case 4: incidence_kernel<4, LISTED><<<blocks, kSpmmThreads, 0, stream>>>(a); break;
+        case 8: incidence_kernel<8, LISTED><<<blocks, kSpmmThreads, 0, stream>>>(a); break;
+        default: incidence_kernel<16, LISTED><<<blocks, kSpmmThreads, 0, stream>>>(a); break;
+    }
+}
+
+// Incidence sums over packed records (see incidence_kernel); returns false when the layout does not qualify.
+static bool try_incidence(SpmmArgs &a, const tango_spmm_plan *plan, cudaStream_t stream, int &rc) {
     const int f = a.f;
-    if (a.indices || a.ld != f || !(f == 1 || f == 2 || f == 4 || f == 8 || f == 16) || !aligned(a.feat, 16)) return false;
+    if (a.ld != f || !(f == 1 || f == 2 || f == 4 || f == 8 || f == 16) || !aligned(a.feat, a.indices ? f : 16)) return false;
+    if (a.indices && plan && (plan->n_skip_rows > 0 || plan->dense_a)) return false;
     a.n_long = a.n_rows;
     rc = take_units(a, plan, stream);
     if (rc) return true;
@@ -949,13 +1005,8 @@ static bool try_incidence_contig(SpmmArgs &a, const tango_spmm_plan *plan, cudaS
     const int64_t blocks = a.long_blocks + (short_vec ? ceil_div((a.n_rows - a.n_long) * a.G, kSpmmThreads) : 0);
     if (blocks > 0x7fffffff) { rc = TANGO_ESIZE; return true; }
     if (blocks > 0) {
-        switch (f) {
-            case 1: incidence_contig_kernel<1><<<(unsigned)blocks, kSpmmThreads, 0, stream>>>(a); break;
-            case 2: incidence_contig_kernel<2><<<(unsigned)blocks, kSpmmThreads, 0, stream>>>(a); break;
-            case 4: incidence_contig_kernel<4><<<(unsigned)blocks, kSpmmThreads, 0, stream>>>(a); break;
-            case 8: incidence_contig_kernel<8><<<(unsigned)blocks, kSpmmThreads, 0, stream>>>(a); break;
-            default: incidence_contig_kernel<16><<<(unsigned)blocks, kSpmmThreads, 0, stream>>>(a); break;
-        }
+        if (a.indices) launch_incidence<true>(a, (unsigned)blocks, stream);
+        else launch_incidence<false>(a, (unsigned)blocks, stream);
         if (cudaPeekAtLastError() != cudaSuccess) { rc = TANGO_ECUDA; return true; }
     }
     if (a.n_units > 0 && !a.arrivals) rc = finalize(a, stream);
@@ -1008,6 +1059,6 @@ extern "C" int tango_spmm_incidence(const int32_t *indptr, const int32_t *edge_i
     a.feat = zq; a.ld = ldz; a.f = (int)f; a.H = 1; a.D = (int)f;
     a.scales = scale; a.out = out; a.ldo = ldo;
     int rc = TANGO_OK;
-    if (try_incidence_contig(a, plan, (cudaStream_t)stream, rc)) return rc;
+    if (try_incidence(a, plan, (cudaStream_t)stream, rc)) return rc;
     return launch_spmm<MODE_COPY>(a, plan, (cudaStream_t)stream);
 }
