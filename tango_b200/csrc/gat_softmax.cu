@@ -50,44 +50,120 @@ enum { FWD_FLOAT = 0, FWD_STATS = 1, FWD_QUANT = 2 };
 
 __device__ __forceinline__ float leaky(float z, float slope) { return z >= 0.f ? z : __fmul_rn(z, slope); }
 
-// z for all heads of slot j of row `row`
+// Heads handled together (HT = 0: any number up to kMaxHeads, element by element) and edges in flight per thread.
+template <int HT> struct Shape {
+    static constexpr int N = HT ? HT : kMaxHeads;
+    static constexpr int U = HT == 1 ? 8 : HT == 2 || HT == 4 ? 4 : 2;
+    static constexpr int kKept = HT == 8 ? 512 : 1024;      // gathered records a warp keeps between its two sweeps
+};
+template <int HT> struct Record { typedef uint8_t T; };
+template <> struct Record<2> { typedef uint16_t T; };
+template <> struct Record<4> { typedef uint32_t T; };
+template <> struct Record<8> { typedef uint2 T; };
+
+// The H floats of an edge, H <= N; the base of the array is aligned to the access.
 template <int HT>
-__device__ __forceinline__ void edge_logits(const GatArgs &a, int j, const float (&er)[kMaxHeads], float sl,
-                                            float (&z)[kMaxHeads]) {
-    if (a.zin) {
-        const int64_t eid = a.edge_ids ? __ldg(a.edge_ids + j) : j;
-        if (HT == 4) {
-            const float4 v = __ldg(reinterpret_cast<const float4 *>(a.zin + eid * 4));
-            z[0] = __fmul_rn(v.x, a.zmul); z[1] = __fmul_rn(v.y, a.zmul);
-            z[2] = __fmul_rn(v.z, a.zmul); z[3] = __fmul_rn(v.w, a.zmul);
-        } else {
-            const int H = HT ? HT : a.H;
+__device__ __forceinline__ void load_heads(const float *p, int H, float (&v)[Shape<HT>::N]) {
+    constexpr int N = Shape<HT>::N;
+    if (HT == 8 || HT == 4) {
 #pragma unroll
-            for (int h = 0; h < kMaxHeads; ++h)
-                if (h < H) z[h] = __fmul_rn(__ldg(a.zin + eid * H + h), a.zmul);
+        for (int i = 0; i < N / 4; ++i) {
+            const float4 t = __ldg(reinterpret_cast<const float4 *>(p) + i);
+            v[4 * i] = t.x; v[(4 * i + 1) % N] = t.y; v[(4 * i + 2) % N] = t.z; v[(4 * i + 3) % N] = t.w;
         }
-        return;
-    }
-    const int64_t s = __ldg(a.indices + j);
-    if (HT == 4) {
-        const uint32_t w = __ldg(reinterpret_cast<const uint32_t *>(a.elq + s * 4));
-#pragma unroll
-        for (int h = 0; h < 4; ++h)
-            z[h] = leaky(__fadd_rn(__fmul_rn((float)(int8_t)(w >> (8 * h)), sl), er[h]), a.slope);
+    } else if (HT == 2) {
+        const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
+        v[0] = t.x; v[1 % N] = t.y;
     } else {
-        const int H = HT ? HT : a.H;
 #pragma unroll
-        for (int h = 0; h < kMaxHeads; ++h)
-            if (h < H) z[h] = leaky(__fadd_rn(__fmul_rn((float)__ldg(a.elq + s * H + h), sl), er[h]), a.slope);
+        for (int h = 0; h < N; ++h) v[h] = h < H ? __ldg(p + h) : 0.f;
+    }
+}
+template <int HT>
+__device__ __forceinline__ void store_heads(float *p, int H, const float (&v)[Shape<HT>::N]) {
+    constexpr int N = Shape<HT>::N;
+    if (HT == 8 || HT == 4) {
+#pragma unroll
+        for (int i = 0; i < N / 4; ++i)
+            reinterpret_cast<float4 *>(p)[i] = make_float4(v[4 * i], v[(4 * i + 1) % N], v[(4 * i + 2) % N], v[(4 * i + 3) % N]);
+    } else if (HT == 2) {
+        *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1 % N]);
+    } else {
+#pragma unroll
+        for (int h = 0; h < N; ++h)
+            if (h < H) p[h] = v[h];
+    }
+}
+// The int8 features of a node, all heads in one record; HT = 0 head by head.
+template <int HT>
+__device__ __forceinline__ void decode(const typename Record<HT>::T &r, float (&v)[Shape<HT>::N]) {
+    constexpr int N = Shape<HT>::N;
+    uint32_t w[2] = {0, 0};
+    if constexpr (HT == 8) { w[0] = r.x; w[1] = r.y; }
+    else w[0] = r;
+#pragma unroll
+    for (int h = 0; h < N; ++h) v[h] = (float)(int8_t)(w[h >> 2] >> (8 * (h & 3)));
+}
+
+// The edges of one trip of a team over a row: thread `tid` takes slots j0 + u * NT.  Their logits for all heads; slots beyond
+// the row get -infinity, which adds nothing to a softmax.  `kept`: records of the row's first `cap` slots in shared memory,
+// written (SAVE) or read instead of gathered (every thread meets its own slots again).
+enum { GATHER = 0, SAVE = 1, REUSE = 2 };
+template <int NT, int HT, int U, bool PLAIN, int KEEP = GATHER>
+__device__ __forceinline__ void trip_logits(const GatArgs &a, int j0, int beg, int end, const float (&er)[Shape<HT>::N], float sl,
+                                            float (&z)[U][Shape<HT>::N], typename Record<HT>::T *kept = nullptr, int cap = 0) {
+    constexpr int N = Shape<HT>::N;
+    typedef typename Record<HT>::T R;
+    const int H = HT ? HT : a.H;
+    int at[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int j = j0 + u * NT;
+        at[u] = j >= end ? -1
+              : PLAIN ? (a.edge_ids ? __ldg(a.edge_ids + j) : j)
+              : KEEP == REUSE && j - beg < cap ? 0 : __ldg(a.indices + j);
+    }
+    R rec[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int h = 0; h < N; ++h) z[u][h] = -INFINITY;
+        rec[u] = R();
+        if (at[u] < 0) continue;
+        if constexpr (PLAIN) {
+            load_heads<HT>(a.zin + (int64_t)at[u] * H, H, z[u]);
+        } else if constexpr (HT == 0) {
+            for (int h = 0; h < N; ++h) z[u][h] = h < H ? (float)__ldg(a.elq + (int64_t)at[u] * H + h) : 0.f;
+        } else {
+            const int slot = j0 + u * NT - beg;
+            if (KEEP == REUSE && slot < cap) rec[u] = kept[slot];
+            else rec[u] = __ldg(reinterpret_cast<const R *>(a.elq) + at[u]);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        if (at[u] < 0) continue;
+        if constexpr (PLAIN) {
+#pragma unroll
+            for (int h = 0; h < N; ++h) z[u][h] = __fmul_rn(z[u][h], a.zmul);
+        } else {
+            if constexpr (HT != 0) {
+                const int slot = j0 + u * NT - beg;
+                if (KEEP == SAVE && slot < cap) kept[slot] = rec[u];
+                decode<HT>(rec[u], z[u]);
+            }
+#pragma unroll
+            for (int h = 0; h < N; ++h) z[u][h] = leaky(__fadd_rn(__fmul_rn(z[u][h], sl), er[h]), a.slope);
+        }
     }
 }
 
-// Fixed-order reductions over a team of NT threads (NT = 32: one warp; else the whole CTA through shared memory).
+// Fixed-order reductions over a team of NT threads (up to 32: aligned lanes of a warp; else the whole CTA through shared memory).
 template <int NT>
 __device__ __forceinline__ float team_sum(float v, float *smem) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (NT == 32) return v;
+    for (int o = NT < 32 ? NT / 2 : 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (NT <= 32) return v;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __syncthreads();
     if (lane == 0) smem[warp] = v;
@@ -101,13 +177,13 @@ __device__ __forceinline__ float team_sum(float v, float *smem) {
 template <int NT>
 __device__ __forceinline__ void team_softmax_merge(float &m, float &s, float *smem) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = NT < 32 ? NT / 2 : 16; o > 0; o >>= 1) {
         const float m2 = __shfl_xor_sync(0xffffffffu, m, o), s2 = __shfl_xor_sync(0xffffffffu, s, o);
         const float mm = fmaxf(m, m2);
         s = (m == -INFINITY ? 0.f : s * __expf(m - mm)) + (m2 == -INFINITY ? 0.f : s2 * __expf(m2 - mm));
         m = mm;
     }
-    if (NT == 32) return;
+    if (NT <= 32) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __syncthreads();
     if (lane == 0) { smem[warp] = m; smem[32 + warp] = s; }
@@ -122,73 +198,88 @@ __device__ __forceinline__ void team_softmax_merge(float &m, float &s, float *sm
     m = mm; s = ss;
 }
 
-template <int NT, int HT, int STAGE>
-__device__ __forceinline__ void softmax_row(const GatArgs &a, int64_t row, int tid, float *smem, float &amax) {
-    const float sl = a.zin ? 0.f : __ldg(a.sl), sr = a.zin ? 0.f : __ldg(a.sr);
-    const int beg = __ldg(a.indptr + row), end = __ldg(a.indptr + row + 1);
+// Slots [beg, end) of row `row` by a team of NT threads.  `kept`: cap records of shared memory (FWD_FLOAT).
+template <int NT, int HT, int U, bool PLAIN, int STAGE>
+__device__ __forceinline__ void softmax_row(const GatArgs &a, int64_t row, int beg, int end, int tid, float *smem,
+                                            typename Record<HT>::T *kept, int cap, float &amax) {
+    constexpr int N = Shape<HT>::N;
+    constexpr bool kKeep = STAGE == FWD_FLOAT && !PLAIN && HT != 0 && NT >= 32;
+    const float sl = PLAIN ? 0.f : __ldg(a.sl), sr = PLAIN ? 0.f : __ldg(a.sr);
     const int H = HT ? HT : a.H;
-    float er[kMaxHeads], m[kMaxHeads], s[kMaxHeads];
+    const int trips = (end - beg + NT * U - 1) / (NT * U);
+    float er[N], m[N], s[N], inv[N], z[U][N];
 #pragma unroll
-    for (int h = 0; h < kMaxHeads; ++h) {
-        er[h] = (h < H && !a.zin) ? __fmul_rn((float)__ldg(a.erq + row * H + h), sr) : 0.f;
+    for (int h = 0; h < N; ++h) {
+        er[h] = (h < H && !PLAIN) ? __fmul_rn((float)__ldg(a.erq + row * H + h), sr) : 0.f;
         m[h] = -INFINITY; s[h] = 0.f;
     }
     if (STAGE == FWD_QUANT) {
         // second step: statistics from the first step, int8 weights out
-        float inv[kMaxHeads];
 #pragma unroll
-        for (int h = 0; h < kMaxHeads; ++h) {
+        for (int h = 0; h < N; ++h) {
             m[h] = h < H ? __ldg(a.row_m + row * H + h) : 0.f;
             inv[h] = h < H ? __ldg(a.row_inv + row * H + h) : 0.f;
         }
         const float inv_s = inv_scale(__ldg(a.att_scale));
         const uint64_t call = effective_call(a.call, a.step);
         const Philox ph{(uint32_t)a.seed, (uint32_t)(a.seed >> 32)};
-        for (int j = beg + tid; j < end; j += NT) {
-            float z[kMaxHeads];
-            edge_logits<HT>(a, j, er, sl, z);
-            const int64_t eid = a.edge_ids ? __ldg(a.edge_ids + j) : j;
-            uint32_t packed = 0;
-            uint64_t cached_blk = ~0ull;
-            uint4 rnd = make_uint4(0, 0, 0, 0);
+        for (int t = 0; t < trips; ++t) {
+            const int j0 = beg + tid + t * NT * U;
+            trip_logits<NT, HT, U, PLAIN>(a, j0, beg, end, er, sl, z);
 #pragma unroll
-            for (int h = 0; h < kMaxHeads; ++h) {
-                if (h < H) {
-                    const float t = __fmul_rn(__expf(z[h] - m[h]) * inv[h], inv_s);
-                    float u = 0.f;
-                    if (a.round_mode == TANGO_ROUND_STOCHASTIC)
-                        u = sr_uniform(ph, (uint64_t)eid * (uint64_t)H + (uint64_t)h, call, cached_blk, rnd);
-                    const int qi = round_to_i8(t, a.round_mode, u);
-                    if (HT == 4) packed |= ((uint32_t)qi & 0xffu) << (8 * h);
-                    else a.att_q[eid * H + h] = (int8_t)qi;
+            for (int u = 0; u < U; ++u) {
+                const int j = j0 + u * NT;
+                if (j >= end) break;
+                const int64_t eid = a.edge_ids ? __ldg(a.edge_ids + j) : j;
+                uint32_t packed[2] = {0, 0};
+                uint64_t cached_blk = ~0ull;
+                uint4 rnd = make_uint4(0, 0, 0, 0);
+#pragma unroll
+                for (int h = 0; h < N; ++h) {
+                    if (h < H) {
+                        const float v = __fmul_rn(__expf(z[u][h] - m[h]) * inv[h], inv_s);
+                        float r = 0.f;
+                        if (a.round_mode == TANGO_ROUND_STOCHASTIC)
+                            r = sr_uniform(ph, (uint64_t)eid * (uint64_t)H + (uint64_t)h, call, cached_blk, rnd);
+                        const int qi = round_to_i8(v, a.round_mode, r);
+                        if (HT >= 2) packed[h >> 2] |= ((uint32_t)qi & 0xffu) << (8 * (h & 3));
+                        else a.att_q[eid * H + h] = (int8_t)qi;
+                    }
                 }
+                if (HT == 8) *reinterpret_cast<uint2 *>(a.att_q + eid * 8) = make_uint2(packed[0], packed[1]);
+                if (HT == 4) *reinterpret_cast<uint32_t *>(a.att_q + eid * 4) = packed[0];
+                if (HT == 2) *reinterpret_cast<uint16_t *>(a.att_q + eid * 2) = (uint16_t)packed[0];
             }
-            if (HT == 4) *reinterpret_cast<uint32_t *>(a.att_q + eid * 4) = packed;
         }
         return;
     }
-    for (int j = beg + tid; j < end; j += NT) {
-        float z[kMaxHeads];
-        edge_logits<HT>(a, j, er, sl, z);
+    for (int t = 0; t < trips; ++t) {
+        trip_logits<NT, HT, U, PLAIN, kKeep ? SAVE : GATHER>(a, beg + tid + t * NT * U, beg, end, er, sl, z, kept, cap);
 #pragma unroll
-        for (int h = 0; h < kMaxHeads; ++h) {
+        for (int h = 0; h < N; ++h) {
             if (h < H) {
-                if (z[h] > m[h]) { s[h] = s[h] * __expf(m[h] - z[h]) + 1.f; m[h] = z[h]; }
-                else s[h] += __expf(z[h] - m[h]);
+                float mx = m[h];
+#pragma unroll
+                for (int u = 0; u < U; ++u) mx = fmaxf(mx, z[u][h]);
+                // nothing but -infinity so far: the sum stays 0 (a NaN, which fmaxf passes over, still reaches the sum)
+                const float base = mx == -INFINITY ? 0.f : mx;
+                float sum = s[h] * __expf(m[h] - base);
+#pragma unroll
+                for (int u = 0; u < U; ++u) sum += __expf(z[u][h] - base);
+                s[h] = sum; m[h] = mx;
             }
         }
     }
 #pragma unroll
-    for (int h = 0; h < kMaxHeads; ++h)
+    for (int h = 0; h < N; ++h)
         if (h < H) team_softmax_merge<NT>(m[h], s[h], smem);
-    float inv[kMaxHeads];
 #pragma unroll
-    for (int h = 0; h < kMaxHeads; ++h) inv[h] = h < H ? 1.f / s[h] : 0.f;
+    for (int h = 0; h < N; ++h) inv[h] = h < H ? 1.f / s[h] : 0.f;
     if (STAGE == FWD_STATS) {
         // first step: keep (m, inv); the row's largest weight is exp(0) * inv = inv
         if (tid == 0 && end > beg) {
 #pragma unroll
-            for (int h = 0; h < kMaxHeads; ++h) {
+            for (int h = 0; h < N; ++h) {
                 if (h < H) {
                     a.row_m[row * H + h] = m[h];
                     a.row_inv[row * H + h] = inv[h];
@@ -198,123 +289,149 @@ __device__ __forceinline__ void softmax_row(const GatArgs &a, int64_t row, int t
         }
         return;
     }
-    for (int j = beg + tid; j < end; j += NT) {
-        float z[kMaxHeads];
-        edge_logits<HT>(a, j, er, sl, z);
-        const int64_t eid = a.edge_ids ? __ldg(a.edge_ids + j) : j;
-        if (HT == 4) {
-            const float4 o = make_float4(__expf(z[0] - m[0]) * inv[0], __expf(z[1] - m[1]) * inv[1],
-                                         __expf(z[2] - m[2]) * inv[2], __expf(z[3] - m[3]) * inv[3]);
-            *reinterpret_cast<float4 *>(a.att + eid * 4) = o;
-            amax = fmaxf(fmaxf(amax, fmaxf(o.x, o.y)), fmaxf(o.z, o.w));
-        } else {
+    for (int t = trips - 1; t >= 0; --t) {          // the last trip's logits are still in registers
+        const int j0 = beg + tid + t * NT * U;
+        if (t != trips - 1) trip_logits<NT, HT, U, PLAIN, kKeep ? REUSE : GATHER>(a, j0, beg, end, er, sl, z, kept, cap);
 #pragma unroll
-            for (int h = 0; h < kMaxHeads; ++h) {
-                if (h < H) {
-                    const float o = __expf(z[h] - m[h]) * inv[h];
-                    a.att[eid * H + h] = o;
-                    amax = fmaxf(amax, o);
-                }
+        for (int u = 0; u < U; ++u) {
+            const int j = j0 + u * NT;
+            if (j >= end) break;
+            const int64_t eid = a.edge_ids ? __ldg(a.edge_ids + j) : j;
+            float o[N];
+#pragma unroll
+            for (int h = 0; h < N; ++h) {
+                o[h] = h < H ? __expf(z[u][h] - m[h]) * inv[h] : 0.f;
+                amax = fmaxf(amax, o[h]);
             }
+            store_heads<HT>(a.att + eid * H, H, o);
         }
     }
 }
 
 // RECOMPUTE: the attention weights are not read but recomputed as exp(z - m) * inv from the forward's statistics.
-template <int NT, int HT, bool RECOMPUTE>
-__device__ __forceinline__ void softmax_bwd_row(const GatArgs &a, int64_t row, int tid, float *smem, float &amax) {
-    const bool plain = a.zin != nullptr;   // backward of the plain flavour: zin is only a marker, never read
-    const float sl = plain ? 0.f : __ldg(a.sl), sr = plain ? 0.f : __ldg(a.sr);
-    const int beg = __ldg(a.indptr + row), end = __ldg(a.indptr + row + 1);
+template <int NT, int HT, int U, bool PLAIN, bool RECOMPUTE>
+__device__ __forceinline__ void softmax_bwd_row(const GatArgs &a, int64_t row, int beg, int end, int tid, float *smem,
+                                                float &amax) {
+    constexpr int N = Shape<HT>::N;
+    const float sl = PLAIN ? 0.f : __ldg(a.sl), sr = PLAIN ? 0.f : __ldg(a.sr);
     const int H = HT ? HT : a.H;
-    float er[kMaxHeads], dot[kMaxHeads], m[kMaxHeads], inv[kMaxHeads];
+    const int trips = (end - beg + NT * U - 1) / (NT * U);
+    float er[N], dot[N], m[N], inv[N], z[U][N], p[U][N], g[U][N];
 #pragma unroll
-    for (int h = 0; h < kMaxHeads; ++h) {
-        er[h] = (h < H && !plain) ? __fmul_rn((float)__ldg(a.erq + row * H + h), sr) : 0.f;
+    for (int h = 0; h < N; ++h) {
+        er[h] = (h < H && !PLAIN) ? __fmul_rn((float)__ldg(a.erq + row * H + h), sr) : 0.f;
         dot[h] = 0.f;
         m[h] = (RECOMPUTE && h < H) ? __ldg(a.row_m + row * H + h) : 0.f;
         inv[h] = (RECOMPUTE && h < H) ? __ldg(a.row_inv + row * H + h) : 0.f;
     }
-    for (int j = beg + tid; j < end; j += NT) {
-        const int64_t eid = a.edge_ids ? __ldg(a.edge_ids + j) : j;
-        if (RECOMPUTE) {
-            float z[kMaxHeads];
-            edge_logits<HT>(a, j, er, sl, z);
-            if (HT == 4) {
-                const float4 g = __ldg(reinterpret_cast<const float4 *>(a.datt + eid * 4));
-                dot[0] += __expf(z[0] - m[0]) * inv[0] * g.x; dot[1] += __expf(z[1] - m[1]) * inv[1] * g.y;
-                dot[2] += __expf(z[2] - m[2]) * inv[2] * g.z; dot[3] += __expf(z[3] - m[3]) * inv[3] * g.w;
-            } else {
+    int eid[U];
+    const auto load = [&](int t, bool logits) {
+        const int j0 = beg + tid + t * NT * U;
 #pragma unroll
-                for (int h = 0; h < kMaxHeads; ++h)
-                    if (h < H) dot[h] += __expf(z[h] - m[h]) * inv[h] * __ldg(a.datt + eid * H + h);
-            }
-        } else if (HT == 4) {
-            const float4 p = __ldg(reinterpret_cast<const float4 *>(a.att + eid * 4));
-            const float4 g = __ldg(reinterpret_cast<const float4 *>(a.datt + eid * 4));
-            dot[0] += p.x * g.x; dot[1] += p.y * g.y; dot[2] += p.z * g.z; dot[3] += p.w * g.w;
-        } else {
-#pragma unroll
-            for (int h = 0; h < kMaxHeads; ++h)
-                if (h < H) dot[h] += __ldg(a.att + eid * H + h) * __ldg(a.datt + eid * H + h);
+        for (int u = 0; u < U; ++u) {
+            const int j = j0 + u * NT;
+            eid[u] = j < end ? (a.edge_ids ? __ldg(a.edge_ids + j) : j) : -1;
         }
+        if (!PLAIN && (RECOMPUTE || logits)) trip_logits<NT, HT, U, PLAIN>(a, j0, beg, end, er, sl, z);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+#pragma unroll
+            for (int h = 0; h < N; ++h) p[u][h] = g[u][h] = 0.f;
+            if (eid[u] >= 0) {
+                if (!RECOMPUTE) load_heads<HT>(a.att + (int64_t)eid[u] * H, H, p[u]);
+                load_heads<HT>(a.datt + (int64_t)eid[u] * H, H, g[u]);
+            }
+        }
+        if (RECOMPUTE) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int h = 0; h < N; ++h) p[u][h] = eid[u] >= 0 ? __expf(z[u][h] - m[h]) * inv[h] : 0.f;
+        }
+    };
+    for (int t = 0; t < trips; ++t) {
+        load(t, t == trips - 1);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int h = 0; h < N; ++h)
+                if (h < H) dot[h] += p[u][h] * g[u][h];
     }
 #pragma unroll
-    for (int h = 0; h < kMaxHeads; ++h)
+    for (int h = 0; h < N; ++h)
         if (h < H) dot[h] = team_sum<NT>(dot[h], smem);
-    for (int j = beg + tid; j < end; j += NT) {
-        float z[kMaxHeads];
-        if (!plain) edge_logits<HT>(a, j, er, sl, z);   // leaky(z) has the sign of z
-        const int64_t eid = a.edge_ids ? __ldg(a.edge_ids + j) : j;
-        if (HT == 4) {
-            const float4 p = RECOMPUTE ? make_float4(__expf(z[0] - m[0]) * inv[0], __expf(z[1] - m[1]) * inv[1],
-                                                     __expf(z[2] - m[2]) * inv[2], __expf(z[3] - m[3]) * inv[3])
-                                       : __ldg(reinterpret_cast<const float4 *>(a.att + eid * 4));
-            const float4 g = __ldg(reinterpret_cast<const float4 *>(a.datt + eid * 4));
-            float4 o = make_float4(p.x * (g.x - dot[0]), p.y * (g.y - dot[1]), p.z * (g.z - dot[2]),
-                                   p.w * (g.w - dot[3]));
-            if (plain) {
-                o.x *= a.zmul; o.y *= a.zmul; o.z *= a.zmul; o.w *= a.zmul;
-            } else {
-                if (!(z[0] > 0.f)) o.x *= a.slope;
-                if (!(z[1] > 0.f)) o.y *= a.slope;
-                if (!(z[2] > 0.f)) o.z *= a.slope;
-                if (!(z[3] > 0.f)) o.w *= a.slope;
-            }
-            *reinterpret_cast<float4 *>(a.dz + eid * 4) = o;
-            amax = fmaxf(fmaxf(amax, fmaxf(fabsf(o.x), fabsf(o.y))), fmaxf(fabsf(o.z), fabsf(o.w)));
-        } else {
+    for (int t = trips - 1; t >= 0; --t) {          // the last trip is still in registers
+        if (t != trips - 1) load(t, true);
 #pragma unroll
-            for (int h = 0; h < kMaxHeads; ++h) {
-                if (h < H) {
-                    const float p = RECOMPUTE ? __expf(z[h] - m[h]) * inv[h] : __ldg(a.att + eid * H + h);
-                    float o = p * (__ldg(a.datt + eid * H + h) - dot[h]);
-                    if (plain) o *= a.zmul;
-                    else if (!(z[h] > 0.f)) o *= a.slope;
-                    a.dz[eid * H + h] = o;
-                    amax = fmaxf(amax, fabsf(o));
-                }
+        for (int u = 0; u < U; ++u) {
+            if (eid[u] < 0) break;
+            float o[N];
+#pragma unroll
+            for (int h = 0; h < N; ++h) {
+                o[h] = p[u][h] * (g[u][h] - dot[h]);
+                if (PLAIN) o[h] *= a.zmul;
+                else if (!(z[u][h] > 0.f)) o[h] *= a.slope;      // leaky(z) has the sign of z
+                if (h < H) amax = fmaxf(amax, fabsf(o[h]));
             }
+            store_heads<HT>(a.dz + (int64_t)eid[u] * H, H, o);
         }
     }
 }
 
-// blocks [0, n_block_rows): one CTA per row; the remaining blocks: one warp per row
+template <int NT, int HT, int U, bool PLAIN, bool BWD, int STAGE>
+__device__ __forceinline__ void one_row(const GatArgs &a, int64_t row, int beg, int end, int tid, float *smem,
+                                        typename Record<HT>::T *kept, int cap, float &amax) {
+    if (BWD) softmax_bwd_row<NT, HT, U, PLAIN, STAGE != 0>(a, row, beg, end, tid, smem, amax);
+    else softmax_row<NT, HT, U, PLAIN, STAGE>(a, row, beg, end, tid, smem, kept, cap, amax);
+}
+
+// CTAs [0, n_block_rows): one row each.  In the CTAs behind them a warp takes four rows in a row of the order: side by side
+// with eight lanes each when the longest of them fits one trip of eight lanes, else one after the other with the whole warp.
 // BWD: gradient kernel; STAGE: forward flavour (FWD_*) or, for BWD, 1 = recompute the weights from the statistics
-template <int HT, bool BWD, int STAGE>
-__global__ void __launch_bounds__(256) gat_softmax_kernel(const GatArgs a) {
+//
+// What bounds it: on long rows the [E, H] streams (forward 4 B in and 4 * H out per edge, backward 8 * H in and 4 * H out,
+// less what the second sweep finds in L2) and, in the forward, a warp's load of 32 random int8 records, which takes 32 passes
+// through L1: the records are kept in shared memory between the sweeps.  On short rows it is rows in flight: half the rows
+// of a sparse power-law graph have one edge, and had a warp each.  One edge in flight per thread -> as it is, us:
+//   114.6 M edges, 4 heads: forward 1224 -> 1160, backward 1577 -> 1387;  1 head: 593 -> 409, 668 -> 566
+//   1.3 M edges on 169 K nodes, 4 heads, plain scores: 153 -> 57, 55 -> 34;  0.1 M edges, 8 heads: 53 -> 28, 40 -> 13
+template <int HT, bool PLAIN, bool BWD, int STAGE>
+__global__ void __launch_bounds__(256, HT == 1 || HT == 2 ? (BWD ? 4 : 6) : (HT == 4 ? 4 : 3) - (BWD ? 1 : 0)) gat_softmax_kernel(const GatArgs a) {
+    constexpr int U = Shape<HT>::U;
+    constexpr bool kKeep = !BWD && STAGE == FWD_FLOAT && !PLAIN && HT != 0;
+    constexpr int kCap = kKeep ? Shape<HT>::kKept : 0;
+    typedef typename Record<HT>::T R;
     __shared__ float smem[64];
+    __shared__ R s_kept[kKeep ? 8 * kCap : 1];
     float amax = 0.f;
     if ((int64_t)blockIdx.x < a.n_block_rows) {
         const int64_t row = a.row_order ? (int64_t)__ldg(a.row_order + blockIdx.x) : (int64_t)blockIdx.x;
-        if (BWD) softmax_bwd_row<256, HT, STAGE != 0>(a, row, threadIdx.x, smem, amax);
-        else softmax_row<256, HT, STAGE>(a, row, threadIdx.x, smem, amax);
+        const int beg = __ldg(a.indptr + row), end = __ldg(a.indptr + row + 1);
+        one_row<256, HT, U, PLAIN, BWD, STAGE>(a, row, beg, end, threadIdx.x, smem, s_kept, 8 * kCap, amax);
     } else {
-        const int64_t i = a.n_block_rows + ((int64_t)blockIdx.x - a.n_block_rows) * 8 + (threadIdx.x >> 5);
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int64_t i = a.n_block_rows + (((int64_t)blockIdx.x - a.n_block_rows) * 8 + warp) * 4 + (lane & 3);
+        int row = -1, beg = 0, end = 0;
         if (i < a.n_rows) {
-            const int64_t row = a.row_order ? (int64_t)__ldg(a.row_order + i) : i;
-            if (BWD) softmax_bwd_row<32, HT, STAGE != 0>(a, row, threadIdx.x & 31, smem, amax);
-            else softmax_row<32, HT, STAGE>(a, row, threadIdx.x & 31, smem, amax);
+            row = a.row_order ? __ldg(a.row_order + i) : (int)i;
+            beg = __ldg(a.indptr + row); end = __ldg(a.indptr + row + 1);
+        }
+        int longest = max(end - beg, __shfl_xor_sync(0xffffffffu, end - beg, 1));
+        longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, 2));
+        if (longest <= 8 * U) {
+            const int team = lane >> 3;
+            row = max(0, __shfl_sync(0xffffffffu, row, team));       // (a missing row has no slots)
+            beg = __shfl_sync(0xffffffffu, beg, team);
+            end = __shfl_sync(0xffffffffu, end, team);
+            if (longest <= 8) one_row<8, HT, 1, PLAIN, BWD, STAGE>(a, row, beg, end, lane & 7, smem, nullptr, 0, amax);
+            else one_row<8, HT, U, PLAIN, BWD, STAGE>(a, row, beg, end, lane & 7, smem, nullptr, 0, amax);
+        } else {
+            for (int r = 0; r < 4; ++r) {
+                const int rr = __shfl_sync(0xffffffffu, row, r);
+                if (rr < 0) break;
+                one_row<32, HT, U, PLAIN, BWD, STAGE>(a, rr, __shfl_sync(0xffffffffu, beg, r), __shfl_sync(0xffffffffu, end, r),
+                                                      lane, smem, s_kept + (kKeep ? warp * kCap : 0), kCap, amax);
+            }
         }
     }
     if (a.out_absmax) {
@@ -326,20 +443,30 @@ __global__ void __launch_bounds__(256) gat_softmax_kernel(const GatArgs a) {
     }
 }
 
+template <int HT, bool BWD, int STAGE>
+static void launch_heads(const GatArgs &a, unsigned blocks, cudaStream_t stream) {
+    if (STAGE == 0 && a.zin) gat_softmax_kernel<HT, true, BWD, 0><<<blocks, 256, 0, stream>>>(a);
+    else gat_softmax_kernel<HT, false, BWD, STAGE><<<blocks, 256, 0, stream>>>(a);
+}
+
 template <bool BWD, int STAGE = 0>
 static int launch_gat(GatArgs &a, cudaStream_t stream) {
     if (a.n_rows < 0 || a.H < 1 || a.H > kMaxHeads) return TANGO_EINVAL;
     if (a.n_rows == 0) return TANGO_OK;
     if (!a.row_order) a.n_block_rows = 0;
     if (a.n_block_rows < 0 || a.n_block_rows > a.n_rows) return TANGO_EINVAL;
-    const int64_t blocks = a.n_block_rows + ceil_div(a.n_rows - a.n_block_rows, 8);
-    if (blocks > 0x7fffffff) return TANGO_ESIZE;
-    const bool h4 = a.H == 4 && aligned(a.att, 16) && (a.zin ? aligned(a.zin, 16) : aligned(a.elq, 4)) &&
-                    (!BWD || (aligned(a.datt, 16) && aligned(a.dz, 16))) && aligned(a.att_q, 4);
-    if (h4) gat_softmax_kernel<4, BWD, STAGE><<<(unsigned)blocks, 256, 0, stream>>>(a);
-    else if (a.H == 1) gat_softmax_kernel<1, BWD, STAGE><<<(unsigned)blocks, 256, 0, stream>>>(a);
-    else if (a.H == 2) gat_softmax_kernel<2, BWD, STAGE><<<(unsigned)blocks, 256, 0, stream>>>(a);
-    else gat_softmax_kernel<0, BWD, STAGE><<<(unsigned)blocks, 256, 0, stream>>>(a);
+    const int64_t blocks = a.n_block_rows + ceil_div(a.n_rows - a.n_block_rows, 8 * 4);
+    if (blocks > 0x7fffffff || a.n_rows > 0x7fffffff) return TANGO_ESIZE;
+    // all heads of an edge in one access where every array allows it
+    const int f = 4 * (a.H < 4 ? a.H : 4);
+    const bool whole = (a.H == 1 || a.H == 2 || a.H == 4 || a.H == 8) && aligned(a.att, f) && aligned(a.zin, f) &&
+                       aligned(a.datt, f) && aligned(a.dz, f) && aligned(a.elq, a.H) && aligned(a.att_q, a.H);
+    const unsigned nb = (unsigned)blocks;
+    if (whole && a.H == 1) launch_heads<1, BWD, STAGE>(a, nb, stream);
+    else if (whole && a.H == 2) launch_heads<2, BWD, STAGE>(a, nb, stream);
+    else if (whole && a.H == 4) launch_heads<4, BWD, STAGE>(a, nb, stream);
+    else if (whole && a.H == 8) launch_heads<8, BWD, STAGE>(a, nb, stream);
+    else launch_heads<0, BWD, STAGE>(a, nb, stream);
     TANGO_LAUNCH_CHECK();
     return TANGO_OK;
 }

@@ -203,3 +203,40 @@ def test_widths_that_do_not_match_are_refused(cuda):
     for feats, hidden in ((40, 8), (8, 40)):
         with pytest.raises(AssertionError):
             QGraphConv(feats, hidden).cuda()(g, torch.randn(300, feats - 1, device="cuda"))
+
+
+@pytest.mark.parametrize("heads", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("order", ["rows", "shuffled"])
+def test_edge_softmax_of_row_lengths_around_the_trips(cuda, heads, order):
+    """Rows of 0 to 3000 edges, with the edge numbers along the rows and not.  __expf of an argument of at most 40 is off by
+    40 * 2^-23 + 2^-21 relative, the sum of up to 3000 positive terms by less than that again: 2e-5 in all."""
+    import tango_b200 as T
+    from tango_b200.gnn import edge_softmax
+    from tango_b200.graph import Graph
+    deg = np.array([0, 1, 2, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 257, 1023, 1024, 1025, 2049, 3000])
+    dst = np.repeat(np.arange(deg.size), deg)
+    rng = np.random.default_rng(heads)
+    if order == "shuffled":
+        dst = rng.permutation(dst)
+    src = rng.integers(0, deg.size, dst.size)
+    g = T.graph_preprocess(Graph(torch.from_numpy(src.astype(np.int32)), torch.from_numpy(dst.astype(np.int32)), deg.size).to("cuda"))
+    z = rng.uniform(-20, 20, (dst.size, heads, 1)).astype(np.float32)
+    z[rng.random(z.shape) < 0.02] = -np.inf
+    z[dst == 1] = 0.5
+    da = rng.standard_normal(z.shape).astype(np.float32)
+    zt = torch.from_numpy(z).cuda().requires_grad_()
+    a, sa = edge_softmax(g, zt, 0.5, True)
+    a.backward(torch.from_numpy(da).cuda())
+    want, grad, size = (np.zeros(z.shape) for _ in range(3))
+    for v in range(deg.size):
+        e = dst == v
+        if e.any():
+            w = np.exp(z[e] * 0.5 - (z[e] * 0.5).max(0))
+            want[e] = w = w / w.sum(0)
+            dot = (w * da[e]).sum(0)
+            grad[e] = w * (da[e] - dot) * 0.5
+            size[e] = w * (np.abs(da[e]) + (w * np.abs(da[e])).sum(0)) * 0.5
+    tiny = 1e-37                                        # (weights below the normal range are flushed)
+    assert (np.abs(_np(a) - want) <= 2e-5 * want + tiny).all()
+    assert (np.abs(_np(zt.grad) - grad) <= 4e-5 * size + tiny).all()
+    assert sa.item() == np.float32(_np(a).max()) / np.float32(127)
