@@ -280,6 +280,12 @@ int tango_spmm_u_mul_e(const int32_t *indptr, const int32_t *indices, const int3
                        const int8_t *nq, int64_t ldn, int h, int d, const int8_t *eq, const float *scale, float *out,
                        int64_t ldo, const tango_spmm_plan *plan /* host */, tango_stream_t stream);
 
+/* The same plus bias[h*D + d] (optional). */
+int tango_spmm_u_mul_e_bias(const int32_t *indptr, const int32_t *indices, const int32_t *edge_ids, int64_t n_rows,
+                            const int8_t *nq, int64_t ldn, int h, int d, const int8_t *eq, const float *scale,
+                            const float *bias, float *out, int64_t ldo, const tango_spmm_plan *plan /* host */,
+                            tango_stream_t stream);
+
 /* out[v,:] = scale[0] * float(sum_{j in row v} Zq[eid(j), :]) -- sum of the int8 edge features incident to a node.
  * Replaces incidence_SPMM (cuda/src/cuda.cpp:198, cuda/src/SPMM.cu:259-303). */
 int tango_spmm_incidence(const int32_t *indptr, const int32_t *edge_ids, int64_t n_rows, const int8_t *zq, int64_t ldz,
@@ -364,6 +370,18 @@ int tango_gat_edge_softmax_bwd_stats(const int32_t *indptr, const int32_t *indic
                                      const int8_t *erq, int h, const float *sl, const float *sr, float slope,
                                      const float *row_m, const float *row_inv, const float *da, float *dz,
                                      float *dz_absmax, tango_stream_t stream);
+
+/* Attention projections of a GAT layer: el[n,h] = <x[n,h,:], al[h,:]> and er with ar, x fp32 [N, H, D] contiguous
+ * (evaluation/test_gat.py:127-128). */
+int tango_gat_project(const float *x, int64_t n, int h, int d, const float *al, const float *ar, float *el, float *er,
+                      tango_stream_t stream);
+
+/* Their gradients: dx[n,h,:] += dl[n,h] * al[h,:] + dr[n,h] * ar[h,:] (dx optional) and dal[h,:] = sum_n dl[n,h] *
+ * x[n,h,:], dar likewise (both or neither; they need `scratch` of tango_gat_project_bwd_scratch_bytes, 4-byte aligned). */
+int64_t tango_gat_project_bwd_scratch_bytes(int64_t n, int h, int d);
+int tango_gat_project_bwd(const float *x, int64_t n, int h, int d, const float *al, const float *ar, const float *dl,
+                          const float *dr, float *dx, float *dal, float *dar, void *scratch, int64_t scratch_bytes,
+                          tango_stream_t stream);
 
 /* Edge softmax of plain fp32 scores: for every destination row v (CSC order) and head h
  *   a[eid(j),h] = softmax_j( z[eid(j),h] * zmul )     over the incoming edges j of v,

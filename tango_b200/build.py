@@ -22,7 +22,7 @@ LIB_DIR = os.path.join(HERE, "lib")
 HEADER = os.path.join(ROOT, "include", "tango_b200.h")
 CUDA_HOME = os.environ.get("CUDA_HOME") or "/usr/local/cuda"
 LIB_PATH = os.path.join(LIB_DIR, "libtango_b200.so")
-SOURCES = ["quantize.cu", "quantize_fused.cu", "spmm.cu", "sddmm.cu", "gat_softmax.cu", "igemm_tcgen05.cu", "peer.cu"]
+SOURCES = ["quantize.cu", "quantize_fused.cu", "spmm.cu", "sddmm.cu", "gat_softmax.cu", "gat_project.cu", "igemm_tcgen05.cu", "peer.cu"]
 HOST_SOURCES = ["torch_ops.cpp", "torch_autograd.cpp", "torch_bind.cpp"]
 HOST_LIB_PATH = os.path.join(LIB_DIR, "_torch_ops.so")
 # measurement aid of the benchmark, a library of its own (not part of the product ABI)

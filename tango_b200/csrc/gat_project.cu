@@ -36,49 +36,50 @@ __device__ __forceinline__ void load(const float *p, float (&v)[VEC]) {
     }
 }
 
-// 2^groups_log2 lanes share an item and reduce with a fixed butterfly.
-template <int VEC>
+// 2^groups_log2 lanes share an item and reduce with a fixed butterfly.  Groups advance by a multiple of H items, so that each
+// keeps its head's weights in registers when they fit one piece per lane (SINGLE).
+template <int VEC, bool SINGLE>
 __global__ void __launch_bounds__(kThreads) project_kernel(const ProjArgs a) {
     const int G = 1 << a.groups_log2, sub = threadIdx.x & (G - 1);
-    const int per_cta = kThreads >> a.groups_log2;
-    const int64_t i0 = (int64_t)blockIdx.x * per_cta * kItems + (threadIdx.x >> a.groups_log2);
-    float l[kItems], r[kItems];
-    int head[kItems];
+    const int64_t groups = (int64_t)gridDim.x * (kThreads >> a.groups_log2), step = groups - groups % a.H;
+    const int64_t gid = (int64_t)blockIdx.x * (kThreads >> a.groups_log2) + (threadIdx.x >> a.groups_log2);
+    const int head = (int)(gid % a.H);
+    const float *al = a.al + (int64_t)head * a.D, *ar = a.ar + (int64_t)head * a.D;
+    float wl[VEC], wr[VEC];
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        const int64_t i = i0 + (int64_t)k * per_cta;
-        l[k] = r[k] = 0.f;
-        head[k] = a.items <= 0xffffffffll ? (int)((uint32_t)i % (uint32_t)a.H) : (int)(i % a.H);
-    }
-    for (int c = sub * VEC; c < a.D; c += G * VEC) {
-        float v[kItems][VEC];
+    for (int e = 0; e < VEC; ++e) wl[e] = wr[e] = 0.f;
+    if (SINGLE && sub * VEC < a.D) { load<VEC>(al + sub * VEC, wl); load<VEC>(ar + sub * VEC, wr); }
+    for (int64_t base = 0; base < a.items; base += step * kItems) {          // the same trips for every lane of a warp
+        float l[kItems], r[kItems];
 #pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const int64_t i = i0 + (int64_t)k * per_cta;
+        for (int k = 0; k < kItems; ++k) l[k] = r[k] = 0.f;
+        for (int c = sub * VEC; c < a.D; c += G * VEC) {
+            float v[kItems][VEC];
 #pragma unroll
-            for (int e = 0; e < VEC; ++e) v[k][e] = 0.f;
-            if (i < a.items) load<VEC>(a.x + i * a.D + c, v[k]);
-        }
+            for (int k = 0; k < kItems; ++k) {
+                const int64_t i = base + k * step + gid;
 #pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            float wl[VEC], wr[VEC];
-            load<VEC>(a.al + (int64_t)head[k] * a.D + c, wl);
-            load<VEC>(a.ar + (int64_t)head[k] * a.D + c, wr);
-#pragma unroll
-            for (int e = 0; e < VEC; ++e) {
-                l[k] += v[k][e] * wl[e];
-                r[k] += v[k][e] * wr[e];
+                for (int e = 0; e < VEC; ++e) v[k][e] = 0.f;
+                if (gid < step && i < a.items) load<VEC>(a.x + i * a.D + c, v[k]);
             }
-        }
-    }
+            if (!SINGLE) { load<VEC>(al + c, wl); load<VEC>(ar + c, wr); }
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        for (int o = G >> 1; o > 0; o >>= 1) {
-            l[k] += __shfl_xor_sync(0xffffffffu, l[k], o);
-            r[k] += __shfl_xor_sync(0xffffffffu, r[k], o);
+            for (int k = 0; k < kItems; ++k)
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) {
+                    l[k] += v[k][e] * wl[e];
+                    r[k] += v[k][e] * wr[e];
+                }
         }
-        const int64_t i = i0 + (int64_t)k * per_cta;
-        if (sub == 0 && i < a.items) { a.el[i] = l[k]; a.er[i] = r[k]; }
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            for (int o = G >> 1; o > 0; o >>= 1) {
+                l[k] += __shfl_xor_sync(0xffffffffu, l[k], o);
+                r[k] += __shfl_xor_sync(0xffffffffu, r[k], o);
+            }
+            const int64_t i = base + k * step + gid;
+            if (sub == 0 && gid < step && i < a.items) { a.el[i] = l[k]; a.er[i] = r[k]; }
+        }
     }
 }
 
@@ -211,10 +212,13 @@ extern "C" int tango_gat_project(const float *x, int64_t n, int h, int d, const 
     const bool wide = d % 4 == 0 && aligned(x, 16) && aligned(al, 16) && aligned(ar, 16);
     const int pieces = wide ? d / 4 : d;
     while ((1 << a.groups_log2) < pieces && a.groups_log2 < 5) ++a.groups_log2;
-    const int64_t blocks = ceil_div(a.items, (int64_t)(kThreads >> a.groups_log2) * kItems);
-    if (blocks > 0x7fffffff) return TANGO_ESIZE;
-    if (wide) project_kernel<4><<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
-    else project_kernel<1><<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
+    const int64_t blocks = ceil_div(a.items, kThreads >> a.groups_log2);       // items >= H: there is a whole step
+    const unsigned nb = (unsigned)(blocks < kNumSMs * 8 ? blocks : kNumSMs * 8);
+    const bool single = pieces <= 1 << a.groups_log2;
+    if (wide && single) project_kernel<4, true><<<nb, kThreads, 0, (cudaStream_t)stream>>>(a);
+    else if (wide) project_kernel<4, false><<<nb, kThreads, 0, (cudaStream_t)stream>>>(a);
+    else if (single) project_kernel<1, true><<<nb, kThreads, 0, (cudaStream_t)stream>>>(a);
+    else project_kernel<1, false><<<nb, kThreads, 0, (cudaStream_t)stream>>>(a);
     TANGO_LAUNCH_CHECK();
     return TANGO_OK;
 }

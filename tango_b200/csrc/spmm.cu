@@ -1032,10 +1032,10 @@ extern "C" int tango_spmm_copy_u(const int32_t *indptr, const int32_t *indices, 
     return launch_spmm<MODE_COPY>(a, plan, (cudaStream_t)stream);
 }
 
-extern "C" int tango_spmm_u_mul_e(const int32_t *indptr, const int32_t *indices, const int32_t *edge_ids,
-                                  int64_t n_rows, const int8_t *nq, int64_t ldn, int h, int d, const int8_t *eq,
-                                  const float *scale, float *out, int64_t ldo, const tango_spmm_plan *plan,
-                                  tango_stream_t stream) {
+extern "C" int tango_spmm_u_mul_e_bias(const int32_t *indptr, const int32_t *indices, const int32_t *edge_ids,
+                                       int64_t n_rows, const int8_t *nq, int64_t ldn, int h, int d, const int8_t *eq,
+                                       const float *scale, const float *bias, float *out, int64_t ldo, const tango_spmm_plan *plan,
+                                       tango_stream_t stream) {
     if (n_rows < 0 || h < 1 || d < 1) return TANGO_EINVAL;
     const int64_t f = (int64_t)h * d;
     if (ldn < f || ldo < f || f > (1 << 20)) return TANGO_EINVAL;
@@ -1044,8 +1044,15 @@ extern "C" int tango_spmm_u_mul_e(const int32_t *indptr, const int32_t *indices,
     SpmmArgs a{};
     a.indptr = indptr; a.indices = indices; a.edge_ids = edge_ids; a.n_rows = n_rows; a.nseg = 1;
     a.feat = nq; a.ld = ldn; a.f = (int)f; a.ew = eq; a.H = h; a.D = d;
-    a.scales = scale; a.out = out; a.ldo = ldo;
+    a.scales = scale; a.bias = bias; a.out = out; a.ldo = ldo;
     return launch_spmm<MODE_WEIGHT_LANE>(a, plan, (cudaStream_t)stream);
+}
+
+extern "C" int tango_spmm_u_mul_e(const int32_t *indptr, const int32_t *indices, const int32_t *edge_ids,
+                                  int64_t n_rows, const int8_t *nq, int64_t ldn, int h, int d, const int8_t *eq,
+                                  const float *scale, float *out, int64_t ldo, const tango_spmm_plan *plan,
+                                  tango_stream_t stream) {
+    return tango_spmm_u_mul_e_bias(indptr, indices, edge_ids, n_rows, nq, ldn, h, d, eq, scale, nullptr, out, ldo, plan, stream);
 }
 
 extern "C" int tango_spmm_incidence(const int32_t *indptr, const int32_t *edge_ids, int64_t n_rows, const int8_t *zq,

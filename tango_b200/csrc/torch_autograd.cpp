@@ -498,9 +498,12 @@ struct GatLogits {
     int64_t n_block() const { return d().sched.n_block_rows; }
 };
 
-static GatLogits gat_logits(const GraphPtr &g, const Tensor &el, const Tensor &er, double slope) {
+// `clear`: set to zero by the same launch.
+static GatLogits gat_logits(const GraphPtr &g, const Tensor &el, const Tensor &er, double slope, const Tensor &clear) {
     const int64_t n = el.size(0), h = el.size(1);
-    const QuantJob jl = quant_job(el.reshape({n, h}), 1), jr = quant_job(er.reshape({n, h}), 1);
+    QuantJob jl = quant_job(el.reshape({n, h}), 1);
+    const QuantJob jr = quant_job(er.reshape({n, h}), 1);
+    jl.clear = clear;
     const auto q = quantize_all({jl, jr});
     return {g, q[0], q[1], (float)slope, (int)h};
 }
@@ -518,6 +521,30 @@ static std::pair<Tensor, Tensor> gat_logit_grads(const GatLogits &a, const Tenso
     return {dl, dr};
 }
 
+// fp32 weights [E, H]; `sa` holds 0 and receives their scale.
+static Tensor gat_softmax(const GatLogits &l, const Tensor &sa) {
+    const Tensor a = floats({l.g->n_edges(), l.h}, sa);
+    const Direction &d = l.d();
+    check(tango_gat_edge_softmax(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), ptr<int32_t>(d.edge_ids), row_order(d),
+                                 l.n_block(), l.g->n_nodes, ptr<int8_t>(l.el.q), ptr<int8_t>(l.er.q), l.h,
+                                 ptr<float>(l.el.scale), ptr<float>(l.er.scale), l.slope, ptr<float>(a), ptr<float>(sa),
+                                 cuda_stream()), "gat_edge_softmax");
+    count(1);
+    return a;
+}
+
+// Gradient of the logits from the weights `a` and their gradient, both [E, H]; `sdz` holds 0 and receives its scale.
+static Tensor gat_softmax_bwd(const GatLogits &l, const Tensor &a, const Tensor &da, const Tensor &sdz) {
+    const Tensor dz = at::empty_like(a);
+    const Direction &d = l.d();
+    check(tango_gat_edge_softmax_bwd(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), ptr<int32_t>(d.edge_ids), row_order(d),
+                                     l.n_block(), l.g->n_nodes, ptr<int8_t>(l.el.q), ptr<int8_t>(l.er.q), l.h,
+                                     ptr<float>(l.el.scale), ptr<float>(l.er.scale), l.slope, ptr<float>(a),
+                                     ptr<float>(da), ptr<float>(dz), ptr<float>(sdz), cuda_stream()), "gat_edge_softmax_bwd");
+    count(1);
+    return dz;
+}
+
 struct GatAttentionBackward : SavingNode {
     std::string name() const override { return "GatAttentionBackward"; }
     GatLogits l;                               // without el and er, which are saved
@@ -529,14 +556,8 @@ struct GatAttentionBackward : SavingNode {
         GatLogits l = this->l;
         l.el.q = k[1]; l.el.scale = k[2]; l.er.q = k[3]; l.er.scale = k[4];
         const c10::cuda::CUDAGuard guard(at.device());
-        const Tensor a2 = at.reshape({-1, l.h}), da = grads[0].reshape({-1, l.h}).contiguous(), dz = at::empty_like(a2);
-        const Tensor sdz = zeros1(a2);
-        const Direction &d = l.d();
-        check(tango_gat_edge_softmax_bwd(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), ptr<int32_t>(d.edge_ids), row_order(d),
-                                         l.n_block(), l.g->n_nodes, ptr<int8_t>(l.el.q), ptr<int8_t>(l.er.q), l.h,
-                                         ptr<float>(l.el.scale), ptr<float>(l.er.scale), l.slope, ptr<float>(a2),
-                                         ptr<float>(da), ptr<float>(dz), ptr<float>(sdz), cuda_stream()), "gat_edge_softmax_bwd");
-        count(1);
+        const Tensor sdz = zeros1(at);
+        const Tensor dz = gat_softmax_bwd(l, at.reshape({-1, l.h}), grads[0].reshape({-1, l.h}).contiguous(), sdz);
         const auto [dl, dr] = gat_logit_grads(l, dz, sdz, needs(0), needs(1), shape_l, shape_r);
         return {dl, dr};
     }
@@ -548,15 +569,9 @@ std::tuple<Tensor, Tensor> gat_attention_fn(const GraphPtr &g, const Tensor &el,
     {
         const Raw raw;
         const c10::cuda::CUDAGuard guard(el.device());
-        l = gat_logits(g, el, er, slope);
-        a = floats({g->n_edges(), l.h, 1}, el);
-        sa = zeros1(el);
-        const Direction &d = l.d();
-        check(tango_gat_edge_softmax(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), ptr<int32_t>(d.edge_ids), row_order(d),
-                                     l.n_block(), g->n_nodes, ptr<int8_t>(l.el.q), ptr<int8_t>(l.er.q), l.h,
-                                     ptr<float>(l.el.scale), ptr<float>(l.er.scale), l.slope, ptr<float>(a), ptr<float>(sa),
-                                     cuda_stream()), "gat_edge_softmax");
-        count(1);
+        sa = floats({1}, el);
+        l = gat_logits(g, el, er, slope, sa);
+        a = gat_softmax(l, sa).view({-1, l.h, 1});
     }
     if (auto node = make_node<GatAttentionBackward>(el, er)) {
         node->l = l; node->l.el = node->l.er = {};
@@ -567,75 +582,122 @@ std::tuple<Tensor, Tensor> gat_attention_fn(const GraphPtr &g, const Tensor &el,
     return {a, sa};
 }
 
-struct GatAggregateBackward : SavingNode {
-    std::string name() const override { return "GatAggregateBackward"; }
+// The layer behind the linear projection, in two forms that differ in where the attention weights live.
+struct GatLayerBackward : SavingNode {
+    std::string name() const override { return "GatLayerBackward"; }
     GatLogits l;                               // without el and er, which are saved
-    std::vector<int64_t> shape_l, shape_r;
+    bool int8_weights = false, compat = false, has_bias = false;
     variable_list backward(const variable_list &grads) override {
         const std::vector<Tensor> k = kept();
-        if (!grads[0].defined()) return variable_list(3);
+        if (!grads[0].defined()) return variable_list(4);
+        const c10::cuda::CUDAGuard guard(grads[0].device());
         GatLogits l = this->l;
         l.el.q = k[0]; l.el.scale = k[1]; l.er.q = k[2]; l.er.scale = k[3];
-        const Tensor &m = k[4], &inv = k[5], &sa = k[6], &aq = k[7], &nq = k[8], &sn = k[9];
-        const c10::cuda::CUDAGuard guard(grads[0].device());
+        const Tensor &eq = k[4], &se = k[5], nq = padded(k[6]), &sn = k[7], &ft = k[8], &al = k[9], &ar = k[10];
+        const int64_t n = l.g->n_nodes, dim = nq.size(2);
+        const bool logits = needs(0) || needs(1) || needs(2), project = needs(1) || needs(2);
+
         QuantJob job = quant_job(grads[0]);
-        job.times[0] = sa;
+        job.colsum = has_bias && needs(3);
+        if (!compat) job.times[0] = se;
         if (needs(0)) job.clear = aggregation_scratch(*l.g, true, grads[0]);
+        const Tensor sdz = job.clear2 = floats({1}, grads[0]);
         const Quantized z = quantize(job);
-        Tensor d_ft, dl, dr;
-        if (needs(0)) d_ft = spmm_u_mul_e(*l.g, true, z.q, aq, z.product[0], job.clear);
-        if (needs(1) || needs(2)) {
-            const Tensor da = sddmm(*l.g, "dot", nq, z.q, sn, z.scale, {}, false).reshape({-1, l.h});
-            const Tensor dz = at::empty_like(da), sdz = zeros1(da);
-            const Direction &d = l.d();
-            check(tango_gat_edge_softmax_bwd_stats(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), ptr<int32_t>(d.edge_ids),
-                                                   row_order(d), l.n_block(), l.g->n_nodes, ptr<int8_t>(l.el.q),
-                                                   ptr<int8_t>(l.er.q), l.h, ptr<float>(l.el.scale), ptr<float>(l.er.scale),
-                                                   l.slope, ptr<float>(m), ptr<float>(inv), ptr<float>(da), ptr<float>(dz),
-                                                   ptr<float>(sdz), cuda_stream()), "gat_edge_softmax_bwd_stats");
-            count(1);
-            std::tie(dl, dr) = gat_logit_grads(l, dz, sdz, needs(1), needs(2), shape_l, shape_r);
+        Tensor d_ft, dal, dar;
+        if (needs(0)) d_ft = spmm_u_mul_e(*l.g, true, z.q, eq, compat ? k[12] : z.product[0], job.clear);
+        if (logits) {
+            const Tensor da = sddmm(*l.g, int8_weights || dim > 1 ? "dot" : "mul", nq, z.q, sn, z.scale, {}, false)
+                                  .reshape({l.g->n_edges(), l.h});
+            Tensor dz;
+            if (int8_weights) {
+                dz = at::empty_like(da);
+                const Direction &d = l.d();
+                check(tango_gat_edge_softmax_bwd_stats(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), ptr<int32_t>(d.edge_ids),
+                                                       row_order(d), l.n_block(), n, ptr<int8_t>(l.el.q), ptr<int8_t>(l.er.q),
+                                                       l.h, ptr<float>(l.el.scale), ptr<float>(l.er.scale), l.slope,
+                                                       ptr<float>(k[11]), ptr<float>(k[12]), ptr<float>(da), ptr<float>(dz),
+                                                       ptr<float>(sdz), cuda_stream()), "gat_edge_softmax_bwd_stats");
+                count(1);
+            } else {
+                dz = gat_softmax_bwd(l, k[11], da, sdz);
+            }
+            const auto [dl, dr] = gat_logit_grads(l, dz, sdz, true, true, {n, l.h}, {n, l.h});
+            if (project) { dal = at::empty_like(al); dar = at::empty_like(ar); }
+            const Matrix x = matrix(ft);
+            const int64_t bytes = project ? tango_gat_project_bwd_scratch_bytes(n, l.h, (int)dim) : 0;
+            const Tensor scratch = at::empty({std::max<int64_t>(bytes, 16)}, dl.options().dtype(at::kByte));
+            check(tango_gat_project_bwd(ptr<float>(x.t), n, l.h, (int)dim, ptr<float>(al), ptr<float>(ar), ptr<float>(dl),
+                                        ptr<float>(dr), ptr<float>(d_ft), ptr<float>(dal), ptr<float>(dar), ptr(scratch), bytes,
+                                        cuda_stream()), "gat_project_bwd");
+            count(1 + project);
         }
-        return {d_ft, dl, dr};
+        return {d_ft, needs(1) ? dal : Tensor(), needs(2) ? dar : Tensor(), z.colsum};
     }
 };
 
-Tensor gat_aggregate_fn(const GraphPtr &g, const Tensor &ft, const Tensor &el, const Tensor &er, double slope) {
-    Tensor out, m, inv, sa, aq;
+Tensor gat_layer_fn(const GraphPtr &g, const Tensor &ft_, const Tensor &al_, const Tensor &ar_, const Tensor &bias, double slope,
+                    bool int8_weights, bool compat_dn_scale) {
+    require(ft_.is_cuda() && ft_.dim() == 3 && ft_.scalar_type() == at::kFloat, "fp32 CUDA features [N, H, D] expected");
+    const int64_t n = ft_.size(0), h = ft_.size(1), dim = ft_.size(2);
+    require(n == g->n_nodes, "one feature row per node");
+    for (const Tensor *t : {&al_, &ar_, &bias})
+        require((t == &bias && !bias.defined()) || (t->is_cuda() && t->scalar_type() == at::kFloat && t->numel() == h * dim),
+                "fp32 CUDA parameters of H * D elements expected");
+    Tensor out, ft, al, ar, weights, inv, scale;
     GatLogits l;
-    Quantized nq;
+    Quantized eq, nq;
     {
         const Raw raw;
-        const c10::cuda::CUDAGuard guard(ft.device());
-        l = gat_logits(g, el, er, slope);
-        const Direction &d = l.d();
-        m = floats({g->n_nodes, l.h}, ft);
-        inv = at::empty_like(m);
-        sa = zeros1(ft);
-        check(tango_gat_edge_softmax_stats(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), row_order(d), l.n_block(),
-                                           g->n_nodes, ptr<int8_t>(l.el.q), ptr<int8_t>(l.er.q), l.h, ptr<float>(l.el.scale),
-                                           ptr<float>(l.er.scale), l.slope, ptr<float>(m), ptr<float>(inv), ptr<float>(sa),
-                                           cuda_stream()), "gat_edge_softmax_stats");
-        const int mode = settings().mode_quantize;
-        const uint64_t call = call_if(mode);
-        aq = at::empty({g->n_edges(), l.h}, ft.options().dtype(at::kChar));
-        check(tango_gat_edge_softmax_quantized(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), ptr<int32_t>(d.edge_ids),
-                                               row_order(d), l.n_block(), g->n_nodes, ptr<int8_t>(l.el.q), ptr<int8_t>(l.er.q),
-                                               l.h, ptr<float>(l.el.scale), ptr<float>(l.er.scale), l.slope, ptr<float>(m),
-                                               ptr<float>(inv), ptr<float>(sa), ptr<int8_t>(aq), mode, settings().seed, call,
-                                               settings().step, cuda_stream()), "gat_edge_softmax_quantized");
-        count(2);
-        QuantJob jn = quant_job(ft);
-        jn.times[0] = sa;
-        jn.clear = aggregation_scratch(*g, false, ft);
-        nq = quantize(jn);
-        out = spmm_u_mul_e(*g, false, nq.q, aq, nq.product[0], jn.clear);
+        const c10::cuda::CUDAGuard guard(ft_.device());
+        ft = ft_.contiguous(); al = al_.contiguous(); ar = ar_.contiguous();
+        const Tensor el = floats({n, h}, ft), er = floats({n, h}, ft), sa = floats({1}, ft);
+        check(tango_gat_project(ptr<float>(ft), n, (int)h, (int)dim, ptr<float>(al), ptr<float>(ar), ptr<float>(el),
+                                ptr<float>(er), cuda_stream()), "gat_project");
+        count(1);
+        l = gat_logits(g, el, er, slope, sa);
+        QuantJob jn;
+        if (int8_weights) {
+            const Direction &d = l.d();
+            weights = floats({n, h}, ft);
+            inv = at::empty_like(weights);
+            eq.scale = sa;
+            check(tango_gat_edge_softmax_stats(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), row_order(d), l.n_block(), n,
+                                               ptr<int8_t>(l.el.q), ptr<int8_t>(l.er.q), l.h, ptr<float>(l.el.scale),
+                                               ptr<float>(l.er.scale), l.slope, ptr<float>(weights), ptr<float>(inv),
+                                               ptr<float>(eq.scale), cuda_stream()), "gat_edge_softmax_stats");
+            const int mode = settings().mode_quantize;
+            const uint64_t call = call_if(mode);
+            eq.q = at::empty({g->n_edges(), h}, ft.options().dtype(at::kChar));
+            check(tango_gat_edge_softmax_quantized(ptr<int32_t>(d.indptr), ptr<int32_t>(d.indices), ptr<int32_t>(d.edge_ids),
+                                                   row_order(d), l.n_block(), n, ptr<int8_t>(l.el.q), ptr<int8_t>(l.er.q), l.h,
+                                                   ptr<float>(l.el.scale), ptr<float>(l.er.scale), l.slope, ptr<float>(weights),
+                                                   ptr<float>(inv), ptr<float>(eq.scale), ptr<int8_t>(eq.q), mode,
+                                                   settings().seed, call, settings().step, cuda_stream()),
+                  "gat_edge_softmax_quantized");
+            count(2);
+            jn = quant_job(ft);
+            jn.times[0] = eq.scale;
+            jn.clear = aggregation_scratch(*g, false, ft);
+            nq = quantize(jn);
+        } else {
+            weights = gat_softmax(l, sa);
+            QuantJob je = quant_job(weights, 1);
+            je.scale = sa;
+            jn = quant_job(ft);
+            jn.times_job = 0;
+            jn.clear = aggregation_scratch(*g, false, ft);
+            const auto q = quantize_all({je, jn});
+            eq = q[0]; nq = q[1];
+        }
+        scale = nq.product[0];
+        out = spmm_u_mul_e(*g, false, nq.q, eq.q, scale, jn.clear, bias.defined() ? bias.contiguous() : bias);
     }
-    if (auto node = make_node<GatAggregateBackward>(ft, el, er)) {
+    if (auto node = make_node<GatLayerBackward>(ft_, al_, ar_, bias)) {
         node->l = l; node->l.el = node->l.er = {};
-        node->shape_l = el.sizes().vec(); node->shape_r = er.sizes().vec();
+        node->int8_weights = int8_weights; node->compat = compat_dn_scale && !int8_weights; node->has_bias = bias.defined();
         torch::autograd::set_history(out, node);
-        node->keep({l.el.q, l.el.scale, l.er.q, l.er.scale, m, inv, sa, aq, nq.q, nq.scale});
+        node->keep({l.el.q, l.el.scale, l.er.q, l.er.scale, eq.q, eq.scale, nq.q, nq.scale, ft, al, ar, weights,
+                    int8_weights ? inv : scale});
     }
     return out;
 }

@@ -26,7 +26,9 @@ Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x, const Tensor &w, const Te
 std::tuple<Tensor, Tensor> edge_softmax_fn(const GraphPtr &g, const Tensor &z, double factor);
 // edge_softmax(leaky_relu(Q(el)[src] + Q(er)[dst])); (weights [E, H, 1], max|weight| / 127).
 std::tuple<Tensor, Tensor> gat_attention_fn(const GraphPtr &g, const Tensor &el, const Tensor &er, double slope);
-// the same weights applied to Q(ft), without an fp32 copy of them.
-Tensor gat_aggregate_fn(const GraphPtr &g, const Tensor &ft, const Tensor &el, const Tensor &er, double slope);
+// A whole GAT layer behind its linear projection: el = <ft, al>, er = <ft, ar> per head, the weights above, and their
+// aggregation of Q(ft) plus bias.  int8_weights: without an fp32 copy of the weights.  compat_dn_scale as in spmm_u_mul_e_fn.
+Tensor gat_layer_fn(const GraphPtr &g, const Tensor &ft, const Tensor &al, const Tensor &ar, const Tensor &bias, double slope,
+                    bool int8_weights, bool compat_dn_scale);
 
 }  // namespace tango_host

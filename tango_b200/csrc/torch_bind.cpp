@@ -123,5 +123,8 @@ PYBIND11_MODULE(_torch_ops, m) {
     });
     m.def("edge_softmax", &edge_softmax_fn);
     m.def("gat_attention", &gat_attention_fn);
-    m.def("gat_aggregate", &gat_aggregate_fn);
+    m.def("gat_layer", [](const GraphPtr &g, const Tensor &ft, const Tensor &al, const Tensor &ar, const py::object &bias,
+                          double slope, bool int8_weights, bool compat) {
+        return gat_layer_fn(g, ft, al, ar, optional(bias), slope, int8_weights, compat);
+    });
 }

@@ -289,7 +289,7 @@ Tensor spmm_copy_u(const Graph &g, bool reverse, const Quantized &nq, const Tens
 }
 
 Tensor spmm_u_mul_e(const Graph &g, bool reverse, const Tensor &nq, const Tensor &eq, const Tensor &scale,
-                    const Tensor &scratch) {
+                    const Tensor &scratch, const Tensor &bias) {
     require(nq.dim() == 3, "node features must be [N, H, D]");
     const c10::cuda::CUDAGuard guard(nq.device());
     const Direction &d = g.dir(reverse);
@@ -297,9 +297,10 @@ Tensor spmm_u_mul_e(const Graph &g, bool reverse, const Tensor &nq, const Tensor
     const Tensor e = eq.numel() ? eq.contiguous() : at::zeros({1}, nq.options());
     Tensor out = floats({d.n_rows(), nq.size(1), nq.size(2)}, scale);
     const Plan plan = make_plan(d.sched, n.cols, nq, scratch);
-    check(tango_spmm_u_mul_e(ptr<int32_t>(d.indptr), index_ptr(d.indices, d.indptr), ptr<int32_t>(d.edge_ids), d.n_rows(),
-                             ptr<int8_t>(n.t), n.ld, (int)nq.size(1), (int)nq.size(2), ptr<int8_t>(e), ptr<float>(scale),
-                             ptr<float>(out), n.cols, plan.get(d.sched), cuda_stream()), "multi_cusparse_SPMM");
+    check(tango_spmm_u_mul_e_bias(ptr<int32_t>(d.indptr), index_ptr(d.indices, d.indptr), ptr<int32_t>(d.edge_ids), d.n_rows(),
+                                  ptr<int8_t>(n.t), n.ld, (int)nq.size(1), (int)nq.size(2), ptr<int8_t>(e), ptr<float>(scale),
+                                  ptr<float>(bias), ptr<float>(out), n.cols, plan.get(d.sched), cuda_stream()),
+          "multi_cusparse_SPMM");
     count(1 + (d.sched.n_units > 0 && !plan.p.arrivals));
     return out;
 }

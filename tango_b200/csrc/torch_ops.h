@@ -136,7 +136,8 @@ Tensor spmm_scratch(const Graph &g, bool reverse, int64_t f, const Tensor &like)
 Tensor spmm_copy_u(const Graph &g, bool reverse, const Quantized &n, const Tensor &scratch, const Tensor &row_scale = {},
                    const Tensor &bias = {}, bool relu = false, const Tensor &scale_out = {});
 // `n` int8 [N, H, D], `e` int8 [E, H]; `scale` multiplies the integer sums
-Tensor spmm_u_mul_e(const Graph &g, bool reverse, const Tensor &n, const Tensor &e, const Tensor &scale, const Tensor &scratch);
+Tensor spmm_u_mul_e(const Graph &g, bool reverse, const Tensor &n, const Tensor &e, const Tensor &scale, const Tensor &scratch,
+                    const Tensor &bias = {});
 Tensor incidence_sum(const Graph &g, bool reverse, const Quantized &z, const Tensor &scratch);
 // op: "dot", "add", "sub", "mul", "div"; U and V 2-D or 3-D; `scale` (optional, holding 0) receives max|out| / 127
 Tensor sddmm(const Graph &g, const std::string &op, const Tensor &u, const Tensor &v, const Tensor &su,

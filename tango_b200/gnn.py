@@ -154,17 +154,20 @@ def _gat_attention_fused(g, el, er, slope):
     return _native.call(_native.ops.gat_attention, _native.graph(g), el, er, slope)
 
 
-def _gat_aggregate_fused(g, ft, el, er, slope):
-    """Attention + aggregation of a GAT layer with no fp32 copy of the attention weights:
+def _gat_layer_fused(g, ft, attn_l, attn_r, bias, slope, int8_weights):
+    """A GAT layer behind its linear projection as a single autograd node, from ft [N, H, D]:
 
-        out[v,h,:] = sum_e Q(a)[e,h] * Q(ft)[src(e),h,:],   a = edge_softmax(leaky_relu(Q(el)[src] + Q(er)[dst]))
+        out[v,h,:] = sum_e Q(a)[e,h] * Q(ft)[src(e),h,:] + bias,   a = edge_softmax(leaky_relu(Q(el)[src] + Q(er)[dst])),
+        el = (ft * attn_l).sum(-1),  er = (ft * attn_r).sum(-1)
 
-    Same arithmetic, bit for bit, as _gat_attention_fused followed by spmm_u_mul_e (and hence the same int8 weights
-    as the reference's sddmm_u_add_v -> LeakyReLU -> edge_softmax -> quantize chain, evaluation/test_gat.py:141-152,
-    cuda/SPMM.py:38-47), but the weights exist only as the int8 tensor the aggregation reads: one pass keeps the
-    softmax statistics of every destination (which already fix the int8 scale), a second writes the int8 weights,
-    and the backward pass recomputes the weights from the statistics."""
-    return _native.call(_native.ops.gat_aggregate, _native.graph(g), ft, el, er, slope)
+    The arithmetic of _gat_attention_fused followed by spmm_u_mul_e (evaluation/test_gat.py:127-150,
+    cuda/SPMM.py:38-47); both projections are one sweep over ft, the bias sits in the epilogue of the aggregation, and
+    their gradients take one sweep more.  int8_weights: the same int8 weights and results, but the weights exist only
+    as the int8 tensor the aggregation reads: one pass keeps the softmax statistics of every destination (which already
+    fix the int8 scale), a second writes the int8 weights, and the backward pass recomputes the weights from the
+    statistics."""
+    return _native.call(_native.ops.gat_layer, _native.graph(g), ft, attn_l, attn_r, bias, slope, int8_weights,
+                        spmm_u_mul_e.compat_dn_scale)
 
 
 class QGATConv(nn.Module):
@@ -208,20 +211,22 @@ class QGATConv(nn.Module):
         prefix = feat.shape[:-1]
         h = self.feat_drop(feat).contiguous()
         ft = self.fc(h).view(*prefix, self._num_heads, self._out_feats)
-        el = (ft * self.attn_l).sum(dim=-1).unsqueeze(-1)
-        er = (ft * self.attn_r).sum(dim=-1).unsqueeze(-1)
-        sa = None
-        # fused="int8": the attention weights never exist in fp32 (needs no attention dropout and no caller that wants
-        # the weights back); fused=True: one fused softmax pass writes them as fp32 [E, H]; fused=False: the
-        # reference's operator-by-operator chain
-        int8_path = (self._fused == "int8" and not get_attention
-                     and not (self.training and self.attn_drop.p > 0))
-        if int8_path:
-            rst = _gat_aggregate_fused(graph, ft, el, er, self._slope)
+        # The whole layer as one node where nobody needs the attention weights in between (attention dropout, a caller that
+        # wants them back): with fused="int8" they never exist in fp32.  fused=True with such a need: one fused softmax
+        # pass; fused=False: the reference's operator-by-operator chain
+        dropping = self.training and self.attn_drop.p > 0
+        bias = self.bias
+        if self._fused and not get_attention and not dropping and feat.dim() == 2:
+            inside = bias if self.res_fc is None else None       # (a residual is added before the bias)
+            rst = _gat_layer_fused(graph, ft, self.attn_l, self.attn_r, inside, self._slope, self._fused == "int8")
+            bias = None if inside is not None else bias
         else:
+            el = (ft * self.attn_l).sum(dim=-1).unsqueeze(-1)
+            er = (ft * self.attn_r).sum(dim=-1).unsqueeze(-1)
+            sa = None
             if self._fused:
                 a, sa = _gat_attention_fused(graph, el, er, self._slope)
-                if self.training and self.attn_drop.p > 0:
+                if dropping:
                     a, sa = self.attn_drop(a), None   # dropout rescales a: its absmax has to be taken again
             else:
                 e = self.leaky_relu(sddmm_u_add_v.apply(graph, el, er))
@@ -229,11 +234,11 @@ class QGATConv(nn.Module):
             rst = spmm_u_mul_e.apply(graph, ft, a, sa)
         if self.res_fc is not None:
             rst = rst + self.res_fc(h).view(*prefix, -1, self._out_feats)
-        if self.bias is not None:
-            rst = rst + self.bias.view(*((1,) * len(prefix)), self._num_heads, self._out_feats)
+        if bias is not None:
+            rst = rst + bias.view(*((1,) * len(prefix)), self._num_heads, self._out_feats)
         if self.activation:
             rst = self.activation(rst)
-        return (rst, a) if get_attention else rst      # (get_attention never takes the int8 path, so `a` exists)
+        return (rst, a) if get_attention else rst
 
 
 class GAT(nn.Module):

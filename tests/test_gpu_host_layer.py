@@ -240,3 +240,62 @@ def test_edge_softmax_of_row_lengths_around_the_trips(cuda, heads, order):
     assert (np.abs(_np(a) - want) <= 2e-5 * want + tiny).all()
     assert (np.abs(_np(zt.grad) - grad) <= 4e-5 * size + tiny).all()
     assert sa.item() == np.float32(_np(a).max()) / np.float32(127)
+
+
+@pytest.mark.parametrize("n,h,d", [(1, 1, 1), (5, 3, 5), (130, 4, 64), (1000, 8, 8), (257, 1, 41), (63, 2, 600), (3001, 4, 63)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_attention_projections(cuda, n, h, d, offset):
+    """Sums of k terms within k * 2^-24 of the sum of their magnitudes, any order; offset: only 4-byte aligned features."""
+    from tango_b200 import _lib
+    rng = np.random.default_rng(n + d)
+
+    def dev(*shape):
+        t = torch.empty(offset + int(np.prod(shape)), device="cuda")[offset:].view(shape)
+        return t.copy_(torch.from_numpy(rng.standard_normal(shape).astype(np.float32)))
+
+    x, al, ar, dl, dr, dx0 = dev(n, h, d), dev(h, d), dev(h, d), dev(n, h), dev(n, h), dev(n, h, d)
+    el, er, dx, dal, dar = torch.empty(n, h, device="cuda"), torch.empty(n, h, device="cuda"), dx0.clone(), dev(h, d), dev(h, d)
+    scratch = torch.empty(_lib.lib.tango_gat_project_bwd_scratch_bytes(n, h, d) // 4, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    p = [t.data_ptr() for t in (x, al, ar, el, er, dl, dr, dx, dal, dar, scratch)]
+    _lib.check(_lib.lib.tango_gat_project(p[0], n, h, d, p[1], p[2], p[3], p[4], stream), "project")
+    _lib.check(_lib.lib.tango_gat_project_bwd(p[0], n, h, d, p[1], p[2], p[5], p[6], p[7], p[8], p[9], p[10], scratch.numel() * 4,
+                                              stream), "project_bwd")
+    x, al, ar, dl, dr, dx0 = (_np(t).astype(np.float64) for t in (x, al, ar, dl, dr, dx0))
+    u = 2.0 ** -24
+
+    def close(got, terms, axis, k):
+        assert (np.abs(_np(got) - terms.sum(axis)) <= (k + 1) * u * np.abs(terms).sum(axis)).all()
+
+    close(el, x * al, -1, d)
+    close(er, x * ar, -1, d)
+    close(dal, dl[:, :, None] * x, 0, n)
+    close(dar, dr[:, :, None] * x, 0, n)
+    close(dx, np.stack([dx0, dl[:, :, None] * al, dr[:, :, None] * ar]), 0, 3)
+
+
+@pytest.mark.parametrize("residual,bias", [(False, True), (True, True), (False, False)])
+@pytest.mark.parametrize("heads,dim", [(1, 7), (2, 1), (4, 16), (8, 8), (3, 5)])
+def test_gat_layer_as_one_node_against_the_chain(cuda, residual, bias, heads, dim):
+    """int8 weights and fp32 weights give the same layer; the operator-by-operator chain differs by the order of fp32 sums,
+    which moves a few int8 codes by one step (1/127 of the largest value, rarely)."""
+    from tango_b200.gnn import QGATConv
+    g = _graph(600, 6000)
+    x0 = torch.randn(600, 24, device="cuda")
+    res = []
+    for fused in (True, "int8", False):
+        torch.manual_seed(1)
+        m = QGATConv(24, dim, heads, residual=residual, bias=bias, activation=F.elu, fused=fused).cuda()
+        if bias:
+            torch.nn.init.normal_(m.bias)
+        x = x0.clone().requires_grad_()
+        out = m(g, x)
+        torch.manual_seed(2)
+        out.backward(torch.randn_like(out))
+        res.append([out, x.grad] + [p.grad for p in m.parameters()])
+        for p in m.parameters():
+            p.requires_grad_(False)
+        assert not m(g, x0).requires_grad and torch.equal(m(g, x0), out)
+    for a, b, c in zip(*res):
+        scale = c.norm()
+        assert (a - b).norm() <= 1e-3 * scale and (a - c).norm() <= 1e-2 * scale
