@@ -6,7 +6,8 @@
 //   forward  Y [M,N]  = Xq[M,K]  . Wq[N,K]^T   A K-major,  B K-major
 //   dX       dX[M,K]  = dYq[M,N] . Wq[N,K]     A K-major,  B MN-major (reduction index is the row of Wq)
 //   dW       dW[N,K]  = dYq^T    . Xq[M,K]     A MN-major, B MN-major, split over the long reduction (M) with
-//                                              int32 atomics into scratch, then a small dequantising kernel.
+//                                              int32 atomics into scratch; the CTA that completes a tile dequantises
+//                                              it (callers with uncleared scratch: a small kernel does).
 // so no transposed copies of the quantized tensors are ever written.
 //
 // One persistent kernel, one CTA of 18 warps per SM: warp 0 issues TMA loads, warp 1 owns tensor memory and issues the
