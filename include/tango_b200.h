@@ -371,13 +371,10 @@ int tango_gat_edge_softmax_bwd_stats(const int32_t *indptr, const int32_t *indic
                                      const float *row_m, const float *row_inv, const float *da, float *dz,
                                      float *dz_absmax, tango_stream_t stream);
 
-/* Attention projections of a GAT layer: el[n,h] = <x[n,h,:], al[h,:]> and er with ar, x fp32 [N, H, D] contiguous
- * (evaluation/test_gat.py:127-128). */
-int tango_gat_project(const float *x, int64_t n, int h, int d, const float *al, const float *ar, float *el, float *er,
-                      tango_stream_t stream);
-
-/* Their gradients: dx[n,h,:] += dl[n,h] * al[h,:] + dr[n,h] * ar[h,:] (dx optional) and dal[h,:] = sum_n dl[n,h] *
- * x[n,h,:], dar likewise (both or neither; they need `scratch` of tango_gat_project_bwd_scratch_bytes, 4-byte aligned). */
+/* Gradients of the attention projections el[n,h] = <x[n,h,:], al[h,:]> and er with ar of a GAT layer, x fp32 [N, H, D]
+ * contiguous (evaluation/test_gat.py:127-128): dx[n,h,:] = (dx + dr[n,h] * ar[h,:]) + dl[n,h] * al[h,:] (dx optional) and
+ * dal[h,:] = sum_n dl[n,h] * x[n,h,:], dar likewise (both or neither; they need `scratch` of
+ * tango_gat_project_bwd_scratch_bytes, 4-byte aligned). */
 int64_t tango_gat_project_bwd_scratch_bytes(int64_t n, int h, int d);
 int tango_gat_project_bwd(const float *x, int64_t n, int h, int d, const float *al, const float *ar, const float *dl,
                           const float *dr, float *dx, float *dal, float *dar, void *scratch, int64_t scratch_bytes,

@@ -97,7 +97,6 @@ _SIGS = {
                                           c_uint64, c_uint64, P, P], c_int),
     "tango_gat_edge_softmax_bwd_stats": ([P, P, P, P, c_int64, c_int64, P, P, c_int, P, P, c_float, P, P, P, P, P, P],
                                          c_int),
-    "tango_gat_project": ([P, c_int64, c_int, c_int, P, P, P, P, P], c_int),
     "tango_gat_project_bwd_scratch_bytes": ([c_int64, c_int, c_int], c_int64),
     "tango_gat_project_bwd": ([P, c_int64, c_int, c_int, P, P, P, P, P, P, P, P, c_int64, P], c_int),
     "tango_quantize_push": ([P, c_int64, c_int64, c_int64, P, P, P, c_int, c_int64, c_int64, c_int, c_uint64, c_uint64,

@@ -1,29 +1,24 @@
-// The attention projections of a GAT layer and their gradients, fp32 throughout:
-//   forward : el[n,h] = <x[n,h,:], al[h,:]>,  er[n,h] = <x[n,h,:], ar[h,:]>
-//   backward: dx[n,h,:] += dl[n,h] * al[h,:] + dr[n,h] * ar[h,:],  dal[h,:] = sum_n dl[n,h] * x[n,h,:],  dar likewise
+// Gradients of the attention projections of a GAT layer, el[n,h] = <x[n,h,:], al[h,:]> and er with ar, fp32 throughout:
+//   dx[n,h,:] = (dx + dr[n,h] * ar[h,:]) + dl[n,h] * al[h,:],  dal[h,:] = sum_n dl[n,h] * x[n,h,:],  dar likewise
 //
-// Bound: HBM.  Forward reads x once (both projections take the same registers); backward reads x and dx and writes dx.
-// Operator by operator each projection is a product of the size of x and a reduction over it, and the backward pass four
-// more products, two reductions and two sums: some 24 sweeps instead of four.
+// Bound: HBM, one sweep that reads x and dx and writes dx.  Operator by operator it is four products of the size of x, two
+// reductions over them and two sums.
 #include "common.cuh"
 
 namespace tango {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kItems = 4;      // (node, head) pairs in flight per lane group
-constexpr int kRows = 4;       // rows in flight per thread of the backward kernel
+constexpr int kRows = 4;       // rows in flight per thread
 
 struct ProjArgs {
     const float *x, *al, *ar;
-    int64_t items, rows;
+    int64_t rows;
     int H, D, F;
-    float *el, *er;            // forward
-    const float *dl, *dr;      // backward
+    const float *dl, *dr;
     float *dx;
     float *part;               // [bands, 2, F]
     int64_t band;              // rows per CTA
-    int groups_log2;           // forward: log2 of the lanes per item
 };
 
 template <int VEC>
@@ -33,53 +28,6 @@ __device__ __forceinline__ void load(const float *p, float (&v)[VEC]) {
         v[0] = t.x; v[1 % VEC] = t.y; v[2 % VEC] = t.z; v[3 % VEC] = t.w;
     } else {
         v[0] = __ldg(p);
-    }
-}
-
-// 2^groups_log2 lanes share an item and reduce with a fixed butterfly.  Groups advance by a multiple of H items, so that each
-// keeps its head's weights in registers when they fit one piece per lane (SINGLE).
-template <int VEC, bool SINGLE>
-__global__ void __launch_bounds__(kThreads) project_kernel(const ProjArgs a) {
-    const int G = 1 << a.groups_log2, sub = threadIdx.x & (G - 1);
-    const int64_t groups = (int64_t)gridDim.x * (kThreads >> a.groups_log2), step = groups - groups % a.H;
-    const int64_t gid = (int64_t)blockIdx.x * (kThreads >> a.groups_log2) + (threadIdx.x >> a.groups_log2);
-    const int head = (int)(gid % a.H);
-    const float *al = a.al + (int64_t)head * a.D, *ar = a.ar + (int64_t)head * a.D;
-    float wl[VEC], wr[VEC];
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) wl[e] = wr[e] = 0.f;
-    if (SINGLE && sub * VEC < a.D) { load<VEC>(al + sub * VEC, wl); load<VEC>(ar + sub * VEC, wr); }
-    for (int64_t base = 0; base < a.items; base += step * kItems) {          // the same trips for every lane of a warp
-        float l[kItems], r[kItems];
-#pragma unroll
-        for (int k = 0; k < kItems; ++k) l[k] = r[k] = 0.f;
-        for (int c = sub * VEC; c < a.D; c += G * VEC) {
-            float v[kItems][VEC];
-#pragma unroll
-            for (int k = 0; k < kItems; ++k) {
-                const int64_t i = base + k * step + gid;
-#pragma unroll
-                for (int e = 0; e < VEC; ++e) v[k][e] = 0.f;
-                if (gid < step && i < a.items) load<VEC>(a.x + i * a.D + c, v[k]);
-            }
-            if (!SINGLE) { load<VEC>(al + c, wl); load<VEC>(ar + c, wr); }
-#pragma unroll
-            for (int k = 0; k < kItems; ++k)
-#pragma unroll
-                for (int e = 0; e < VEC; ++e) {
-                    l[k] += v[k][e] * wl[e];
-                    r[k] += v[k][e] * wr[e];
-                }
-        }
-#pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            for (int o = G >> 1; o > 0; o >>= 1) {
-                l[k] += __shfl_xor_sync(0xffffffffu, l[k], o);
-                r[k] += __shfl_xor_sync(0xffffffffu, r[k], o);
-            }
-            const int64_t i = base + k * step + gid;
-            if (sub == 0 && gid < step && i < a.items) { a.el[i] = l[k]; a.er[i] = r[k]; }
-        }
     }
 }
 
@@ -130,8 +78,8 @@ __global__ void __launch_bounds__(kThreads) project_bwd_kernel(const ProjArgs a,
                 for (int e = 0; e < VEC; ++e) {
                     sl[e] += gl[k] * v[k][e];
                     sr[e] += gr[k] * v[k][e];
+                    d[k][e] += gr[k] * wr[e];      // the order in which the operator chain's gradients of x meet
                     d[k][e] += gl[k] * wl[e];
-                    d[k][e] += gr[k] * wr[e];
                 }
                 if (a.dx) {
                     float *o = a.dx + rr * a.F + c;
@@ -201,27 +149,6 @@ bool valid(int64_t n, int h, int d) { return n >= 0 && h >= 1 && d >= 1 && (int6
 }  // namespace tango
 
 using namespace tango;
-
-extern "C" int tango_gat_project(const float *x, int64_t n, int h, int d, const float *al, const float *ar, float *el,
-                                 float *er, tango_stream_t stream) {
-    if (!valid(n, h, d)) return TANGO_EINVAL;
-    if (n == 0) return TANGO_OK;
-    if (!x || !al || !ar || !el || !er) return TANGO_EINVAL;
-    ProjArgs a{};
-    a.x = x; a.al = al; a.ar = ar; a.items = n * h; a.H = h; a.D = d; a.el = el; a.er = er;
-    const bool wide = d % 4 == 0 && aligned(x, 16) && aligned(al, 16) && aligned(ar, 16);
-    const int pieces = wide ? d / 4 : d;
-    while ((1 << a.groups_log2) < pieces && a.groups_log2 < 5) ++a.groups_log2;
-    const int64_t blocks = ceil_div(a.items, kThreads >> a.groups_log2);       // items >= H: there is a whole step
-    const unsigned nb = (unsigned)(blocks < kNumSMs * 8 ? blocks : kNumSMs * 8);
-    const bool single = pieces <= 1 << a.groups_log2;
-    if (wide && single) project_kernel<4, true><<<nb, kThreads, 0, (cudaStream_t)stream>>>(a);
-    else if (wide) project_kernel<4, false><<<nb, kThreads, 0, (cudaStream_t)stream>>>(a);
-    else if (single) project_kernel<1, true><<<nb, kThreads, 0, (cudaStream_t)stream>>>(a);
-    else project_kernel<1, false><<<nb, kThreads, 0, (cudaStream_t)stream>>>(a);
-    TANGO_LAUNCH_CHECK();
-    return TANGO_OK;
-}
 
 extern "C" int64_t tango_gat_project_bwd_scratch_bytes(int64_t n, int h, int d) {
     if (!valid(n, h, d)) return TANGO_EINVAL;

@@ -16,8 +16,14 @@
 // A destination row is owned by a thread team: a whole CTA for the rows at the head of the degree-sorted order (a
 // power-law graph has rows with 10^5 incoming edges; one warp would serialise them), a warp for the rest.  All heads
 // of an edge are handled together (one 128-bit access per edge when H == 4).  The softmax statistics are
-// accumulated "online" (running maximum with rescaling), so the forward needs two sweeps over a row, and every
-// reduction runs in a fixed order, which makes the result deterministic.
+// accumulated "online" (running maximum with rescaling), so the forward needs two sweeps over a row.
+//
+// Every sum over a row runs in ONE order that depends on the row's length alone: up to 1024 slots (rows behind
+// n_block_rows), lane l of 32 takes slots l, l + 32, ... one after the other and the lanes meet in a butterfly (16, 8, 4, 2,
+// 1); longer rows have 256 lanes, a butterfly per 32 of them, then the eight results in turn.  Narrower teams (short rows,
+// below) keep the lanes they stand in for apart and follow the same tree.  The weights are quantized to int8 behind this
+// kernel, and one ulp in the largest of them can move every code: a layer must not change with the graph around a row or
+// with the launch shape.
 #include "common.cuh"
 
 namespace tango {
@@ -173,15 +179,37 @@ __device__ __forceinline__ float team_sum(float v, float *smem) {
     return t;
 }
 
+// Takes in the logits z[0..U) one after the other: s = s * exp(m - z) + 1 at a new maximum z, else s + exp(z - m); -infinity
+// adds nothing, NaN stays in the sum.  The maxima come first, so that only a product and a sum per logit are a chain.
+template <int U>
+__device__ __forceinline__ void online_softmax(const float (&z)[U], float &m, float &s) {
+    float keep[U], e[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const bool up = z[u] > m;
+        const float d = __expf(-fabsf(z[u] - fmaxf(m, -3.402823466e+38f)));     // (a finite base: -infinity twice is no NaN)
+        keep[u] = up ? d : 1.f;
+        e[u] = up ? 1.f : d;
+        m = up ? z[u] : m;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) s = __fadd_rn(__fmul_rn(s, keep[u]), e[u]);
+}
+
+// (m, s) of two disjoint sets of logits; symmetric in them
+__device__ __forceinline__ void merge_softmax(float &m, float &s, float m2, float s2) {
+    const float mm = fmaxf(m, m2);
+    s = (m == -INFINITY ? 0.f : s * __expf(m - mm)) + (m2 == -INFINITY ? 0.f : s2 * __expf(m2 - mm));
+    m = mm;
+}
+
 // merges online-softmax states (m, s): fixed butterfly inside a warp, then warp 0..n in order
 template <int NT>
 __device__ __forceinline__ void team_softmax_merge(float &m, float &s, float *smem) {
 #pragma unroll
     for (int o = NT < 32 ? NT / 2 : 16; o > 0; o >>= 1) {
         const float m2 = __shfl_xor_sync(0xffffffffu, m, o), s2 = __shfl_xor_sync(0xffffffffu, s, o);
-        const float mm = fmaxf(m, m2);
-        s = (m == -INFINITY ? 0.f : s * __expf(m - mm)) + (m2 == -INFINITY ? 0.f : s2 * __expf(m2 - mm));
-        m = mm;
+        merge_softmax(m, s, m2, s2);
     }
     if (NT <= 32) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -189,12 +217,7 @@ __device__ __forceinline__ void team_softmax_merge(float &m, float &s, float *sm
     if (lane == 0) { smem[warp] = m; smem[32 + warp] = s; }
     __syncthreads();
     float mm = -INFINITY, ss = 0.f;
-    for (int w = 0; w < NT / 32; ++w) {
-        const float m2 = smem[w], s2 = smem[32 + w];
-        const float mx = fmaxf(mm, m2);
-        ss = (mm == -INFINITY ? 0.f : ss * __expf(mm - mx)) + (m2 == -INFINITY ? 0.f : s2 * __expf(m2 - mx));
-        mm = mx;
-    }
+    for (int w = 0; w < NT / 32; ++w) merge_softmax(mm, ss, smem[w], smem[32 + w]);
     m = mm; s = ss;
 }
 
@@ -202,7 +225,8 @@ __device__ __forceinline__ void team_softmax_merge(float &m, float &s, float *sm
 template <int NT, int HT, int U, bool PLAIN, int STAGE>
 __device__ __forceinline__ void softmax_row(const GatArgs &a, int64_t row, int beg, int end, int tid, float *smem,
                                             typename Record<HT>::T *kept, int cap, float &amax) {
-    constexpr int N = Shape<HT>::N;
+    constexpr int N = Shape<HT>::N, K = U < 4 ? U : 4;
+    static_assert(NT == 8 || NT >= 32, "eight lanes stand in for 32");
     constexpr bool kKeep = STAGE == FWD_FLOAT && !PLAIN && HT != 0 && NT >= 32;
     const float sl = PLAIN ? 0.f : __ldg(a.sl), sr = PLAIN ? 0.f : __ldg(a.sr);
     const int H = HT ? HT : a.H;
@@ -257,16 +281,28 @@ __device__ __forceinline__ void softmax_row(const GatArgs &a, int64_t row, int b
         trip_logits<NT, HT, U, PLAIN, kKeep ? SAVE : GATHER>(a, beg + tid + t * NT * U, beg, end, er, sl, z, kept, cap);
 #pragma unroll
         for (int h = 0; h < N; ++h) {
-            if (h < H) {
-                float mx = m[h];
+            if (h >= H) continue;
+            if (NT >= 32) {
+                float zh[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u) mx = fmaxf(mx, z[u][h]);
-                // nothing but -infinity so far: the sum stays 0 (a NaN, which fmaxf passes over, still reaches the sum)
-                const float base = mx == -INFINITY ? 0.f : mx;
-                float sum = s[h] * __expf(m[h] - base);
+                for (int u = 0; u < U; ++u) zh[u] = z[u][h];
+                online_softmax<U>(zh, m[h], s[h]);
+            } else {
+                // the only trip: logit u belongs to lane tid + 8 * (u % 4) of 32
+                float mk[K], sk[K];
 #pragma unroll
-                for (int u = 0; u < U; ++u) sum += __expf(z[u][h] - base);
-                s[h] = sum; m[h] = mx;
+                for (int k = 0; k < K; ++k) {
+                    float zk[U / K];
+#pragma unroll
+                    for (int i = 0; i < U / K; ++i) zk[i] = z[i * K + k][h];
+                    mk[k] = -INFINITY; sk[k] = 0.f;
+                    online_softmax<U / K>(zk, mk[k], sk[k]);
+                }
+#pragma unroll
+                for (int o = K / 2; o > 0; o >>= 1)
+#pragma unroll
+                    for (int k = 0; k < o; ++k) merge_softmax(mk[k], sk[k], mk[(k + o) % K], sk[(k + o) % K]);
+                m[h] = mk[0]; s[h] = sk[0];
             }
         }
     }
@@ -312,7 +348,7 @@ __device__ __forceinline__ void softmax_row(const GatArgs &a, int64_t row, int b
 template <int NT, int HT, int U, bool PLAIN, bool RECOMPUTE>
 __device__ __forceinline__ void softmax_bwd_row(const GatArgs &a, int64_t row, int beg, int end, int tid, float *smem,
                                                 float &amax) {
-    constexpr int N = Shape<HT>::N;
+    constexpr int N = Shape<HT>::N, K = U < 4 ? U : 4;
     const float sl = PLAIN ? 0.f : __ldg(a.sl), sr = PLAIN ? 0.f : __ldg(a.sr);
     const int H = HT ? HT : a.H;
     const int trips = (end - beg + NT * U - 1) / (NT * U);
@@ -352,10 +388,26 @@ __device__ __forceinline__ void softmax_bwd_row(const GatArgs &a, int64_t row, i
     for (int t = 0; t < trips; ++t) {
         load(t, t == trips - 1);
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int h = 0; h < N; ++h) {
+            if (h >= H) continue;
+            if (NT >= 32) {
 #pragma unroll
-            for (int h = 0; h < N; ++h)
-                if (h < H) dot[h] += p[u][h] * g[u][h];
+                for (int u = 0; u < U; ++u) dot[h] += p[u][h] * g[u][h];
+            } else {                               // the only trip, as in the forward
+                float d[K];
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    d[k] = p[k][h] * g[k][h];
+#pragma unroll
+                    for (int u = k + K; u < U; u += K) d[k] += p[u][h] * g[u][h];
+                }
+#pragma unroll
+                for (int o = K / 2; o > 0; o >>= 1)
+#pragma unroll
+                    for (int k = 0; k < o; ++k) d[k] += d[(k + o) % K];
+                dot[h] = d[0];
+            }
+        }
     }
 #pragma unroll
     for (int h = 0; h < N; ++h)

@@ -650,10 +650,9 @@ Tensor gat_layer_fn(const GraphPtr &g, const Tensor &ft_, const Tensor &al_, con
         const Raw raw;
         const c10::cuda::CUDAGuard guard(ft_.device());
         ft = ft_.contiguous(); al = al_.contiguous(); ar = ar_.contiguous();
-        const Tensor el = floats({n, h}, ft), er = floats({n, h}, ft), sa = floats({1}, ft);
-        check(tango_gat_project(ptr<float>(ft), n, (int)h, (int)dim, ptr<float>(al), ptr<float>(ar), ptr<float>(el),
-                                ptr<float>(er), cuda_stream()), "gat_project");
-        count(1);
+        // the sums of the operator chain: the codes of el and er, and with them every gradient, hang on their last bit
+        const Tensor el = at::mul(ft, al.view({1, h, dim})).sum(-1), er = at::mul(ft, ar.view({1, h, dim})).sum(-1);
+        const Tensor sa = floats({1}, ft);
         l = gat_logits(g, el, er, slope, sa);
         QuantJob jn;
         if (int8_weights) {

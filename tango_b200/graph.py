@@ -299,15 +299,9 @@ class SpmmSchedule:
         ranked = row_deg[order[self.n_skip:]]
         self.n_over_few, self.n_over_one = [self.n_skip + c for c in
                                             torch.stack([(ranked > 4).sum(), (ranked > 1).sum()]).tolist()]
-        # Rows that deserve a whole CTA in row-team kernels.  A warp's longest row is the critical path there as well, so the
-        # line follows the total work (slots / 16384) like the threshold above, between 128 and BLOCK_ROW_NNZ slots: at
-        # 114.6 M slots 256 measured 30 % slower than 1024 (fewer rows in flight), at
-        # 0.1 M slots 128 took the 8-head kernels from 56 / 43 to 28 / 13 us.
-        slots = int(indptr[-1]) if indptr.numel() else 0
-        block_row = 128
-        while block_row < BLOCK_ROW_NNZ and block_row * 16384 < slots:
-            block_row *= 2
-        self.n_block_rows = int((row_deg > block_row).sum())
+        # Rows that deserve a whole CTA in row-team kernels.  The line is the same for every graph: the order in which a row's
+        # softmax terms are added depends on it.
+        self.n_block_rows = int((row_deg > BLOCK_ROW_NNZ).sum())
         self.n_heavy = int(heavy.numel())
         self.heavy_rows = heavy.to(torch.int32)
         if self.n_heavy == 0:
