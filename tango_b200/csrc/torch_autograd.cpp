@@ -394,7 +394,14 @@ struct GcnConvBackward : SavingNode {
 
 Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x_, const Tensor &w, const Tensor &b, const Tensor &out_norm,
                    const Tensor &in_norm, bool relu, bool linear_first) {
-    require(x_.size(1) == w.size(1), "features and weight must have the same number of columns");
+    require(x_.dim() == 2 && w.dim() == 2 && x_.size(1) == w.size(1), "features and weight must have the same number of columns");
+    require(x_.size(0) == g->n_nodes, "one feature row per node expected");
+    require(out_norm.numel() == g->n_nodes && in_norm.numel() == g->n_nodes, "one norm per node expected");
+    require(!b.defined() || b.numel() == w.size(0), "one bias per output feature expected");
+    for (const Tensor *t : {&x_, &w, &out_norm, &in_norm, &b})
+        require(!t->defined() || (t->is_cuda() && t->scalar_type() == at::kFloat && t->device() == x_.device()),
+                "fp32 tensors on one CUDA device expected");
+    const Tensor bias = b.defined() ? b.detach().contiguous() : b, out_n = out_norm.contiguous(), in_n = in_norm.contiguous();
     Tensor out;
     Quantized x, wq;
     {
@@ -406,7 +413,7 @@ Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x_, const Tensor &w, const T
             const uint64_t call = call_if(mode);
             if (mode == TANGO_ROUND_STOCHASTIC) next_call();
             QuantJob jx{x_, mode, seed, call};
-            jx.row_scale = out_norm;
+            jx.row_scale = out_n;
             jx.clear = scale;
             const auto q = quantize_all({{w, mode, seed, call + 1}, jx});
             wq = q[0]; x = q[1];
@@ -414,10 +421,10 @@ Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x_, const Tensor &w, const T
             QuantJob jh = quant_job(h);
             jh.scale = scale;
             jh.clear = aggregation_scratch(*g, false, h);
-            out = spmm_copy_u(*g, false, quantize(jh), jh.clear, in_norm, b, relu);
+            out = spmm_copy_u(*g, false, quantize(jh), jh.clear, in_n, bias, relu);
         } else {
             QuantJob jx = quant_job(x_);
-            jx.row_scale = out_norm;
+            jx.row_scale = out_n;
             jx.clear = scale;
             jx.clear2 = aggregation_scratch(*g, false, x_);
             const Tensor a = spmm_copy_u(*g, false, quantize(jx), jx.clear2, {}, {}, false, scale);
@@ -427,14 +434,14 @@ Tensor gcn_conv_fn(const GraphPtr &g, const Tensor &x_, const Tensor &w, const T
             ja.scale = scale;
             const auto q = quantize_all({{w, mode, seed, call + 1}, ja});
             wq = q[0]; x = q[1];
-            out = gemm_nt(x, wq, b, {}, in_norm, relu);
+            out = gemm_nt(x, wq, bias, {}, in_n, relu);
         }
     }
     if (auto node = make_node<GcnConvBackward>(x_, w, b)) {
         node->g = g; node->first = linear_first ? First::linear : First::aggregate;
         node->relu = relu; node->has_bias = b.defined();
         torch::autograd::set_history(out, node);
-        node->keep({relu ? out : Tensor(), x.q, x.scale, wq.q, wq.scale, out_norm, in_norm}, 1);
+        node->keep({relu ? out : Tensor(), x.q, x.scale, wq.q, wq.scale, out_n, in_n}, 1);
     }
     return out;
 }

@@ -40,7 +40,7 @@ def _cached_norm(graph, which: str) -> torch.Tensor:
     return cache[which]
 
 
-def _gcn_conv_fused(graph, X, W, b, out_norm, in_norm, relu):
+def _gcn_conv_fused(graph, X, W, b, out_norm, in_norm, relu, linear_first):
     """One graph convolution (norm='both') as a single autograd node, the linear layer first where it shrinks the features,
     else the aggregation:
 
@@ -51,7 +51,7 @@ def _gcn_conv_fused(graph, X, W, b, out_norm, in_norm, relu):
     into the kernels next to them: the left norm into the absmax/quantize of X, the right norm + bias + ReLU into the
     epilogue of the aggregation or of the GEMM, and the right norm of the backward pass into the quantizer of the
     incoming gradient."""
-    return _native.call(_native.ops.gcn_conv, _native.graph(graph), X, W, b, out_norm, in_norm, relu, W.size(1) > W.size(0))
+    return _native.call(_native.ops.gcn_conv, _native.graph(graph), X, W, b, out_norm, in_norm, relu, linear_first)
 
 
 class QGraphConv(nn.Module):
@@ -78,13 +78,23 @@ class QGraphConv(nn.Module):
         if self.bias is not None:
             nn.init.zeros_(self.bias)
 
+    def _is_one_node(self, graph, feat):
+        """Whether the layer runs as one native node.  Where the aggregation comes first, what that node does not take (rows
+        or a bias that only fit by broadcasting, half-precision features that the norm promotes) stays with the operators."""
+        if not (self._fused and self._norm == "both" and self.weight is not None and feat.dim() == 2):
+            return False
+        b = self.bias
+        return self._in_feats > self._out_feats or (
+            feat.dtype == torch.float32 and feat.size(0) == graph.num_nodes()
+            and (b is None or b.dtype == torch.float32 and b.shape == (self._out_feats,)))
+
     def forward(self, graph, feat):
         if not self._allow_zero_in_degree and _has_zero_in_degree(graph):
             raise RuntimeError("There are 0-in-degree nodes in the graph; add self loops first")
-        if self._fused and self._norm == "both" and self.weight is not None and feat.dim() == 2:
+        if self._is_one_node(graph, feat):
             relu = self._activation in (F.relu, torch.relu)
             rst = _gcn_conv_fused(graph, feat, self.weight, self.bias, _cached_norm(graph, "out"),
-                                  _cached_norm(graph, "in"), relu)
+                                  _cached_norm(graph, "in"), relu, self._in_feats > self._out_feats)
             if self._activation is not None and not relu:
                 rst = self._activation(rst)
             return rst

@@ -203,6 +203,20 @@ def test_widths_that_do_not_match_are_refused(cuda):
     for feats, hidden in ((40, 8), (8, 40)):
         with pytest.raises(AssertionError):
             QGraphConv(feats, hidden).cuda()(g, torch.randn(300, feats - 1, device="cuda"))
+    # what broadcasts or promotes in a layer that aggregates first is taken by the operators, the rest refused by them
+    m = QGraphConv(8, 40).cuda()
+    x = torch.randn(300, 8, device="cuda").half()
+    assert torch.equal(m(g, x), m(g, x.float()))
+    assert torch.equal(m(g, x[:1].float()), m(g, x[:1].float().repeat(300, 1)))
+    for rows in (299, 301):
+        with pytest.raises(RuntimeError):
+            m(g, torch.randn(rows, 8, device="cuda"))
+    y = m(g, x.float())
+    m.bias = torch.nn.Parameter(torch.full((1,), 2.0, device="cuda"))
+    assert torch.equal(m(g, x.float()), y + 2)
+    m.bias = torch.nn.Parameter(torch.zeros(39, device="cuda"))
+    with pytest.raises(RuntimeError):
+        m(g, x.float())
 
 
 @pytest.mark.parametrize("heads", [1, 2, 3, 4, 5, 8])

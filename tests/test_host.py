@@ -472,3 +472,29 @@ def test_hub_self_check_accepts_a_faithful_region_and_rejects_a_lossy_one(monkey
     assert K.hub_self_check(hub, ip, idx, SpmmSchedule(ip), 2000, f=16)
     monkeypatch.setattr(K, "_csr_spmm", fake(True))
     assert not K.hub_self_check(hub, ip, idx, SpmmSchedule(ip), 2000, f=16)
+
+
+def _native_graph(n=30):
+    from tango_b200 import _native
+    return _native.ops, _native.graph(rmat_graph(n, 4 * n, 1))
+
+
+@pytest.mark.parametrize("linear_first", [False, True])
+def test_graph_convolution_refuses_sizes_that_do_not_match_before_any_launch(linear_first):
+    ops, g = _native_graph(30)
+    x, w, b, norm = torch.ones(30, 8), torch.ones(4, 8), torch.ones(4), torch.ones(30)
+
+    def refused(why, **changed):
+        a = {"x": x, "w": w, "b": b, "out": norm, "in": norm, **changed}
+        with pytest.raises(AssertionError, match=why):
+            ops.gcn_conv(g, a["x"], a["w"], a["b"], a["out"], a["in"], True, linear_first)
+
+    for rows in (29, 31):
+        refused("row per node", x=torch.ones(rows, 8))
+        refused("norm per node", out=torch.ones(rows))
+        refused("norm per node", **{"in": torch.ones(rows)})
+    refused("columns", x=torch.ones(30, 7))
+    refused("columns", x=torch.ones(30, 2, 4))
+    for n in (3, 5):
+        refused("bias", b=torch.ones(n))
+    refused("CUDA")                                   # right sizes, wrong place
