@@ -113,10 +113,19 @@ struct QLinearBackward : OnceNode {
     }
 };
 
+// The GEMM's epilogue reads the bias by its address: one contiguous fp32 value per row of w.
+static Tensor checked_bias(const Tensor &x, const Tensor &w, const Tensor &b) {
+    require(x.size(1) == w.size(1), "x and w must have the same number of columns");
+    require(!b.defined() || b.numel() == w.size(0), "one bias per row of w expected");
+    require(!b.defined() || b.scalar_type() == at::kFloat, "fp32 bias expected");
+    require(x.is_cuda() && w.device() == x.device() && (!b.defined() || b.device() == x.device()),
+            "x, w and b must be on the same GPU");
+    return b.defined() ? b.detach().contiguous() : b;
+}
+
 std::tuple<Tensor, Tensor, Tensor, Tensor> qlinear(const Tensor &x, const Tensor &w, const Tensor &b, bool want_scale,
                                                    const Tensor &xq_, const Tensor &sx_) {
-    require(x.is_cuda() && w.is_cuda() && (!b.defined() || b.is_cuda()), "x, w and b must be on the GPU");
-    require(x.size(1) == w.size(1), "x and w must have the same number of columns");
+    const Tensor bias = checked_bias(x, w, b);
     Tensor y, sy;
     Quantized xq, wq;
     {
@@ -133,7 +142,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> qlinear(const Tensor &x, const Tensor
             const auto q = quantize_all({jw, {x, mode, seed, call}});
             wq = q[0]; xq = q[1];
         }
-        y = gemm_nt(xq, wq, b, sy);
+        y = gemm_nt(xq, wq, bias, sy);
     }
     if (auto node = make_node<QLinearBackward>(x, w, b)) {
         node->x = xq; node->w = wq; node->has_bias = b.defined();
@@ -147,18 +156,16 @@ std::vector<Tensor> qlinear_group(const Tensor &x, const std::vector<Tensor> &w,
     const uint64_t seed = settings().seed;
     require(w.size() >= 1 && w.size() <= 3 && w.size() == b.size(), "one to three layers");
     require(mode != TANGO_ROUND_STOCHASTIC, "stochastic rounding draws anew for every layer");
-    std::vector<Tensor> y;
+    std::vector<Tensor> y, bias;
     std::vector<Quantized> q;
+    for (size_t k = 0; k < w.size(); ++k) bias.push_back(checked_bias(x, w[k], b[k]));
     {
         const Raw raw;
         std::vector<QuantJob> jobs;
-        for (const Tensor &t : w) {
-            require(x.is_cuda() && t.is_cuda() && x.size(1) == t.size(1), "x and w must be on the GPU and agree in columns");
-            jobs.push_back({t, mode, seed, 0});
-        }
+        for (const Tensor &t : w) jobs.push_back({t, mode, seed, 0});
         jobs.push_back({x, mode, seed, 0});
         q = quantize_all(jobs);
-        for (size_t k = 0; k < w.size(); ++k) y.push_back(gemm_nt(q.back(), q[k], b[k]));
+        for (size_t k = 0; k < w.size(); ++k) y.push_back(gemm_nt(q.back(), q[k], bias[k]));
     }
     for (size_t k = 0; k < w.size(); ++k)
         if (auto node = make_node<QLinearBackward>(x, w[k], b[k])) {

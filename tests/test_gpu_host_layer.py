@@ -197,6 +197,13 @@ def test_module_hooks_of_projections_that_share_their_input(cuda, share):
         config.share_quantized_inputs(False)
 
 
+def test_linear_layer_with_a_strided_bias(cuda):
+    import tango_b200 as T
+    x, w = torch.randn(33, 24, device="cuda"), torch.randn(16, 24, device="cuda")
+    b = torch.randn(32, device="cuda")[::2].requires_grad_()
+    assert torch.equal(T.Qlinear_func.apply(x, w, b), T.Qlinear_func.apply(x, w, b.detach().contiguous()))
+
+
 def test_widths_that_do_not_match_are_refused(cuda):
     from tango_b200.gnn import QGraphConv
     g = _graph(300, 3000)

@@ -498,3 +498,14 @@ def test_graph_convolution_refuses_sizes_that_do_not_match_before_any_launch(lin
     for n in (3, 5):
         refused("bias", b=torch.ones(n))
     refused("CUDA")                                   # right sizes, wrong place
+
+
+def test_linear_layers_refuse_a_bias_that_does_not_match_before_any_launch():
+    ops, _ = _native_graph(30)
+    x, w = torch.ones(6, 8), torch.ones(4, 8)
+    for b, why in ((torch.ones(3), "one bias"), (torch.ones(5), "one bias"), (torch.ones(4).half(), "fp32 bias"),
+                   (torch.ones(4), "GPU"), (None, "GPU")):
+        with pytest.raises(AssertionError, match=why):
+            ops.qlinear(x, w, b, False, None, None)
+        with pytest.raises(AssertionError, match=why):
+            ops.qlinear_group(x, [w], [b])
