@@ -502,6 +502,8 @@ std::tuple<Tensor, Tensor> edge_softmax_fn(const GraphPtr &g, const Tensor &z, d
 }
 
 // ------------------------------------------------------------------------------------------------ graph attention
+constexpr int64_t kMaxHeads = 8;       // of the softmax kernels
+
 // The two softmax flavours share everything but where the weights live; g, el, er as int8 [N, H] with their scales.
 struct GatLogits {
     GraphPtr g;
@@ -515,6 +517,7 @@ struct GatLogits {
 // `clear`: set to zero by the same launch.
 static GatLogits gat_logits(const GraphPtr &g, const Tensor &el, const Tensor &er, double slope, const Tensor &clear) {
     const int64_t n = el.size(0), h = el.size(1);
+    if (h < 1 || h > kMaxHeads) throw Failure("gat_attention: 1 to 8 heads");
     QuantJob jl = quant_job(el.reshape({n, h}), 1);
     const QuantJob jr = quant_job(er.reshape({n, h}), 1);
     jl.clear = clear;
@@ -651,12 +654,15 @@ struct GatLayerBackward : SavingNode {
 
 Tensor gat_layer_fn(const GraphPtr &g, const Tensor &ft_, const Tensor &al_, const Tensor &ar_, const Tensor &bias, double slope,
                     bool int8_weights, bool compat_dn_scale) {
-    require(ft_.is_cuda() && ft_.dim() == 3 && ft_.scalar_type() == at::kFloat, "fp32 CUDA features [N, H, D] expected");
+    require(ft_.dim() == 3, "features [N, H, D] expected");
     const int64_t n = ft_.size(0), h = ft_.size(1), dim = ft_.size(2);
-    require(n == g->n_nodes, "one feature row per node");
+    require(n == g->n_nodes, "one feature row per node expected");
+    if (h < 1 || h > kMaxHeads) throw Failure("gat_layer: 1 to 8 heads");      // before the first launch
     for (const Tensor *t : {&al_, &ar_, &bias})
-        require((t == &bias && !bias.defined()) || (t->is_cuda() && t->scalar_type() == at::kFloat && t->numel() == h * dim),
-                "fp32 CUDA parameters of H * D elements expected");
+        require(!t->defined() || t->numel() == h * dim, "parameters of H * D elements expected");
+    for (const Tensor *t : {&ft_, &al_, &ar_, &bias})
+        require(!t->defined() || (t->is_cuda() && t->scalar_type() == at::kFloat && t->device() == ft_.device()),
+                "fp32 tensors on one CUDA device expected");
     Tensor out, ft, al, ar, weights, inv, scale;
     GatLogits l;
     Quantized eq, nq;

@@ -226,7 +226,7 @@ class QGATConv(nn.Module):
         # pass; fused=False: the reference's operator-by-operator chain
         dropping = self.training and self.attn_drop.p > 0
         bias = self.bias
-        if self._fused and not get_attention and not dropping and feat.dim() == 2:
+        if self._fused and not get_attention and not dropping and feat.dim() == 2 and feat.size(0) == graph.num_nodes():
             inside = bias if self.res_fc is None else None       # (a residual is added before the bias)
             rst = _gat_layer_fused(graph, ft, self.attn_l, self.attn_r, inside, self._slope, self._fused == "int8")
             bias = None if inside is not None else bias

@@ -509,3 +509,17 @@ def test_linear_layers_refuse_a_bias_that_does_not_match_before_any_launch():
             ops.qlinear(x, w, b, False, None, None)
         with pytest.raises(AssertionError, match=why):
             ops.qlinear_group(x, [w], [b])
+
+
+@pytest.mark.parametrize("heads", [9, 16, 10000, 400000])
+def test_attention_layers_refuse_more_heads_than_the_softmax_takes_before_any_launch(heads):
+    from tango_b200._lib import TangoError
+    ops, g = _native_graph(30)
+    ft = torch.ones(30, heads, 1)
+    p = torch.ones(1, heads, 1)
+    for int8_weights in (False, True):
+        with pytest.raises(TangoError, match="heads"):
+            ops.gat_layer(g, ft, p, p, None, 0.2, int8_weights, False)
+    for bad, why in ((torch.ones(29, 2, 3), "row per node"), (torch.ones(31, 2, 3), "row per node"), (torch.ones(30, 2, 4), "H . D")):
+        with pytest.raises(AssertionError, match=why):
+            ops.gat_layer(g, bad, torch.ones(1, 2, 3), torch.ones(1, 2, 3), None, 0.2, False, False)
