@@ -15,14 +15,29 @@ class spmm_copy_u:
         return _native.call(_native.ops.spmm_copy_u, _native.graph(g), N, scaleN)
 
 
-class spmm_u_mul_e:
+class _WithScaleSwitch(type):
+    """The class attribute `compat_dn_scale` is kept by the host layer, whose backward pass reads it."""
+
+    @property
+    def compat_dn_scale(cls) -> bool:
+        return _native.ops.compat_dn_scale()
+
+    @compat_dn_scale.setter
+    def compat_dn_scale(cls, value) -> None:
+        _native.ops.set_compat_dn_scale(bool(value))
+
+    @compat_dn_scale.deleter
+    def compat_dn_scale(cls) -> None:
+        _native.ops.set_compat_dn_scale(False)
+
+
+class spmm_u_mul_e(metaclass=_WithScaleSwitch):
     """out[v,h,:] = sum_e E[e,h] * N[src(e),h,:] with both operands int8 (cuda/SPMM.py:36-62).
 
-    `compat_dn_scale=True` reproduces the reference's backward, which scales dN with the forward product
-    s(N)*s(E) (cuda/SPMM.py:52,56) instead of s(dZ)*s(E); the default uses the consistent scale."""
-
-    compat_dn_scale = False
+    `spmm_u_mul_e.compat_dn_scale = True` reproduces the reference's backward, which scales dN with the forward product
+    s(N)*s(E) (cuda/SPMM.py:52,56) instead of s(dZ)*s(E); the default uses the consistent scale.  What counts is its value
+    when the backward pass runs."""
 
     @staticmethod
     def apply(g, N, E, scaleE_=None):
-        return _native.call(_native.ops.spmm_u_mul_e, _native.graph(g), N, E, scaleE_, spmm_u_mul_e.compat_dn_scale)
+        return _native.call(_native.ops.spmm_u_mul_e, _native.graph(g), N, E, scaleE_)

@@ -216,10 +216,11 @@ struct SpmmUMulEBackward : OnceNode {
     std::string name() const override { return "SpmmUMulEBackward"; }
     GraphPtr g;
     Tensor nq, sn, eq, se, scale;
-    bool reduce_last = false, compat = false;
+    bool reduce_last = false;
     std::vector<int64_t> e_shape;
     variable_list backward(const variable_list &grads) override {
         if (!grads[0].defined()) return variable_list(2);
+        const bool compat = settings().compat_dn_scale;
         QuantJob job = quant_job(grads[0]);
         if (!compat) job.times[0] = se;
         if (needs(0)) job.clear = aggregation_scratch(*g, true, grads[0]);
@@ -231,7 +232,7 @@ struct SpmmUMulEBackward : OnceNode {
     }
 };
 
-Tensor spmm_u_mul_e_fn(const GraphPtr &g, const Tensor &n, const Tensor &e, const Tensor &scale_e, bool compat_dn_scale) {
+Tensor spmm_u_mul_e_fn(const GraphPtr &g, const Tensor &n, const Tensor &e, const Tensor &scale_e) {
     Tensor out, sn, se, scale;
     Quantized eq, nq;
     {
@@ -249,7 +250,6 @@ Tensor spmm_u_mul_e_fn(const GraphPtr &g, const Tensor &n, const Tensor &e, cons
     if (auto node = make_node<SpmmUMulEBackward>(n, e)) {
         node->g = g; node->nq = nq.q; node->sn = sn; node->eq = eq.q; node->se = se; node->scale = scale;
         node->reduce_last = reduces_last_dim(n, e);
-        node->compat = compat_dn_scale;
         node->e_shape = e.sizes().vec();
         torch::autograd::set_history(out, node);
     }
@@ -603,7 +603,7 @@ std::tuple<Tensor, Tensor> gat_attention_fn(const GraphPtr &g, const Tensor &el,
 struct GatLayerBackward : SavingNode {
     std::string name() const override { return "GatLayerBackward"; }
     GatLogits l;                               // without el and er, which are saved
-    bool int8_weights = false, compat = false, has_bias = false;
+    bool int8_weights = false, has_bias = false;
     variable_list backward(const variable_list &grads) override {
         const std::vector<Tensor> k = kept();
         if (!grads[0].defined()) return variable_list(4);
@@ -613,6 +613,7 @@ struct GatLayerBackward : SavingNode {
         const Tensor &eq = k[4], &se = k[5], nq = padded(k[6]), &sn = k[7], &ft = k[8], &al = k[9], &ar = k[10];
         const int64_t n = l.g->n_nodes, dim = nq.size(2);
         const bool logits = needs(0) || needs(1) || needs(2), project = needs(1) || needs(2);
+        const bool compat = !int8_weights && settings().compat_dn_scale;
 
         QuantJob job = quant_job(grads[0]);
         job.colsum = has_bias && needs(3);
@@ -653,7 +654,7 @@ struct GatLayerBackward : SavingNode {
 };
 
 Tensor gat_layer_fn(const GraphPtr &g, const Tensor &ft_, const Tensor &al_, const Tensor &ar_, const Tensor &bias, double slope,
-                    bool int8_weights, bool compat_dn_scale) {
+                    bool int8_weights) {
     require(ft_.dim() == 3, "features [N, H, D] expected");
     const int64_t n = ft_.size(0), h = ft_.size(1), dim = ft_.size(2);
     require(n == g->n_nodes, "one feature row per node expected");
@@ -713,7 +714,7 @@ Tensor gat_layer_fn(const GraphPtr &g, const Tensor &ft_, const Tensor &al_, con
     }
     if (auto node = make_node<GatLayerBackward>(ft_, al_, ar_, bias)) {
         node->l = l; node->l.el = node->l.er = {};
-        node->int8_weights = int8_weights; node->compat = compat_dn_scale && !int8_weights; node->has_bias = bias.defined();
+        node->int8_weights = int8_weights; node->has_bias = bias.defined();
         torch::autograd::set_history(out, node);
         node->keep({l.el.q, l.el.scale, l.er.q, l.er.scale, eq.q, eq.scale, nq.q, nq.scale, ft, al, ar, weights,
                     int8_weights ? inv : scale});

@@ -13,7 +13,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> qlinear(const Tensor &x, const Tensor
 std::vector<Tensor> qlinear_group(const Tensor &x, const std::vector<Tensor> &w, const std::vector<Tensor> &b);
 
 Tensor spmm_copy_u_fn(const GraphPtr &g, const Tensor &n, const Tensor &scale);
-Tensor spmm_u_mul_e_fn(const GraphPtr &g, const Tensor &n, const Tensor &e, const Tensor &scale_e, bool compat_dn_scale);
+Tensor spmm_u_mul_e_fn(const GraphPtr &g, const Tensor &n, const Tensor &e, const Tensor &scale_e);
 Tensor sddmm_u_add_v_fn(const GraphPtr &g, const Tensor &u, const Tensor &v, const Tensor &su, const Tensor &sv);
 Tensor sddmm_u_dot_v_fn(const GraphPtr &g, const Tensor &u, const Tensor &v);
 
@@ -27,8 +27,8 @@ std::tuple<Tensor, Tensor> edge_softmax_fn(const GraphPtr &g, const Tensor &z, d
 // edge_softmax(leaky_relu(Q(el)[src] + Q(er)[dst])); (weights [E, H, 1], max|weight| / 127).
 std::tuple<Tensor, Tensor> gat_attention_fn(const GraphPtr &g, const Tensor &el, const Tensor &er, double slope);
 // A whole GAT layer behind its linear projection: el = <ft, al>, er = <ft, ar> per head, the weights above, and their
-// aggregation of Q(ft) plus bias.  int8_weights: without an fp32 copy of the weights.  compat_dn_scale as in spmm_u_mul_e_fn.
+// aggregation of Q(ft) plus bias.  int8_weights: without an fp32 copy of the weights.
 Tensor gat_layer_fn(const GraphPtr &g, const Tensor &ft, const Tensor &al, const Tensor &ar, const Tensor &bias, double slope,
-                    bool int8_weights, bool compat_dn_scale);
+                    bool int8_weights);
 
 }  // namespace tango_host

@@ -83,6 +83,8 @@ PYBIND11_MODULE(_torch_ops, m) {
     m.def("set_step_counter", [](const py::object &t) {   // the Python side keeps the tensor alive
         settings().step = t.is_none() ? nullptr : reinterpret_cast<const uint64_t *>(t.cast<Tensor>().data_ptr());
     });
+    m.def("compat_dn_scale", [] { return settings().compat_dn_scale.load(); });
+    m.def("set_compat_dn_scale", [](bool on) { settings().compat_dn_scale = on; });
     m.def("next_call", [] { return next_call(); });
     m.def("set_call_counter", [](uint64_t v) { settings().calls = v; });
     m.def("launches", [] { return settings().launches.load(); });
@@ -110,8 +112,8 @@ PYBIND11_MODULE(_torch_ops, m) {
         return qlinear_group(x, w, bias);
     });
     m.def("spmm_copy_u", [](const GraphPtr &g, const Tensor &n, const py::object &s) { return spmm_copy_u_fn(g, n, optional(s)); });
-    m.def("spmm_u_mul_e", [](const GraphPtr &g, const Tensor &n, const Tensor &e, const py::object &s, bool compat) {
-        return spmm_u_mul_e_fn(g, n, e, optional(s), compat);
+    m.def("spmm_u_mul_e", [](const GraphPtr &g, const Tensor &n, const Tensor &e, const py::object &s) {
+        return spmm_u_mul_e_fn(g, n, e, optional(s));
     });
     m.def("sddmm_u_add_v", [](const GraphPtr &g, const Tensor &u, const Tensor &v, const py::object &su, const py::object &sv) {
         return sddmm_u_add_v_fn(g, u, v, optional(su), optional(sv));
@@ -124,7 +126,7 @@ PYBIND11_MODULE(_torch_ops, m) {
     m.def("edge_softmax", &edge_softmax_fn);
     m.def("gat_attention", &gat_attention_fn);
     m.def("gat_layer", [](const GraphPtr &g, const Tensor &ft, const Tensor &al, const Tensor &ar, const py::object &bias,
-                          double slope, bool int8_weights, bool compat) {
-        return gat_layer_fn(g, ft, al, ar, optional(bias), slope, int8_weights, compat);
+                          double slope, bool int8_weights) {
+        return gat_layer_fn(g, ft, al, ar, optional(bias), slope, int8_weights);
     });
 }

@@ -37,6 +37,7 @@ struct Settings {
     std::atomic<int> mode_gemm{TANGO_ROUND_TRUNC}, mode_quantize{TANGO_ROUND_NEAREST};
     std::atomic<uint64_t> seed{0};
     std::atomic<const uint64_t *> step{nullptr};
+    std::atomic<bool> compat_dn_scale{false};      // read by the backward passes
     std::atomic<uint64_t> calls{0};      // keys the stochastic-rounding stream of successive calls
     std::atomic<int64_t> launches{0};    // kernels launched so far
 };

@@ -176,8 +176,7 @@ def _gat_layer_fused(g, ft, attn_l, attn_r, bias, slope, int8_weights):
     as the int8 tensor the aggregation reads: one pass keeps the softmax statistics of every destination (which already
     fix the int8 scale), a second writes the int8 weights, and the backward pass recomputes the weights from the
     statistics."""
-    return _native.call(_native.ops.gat_layer, _native.graph(g), ft, attn_l, attn_r, bias, slope, int8_weights,
-                        spmm_u_mul_e.compat_dn_scale)
+    return _native.call(_native.ops.gat_layer, _native.graph(g), ft, attn_l, attn_r, bias, slope, int8_weights)
 
 
 class QGATConv(nn.Module):

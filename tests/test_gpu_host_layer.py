@@ -357,3 +357,33 @@ def test_edge_softmax_of_a_row_does_not_depend_on_the_rows_beside_it(cuda, heads
         for i in range(2):
             np.testing.assert_array_equal(equals[i][:k], beside[i][:k], err_msg=str(k))
             np.testing.assert_array_equal(equals[i][:k], among[i][:k], err_msg=str(k))
+
+
+def test_scale_switch_of_the_weighted_sum_is_read_in_the_backward_pass(cuda, monkeypatch):
+    """Flipped between forward and backward, dN is the integer sum times the forward scales; also inside a GAT layer."""
+    import tango_b200 as T
+    from tango_b200.gnn import QGATConv
+    g = _graph(200, 2000)
+    n0, e = torch.randn(200, 2, 8, device="cuda"), torch.rand(g.num_edges(), 2, 1, device="cuda")
+    dz = torch.randn(200, 2, 8, device="cuda") * 3
+    layer = QGATConv(24, 8, 2).cuda()
+    x0 = torch.randn(200, 24, device="cuda")
+
+    def grads(forward, backward):
+        monkeypatch.setattr(T.spmm_u_mul_e, "compat_dn_scale", forward)
+        n, x = n0.clone().requires_grad_(), x0.clone().requires_grad_()
+        out, y = T.spmm_u_mul_e.apply(g, n, e), layer(g, x)
+        monkeypatch.setattr(T.spmm_u_mul_e, "compat_dn_scale", backward)
+        out.backward(dz)
+        y.backward(dz)
+        return n.grad, x.grad
+
+    off, on = grads(False, False), grads(True, True)
+    assert not torch.equal(off[0], on[0]) and not torch.equal(off[1], on[1])
+    for forward in (False, True):
+        assert all(torch.equal(a, b) for a, b in zip(off, grads(forward, False)))
+        assert all(torch.equal(a, b) for a, b in zip(on, grads(forward, True)))
+    ratio = T.kernels.cuda_kernels.get_scale(n0) / T.kernels.cuda_kernels.get_scale(dz)
+    torch.testing.assert_close(on[0], off[0] * ratio, rtol=1e-6, atol=0)
+    monkeypatch.undo()
+    assert T.spmm_u_mul_e.compat_dn_scale is False

@@ -519,7 +519,7 @@ def test_attention_layers_refuse_more_heads_than_the_softmax_takes_before_any_la
     p = torch.ones(1, heads, 1)
     for int8_weights in (False, True):
         with pytest.raises(TangoError, match="heads"):
-            ops.gat_layer(g, ft, p, p, None, 0.2, int8_weights, False)
+            ops.gat_layer(g, ft, p, p, None, 0.2, int8_weights)
     for bad, why in ((torch.ones(29, 2, 3), "row per node"), (torch.ones(31, 2, 3), "row per node"), (torch.ones(30, 2, 4), "H . D")):
         with pytest.raises(AssertionError, match=why):
-            ops.gat_layer(g, bad, torch.ones(1, 2, 3), torch.ones(1, 2, 3), None, 0.2, False, False)
+            ops.gat_layer(g, bad, torch.ones(1, 2, 3), torch.ones(1, 2, 3), None, 0.2, False)
