@@ -16,19 +16,22 @@ class spmm_copy_u:
 
 
 class _WithScaleSwitch(type):
-    """The class attribute `compat_dn_scale` is kept by the host layer, whose backward pass reads it."""
+    """The class attribute `compat_dn_scale` is handed to the host layer, whose backward pass reads it."""
+
+    _compat_dn_scale = False
 
     @property
     def compat_dn_scale(cls) -> bool:
-        return _native.ops.compat_dn_scale()
+        return cls._compat_dn_scale
 
     @compat_dn_scale.setter
     def compat_dn_scale(cls, value) -> None:
-        _native.ops.set_compat_dn_scale(bool(value))
+        _WithScaleSwitch._compat_dn_scale = bool(value)
+        _native.setting("set_compat_dn_scale", bool(value))
 
     @compat_dn_scale.deleter
     def compat_dn_scale(cls) -> None:
-        _native.ops.set_compat_dn_scale(False)
+        cls.compat_dn_scale = False
 
 
 class spmm_u_mul_e(metaclass=_WithScaleSwitch):

@@ -1,5 +1,7 @@
 """The native host layer (lib/_torch_ops.so, from csrc/torch_*.cpp): the operators over torch tensors with autograd nodes
-in C++.  Prebuilt in-tree like the CUDA library; importing fails loudly when it is missing."""
+in C++.  Prebuilt in-tree like the CUDA library, for one version of torch with CUDA.  It is loaded when the first operator is
+called, so that graphs, partitions and settings can be used where it cannot be (a CPU build of torch); an operator there, or
+with a build that is missing or belongs to another torch, raises ImportError."""
 from __future__ import annotations
 
 import importlib.machinery
@@ -10,7 +12,7 @@ import sys
 import torch
 from torch.autograd.function import Function, once_differentiable
 
-from . import _lib
+from . import _lib, build
 
 PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "_torch_ops.so")
 
@@ -18,6 +20,9 @@ PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "_torch_o
 def _load():
     if not os.path.exists(PATH):
         raise ImportError(f"{PATH} is missing: build it first with `python tango_b200/build.py`")
+    built, here = build.built_tag(), build.host_tag()
+    if built not in ("", here):
+        raise ImportError(f"{PATH} was built for {built}, not for {here}: build it anew with `python tango_b200/build.py`")
     loader = importlib.machinery.ExtensionFileLoader("_torch_ops", PATH)
     module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_torch_ops", PATH, loader=loader))
     # the extension names its exception class by the package it belongs to, under whatever name that was imported
@@ -26,7 +31,33 @@ def _load():
     return module
 
 
-ops = _load()
+class _NotLoaded:
+    """Takes the place of the extension until something of it is asked for."""
+
+    def __getattr__(self, name):
+        return getattr(load(), name)
+
+
+ops = _NotLoaded()
+_settings = {}        # setter of the extension -> its arguments, for settings made before it is loaded
+
+
+def load():
+    """The extension; raises ImportError where it cannot be loaded."""
+    global ops
+    if isinstance(ops, _NotLoaded):
+        module = _load()
+        for name, args in _settings.items():
+            getattr(module, name)(*args)
+        ops = module
+    return ops
+
+
+def setting(name, *args) -> None:
+    """ops.<name>(*args) for a setter, now or when the extension is loaded."""
+    _settings[name] = args
+    if not isinstance(ops, _NotLoaded):
+        getattr(ops, name)(*args)
 
 
 def transformed() -> bool:

@@ -13,6 +13,7 @@ import os
 import subprocess
 import sys
 import sysconfig
+from importlib import metadata
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -25,6 +26,7 @@ LIB_PATH = os.path.join(LIB_DIR, "libtango_b200.so")
 SOURCES = ["quantize.cu", "quantize_fused.cu", "spmm.cu", "sddmm.cu", "gat_softmax.cu", "gat_project.cu", "igemm_tcgen05.cu", "peer.cu"]
 HOST_SOURCES = ["torch_ops.cpp", "torch_autograd.cpp", "torch_bind.cpp"]
 HOST_LIB_PATH = os.path.join(LIB_DIR, "_torch_ops.so")
+HOST_TAG_PATH = os.path.join(LIB_DIR, "_torch_ops.tag")     # what the host layer was built for
 # measurement aid of the benchmark, a library of its own (not part of the product ABI)
 PROBE_SRC = os.path.join(CSRC, "bench", "row_gather_probe.cu")
 PROBE_LIB_PATH = os.path.join(LIB_DIR, "libtango_bench_probe.so")
@@ -51,15 +53,34 @@ def _sources(*suffixes):
     return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(suffixes)] + [HEADER]
 
 
+def host_tag() -> str:
+    """The versions that the host layer depends on: it is compiled against torch's C++ headers for one interpreter."""
+    return f"torch {metadata.version('torch')} {sysconfig.get_config_var('SOABI')}"
+
+
+def built_tag() -> str:
+    try:
+        with open(HOST_TAG_PATH) as f:
+            return f.read().strip()
+    except OSError:
+        return ""
+
+
+def _host_outdated() -> bool:
+    return built_tag() != host_tag() or _newer(HOST_LIB_PATH, _sources(".cpp", "torch_ops.h", "torch_autograd.h"))
+
+
 def needs_build() -> bool:
-    return (_newer(LIB_PATH, _sources(".cu", ".cuh")) or _newer(PROBE_LIB_PATH, [PROBE_SRC])
-            or _newer(HOST_LIB_PATH, _sources(".cpp", "torch_ops.h", "torch_autograd.h")))
+    return _newer(LIB_PATH, _sources(".cu", ".cuh")) or _newer(PROBE_LIB_PATH, [PROBE_SRC]) or _host_outdated()
 
 
 def _build_host() -> None:
     """g++ over the torch headers (no nvcc: the host layer holds no device code)."""
     from torch.utils.cpp_extension import include_paths, library_paths
     import torch
+    if torch.version.cuda is None:
+        sys.stderr.write("the host layer is not built: this torch has no CUDA (graphs and settings work, operators do not)\n")
+        return
     flags = ["-O2", "-fPIC", "-std=c++17", "-fvisibility=hidden", "-DTORCH_API_INCLUDE_EXTENSION_H",
              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I" + os.path.dirname(HEADER),
              "-I" + os.path.join(CUDA_HOME, "include"), "-I" + sysconfig.get_paths()["include"]]
@@ -73,6 +94,8 @@ def _build_host() -> None:
     _run(link + ["-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda"], "_torch_ops.so")
     for o in objects:
         os.remove(o)
+    with open(HOST_TAG_PATH, "w") as f:
+        f.write(host_tag() + "\n")
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -89,7 +112,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(res.stderr)
     if force or _newer(PROBE_LIB_PATH, [PROBE_SRC]):
         _run(nvcc + ["-o", PROBE_LIB_PATH, PROBE_SRC], "libtango_bench_probe.so")
-    if force or _newer(HOST_LIB_PATH, _sources(".cpp", "torch_ops.h", "torch_autograd.h")):
+    if force or _host_outdated():
         _build_host()
     return LIB_PATH
 

@@ -7,7 +7,7 @@ fused forward GEMM truncates (cuda/src/iterator.h:155-164).  `reference` keeps e
 from __future__ import annotations
 
 from ._lib import ROUND_NEAREST, ROUND_STOCHASTIC, ROUND_TRUNC
-from ._native import ops as _ops
+from ._native import setting as _setting
 
 _state = {"rounding": "reference", "seed": 0, "share_quantized_inputs": False, "step_counter": None,
           "hub_block": 163840}
@@ -18,7 +18,7 @@ def set_rounding(mode: str = "reference", seed: int = 0) -> None:
         raise ValueError(mode)
     _state["rounding"] = mode
     _state["seed"] = int(seed)
-    _ops.set_rounding(mode_for("gemm_fwd"), mode_for("quantize"), int(seed) & 0xFFFFFFFFFFFFFFFF)
+    _setting("set_rounding", mode_for("gemm_fwd"), mode_for("quantize"), int(seed) & 0xFFFFFFFFFFFFFFFF)
 
 
 def get_rounding() -> str:
@@ -62,7 +62,7 @@ def set_step_counter(counter) -> None:
         import torch
         assert counter.is_cuda and counter.dtype == torch.int64 and counter.numel() == 1
     _state["step_counter"] = counter
-    _ops.set_step_counter(counter)
+    _setting("set_step_counter", counter)
 
 
 def step_counter():

@@ -83,7 +83,6 @@ PYBIND11_MODULE(_torch_ops, m) {
     m.def("set_step_counter", [](const py::object &t) {   // the Python side keeps the tensor alive
         settings().step = t.is_none() ? nullptr : reinterpret_cast<const uint64_t *>(t.cast<Tensor>().data_ptr());
     });
-    m.def("compat_dn_scale", [] { return settings().compat_dn_scale.load(); });
     m.def("set_compat_dn_scale", [](bool on) { settings().compat_dn_scale = on; });
     m.def("next_call", [] { return next_call(); });
     m.def("set_call_counter", [](uint64_t v) { settings().calls = v; });

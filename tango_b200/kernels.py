@@ -120,7 +120,7 @@ def next_call() -> int:
 
 
 def set_call_counter(v: int) -> None:
-    _native.ops.set_call_counter(int(v))
+    _native.setting("set_call_counter", int(v))
 
 
 def infer_broadcast_shape(op, ushape, vshape):

@@ -523,3 +523,66 @@ def test_attention_layers_refuse_more_heads_than_the_softmax_takes_before_any_la
     for bad, why in ((torch.ones(29, 2, 3), "row per node"), (torch.ones(31, 2, 3), "row per node"), (torch.ones(30, 2, 4), "H . D")):
         with pytest.raises(AssertionError, match=why):
             ops.gat_layer(g, bad, torch.ones(1, 2, 3), torch.ones(1, 2, 3), None, 0.2, False)
+
+
+def _fresh_python(code, tmp_path):
+    """Runs `code` in a process of its own with a copy of the package whose host layer is a file that cannot be loaded."""
+    import shutil
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    for part in ("tango_b200", "include"):
+        shutil.copytree(os.path.join(root, part), tmp_path / part, ignore=shutil.ignore_patterns("__pycache__"))
+    return subprocess.run([sys.executable, "-c", code], cwd=tmp_path, capture_output=True, text=True, timeout=300)
+
+
+@pytest.mark.parametrize("damage", ["missing", "not loadable", "another torch"])
+def test_package_without_its_host_layer_imports_and_raises_at_the_first_operator(tmp_path, damage):
+    res = _fresh_python(f"""
+import os, torch
+lib = os.path.join("tango_b200", "lib")
+if {damage!r} == "missing":
+    os.remove(os.path.join(lib, "_torch_ops.so"))
+elif {damage!r} == "not loadable":
+    open(os.path.join(lib, "_torch_ops.so"), "w").write("no library")
+else:
+    open(os.path.join(lib, "_torch_ops.tag"), "w").write("torch 1.0 cpython")
+import tango_b200 as T
+from tango_b200 import build, config
+from tango_b200.graph import rmat_graph
+assert T.__file__.startswith(os.getcwd())
+config.set_rounding("nearest", 3)
+config.set_rounding("reference")
+T.spmm_u_mul_e.compat_dn_scale = False
+g = rmat_graph(50, 200, 1)
+assert g.num_edges() >= 200
+assert build.needs_build() == ({damage!r} != "not loadable")
+for op in (lambda: T.spmm_copy_u.apply(g, torch.ones(50, 4)), lambda: T.QLinear(4, 4)(torch.ones(2, 4))):
+    try:
+        op()
+    except ImportError as e:
+        assert "_torch_ops" in str(e), e
+    else:
+        raise SystemExit("no ImportError")
+""", tmp_path)
+    assert res.returncode == 0, res.stderr
+
+
+def test_settings_made_before_the_host_layer_is_loaded_reach_it(tmp_path):
+    res = _fresh_python("""
+import tango_b200 as T
+from tango_b200 import _native, config
+config.set_rounding("stochastic", 5)
+T.spmm_u_mul_e.compat_dn_scale = True
+assert type(_native.ops).__name__ == "_NotLoaded"
+calls = []
+real = _native._load
+_native._load = lambda: type("M", (), {k: staticmethod(lambda *a, k=k: calls.append((k, a))) for k in ("set_rounding", "set_compat_dn_scale")})
+_native.load()
+assert ("set_rounding", (config.mode_for("gemm_fwd"), config.mode_for("quantize"), 5)) in calls, calls
+assert ("set_compat_dn_scale", (True,)) in calls, calls
+_native.ops = _native._NotLoaded()
+_native._load = real
+_native.load().next_call()
+""", tmp_path)
+    assert res.returncode == 0, res.stderr
