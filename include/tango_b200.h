@@ -135,6 +135,11 @@ int64_t tango_quantize_fused_scratch_bytes(const tango_quant_job *jobs, int n_jo
 int tango_quantize_fused(const tango_quant_job *jobs, int n_jobs, const uint64_t *step, void *scratch,
                          int64_t scratch_bytes, tango_stream_t stream);
 
+/* The same, bit for bit, with one ordinary launch per sweep: tango_quantize_fused does this by itself where a cooperative
+ * launch is refused (a context with fewer SMs than the device reports). */
+int tango_quantize_two_launches(const tango_quant_job *jobs, int n_jobs, const uint64_t *step, void *scratch,
+                                int64_t scratch_bytes, tango_stream_t stream);
+
 /* ---------------------------------------------------------------- int8 GEMMs (tcgen05 kind::i8) */
 
 /* Bytes of scratch tango_qgemm_dw needs for an [n, k] weight gradient. */

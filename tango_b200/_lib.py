@@ -15,6 +15,7 @@ LIB_PATH = os.environ.get("TANGO_B200_LIB") or os.path.join(_HERE, "lib", "libta
 TANGO_OK = 0
 TANGO_EALIGN = -2
 TANGO_ETIMEOUT = -4
+TANGO_ESIZE = -5
 ROUND_TRUNC, ROUND_NEAREST, ROUND_STOCHASTIC = 0, 1, 2
 OPS = {"add": 0, "sub": 1, "mul": 2, "div": 3}
 
@@ -56,6 +57,21 @@ if not os.path.exists(LIB_PATH):
 lib = ctypes.CDLL(LIB_PATH)
 
 P = c_void_p
+class QuantJob(Structure):
+    """tango_quant_job"""
+    _fields_ = [
+        ("x", c_void_p), ("rows", c_int64), ("cols", c_int64), ("ldx", c_int64),
+        ("gate", c_void_p), ("ldgate", c_int64),
+        ("row_scale", c_void_p),
+        ("scale", c_void_p), ("fixed_scale", c_int), ("times_job", c_int),
+        ("times", c_void_p * 2), ("product", c_void_p * 2),
+        ("colsum", c_void_p),
+        ("clear", c_void_p * 2), ("clear_words", c_int64 * 2),
+        ("q", c_void_p), ("ldq", c_int64),
+        ("mode", c_int), ("seed", c_uint64), ("call", c_uint64),
+    ]
+
+
 _SIGS = {
     "tango_version": ([], c_int),
     "tango_strerror": ([c_int], c_char_p),
@@ -69,6 +85,7 @@ _SIGS = {
                                   c_uint64, P, P], c_int),
     "tango_quantize_fused_scratch_bytes": ([P, c_int], c_int64),
     "tango_quantize_fused": ([P, c_int, P, P, c_int64, P], c_int),
+    "tango_quantize_two_launches": ([P, c_int, P, P, c_int64, P], c_int),
     "tango_qgemm_dw_workspace_bytes": ([c_int64, c_int64], c_int64),
     "tango_qgemm_nt": ([P, c_int64, P, c_int64, c_int64, c_int64, c_int64, P, P, P, P, c_int64, P, P, P], c_int),
     "tango_qgemm_layer": ([P, c_int64, P, c_int64, c_int64, c_int64, c_int64, P, P, P, P, c_int, P, c_int64, P, P, P, P], c_int),

@@ -64,9 +64,13 @@ struct Job {
     uint64_t seed, call;
 };
 
+// Both sweeps in one launch, or one of them.
+enum { BOTH_SWEEPS = 0, FIRST_SWEEP = 1, SECOND_SWEEP = 2 };
+
 struct Params {
     Job job[kMaxJobs];
     int n_jobs;
+    int sweeps;
     const unsigned long long *step;
 };
 
@@ -349,19 +353,24 @@ __global__ void __launch_bounds__(kThreads, MODE == TANGO_ROUND_STOCHASTIC && EX
     while (ji + 1 < p.n_jobs && (int)blockIdx.x >= p.job[ji + 1].first_block) ++ji;
     const Job &j = p.job[ji];
     const int block = blockIdx.x - j.first_block;
+    if (!STATS || p.sweeps != SECOND_SWEEP) {
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
-        for (int64_t i = (int64_t)block * kThreads + threadIdx.x; i < j.clear_words[k]; i += (int64_t)j.n_blocks * kThreads)
-            j.clear[k][i] = 0;
+        for (int k = 0; k < 2; ++k)
+            for (int64_t i = (int64_t)block * kThreads + threadIdx.x; i < j.clear_words[k]; i += (int64_t)j.n_blocks * kThreads)
+                j.clear[k][i] = 0;
+    }
     float scale;
     if (STATS) {
-        float m = 0.f;
-        if (EXT && j.colsum) m = j.vec == 4 && j.cols % 4 == 0 ? band_stats<4>(j, block, s_part) : band_stats<1>(j, block, s_part);
-        else if (!j.fixed) m = band_absmax<EXT>(j, block);
-        m = block_max(m, s_warp);
-        if (threadIdx.x == 0) j.part_max[block] = m;
-        if (gridDim.x > 1) cooperative_groups::this_grid().sync();
-        else __syncthreads();
+        if (p.sweeps != SECOND_SWEEP) {
+            float m = 0.f;
+            if (EXT && j.colsum) m = j.vec == 4 && j.cols % 4 == 0 ? band_stats<4>(j, block, s_part) : band_stats<1>(j, block, s_part);
+            else if (!j.fixed) m = band_absmax<EXT>(j, block);
+            m = block_max(m, s_warp);
+            if (threadIdx.x == 0) j.part_max[block] = m;
+            if (p.sweeps == FIRST_SWEEP) return;
+            if (gridDim.x > 1) cooperative_groups::this_grid().sync();
+            else __syncthreads();
+        }
         if (j.fixed) {
             scale = __ldg(j.scale);
         } else {
@@ -440,6 +449,16 @@ int occupancy(KernelFn fn, int variant) {
     return known[variant];
 }
 
+// SMs of the current device, asked for once per device; a B200's where there is none to ask (size queries on a host).
+int device_sms() {
+    constexpr int kDevices = 64;
+    static int known[kDevices] = {0};      // benign race: every thread stores the same value
+    int dev = -1, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return kNumSMs;
+    if (!known[dev] && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0) known[dev] = n;
+    return known[dev] ? known[dev] : kNumSMs;
+}
+
 int plan(const tango_quant_job *jobs, int n, const uint64_t *step, Launch &l) {
     if (!jobs || n < 1 || n > kMaxJobs) return TANGO_EINVAL;
     l.p = Params{};
@@ -491,7 +510,7 @@ int plan(const tango_quant_job *jobs, int n, const uint64_t *step, Launch &l) {
     l.p.n_jobs = m;
     l.fn = pick(stats, jobs[0].mode, ext);
     // enough CTAs to fill the device with four units per thread, never more than are resident at once (the barrier)
-    const int64_t resident = (int64_t)kNumSMs * occupancy(l.fn, (stats ? 6 : 0) + (ext ? 3 : 0) + jobs[0].mode);
+    const int64_t resident = (int64_t)device_sms() * occupancy(l.fn, (stats ? 6 : 0) + (ext ? 3 : 0) + jobs[0].mode);
     int64_t want = ceil_div(total, kThreads * (total < 148 * 4 * kThreads ? 2 : kSteps));
     if (stats && want > resident) want = resident;
     if (want > (1 << 20)) want = 1 << 20;
@@ -534,8 +553,8 @@ extern "C" int64_t tango_quantize_fused_scratch_bytes(const tango_quant_job *job
     return rc == TANGO_OK ? l.scratch_floats * (int64_t)sizeof(float) : rc;
 }
 
-extern "C" int tango_quantize_fused(const tango_quant_job *jobs, int n_jobs, const uint64_t *step, void *scratch,
-                                    int64_t scratch_bytes, tango_stream_t stream) {
+static int run(const tango_quant_job *jobs, int n_jobs, const uint64_t *step, void *scratch, int64_t scratch_bytes,
+               bool one_launch, cudaStream_t stream) {
     Launch l;
     const int rc = plan(jobs, n_jobs, step, l);
     if (rc) return rc;
@@ -549,9 +568,32 @@ extern "C" int tango_quantize_fused(const tango_quant_job *jobs, int n_jobs, con
         if (j.colsum) f += (int64_t)j.n_blocks * j.cols;
     }
     void *args[] = {&l.p};
-    if (l.cooperative)
-        TANGO_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)l.fn, dim3(l.blocks), dim3(kThreads), args, 0, (cudaStream_t)stream));
-    else
-        TANGO_CUDA_TRY(cudaLaunchKernel((const void *)l.fn, dim3(l.blocks), dim3(kThreads), args, 0, (cudaStream_t)stream));
+    const dim3 grid(l.blocks), block(kThreads);
+    if (!l.cooperative) {
+        TANGO_CUDA_TRY(cudaLaunchKernel((const void *)l.fn, grid, block, args, 0, stream));
+        return TANGO_OK;
+    }
+    if (one_launch) {
+        const cudaError_t e = cudaLaunchCooperativeKernel((const void *)l.fn, grid, block, args, 0, stream);
+        if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported) {
+            TANGO_CUDA_TRY(e);
+            return TANGO_OK;
+        }
+        (void)cudaGetLastError();        // fewer SMs for this process than the device has: no barrier then
+    }
+    for (int sweeps : {FIRST_SWEEP, SECOND_SWEEP}) {
+        l.p.sweeps = sweeps;
+        TANGO_CUDA_TRY(cudaLaunchKernel((const void *)l.fn, grid, block, args, 0, stream));
+    }
     return TANGO_OK;
+}
+
+extern "C" int tango_quantize_fused(const tango_quant_job *jobs, int n_jobs, const uint64_t *step, void *scratch,
+                                    int64_t scratch_bytes, tango_stream_t stream) {
+    return run(jobs, n_jobs, step, scratch, scratch_bytes, true, (cudaStream_t)stream);
+}
+
+extern "C" int tango_quantize_two_launches(const tango_quant_job *jobs, int n_jobs, const uint64_t *step, void *scratch,
+                                           int64_t scratch_bytes, tango_stream_t stream) {
+    return run(jobs, n_jobs, step, scratch, scratch_bytes, false, (cudaStream_t)stream);
 }

@@ -387,3 +387,38 @@ def test_scale_switch_of_the_weighted_sum_is_read_in_the_backward_pass(cuda, mon
     torch.testing.assert_close(on[0], off[0] * ratio, rtol=1e-6, atol=0)
     monkeypatch.undo()
     assert T.spmm_u_mul_e.compat_dn_scale is False
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 5), (300, 7), (2001, 130), (70000, 64)])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_quantizer_in_two_launches_equals_the_cooperative_one(cuda, rows, cols, mode):
+    """What a context with too few SMs for the grid barrier runs: gate, row factor, column sums, products and clears."""
+    from tango_b200 import _lib
+    ld = (cols + 15) // 16 * 16
+    x, gate, y = torch.randn(3, rows, cols, device="cuda")
+    factor = torch.rand(rows, device="cuda") + 0.5
+    res = []
+    for entry in (_lib.lib.tango_quantize_fused, _lib.lib.tango_quantize_two_launches):
+        q = torch.full((2, rows, ld), 99, dtype=torch.int8, device="cuda")
+        scales, product, colsum = torch.zeros(2, device="cuda"), torch.zeros(2, device="cuda"), torch.zeros(cols, device="cuda")
+        words = torch.full((1000,), 7, dtype=torch.int32, device="cuda")
+        jobs = (_lib.QuantJob * 2)(
+            _lib.QuantJob(x=x.data_ptr(), rows=rows, cols=cols, ldx=cols, gate=gate.data_ptr(), ldgate=cols,
+                          row_scale=factor.data_ptr(), scale=scales[0:].data_ptr(), times_job=-1, colsum=colsum.data_ptr(),
+                          clear=(words.data_ptr(), None), clear_words=(999, 0), q=q[0].data_ptr(), ldq=ld, mode=mode, seed=3, call=1),
+            _lib.QuantJob(x=y.data_ptr(), rows=rows, cols=cols, ldx=cols, scale=scales[1:].data_ptr(), times_job=0,
+                          times=(None, factor.data_ptr()), product=(product[0:].data_ptr(), product[1:].data_ptr()),
+                          q=q[1].data_ptr(), ldq=ld, mode=mode, seed=3, call=2))
+        n = _lib.lib.tango_quantize_fused_scratch_bytes(jobs, 2)
+        scratch = torch.empty(n, dtype=torch.uint8, device="cuda")
+        _lib.check(entry(jobs, 2, None, scratch.data_ptr(), n, torch.cuda.current_stream().cuda_stream), "quantize")
+        res.append((q, scales, product, colsum, words))
+    assert all(torch.equal(a, b) for a, b in zip(*res))
+    q, scales, product, colsum, words = (_np(t) for t in res[1])
+    masked = np.where(_np(gate) > 0, _np(x), np.float32(0))
+    assert scales[0] == O.absmax_scale(masked * _np(factor)[:, None]) and scales[1] == O.absmax_scale(_np(y))
+    assert product[0] == scales[1] * scales[0] and product[1] == scales[1] * _np(factor)[0]
+    assert (words == np.concatenate([np.zeros(999), [7]])).all() and (q[:, :, cols:] == 0).all()
+    assert (np.abs(colsum - masked.astype(np.float64).sum(0)) <= rows * 2.0 ** -24 * np.abs(masked).astype(np.float64).sum(0)).all()
+    if mode == 1:
+        np.testing.assert_array_equal(q[1, :, :cols], O.quantize(_np(y), scales[1]))
