@@ -129,8 +129,8 @@ typedef struct tango_quant_job {
 /* Up to four jobs of one rounding mode in one launch (a cooperative one: its CTAs meet once between the two sweeps).  Replaces the
  * get_scale + quantize pairs in front of every int8 operator (cuda/QLinear.py:29-35, cuda/SPMM.py:9-20) and, with
  * `gate` / `colsum`, the ReLU backward and bias gradient before them.  The scratch query returns a byte count or a
- * negative error code; TANGO_ESIZE: a matrix of 2^32 elements or more in a row, or about 2^33 in all (use the calls
- * above and below). */
+ * negative error code; TANGO_ESIZE: a matrix of 2^32 elements or more in a row, or about 2^33 in all, or column sums
+ * whose partial sums would take more than 64 MB of scratch (use the calls above and below). */
 int64_t tango_quantize_fused_scratch_bytes(const tango_quant_job *jobs, int n_jobs);
 int tango_quantize_fused(const tango_quant_job *jobs, int n_jobs, const uint64_t *step, void *scratch,
                          int64_t scratch_bytes, tango_stream_t stream);

@@ -459,6 +459,10 @@ int device_sms() {
     return known[dev] ? known[dev] : kNumSMs;
 }
 
+// Column sums: every CTA writes one row of them to scratch.  Beyond 2^24 floats (64 MB; rows of 28,000 columns and more where
+// the matrix fills the device) the caller sums the columns apart.
+constexpr int64_t kMaxPartSums = 1 << 24;
+
 int plan(const tango_quant_job *jobs, int n, const uint64_t *step, Launch &l) {
     if (!jobs || n < 1 || n > kMaxJobs) return TANGO_EINVAL;
     l.p = Params{};
@@ -534,6 +538,7 @@ int plan(const tango_quant_job *jobs, int n, const uint64_t *step, Launch &l) {
         j.first_block = first;
         j.n_blocks = (int)nb;
         first += (int)nb;
+        if (j.colsum && nb * (int64_t)j.cols > kMaxPartSums) return TANGO_ESIZE;
         l.scratch_floats += nb + (j.colsum ? nb * (int64_t)j.cols : 0);
     }
     l.blocks = first;

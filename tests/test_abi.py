@@ -142,3 +142,22 @@ def test_dense_hub_region_arguments_are_validated_before_any_cuda_call():
     # the quantised attention entry point rejects an unknown rounding mode outright
     assert L.tango_gat_edge_softmax_quantized(None, None, None, None, 0, 0, None, None, 4, None, None, 0.2, None, None,
                                               None, None, 7, 0, 0, None, None) == -1
+
+
+def test_scratch_of_the_fused_quantizer_is_bounded_and_bad_jobs_are_refused():
+    """The size query plans the launch; no pointer is followed."""
+    from tango_b200 import _lib
+
+    def job(rows, cols, colsum=0, **more):
+        return _lib.QuantJob(x=64, rows=rows, cols=cols, ldx=cols, scale=64, times_job=-1, colsum=colsum, q=64, ldq=cols, mode=1, **more)
+
+    def bytes_of(*jobs):
+        return _lib.lib.tango_quantize_fused_scratch_bytes((_lib.QuantJob * len(jobs))(*jobs), len(jobs))
+
+    for rows, cols in ((1, 1), (2000, 32), (131072, 1024), (232965, 602), (1000, 10000), (10, 1000000)):
+        assert 0 < bytes_of(job(rows, cols, 64)) <= 2 ** 26 + 2 ** 16, (rows, cols)
+    assert bytes_of(job(1000, 1000000, 64)) == _lib.TANGO_ESIZE          # 148 partial sums and more of a million columns
+    assert 0 < bytes_of(job(1000, 1000000)) <= 2 ** 16
+    assert bytes_of(job(1, 2 ** 32)) == _lib.TANGO_ESIZE
+    assert bytes_of(job(8, 8), job(8, 8, gate=64, ldgate=7)) == -1       # gate pitch below the width
+    assert bytes_of(job(8, 8, 64, fixed_scale=1)) == -1                  # column sums come from the sweep for the scale

@@ -41,7 +41,8 @@ def _index(g, fmt):
     return [_np(t).astype(np.int64) for t in (g.adj_csr if fmt == "csr" else g.adj_csc)]
 
 
-@pytest.mark.parametrize("m,k,n", [(2, 1, 2), (3, 5, 2), (127, 16, 33), (129, 130, 41), (1000, 602, 64), (4099, 31, 257)])
+@pytest.mark.parametrize("m,k,n", [(2, 1, 2), (3, 5, 2), (127, 16, 33), (129, 130, 41), (1000, 602, 64), (4099, 31, 257),
+                                   (700, 5, 40000)])         # too many columns for the partial sums of one launch
 @pytest.mark.parametrize("expanded", [False, True])
 def test_linear_layer_against_oracle(cuda, m, k, n, expanded):
     """Forward, dX and dW bit for bit; the bias gradient is an fp32 sum, in any order within m * 2^-24 * sum|dY|."""
@@ -387,6 +388,27 @@ def test_scale_switch_of_the_weighted_sum_is_read_in_the_backward_pass(cuda, mon
     torch.testing.assert_close(on[0], off[0] * ratio, rtol=1e-6, atol=0)
     monkeypatch.undo()
     assert T.spmm_u_mul_e.compat_dn_scale is False
+
+
+def test_wide_layer_behind_relu_sums_its_columns_apart(cuda):
+    """40,000 outputs: gate, column sums and quantisation of the gradient are separate kernels; same layer as the operators."""
+    from tango_b200.gnn import QGraphConv
+    g = _graph(700, 4000)
+    x0 = torch.randn(700, 8, device="cuda")
+    res = []
+    for fused in (True, False):
+        torch.manual_seed(1)
+        m = QGraphConv(8, 40000, activation=F.relu, fused=fused).cuda()
+        torch.nn.init.normal_(m.bias)
+        x = x0.clone().requires_grad_()
+        out = m(g, x)
+        torch.manual_seed(2)
+        dy = torch.randn_like(out)
+        out.backward(dy)
+        res.append((out, x.grad, m.weight.grad))
+        d64 = torch.where(out > 0, dy, 0).double()
+        assert ((m.bias.grad - d64.sum(0)).abs() <= 700 * 2.0 ** -24 * d64.abs().sum(0)).all()
+    assert all(torch.equal(a, b) for a, b in zip(*res))
 
 
 @pytest.mark.parametrize("rows,cols", [(1, 5), (300, 7), (2001, 130), (70000, 64)])
