@@ -25,7 +25,7 @@ Matrix matrix(const Tensor &t) {
         return {c, 1, n, std::max<int64_t>(n, 1)};
     }
     const int64_t rows = t.size(0), cols = rows ? t.numel() / rows : 0;
-    if (t.is_contiguous()) return {t, rows, cols, std::max<int64_t>(cols, 1)};
+    // the row stride comes first: a single row of a padded tensor counts as contiguous, but its pitch is the padded one
     if (rows > 0 && t.stride(0) >= cols) {
         int64_t want = 1;
         bool packed = true;
@@ -33,8 +33,9 @@ Matrix matrix(const Tensor &t) {
             packed = t.size(d) == 1 || t.stride(d) == want;
             want *= t.size(d);
         }
-        if (packed) return {t, rows, cols, t.stride(0)};
+        if (packed) return {t, rows, cols, std::max<int64_t>(t.stride(0), 1)};
     }
+    if (t.is_contiguous()) return {t, rows, cols, std::max<int64_t>(cols, 1)};
     return {t.contiguous(), rows, cols, std::max<int64_t>(cols, 1)};
 }
 

@@ -61,10 +61,11 @@ def _matrix(t: torch.Tensor):
     if t.dim() <= 1:
         t = t.contiguous()
         return t, 1, t.numel(), max(t.numel(), 1)
+    # the row stride comes first: a single row of a padded tensor counts as contiguous, but its pitch is the padded one
+    if rows > 0 and t[0].is_contiguous() and t.stride(0) >= cols:
+        return t, rows, cols, max(t.stride(0), 1)
     if t.is_contiguous():
         return t, rows, cols, max(cols, 1)
-    if rows > 0 and t[0].is_contiguous() and t.stride(0) >= cols:
-        return t, rows, cols, t.stride(0)
     t = t.contiguous()
     return t, rows, cols, max(cols, 1)
 

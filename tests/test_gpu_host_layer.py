@@ -41,7 +41,7 @@ def _index(g, fmt):
     return [_np(t).astype(np.int64) for t in (g.adj_csr if fmt == "csr" else g.adj_csc)]
 
 
-@pytest.mark.parametrize("m,k,n", [(2, 1, 2), (3, 5, 2), (127, 16, 33), (129, 130, 41), (1000, 602, 64), (4099, 31, 257),
+@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (1, 5, 1), (1, 100, 32), (7, 100, 1), (1, 33, 20), (2, 1, 2), (3, 5, 2), (127, 16, 33), (129, 130, 41), (1000, 602, 64), (4099, 31, 257),
                                    (700, 5, 40000)])         # too many columns for the partial sums of one launch
 @pytest.mark.parametrize("expanded", [False, True])
 def test_linear_layer_against_oracle(cuda, m, k, n, expanded):
@@ -64,6 +64,25 @@ def test_linear_layer_against_oracle(cuda, m, k, n, expanded):
     np.testing.assert_array_equal(_np(layer.weight.grad), O.qgemm_backward_dw(dyq, xq, sdy, sx))
     d64 = dy.astype(np.float64)
     assert (np.abs(_np(layer.bias.grad) - d64.sum(0)) <= m * 2.0 ** -24 * np.abs(d64).sum(0)).all()
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 100, 32), (7, 100, 1), (1, 5, 1)])
+def test_reference_gemm_calls_with_one_row(cuda, m, k, n):
+    """The one-row operands of the kernel module's own calls: a padded pitch, although the tensor counts as contiguous."""
+    from tango_b200 import kernels as K
+    rng = np.random.default_rng(m + n)
+    x, w, dy = (rng.standard_normal(s).astype(np.float32) for s in ((m, k), (n, k), (m, n)))
+    xt, wt = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    sx, sw = K.cuda_kernels.get_scale(xt), K.cuda_kernels.get_scale(wt)
+    xq, wq = K.alloc_int8(xt.shape, xt.device), K.alloc_int8(wt.shape, wt.device)
+    y = K.QGEMM_forward(xt, xq, sx, wt, wq, sw, None, False)
+    ry, rxq, rwq, rsx, rsw, *_ = O.qgemm_forward(x, w)
+    np.testing.assert_array_equal(_np(y), ry)
+    dyq, sdy = K.quantize(torch.from_numpy(dy).cuda())
+    dx, dw = K.QGEMM_backward(dyq, xq, wq, sdy, sx, sw)
+    rdyq = O.quantize(dy, O.absmax_scale(dy))
+    np.testing.assert_array_equal(_np(dx), O.qgemm_backward_dx(rdyq, rwq, sdy.item(), rsw))
+    np.testing.assert_array_equal(_np(dw), O.qgemm_backward_dw(rdyq, rxq, sdy.item(), rsx))
 
 
 @pytest.mark.parametrize("f", [1, 4, 16, 17, 41, 64, 128, 130, 513, 602])
