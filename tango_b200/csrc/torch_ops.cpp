@@ -85,9 +85,10 @@ QuantJob quant_job(const Tensor &t, int64_t align) {
     return j;
 }
 
-// A matrix too large for the fused kernel's 32-bit indices: scale, then quantize, then column sums, one after the other.
+// A matrix too large for the fused kernel (32-bit indices, scratch of column sums): scale, then quantize, then column sums, one after the other.
 static void quantize_large(const QuantJob &j, const tango_quant_job &c, Quantized &o) {
     if (c.gate) {
+        require(!c.fixed_scale, "a gated matrix of this size finds its own scale");
         const int64_t bytes = tango_relu_grad_stats_scratch_bytes(c.rows, c.cols);
         const Tensor scratch = at::empty({std::max<int64_t>(bytes, 16)}, j.t.options().dtype(at::kByte));
         check(tango_relu_grad_stats(c.x, c.ldx, c.gate, c.ldgate, c.rows, c.cols, c.row_scale, c.scale, c.colsum, ptr(scratch),
@@ -142,6 +143,7 @@ std::vector<Quantized> quantize_all(const std::vector<QuantJob> &jobs) {
         c[k].mode = j.mode; c[k].seed = j.seed; c[k].call = j.call;
     }
     const int64_t bytes = tango_quantize_fused_scratch_bytes(c, (int)n);
+    if (bytes < 0 && bytes != TANGO_ESIZE) check((int)bytes, "quantize");
     if (bytes < 0) {
         for (size_t k = 0; k < n; ++k) {
             for (const Tensor &t : {jobs[k].clear, jobs[k].clear2})

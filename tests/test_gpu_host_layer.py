@@ -463,3 +463,18 @@ def test_quantizer_in_two_launches_equals_the_cooperative_one(cuda, rows, cols, 
     assert (np.abs(colsum - masked.astype(np.float64).sum(0)) <= rows * 2.0 ** -24 * np.abs(masked).astype(np.float64).sum(0)).all()
     if mode == 1:
         np.testing.assert_array_equal(q[1, :, :cols], O.quantize(_np(y), scales[1]))
+
+
+def test_vector_beyond_the_indices_of_the_fused_quantizer(cuda):
+    """2^32 + 8 elements (17 GB): scale and codes as the fused kernel gives them piece by piece."""
+    from tango_b200 import kernels as K
+    n, step = 2 ** 32 + 8, 2 ** 28
+    x = torch.empty(n, device="cuda")
+    for i in range(0, n, step):
+        x[i:i + step].normal_()
+    x[-1] = -40.0
+    q, s = K.quantize(x)
+    assert s.item() == np.float32(40) / np.float32(127)
+    for i in range(0, n, step):
+        assert torch.equal(q[i:i + step], K.quantize(x[i:i + step], s)[0])
+
