@@ -101,6 +101,16 @@ class Graph:
         self._identity = {}   # fmt -> True when slot k of that format holds edge k (edge ids follow the format's order)
         self.n_classes = None
 
+    def __setstate__(self, state):
+        """Row schedules that came out of a file of an earlier layout are made anew from the indices beside them."""
+        self.__dict__.update(state)
+        for fmt, sched in self._plans.items():
+            if getattr(sched, "layout", 0) != SpmmSchedule.LAYOUT:
+                self._plans[fmt] = SpmmSchedule((self.adj_csr if fmt == "csr" else self.adj_csc)[0])
+        for hub in getattr(self, "_hubs", {}).values():
+            if getattr(hub.schedule, "layout", 0) != SpmmSchedule.LAYOUT:
+                hub.make_schedule()
+
     # ---- DGL-like surface used by the operators and the layers
     @property
     def device(self):
@@ -249,6 +259,8 @@ class SpmmSchedule:
     rows of a dense hub block, in the block's row order); they come first in `heavy_rows`, every heavy row comes
     first in `row_order`, and `n_skip` = n_heavy tells the row kernels to start after them."""
 
+    LAYOUT = 3      # counts up when the fields or their meaning change: see Graph.__setstate__
+
     def __init__(self, indptr: torch.Tensor, nseg: int = 1, threshold: Optional[int] = None,
                  unit: Optional[int] = None, force_heavy: Optional[torch.Tensor] = None):
         if threshold is None:
@@ -262,6 +274,7 @@ class SpmmSchedule:
                 threshold *= 2
         if unit is None:
             unit = max(128, threshold // 2)
+        self.layout = self.LAYOUT
         self.nseg = nseg
         self.threshold = threshold
         self.unit = unit
@@ -415,9 +428,12 @@ class HubBlock:
         self.indptr = tip.to(torch.int32)
         self.rows = rows[:ntr * T].to(torch.int32)
         self.cols = cols[:ks].to(torch.int32).contiguous()
-        self.schedule = SpmmSchedule(self.indptr, force_heavy=rows[:ntr * T])
-        self.schedule.hub = self
+        self.make_schedule()
         self.ok = True
+
+    def make_schedule(self):
+        self.schedule = SpmmSchedule(self.indptr, force_heavy=self.rows)
+        self.schedule.hub = self
 
     def to_dense(self) -> torch.Tensor:
         """The region as an ordinary [rows, cols] int32 matrix (zero outside the staircase); for tests."""

@@ -1,5 +1,6 @@
 """Host-side logic that needs no GPU: graph generator and index bundles, long-row schedules, row partitions, shape
 helpers, rounding-mode switch, and the 2-rank all-gather path over gloo."""
+import copy
 import os
 import socket
 
@@ -586,3 +587,32 @@ _native._load = real
 _native.load().next_call()
 """, tmp_path)
     assert res.returncode == 0, res.stderr
+
+
+def test_graph_from_a_file_of_an_earlier_layout_gets_new_schedules():
+    """Fields that a schedule gained since, and the rows that deserve a CTA, whose line has moved."""
+    import io
+    from tango_b200 import _native
+    g = rmat_graph(400, 12000, 3)
+    for fmt in ("csc", "csr"):
+        g._plans[fmt] = SpmmSchedule((g.adj_csr if fmt == "csr" else g.adj_csc)[0])
+    hub = HubBlock(*g.adj_csc[:2], 400, min_density=0.0)
+    g._hubs = {"csc": hub}
+    want = copy.deepcopy(g)
+    for sched in (*g._plans.values(), hub.schedule):
+        for name in ("layout", "unit", "row_info", "n_over_few", "n_over_one"):
+            delattr(sched, name)
+        sched.n_block_rows = 17
+    f = io.BytesIO()
+    torch.save(g, f)
+    f.seek(0)
+    got = torch.load(f, weights_only=False)
+    for a, b in ((got._plans["csc"], want._plans["csc"]), (got._plans["csr"], want._plans["csr"]),
+                 (got._hubs["csc"].schedule, want._hubs["csc"].schedule)):
+        assert set(vars(a)) == set(vars(b))
+        for name, v in vars(b).items():
+            if name != "hub":
+                assert torch.equal(getattr(a, name), v) if isinstance(v, torch.Tensor) else getattr(a, name) == v, name
+    assert got._hubs["csc"].schedule.hub is got._hubs["csc"]
+    _native.graph(got)
+    assert copy.deepcopy(got)._plans["csc"].row_info.data_ptr() != got._plans["csc"].row_info.data_ptr()
