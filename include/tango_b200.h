@@ -100,7 +100,7 @@ int tango_quantize_relu_grad(const float *g, int64_t ldg, const float *y, int64_
                              uint64_t seed, uint64_t call, const uint64_t *step, tango_stream_t stream);
 
 /* One matrix of a fused absmax + quantise launch (host struct, read before the call returns): with
- * m[r,c] = (gate ? (gate[r,c] > 0 ? x[r,c] : 0) : x[r,c]),
+ * m[r,c] = (gate ? (gate[r,c] <= 0 ? 0 : x[r,c]) : x[r,c])  (a NaN in the gate lets x pass, as in PyTorch's ReLU gradient),
  *   scale[0]  = max |m[r,c] * row_scale[r]| / 127            (fixed_scale: scale[0] is given instead)
  *   q[r,c]    = round_mode(m[r,c] * row_scale[r] / scale[0])  (columns [cols, ldq) are zero; stream as in tango_quantize)
  *   colsum[c] = sum_r m[r,c], added in a fixed order          (optional, not with fixed_scale)

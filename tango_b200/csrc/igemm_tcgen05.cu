@@ -220,7 +220,7 @@ __device__ __forceinline__ void store_chunk(const GemmParams &p, uint32_t (&r)[3
         }
         if (p.relu) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(fmaxf(__uint_as_float(r[i]), 0.f));
+            for (int i = 0; i < 32; ++i) r[i] = __uint_as_float(r[i]) <= 0.f ? 0u : r[i];      // NaN passes
         }
         if (p.absmax) {
             float m = 0.f;

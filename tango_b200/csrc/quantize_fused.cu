@@ -98,7 +98,7 @@ __device__ __forceinline__ float4 load4(const float *p, int left) {
 }
 
 __device__ __forceinline__ float4 gated(const float4 &v, const float4 &g) {
-    return make_float4(g.x > 0.f ? v.x : 0.f, g.y > 0.f ? v.y : 0.f, g.z > 0.f ? v.z : 0.f, g.w > 0.f ? v.w : 0.f);
+    return make_float4(g.x <= 0.f ? 0.f : v.x, g.y <= 0.f ? 0.f : v.y, g.z <= 0.f ? 0.f : v.z, g.w <= 0.f ? 0.f : v.w);
 }
 __device__ __forceinline__ float4 scaled(const float4 &v, float s) {
     return make_float4(__fmul_rn(v.x, s), __fmul_rn(v.y, s), __fmul_rn(v.z, s), __fmul_rn(v.w, s));
@@ -194,7 +194,7 @@ __device__ __forceinline__ float band_stats(const Job &j, int block, float *s_pa
                         v[k][0] = t.x; v[k][VW > 1 ? 1 : 0] = t.y; v[k][VW > 2 ? 2 : 0] = t.z; v[k][VW > 3 ? 3 : 0] = t.w;
                     } else {
                         v[k][0] = in ? __ldg(x + rr * ldx + c) : 0.f;
-                        if (in && gate && !(__ldg(gate + rr * ldgate + c) > 0.f)) v[k][0] = 0.f;
+                        if (in && gate && __ldg(gate + rr * ldgate + c) <= 0.f) v[k][0] = 0.f;
                     }
                     if (in && row_scale) s[k] = fabsf(__ldg(row_scale + rr));
                 }

@@ -478,3 +478,24 @@ def test_vector_beyond_the_indices_of_the_fused_quantizer(cuda):
     for i in range(0, n, step):
         assert torch.equal(q[i:i + step], K.quantize(x[i:i + step], s)[0])
 
+
+
+@pytest.mark.parametrize("out", [40, 41])
+def test_infinities_and_nan_go_through_a_convolution_as_through_the_operators(cuda, out):
+    """An infinite feature gives infinite scales and NaN sums; ReLU keeps a NaN and lets its gradient pass."""
+    from tango_b200.gnn import QGraphConv
+    g = _graph(200, 1000)
+    x0 = torch.randn(200, 8, device="cuda")
+    x0[3, 2] = float("inf")
+    res = []
+    for fused in (True, False):
+        torch.manual_seed(1)
+        m = QGraphConv(8, out, activation=F.relu, fused=fused).cuda()
+        x = x0.clone().requires_grad_()
+        y = m(g, x)
+        torch.manual_seed(2)
+        y.backward(torch.randn_like(y))
+        res.append((y, x.grad, m.weight.grad, m.bias.grad))
+    assert res[0][0].isnan().any()
+    for a, b in zip(*res):
+        torch.testing.assert_close(a, b, rtol=0, atol=0 if a is not res[0][3] else 1e-4, equal_nan=True)
