@@ -64,13 +64,12 @@ struct Job {
     uint64_t seed, call;
 };
 
-// Both sweeps in one launch, or one of them.
+// The sweeps of a launch.
 enum { BOTH_SWEEPS = 0, FIRST_SWEEP = 1, SECOND_SWEEP = 2 };
 
 struct Params {
     Job job[kMaxJobs];
     int n_jobs;
-    int sweeps;
     const unsigned long long *step;
 };
 
@@ -345,7 +344,8 @@ __device__ __forceinline__ void quantize_band(const Job &j, uint32_t beg, uint32
 }
 
 // EXT: jobs with a gate or column sums take part; STATS: false when every scale is given (no barrier, ordinary launch).
-template <bool STATS, int MODE, bool EXT>
+// SWEEPS is a template parameter because a test of it at run time cost the EXT forms registers (1 % of a launch).
+template <bool STATS, int MODE, bool EXT, int SWEEPS>
 __global__ void __launch_bounds__(kThreads, MODE == TANGO_ROUND_STOCHASTIC && EXT ? 3 : MODE == TANGO_ROUND_STOCHASTIC || EXT ? 4 : 5) quantize_fused_kernel(const __grid_constant__ Params p) {
     __shared__ float s_part[EXT && STATS ? kThreads * 4 : 1];
     __shared__ float s_warp[kThreads / 32];
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, MODE == TANGO_ROUND_STOCHASTIC && EX
     while (ji + 1 < p.n_jobs && (int)blockIdx.x >= p.job[ji + 1].first_block) ++ji;
     const Job &j = p.job[ji];
     const int block = blockIdx.x - j.first_block;
-    if (!STATS || p.sweeps != SECOND_SWEEP) {
+    if (SWEEPS != SECOND_SWEEP) {
 #pragma unroll
         for (int k = 0; k < 2; ++k)
             for (int64_t i = (int64_t)block * kThreads + threadIdx.x; i < j.clear_words[k]; i += (int64_t)j.n_blocks * kThreads)
@@ -361,13 +361,13 @@ __global__ void __launch_bounds__(kThreads, MODE == TANGO_ROUND_STOCHASTIC && EX
     }
     float scale;
     if (STATS) {
-        if (p.sweeps != SECOND_SWEEP) {
+        if (SWEEPS != SECOND_SWEEP) {
             float m = 0.f;
             if (EXT && j.colsum) m = j.vec == 4 && j.cols % 4 == 0 ? band_stats<4>(j, block, s_part) : band_stats<1>(j, block, s_part);
             else if (!j.fixed) m = band_absmax<EXT>(j, block);
             m = block_max(m, s_warp);
             if (threadIdx.x == 0) j.part_max[block] = m;
-            if (p.sweeps == FIRST_SWEEP) return;
+            if (SWEEPS == FIRST_SWEEP) return;
             if (gridDim.x > 1) cooperative_groups::this_grid().sync();
             else __syncthreads();
         }
@@ -423,19 +423,21 @@ struct Launch {
     Params p;
     KernelFn fn;
     int blocks;
-    bool cooperative;
+    bool cooperative, ext;
     int64_t scratch_floats;
 };
 
-template <bool STATS, bool EXT>
+template <bool STATS, bool EXT, int SWEEPS>
 KernelFn pick_mode(int mode) {
-    return mode == TANGO_ROUND_STOCHASTIC ? quantize_fused_kernel<STATS, TANGO_ROUND_STOCHASTIC, EXT>
-         : mode == TANGO_ROUND_NEAREST    ? quantize_fused_kernel<STATS, TANGO_ROUND_NEAREST, EXT>
-                                          : quantize_fused_kernel<STATS, TANGO_ROUND_TRUNC, EXT>;
+    return mode == TANGO_ROUND_STOCHASTIC ? quantize_fused_kernel<STATS, TANGO_ROUND_STOCHASTIC, EXT, SWEEPS>
+         : mode == TANGO_ROUND_NEAREST    ? quantize_fused_kernel<STATS, TANGO_ROUND_NEAREST, EXT, SWEEPS>
+                                          : quantize_fused_kernel<STATS, TANGO_ROUND_TRUNC, EXT, SWEEPS>;
 }
+template <int SWEEPS>
 KernelFn pick(bool stats, int mode, bool ext) {
-    return stats ? (ext ? pick_mode<true, true>(mode) : pick_mode<true, false>(mode))
-                 : (ext ? pick_mode<false, true>(mode) : pick_mode<false, false>(mode));
+    if constexpr (SWEEPS != BOTH_SWEEPS) return ext ? pick_mode<true, true, SWEEPS>(mode) : pick_mode<true, false, SWEEPS>(mode);
+    return stats ? (ext ? pick_mode<true, true, BOTH_SWEEPS>(mode) : pick_mode<true, false, BOTH_SWEEPS>(mode))
+                 : (ext ? pick_mode<false, true, BOTH_SWEEPS>(mode) : pick_mode<false, false, BOTH_SWEEPS>(mode));
 }
 
 // Resident CTAs per SM of a variant; the same on every B200, so one query per variant and process.
@@ -512,7 +514,8 @@ int plan(const tango_quant_job *jobs, int n, const uint64_t *step, Launch &l) {
         l.p.job[m++] = j;
     }
     l.p.n_jobs = m;
-    l.fn = pick(stats, jobs[0].mode, ext);
+    l.fn = pick<BOTH_SWEEPS>(stats, jobs[0].mode, ext);
+    l.ext = ext;
     // enough CTAs to fill the device with four units per thread, never more than are resident at once (the barrier)
     const int64_t resident = (int64_t)device_sms() * occupancy(l.fn, (stats ? 6 : 0) + (ext ? 3 : 0) + jobs[0].mode);
     int64_t want = ceil_div(total, kThreads * (total < 148 * 4 * kThreads ? 2 : kSteps));
@@ -586,10 +589,8 @@ static int run(const tango_quant_job *jobs, int n_jobs, const uint64_t *step, vo
         }
         (void)cudaGetLastError();        // fewer SMs for this process than the device has: no barrier then
     }
-    for (int sweeps : {FIRST_SWEEP, SECOND_SWEEP}) {
-        l.p.sweeps = sweeps;
-        TANGO_CUDA_TRY(cudaLaunchKernel((const void *)l.fn, grid, block, args, 0, stream));
-    }
+    TANGO_CUDA_TRY(cudaLaunchKernel((const void *)pick<FIRST_SWEEP>(true, jobs[0].mode, l.ext), grid, block, args, 0, stream));
+    TANGO_CUDA_TRY(cudaLaunchKernel((const void *)pick<SECOND_SWEEP>(true, jobs[0].mode, l.ext), grid, block, args, 0, stream));
     return TANGO_OK;
 }
 
