@@ -153,12 +153,12 @@ int tango_qgemm_nt(const int8_t *xq, int64_t ldx, const int8_t *wq, int64_t ldw,
                    int *status, tango_stream_t stream);
 
 /* The same product with the element-wise steps around it in the epilogue:
- * Y = act(acc * (sx*sw) * row_scale[r] + bias[c]); scale_y = max|Y| / 127 (every optional argument may be NULL; relu = 0
- * or 1).  They are the norms, bias and activation of a graph convolution that multiplies
+ * Y = act(acc * (sx*sw) * row_scale[r] + bias[c]); scale_y = max|Y[r,c] * scale_row_factor[r]| / 127 (every optional
+ * argument may be NULL; relu = 0 or 1).  They are the norms, bias and activation of a graph convolution that multiplies
  * last (evaluation/test_gcn.py:95-137). */
 int tango_qgemm_layer(const int8_t *xq, int64_t ldx, const int8_t *wq, int64_t ldw, int64_t m, int64_t n, int64_t k,
                       const float *sx, const float *sw, const float *row_scale, const float *bias, int relu, float *y,
-                      int64_t ldy, float *scale_y, int *status, tango_stream_t stream);
+                      int64_t ldy, float *scale_y, const float *scale_row_factor, int *status, tango_stream_t stream);
 
 /* The reference's fused forward: quantises X[M,K] (times row_scale[r] if given) and W[N,K] with the given rounding
  * mode and the scales sx, sw, writes the int8 copies xq, wq that the backward pass re-uses, and computes the GEMM

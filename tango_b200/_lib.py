@@ -88,7 +88,7 @@ _SIGS = {
     "tango_quantize_two_launches": ([P, c_int, P, P, c_int64, P], c_int),
     "tango_qgemm_dw_workspace_bytes": ([c_int64, c_int64], c_int64),
     "tango_qgemm_nt": ([P, c_int64, P, c_int64, c_int64, c_int64, c_int64, P, P, P, P, c_int64, P, P, P], c_int),
-    "tango_qgemm_layer": ([P, c_int64, P, c_int64, c_int64, c_int64, c_int64, P, P, P, P, c_int, P, c_int64, P, P, P], c_int),
+    "tango_qgemm_layer": ([P, c_int64, P, c_int64, c_int64, c_int64, c_int64, P, P, P, P, c_int, P, c_int64, P, P, P, P], c_int),
     "tango_qgemm_dw_scratch_bytes": ([c_int64, c_int64, c_int64], c_int64),
     "tango_qgemm_dw_cleared": ([P, c_int64, P, c_int64, c_int64, c_int64, c_int64, P, P, P, c_int64, P, c_int64, P, P], c_int),
     "tango_qgemm_forward": ([P, c_int64, P, P, c_int64, c_int64, c_int64, c_int64, P, P, P, c_int64, P, c_int64, P, P,

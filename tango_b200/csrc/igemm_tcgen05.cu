@@ -67,7 +67,8 @@ struct GemmParams {
     const float *sa, *sb, *bias;
     const float *out_row_scale;     // optional: output row r is multiplied by out_row_scale[r] after dequantisation
     int relu;
-    float *absmax;                  // optional: receives max|output| / 127
+    float *absmax;                  // optional: receives max|output * absmax_row_scale[r]| / 127
+    const float *absmax_row_scale;  // optional
     int *status;
     uint32_t tmem_cols;
     int wide_store;                 // output rows start on 32-byte boundaries and are whole sectors
@@ -230,7 +231,9 @@ __device__ __forceinline__ void store_chunk(const GemmParams &p, uint32_t (&r)[3
 #pragma unroll
                 for (int i = 0; i < 32; ++i) m = i < width ? fmaxf(m, fabsf(__uint_as_float(r[i]))) : m;
             }
-            if (row < p.M) amax = fmaxf(amax, m);
+            // rounding is monotonic: the largest product is the product of the largest value
+            const float f = row < p.M ? (p.absmax_row_scale ? fabsf(__ldg(p.absmax_row_scale + row)) : 1.f) : 0.f;
+            amax = fmaxf(amax, __fmul_rn(m, f));
         }
     }
     if (p.wide_store) {
@@ -568,7 +571,7 @@ struct GemmCall {
     int mode; int splits;
     float *out; int64_t ldo; int32_t *ws; int64_t ldws; int *arrivals;
     const float *sa, *sb, *bias; float *absmax; int *status;
-    const float *out_row_scale;
+    const float *out_row_scale, *absmax_row_scale;
     int relu;
 };
 
@@ -648,7 +651,7 @@ static int launch_gemm(const GemmCall &c, cudaStream_t stream) {
     p.a_mn = c.a_mn; p.b_mn = c.b_mn;
     p.mode = c.mode; p.out = c.out; p.ldo = c.ldo; p.ws = c.ws; p.ldws = c.ldws; p.arrivals = c.arrivals;
     p.sa = c.sa; p.sb = c.sb; p.bias = c.bias; p.absmax = c.absmax; p.status = c.status;
-    p.out_row_scale = c.out_row_scale; p.relu = c.relu;
+    p.out_row_scale = c.out_row_scale; p.absmax_row_scale = c.absmax_row_scale; p.relu = c.relu;
     p.wide_store = c.ldo % 8 == 0 && c.N % 8 == 0 && aligned(c.out, 32);
     p.pairs = c.ldo % 2 == 0 && c.N % 2 == 0 && aligned(c.out, 8);
 
@@ -707,21 +710,22 @@ extern "C" int64_t tango_qgemm_dw_workspace_bytes(int64_t n, int64_t k) {
 
 extern "C" int tango_qgemm_layer(const int8_t *xq, int64_t ldx, const int8_t *wq, int64_t ldw, int64_t m, int64_t n,
                                  int64_t k, const float *sx, const float *sw, const float *row_scale, const float *bias,
-                                 int relu, float *y, int64_t ldy, float *scale_y, int *status, tango_stream_t stream) {
+                                 int relu, float *y, int64_t ldy, float *scale_y, const float *scale_row_factor,
+                                 int *status, tango_stream_t stream) {
     if (m < 0 || n < 0 || k <= 0 || ldx < k || ldw < k || ldy < n) return TANGO_EINVAL;
     if (m == 0 || n == 0) return TANGO_OK;
     if (!xq || !wq || !sx || !sw || !y) return TANGO_EINVAL;
     GemmCall c{};
     c.a = xq; c.lda = ldx; c.b = wq; c.ldb = ldw; c.M = m; c.N = n; c.K = k; c.mode = MODE_STORE; c.splits = 1;
     c.out = y; c.ldo = ldy; c.sa = sx; c.sb = sw; c.bias = bias; c.relu = relu; c.out_row_scale = row_scale;
-    c.absmax = scale_y; c.status = status;
+    c.absmax = scale_y; c.absmax_row_scale = scale_row_factor; c.status = status;
     return launch_gemm(c, (cudaStream_t)stream);
 }
 
 extern "C" int tango_qgemm_nt(const int8_t *xq, int64_t ldx, const int8_t *wq, int64_t ldw, int64_t m, int64_t n,
                               int64_t k, const float *sx, const float *sw, const float *bias, float *y, int64_t ldy,
                               float *scale_y, int *status, tango_stream_t stream) {
-    return tango_qgemm_layer(xq, ldx, wq, ldw, m, n, k, sx, sw, nullptr, bias, 0, y, ldy, scale_y, status, stream);
+    return tango_qgemm_layer(xq, ldx, wq, ldw, m, n, k, sx, sw, nullptr, bias, 0, y, ldy, scale_y, nullptr, status, stream);
 }
 
 extern "C" int tango_qgemm_forward(const float *x, int64_t ldx_f, const float *row_scale, const float *w,

@@ -172,7 +172,7 @@ Tensor gemm_nt(const Quantized &xq, const Quantized &wq, const Tensor &bias, con
     Tensor y = floats({x.rows, w.rows}, xq.scale);
     check(tango_qgemm_layer(ptr<int8_t>(x.t), x.ld, ptr<int8_t>(w.t), w.ld, x.rows, w.rows, x.cols, ptr<float>(xq.scale),
                             ptr<float>(wq.scale), ptr<float>(row_scale), ptr<float>(bias), relu, ptr<float>(y), w.rows,
-                            ptr<float>(scale_out), ptr<int>(status_word(y.device())), cuda_stream()), "qgemm_nt");
+                            ptr<float>(scale_out), nullptr, ptr<int>(status_word(y.device())), cuda_stream()), "qgemm_nt");
     count(1);
     return y;
 }
