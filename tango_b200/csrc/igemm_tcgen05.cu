@@ -196,6 +196,14 @@ __device__ __forceinline__ void add_chunk(const GemmParams &p, const uint32_t (&
     __syncwarp();
 }
 
+// max(v, 0) that hands a NaN on, in one instruction (a compare and select in its place cost the plain form of the epilogue,
+// which never runs it, 8 %: dX of 232,965 x 602 166 -> 180 us).
+__device__ __forceinline__ float relu_nan(float v) {
+    float t;
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(t) : "f"(v));
+    return t;
+}
+
 // Dequantise and store.  An epilogue warp is a dependent chain with few companions, so instructions count: the optional
 // steps are compiled out of the plain form, and where the rows of the output start on 32-byte boundaries every lane stores
 // its own row's chunk with four 256-bit stores.  Rows of any other pitch are laid out in shared memory first (`line_tile`,
@@ -220,7 +228,7 @@ __device__ __forceinline__ void store_chunk(const GemmParams &p, uint32_t (&r)[3
         }
         if (p.relu) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) r[i] = __uint_as_float(r[i]) <= 0.f ? 0u : r[i];      // NaN passes
+            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(relu_nan(__uint_as_float(r[i])));
         }
         if (p.absmax) {
             float m = 0.f;

@@ -152,7 +152,9 @@ def test_saved_tensor_hooks_and_copies_of_models(cuda):
         with torch.autograd.graph.saved_tensors_hooks(lambda t: seen.append(t.dtype) or t.cpu(), lambda t: t.cuda()):
             got = _step(m, x)
         assert all(torch.equal(a, b) for a, b in zip(want, got)), name
-        assert name == "hgt" or torch.int8 in seen, name          # the int8 operands are offloaded too
+        # the fused layers' int8 operands are offloaded too; the single operators that hgt is made of keep theirs on the node,
+        # as the reference's Functions do, and allow a second backward pass
+        assert name == "hgt" or torch.int8 in seen, name
         for other in (copy.deepcopy(m), torch.load(io.BytesIO(_saved(m)), weights_only=False)):
             assert all(torch.equal(a, b) for a, b in zip(want, _step(other, x))), name
         out = _forward(m, x).sum()
@@ -499,3 +501,26 @@ def test_infinities_and_nan_go_through_a_convolution_as_through_the_operators(cu
     assert res[0][0].isnan().any()
     for a, b in zip(*res):
         torch.testing.assert_close(a, b, rtol=0, atol=0 if a is not res[0][3] else 1e-4, equal_nan=True)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 16), (129, 41, 100), (700, 256, 602)])
+@pytest.mark.parametrize("relu", [0, 1])
+def test_gemm_epilogue_options(cuda, m, n, k, relu):
+    """Row factor, bias, ReLU and the output maximum with its own factor, operation for operation."""
+    import tango_b200 as T
+    from tango_b200 import _lib
+    rng = np.random.default_rng(m)
+    x, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    row, bias, factor = (rng.standard_normal(s).astype(np.float32) for s in (m, n, m))
+    (xq, sx), (wq, sw) = T.kernels.quantize(torch.from_numpy(x).cuda()), T.kernels.quantize(torch.from_numpy(w).cuda())
+    y, sy, st = torch.empty(m, n, device="cuda"), torch.zeros(1, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    rt, bt, ft = (torch.from_numpy(t).cuda() for t in (row, bias, factor))
+    p = [t.data_ptr() for t in (xq, wq, sx, sw, rt, bt, y, sy, ft, st)]
+    ld = (k + 15) // 16 * 16
+    _lib.check(_lib.lib.tango_qgemm_layer(p[0], ld, p[1], ld, m, n, k, p[2], p[3], p[4], p[5], relu, p[6], n, p[7], p[8], p[9],
+                                          torch.cuda.current_stream().cuda_stream), "qgemm_layer")
+    acc = _np(xq).astype(np.int64) @ _np(wq).astype(np.int64).T
+    want = acc.astype(np.float32) * (_np(sx) * _np(sw)) * row[:, None] + bias
+    want = np.maximum(want, np.float32(0)) if relu else want
+    np.testing.assert_array_equal(_np(y), want)
+    assert sy.item() == np.float32(np.abs(want * factor[:, None]).max()) / np.float32(127) and st.item() == 0
