@@ -442,10 +442,9 @@ def run_ours(args):
                           + (" + int8 tensor-core product of the dense hub block" if getattr(g, "_hubs", None) else ""),
                 "bound": "hbm", "achieved": ach,
                 "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": ach / peaks["hbm_gbs"],
-                "traffic": 397_105_920 + 4 * max(0, n_edges - 20_232_965),
-                "traffic_source": "derived, not measured in this run: dram__bytes_read+write of the ncu capture in "
-                                  "profiles/spmm_copy_u_f256_ncu.md (397.1 MB on a 20.2 M-edge graph with the same nodes) "
-                                  "+ 4 B of index stream for every further edge",
+                "traffic": 1_186_173_440 if n_edges == 114_615_892 and hb is not None else None,
+                "traffic_source": "not measured in this run: dram__bytes_read+write of the aggregation's four kernels on this "
+                                  "workload with the hub region on, profiles/spmm_copy_u_f256_ncu.md",
                 "binding_ceiling": "l2_row_gather (see frac_of_l2_row_gather_peak); the HBM fraction is secondary",
                 "peak_source": peak_kind, "kernel_ms": k_ms, "algorithmic_bytes": alg,
                 "gathered_bytes_per_s_GB": touched / (k_ms * 1e-3) / 1e9,

@@ -445,8 +445,9 @@ __device__ __forceinline__ void one_row(const GatArgs &a, int64_t row, int beg, 
 // less what the second sweep finds in L2) and, in the forward, a warp's load of 32 random int8 records, which takes 32 passes
 // through L1: the records are kept in shared memory between the sweeps.  On short rows it is rows in flight: half the rows
 // of a sparse power-law graph have one edge, and had a warp each.  One edge in flight per thread -> as it is, us:
-//   114.6 M edges, 4 heads: forward 1224 -> 1160, backward 1577 -> 1387;  1 head: 593 -> 409, 668 -> 566
-//   1.3 M edges on 169 K nodes, 4 heads, plain scores: 153 -> 57, 55 -> 34;  0.1 M edges, 8 heads: 53 -> 28, 40 -> 13
+//   114.6 M edges, 4 heads: forward 1224 -> 1195, backward 1577 -> 1386;  1 head: 593 -> 427, 668 -> 565
+//   1.3 M edges on 169 K nodes, 4 heads, plain scores: 153 -> 50, 55 -> 39;  0.1 M edges, 8 heads: 53 -> 50, 40 -> 40 (a CTA
+//   for rows of 128 edges and more took 28 and 13 there, but their terms were then added in another order)
 template <int HT, bool PLAIN, bool BWD, int STAGE>
 __global__ void __launch_bounds__(256, HT == 1 || HT == 2 ? (BWD ? 4 : 6) : (HT == 4 ? 4 : 3) - (BWD ? 1 : 0)) gat_softmax_kernel(const GatArgs a) {
     constexpr int U = Shape<HT>::U;
